@@ -2,19 +2,19 @@
 
 Each op is a ``CustomOp`` registered the way the reference registers its op libraries
 (iree/turbine/ops/__init__.py:7-11; e.g. iree/turbine/ops/conv_fwd.py:62-89 for a ``select``):
-a schema string, a ``select`` that types every argument and declares the result meta tensors
-(which also is the Meta implementation, so fake tensors and ``torch.compile`` tracing work), and
-a CUDA implementation.  The CUDA implementation is ``eager_execute`` calling the C ABI on the
-current stream; there is no CPU implementation, so a CPU tensor fails in the dispatcher with
-torch's own "not implemented for CPU" error.
-
-Output shape/dtype rules live in ``select`` only; ``eager_execute`` allocates outputs from the
-same rules.
+a schema string and a ``select`` that types every argument and declares the result meta tensors
+(which also is the Meta implementation, so fake tensors and ``torch.compile`` tracing work).  The
+CUDA implementations are native (``csrc/torch_ops.cpp``, built as ``_native.so``): they call the C
+ABI on the current stream and cost a few microseconds of host time.  There is no CPU
+implementation, so a CPU tensor fails in the dispatcher with torch's own "not implemented for CPU"
+error; without the built ``_native.so`` a CUDA tensor fails there as well.
 """
 
 from __future__ import annotations
 
 import ctypes as C
+import sys
+import types
 from typing import Optional
 
 import torch
@@ -47,35 +47,40 @@ __all__ = [
 
 LIBRARY = def_library("b200k")
 
+try:
+    from . import _native  # registers the CUDA implementations
+except ImportError as _e:
+    _native_error = _e
+
+    class _native:  # every use says what is missing; the ops themselves have no CUDA implementation
+        def __getattr__(self, name):
+            raise RuntimeError(
+                f"the operator implementations (_native.so) cannot be loaded: {_native_error}. Run "
+                "`python csrc/build.py` in the package directory. There is no fallback.")
+
+    _native = _native()
+
 _HALF_TYPES = (torch.float16, torch.bfloat16)
 
-# One int32 status word per device: kernels OR a code into it if a bounded device-side wait gave
-# up (see include/b200k.h).  Reading it synchronizes, so it is only read on request.
-_status_words: dict[int, Tensor] = {}
+
+def _status_word(device) -> Tensor:
+    """The device's int32 status word: kernels OR a code into it if a bounded device-side wait gave up
+    (see include/b200k.h).  Reading it synchronizes, so it is only read on request."""
+    dev = torch.device("cuda") if device is None else torch.device(device)
+    return _native.status_word(dev.index if dev.index is not None else torch.cuda.current_device())
 
 
 def _status_ptr(device: torch.device) -> int:
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    w = _status_words.get(idx)
-    if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status_words[idx] = w
-    return w.data_ptr()
+    return _status_word(device).data_ptr()
 
 
 def device_status(device=None) -> int:
     """Returns the device status word (0 = no kernel reported a timed-out wait).  Synchronizes."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    _status_ptr(dev)
-    idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    return int(_status_words[idx].item())
+    return int(_status_word(device).item())
 
 
 def reset_device_status(device=None) -> None:
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    _status_ptr(dev)
-    idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    _status_words[idx].zero_()
+    _status_word(device).zero_()
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -140,25 +145,7 @@ def _launch_gemm(a: Tensor, b: Tensor, out: Tensor, scale_a, scale_b, tile_n: in
     L.check(L.lib().b200k_gemm_nt(C.byref(args), _stream(a)))
 
 
-def _batched_operand(t: Tensor):
-    """A [B, R, C] operand as the kernel can read it without a copy: (tensor, stored_transposed).
-    Either the last dim is contiguous (rows of the matrix) or the middle one is (the matrix is stored
-    transposed); row pitch and batch stride must be multiples of 16 bytes.  Otherwise a contiguous copy."""
-    es = t.element_size()
-
-    def ok(x):
-        return (x.stride(2) == 1 and (x.stride(1) * es) % 16 == 0 and (x.stride(0) * es) % 16 == 0
-                and x.stride(1) >= x.size(2) and x.data_ptr() % 16 == 0 and x.size(2) % 8 == 0)
-
-    if ok(t):
-        return t, False
-    tt = t.transpose(1, 2)
-    if ok(tt):
-        return tt, True
-    return t.contiguous(), False
-
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class gemm_nt(CustomOp):
     """C[M,N] = A[M,K] @ B[N,K]^T, f16 or bf16 operands, fp32 accumulation.
 
@@ -180,13 +167,8 @@ class gemm_nt(CustomOp):
         b.specialize_dims(1)
         sel.return_new_tensor([a.t.size(0), b.t.size(0)], _gemm_out_dtype(a.t.dtype, od.v))
 
-    def eager_execute(self, a, b, out_dtype=None):
-        out = torch.empty((a.size(0), b.size(0)), dtype=_gemm_out_dtype(a.dtype, out_dtype), device=a.device)
-        _launch_gemm(a, b, out, None, None)
-        return out
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class gemm(CustomOp):
     """C = op(a) @ op(b) with BLAS-style flags: ``a`` is [M, K] ([K, M] with ``trans_a``), ``b`` is
     [K, N] ([N, K] with ``trans_b``); f16 / bf16, fp32 accumulation.  No operand is repacked: the
@@ -216,14 +198,8 @@ class gemm(CustomOp):
                      lambda: "gemm: the contiguous dimension of each operand must be a multiple of 8")
         sel.return_new_tensor([m, n], _gemm_out_dtype(a.t.dtype, od.v))
 
-    def eager_execute(self, a, b, trans_a=False, trans_b=False, out_dtype=None):
-        m, n, _, _ = self._mnk(a, b, trans_a, trans_b)
-        out = torch.empty((m, n), dtype=_gemm_out_dtype(a.dtype, out_dtype), device=a.device)
-        _launch_gemm(a, b, out, None, None, a_km=bool(trans_a), b_kn=not trans_b)
-        return out
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class bmm(CustomOp):
     """Batched product ``a[B, M, K] @ b[B, K, N]`` (aten::bmm; the reference's BOO layer registers it
     beside mm and addmm, kernel/boo/op_exports/registry.py:99-104), f16 / bf16, fp32 accumulation, every
@@ -244,59 +220,31 @@ class bmm(CustomOp):
         torch._check(a.t.size(1) % 8 == 0 or a.t.size(2) % 8 == 0, lambda: "bmm: M or K must be a multiple of 8")
         sel.return_new_tensor([a.t.size(0), a.t.size(1), b.t.size(2)], _gemm_out_dtype(a.t.dtype, od.v))
 
-    def eager_execute(self, a, b, out_dtype=None):
-        bsz, m, k = a.shape
-        n = b.size(2)
-        out = torch.empty((bsz, m, n), dtype=_gemm_out_dtype(a.dtype, out_dtype), device=a.device)
-        if bsz == 0 or m == 0 or n == 0:
-            return out
-        a_s, a_t = _batched_operand(a)   # a_t: stored [B, K, M]
-        b_s, b_t = _batched_operand(b)   # b_t: stored [B, N, K]  (the kernel's native form)
-        args = L.GemmArgs()
-        args.a, args.b, args.c = a_s.data_ptr(), b_s.data_ptr(), out.data_ptr()
-        args.m, args.n, args.k = m, n, k
-        args.a_km, args.b_kn = int(a_t), int(not b_t)
-        args.lda, args.ldb, args.ldc = a_s.stride(1), b_s.stride(1), out.stride(1)
-        args.batch = bsz
-        args.a_batch_stride, args.b_batch_stride, args.c_batch_stride = a_s.stride(0), b_s.stride(0), out.stride(0)
-        args.in_dtype = L.DTYPE_CODES[a.dtype]
-        args.out_dtype = L.DTYPE_CODES[out.dtype]
-        args.status = _status_ptr(a.device)
-        L.check(L.lib().b200k_gemm_nt(C.byref(args), _stream(a)))
-        return out
 
+@CustomOp.register(library=LIBRARY, register_impl=False)
+class linear_op(CustomOp):
+    """``linear`` as an operator (its autograd formula is native, see ``linear`` below)."""
 
-class _LinearFunction(torch.autograd.Function):
-    """y = x @ w^T (+ bias) with both backward products on the same kernel (the reference wraps its
-    own op the same way, kernel/boo/ops/conv.py:313-372; the products are those of
-    kernel/boo/op_exports/gemm.py:233-270): dx = dy @ w, dw = dy^T @ x, db = sum(dy)."""
+    signature = "linear(Tensor x, Tensor w, Tensor? bias=None) -> Tensor"
 
-    @staticmethod
-    def forward(ctx, x, w, bias):
-        ctx.save_for_backward(x, w)
-        ctx.has_bias = bias is not None
-        return torch.ops.b200k.linear_act(x, w, bias, "none", x.dtype)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, w = ctx.saved_tensors
-        dy = dy.contiguous()
-        dx = dw = db = None
-        if ctx.needs_input_grad[0]:
-            dx = torch.ops.b200k.gemm(dy, w, False, False, x.dtype)       # [M, N] @ [N, K]
-        if ctx.needs_input_grad[1]:
-            dw = torch.ops.b200k.gemm(dy, x, True, False, w.dtype)        # [M, N]^T @ [M, K]
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy.float().sum(0).to(dy.dtype)
-        return dx, dw, db
+    def select(self, sel: KernelSelection):
+        x = sel.arg_tensor(0)
+        w = sel.arg_tensor(1)
+        sel.arg_optional_tensor(2)
+        torch._check(x.t.dim() == 2 and w.t.dim() == 2 and x.t.size(1) == w.t.size(1),
+                     lambda: "linear: x must be [M, K] and w [N, K]")
+        sel.return_new_tensor([x.t.size(0), w.t.size(0)], x.t.dtype)
 
 
 def linear(x: Tensor, w: Tensor, bias: Optional[Tensor] = None) -> Tensor:
-    """Differentiable ``x[M, K] @ w[N, K]^T + bias`` (f16 / bf16 CUDA tensors) on the b200k GEMM."""
-    return _LinearFunction.apply(x, w, bias)
+    """Differentiable ``x[M, K] @ w[N, K]^T + bias`` (f16 / bf16 CUDA tensors) on the b200k GEMM, with both
+    backward products on the same kernel (the reference wraps its own op the same way,
+    kernel/boo/ops/conv.py:313-372; the products are those of kernel/boo/op_exports/gemm.py:233-270):
+    dx = dy @ w, dw = dy^T @ x, db = sum(dy)."""
+    return torch.ops.b200k.linear(x, w, bias)
 
 
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class linear_act(CustomOp):
     """act(A[M,K] @ W[N,K]^T + bias[N]) in one kernel: the GEMM with bias and activation applied in
     its epilogue (the shape of a linear layer with trailing optional bias).  ``activation`` is
@@ -323,13 +271,8 @@ class linear_act(CustomOp):
             torch._check(bt.dtype in (torch.float32,) + _HALF_TYPES, lambda: "linear_act: bias must be float32 / float16 / bfloat16")
         sel.return_new_tensor([a.t.size(0), w.t.size(0)], _gemm_out_dtype(a.t.dtype, od.v))
 
-    def eager_execute(self, a, w, bias=None, activation="none", out_dtype=None):
-        out = torch.empty((a.size(0), w.size(0)), dtype=_gemm_out_dtype(a.dtype, out_dtype), device=a.device)
-        _launch_gemm(a, w, out, None, None, bias=bias, activation=activation)
-        return out
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class gemm_fp8_nt(CustomOp):
     """C = (A8 @ B8^T) * scale_a * scale_b with float8_e4m3fn operands and per-tensor fp32 scales.
 
@@ -360,13 +303,8 @@ class gemm_fp8_nt(CustomOp):
         )
         sel.return_new_tensor([a.t.size(0), b.t.size(0)], _gemm_out_dtype(a.t.dtype, od.v))
 
-    def eager_execute(self, a, b, scale_a, scale_b, out_dtype=None):
-        out = torch.empty((a.size(0), b.size(0)), dtype=_gemm_out_dtype(a.dtype, out_dtype), device=a.device)
-        _launch_gemm(a, b, out, scale_a, scale_b)
-        return out
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class quantize_e4m3(CustomOp):
     """Per-tensor quantisation: returns (x / s cast to float8_e4m3fn, s) with s = max|x| / 448."""
 
@@ -378,38 +316,32 @@ class quantize_e4m3(CustomOp):
         sel.return_new_tensor(list(x.t.shape), torch.float8_e4m3fn)
         sel.return_new_tensor([1], torch.float32)
 
-    def eager_execute(self, x):
-        x = x.contiguous()
-        y = torch.empty(x.shape, dtype=torch.float8_e4m3fn, device=x.device)
-        scale = torch.empty(1, dtype=torch.float32, device=x.device)
-        scratch = torch.empty(1, dtype=torch.int32, device=x.device)
-        L.check(
-            L.lib().b200k_quantize_e4m3(
-                x.data_ptr(), y.data_ptr(), scale.data_ptr(), scratch.data_ptr(), x.numel(), _stream(x)
-            )
-        )
-        return y, scale
-
 
 # ---------------------------------------------------------------------------------------------
 # attention forward
 # ---------------------------------------------------------------------------------------------
-def _bhsd(t: Tensor) -> Tensor:
-    s0, s1, s2, s3 = t.stride()
-    ok = (s3 == 1 and s0 > 0 and s1 > 0 and s2 > 0 and (s0 | s1 | s2) % 8 == 0 and t.data_ptr() % 16 == 0)
-    return t if ok else t.contiguous()
+class _OpsModule(types.ModuleType):
+    """This module with one checked attribute.  ``ATTENTION_KERNEL`` says which forward kernel
+    ``attention`` / ``attention_lse`` / ``paged_attention`` ask for: 0 lets the library choose (one-tile or
+    tile-pair kernel, see include/b200k.h), 1 / 2 force one of them (head dim 64 only exists in the pair
+    kernel).  A tuning and testing knob, like the GEMM tile shape; the native implementations keep it."""
+
+    @property
+    def ATTENTION_KERNEL(self) -> int:
+        return _native.attention_kernel()
+
+    @ATTENTION_KERNEL.setter
+    def ATTENTION_KERNEL(self, value: int) -> None:
+        _native.set_attention_kernel(int(value))
 
 
-# Which forward kernel ``attention`` / ``attention_lse`` / ``paged_attention`` ask for: 0 lets the
-# library choose (one-tile or tile-pair kernel, see include/b200k.h), 1 / 2 force one of them
-# (head dim 64 only exists in the pair kernel).  A tuning and testing knob, like the GEMM tile shape.
-ATTENTION_KERNEL = L.ATTN_AUTO
+sys.modules[__name__].__class__ = _OpsModule
 
 
 def _fill_attention_args(q: Tensor, k: Tensor, v: Tensor, o: Tensor, scale: float, causal: bool) -> L.AttentionArgs:
     args = L.AttentionArgs()
     args.batch, args.q_heads, args.seq_q, args.head_dim = q.shape
-    args.kernel = ATTENTION_KERNEL if args.head_dim == 128 else L.ATTN_AUTO
+    args.kernel = _native.attention_kernel() if args.head_dim == 128 else L.ATTN_AUTO
     args.q, args.k, args.v, args.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
     _, args.kv_heads, args.seq_kv, _ = k.shape
     args.q_stride_b, args.q_stride_h, args.q_stride_s, _ = q.stride()
@@ -451,7 +383,7 @@ def _attention_select(sel: KernelSelection):
     return q
 
 
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class attention(CustomOp):
     """O = softmax(scale * Q K^T [causal]) V.  q [B,Hq,Sq,D], k/v [B,Hkv,Skv,D] -> [B,Hq,Sq,D], D = 128 or 64."""
 
@@ -460,16 +392,8 @@ class attention(CustomOp):
     def select(self, sel: KernelSelection):
         _attention_select(sel)
 
-    def eager_execute(self, q, k, v, scale, is_causal):
-        o = _attention_out_like(q, q.device)
-        q, k, v = _bhsd(q), _bhsd(k), _bhsd(v)
-        args = _fill_attention_args(q, k, v, o, scale, is_causal)
-        args.status = _status_ptr(q.device)
-        L.check(L.lib().b200k_attention_fwd(C.byref(args), _stream(q)))
-        return o
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class attention_lse(CustomOp):
     """``attention`` that also returns the row statistic the backward needs:
     lse[b, h, i] = ln sum_j exp(scale * q_i . k_j) over the visible keys (float32, -inf for a row
@@ -480,16 +404,6 @@ class attention_lse(CustomOp):
     def select(self, sel: KernelSelection):
         q = _attention_select(sel)
         sel.return_new_tensor(list(q.t.shape[:3]), torch.float32)
-
-    def eager_execute(self, q, k, v, scale, is_causal):
-        o = _attention_out_like(q, q.device)
-        lse = torch.empty(q.shape[:3], dtype=torch.float32, device=q.device)
-        q, k, v = _bhsd(q), _bhsd(k), _bhsd(v)
-        args = _fill_attention_args(q, k, v, o, scale, is_causal)
-        args.status = _status_ptr(q.device)
-        args.lse = lse.data_ptr()
-        L.check(L.lib().b200k_attention_fwd(C.byref(args), _stream(q)))
-        return o, lse
 
 
 def _attention_bwd_checks(q: Tensor, k: Tensor, v: Tensor, o: Tensor, d_o: Tensor, lse: Optional[Tensor] = None) -> None:
@@ -508,7 +422,7 @@ def _attention_bwd_checks(q: Tensor, k: Tensor, v: Tensor, o: Tensor, d_o: Tenso
                  lambda: "attention_bwd: query heads must be a multiple of kv heads")
 
 
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class attention_bwd(CustomOp):
     """Gradients of ``attention``: (q, k, v, o, d_o) -> (d_q, d_k, d_v).  d_k / d_v are summed over
     the query heads of a group.  Only the forward OUTPUT is needed; row statistics are recomputed."""
@@ -526,50 +440,16 @@ class attention_bwd(CustomOp):
         sel.return_new_tensor(list(k.t.shape), q.t.dtype)
         sel.return_new_tensor(list(k.t.shape), q.t.dtype)
 
-    def eager_execute(self, q, k, v, o, d_o, scale, is_causal, lse=None):
-        _attention_bwd_checks(q, k, v, o, d_o, lse)
-        if lse is not None:
-            lse = lse.contiguous()
-        q, k, v, o, d_o = (_bhsd(t) for t in (q, k, v, o, d_o))
-        d_q, d_k, d_v = torch.empty_like(q, memory_format=torch.contiguous_format), \
-            torch.empty_like(k, memory_format=torch.contiguous_format), \
-            torch.empty_like(v, memory_format=torch.contiguous_format)
-        a = L.AttentionBwdArgs()
-        for name, t in (("q", q), ("k", k), ("v", v), ("o", o), ("do", d_o), ("dq", d_q), ("dk", d_k), ("dv", d_v)):
-            setattr(a, {"do": "d_o", "dq": "d_q", "dk": "d_k", "dv": "d_v"}.get(name, name), t.data_ptr())
-            for d, i in (("b", 0), ("h", 1), ("s", 2)):
-                setattr(a, f"{name}_stride_{d}", t.stride(i))
-        a.batch, a.q_heads, a.seq_q, a.head_dim = q.shape
-        a.kv_heads, a.seq_kv = k.size(1), k.size(2)
-        a.dtype = L.DTYPE_CODES[q.dtype]
-        a.causal = 1 if is_causal else 0
-        a.scale = float(scale)
-        a.status = _status_ptr(q.device)
-        a.lse = lse.data_ptr() if lse is not None else None
-        lib = L.lib()
-        need = lib.b200k_attention_bwd_workspace_bytes(C.byref(a))
-        ws = torch.empty(max(int(need), 16), dtype=torch.uint8, device=q.device)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-        L.check(lib.b200k_attention_bwd(C.byref(a), _stream(q)))
-        return d_q, d_k, d_v
 
+@CustomOp.register(library=LIBRARY, register_impl=False)
+class sdpa_op(CustomOp):
+    """``sdpa`` as an operator (its autograd formula is native: ``attention_lse`` forward, ``attention_bwd``
+    backward)."""
 
-class _AttentionFunction(torch.autograd.Function):
-    """``attention`` with its gradient on the backward kernels (wrapped the way the reference wraps
-    its own forward / backward ops, kernel/boo/ops/conv.py:313-372)."""
+    signature = "sdpa(Tensor q, Tensor k, Tensor v, float scale, bool is_causal) -> Tensor"
 
-    @staticmethod
-    def forward(ctx, q, k, v, scale, is_causal):
-        o, lse = torch.ops.b200k.attention_lse(q, k, v, scale, is_causal)
-        ctx.save_for_backward(q, k, v, o, lse)
-        ctx.scale, ctx.is_causal = scale, is_causal
-        return o
-
-    @staticmethod
-    def backward(ctx, d_o):
-        q, k, v, o, lse = ctx.saved_tensors
-        d_q, d_k, d_v = torch.ops.b200k.attention_bwd(q, k, v, o, d_o, ctx.scale, ctx.is_causal, lse)
-        return d_q, d_k, d_v, None, None
+    def select(self, sel: KernelSelection):
+        _attention_select(sel)
 
 
 def sdpa(q: Tensor, k: Tensor, v: Tensor, scale: Optional[float] = None, is_causal: bool = False) -> Tensor:
@@ -579,7 +459,7 @@ def sdpa(q: Tensor, k: Tensor, v: Tensor, scale: Optional[float] = None, is_caus
         raise ValueError("sdpa: head dim must be 128 or 64")
     if scale is None:
         scale = 1.0 / (q.size(-1) ** 0.5)
-    return _AttentionFunction.apply(q, k, v, float(scale), bool(is_causal))
+    return torch.ops.b200k.sdpa(q, k, v, float(scale), bool(is_causal))
 
 
 # ---------------------------------------------------------------------------------------------
@@ -598,17 +478,7 @@ def _decode_common_checks(name: str, q: Tensor, kc: Tensor, vc: Tensor, lens: Te
                  lambda: f"{name}: query heads must be a multiple (at most 16x) of kv heads")
 
 
-def _launch_decode(args: L.DecodeArgs, q: Tensor) -> None:
-    lib = L.lib()
-    need = lib.b200k_decode_workspace_bytes(C.byref(args))
-    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
-    args.workspace = ws.data_ptr()
-    args.workspace_bytes = need
-    args.status = _status_ptr(q.device)
-    L.check(lib.b200k_decode_attention(C.byref(args), _stream(q)))
-
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class decode_attention(CustomOp):
     """One query token per sequence against a contiguous KV history.
 
@@ -631,25 +501,8 @@ class decode_attention(CustomOp):
         torch._check(k.t.size(0) == q.t.size(0), lambda: "decode_attention: k must have one history per sequence")
         sel.return_new_tensor(list(q.t.shape), q.t.dtype)
 
-    def eager_execute(self, q, k, v, seq_lens, scale, chunk_tokens=0):
-        q, k, v, seq_lens = q.contiguous(), k.contiguous(), v.contiguous(), seq_lens.contiguous()
-        o = torch.empty_like(q)
-        args = L.DecodeArgs()
-        args.q, args.k_cache, args.v_cache, args.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
-        args.block_table = None
-        args.seq_lens = seq_lens.data_ptr()
-        args.num_seqs, args.q_heads, args.head_dim = q.size(0), q.size(1), q.size(2)
-        args.kv_heads = k.size(1)
-        args.max_seq_len = k.size(2)
-        args.kv_batch_stride, args.kv_head_stride = k.stride(0), k.stride(1)
-        args.dtype = L.DTYPE_CODES[q.dtype]
-        args.chunk_tokens = int(chunk_tokens)
-        args.scale = float(scale)
-        _launch_decode(args, q)
-        return o
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class paged_decode_attention(CustomOp):
     """One query token per sequence against a paged KV cache.
 
@@ -677,29 +530,8 @@ class paged_decode_attention(CustomOp):
         torch._check(kc.t.size(2) % 16 == 0, lambda: "paged_decode_attention: page size must be a multiple of 16")
         sel.return_new_tensor(list(q.t.shape), q.t.dtype)
 
-    def eager_execute(self, q, k_cache, v_cache, block_table, seq_lens, scale, chunk_tokens=0):
-        q, k_cache, v_cache = q.contiguous(), k_cache.contiguous(), v_cache.contiguous()
-        block_table, seq_lens = block_table.contiguous(), seq_lens.contiguous()
-        o = torch.empty_like(q)
-        args = L.DecodeArgs()
-        args.q, args.k_cache, args.v_cache, args.o = q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), o.data_ptr()
-        args.block_table = block_table.data_ptr()
-        args.seq_lens = seq_lens.data_ptr()
-        args.num_seqs, args.q_heads, args.head_dim = q.size(0), q.size(1), q.size(2)
-        args.kv_heads = k_cache.size(1)
-        args.page_size = k_cache.size(2)
-        args.num_pages = k_cache.size(0)
-        args.block_table_stride = block_table.stride(0)
-        args.max_seq_len = block_table.size(1) * k_cache.size(2)
-        args.kv_page_stride, args.kv_head_stride = k_cache.stride(0), k_cache.stride(1)
-        args.dtype = L.DTYPE_CODES[q.dtype]
-        args.chunk_tokens = int(chunk_tokens)
-        args.scale = float(scale)
-        _launch_decode(args, q)
-        return o
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class paged_gather(CustomOp):
     """out[s, h, t, :] = cache[block_table[s, t // page], h, t % page, :] for t < seq_lens[s].
 
@@ -718,22 +550,8 @@ class paged_gather(CustomOp):
         torch._check(lens.t.dtype == torch.int32 and lens.t.dim() == 1, lambda: "paged_gather: seq_lens must be int32 1-D")
         sel.return_new_tensor([bt.t.size(0), c.t.size(1), n.v, c.t.size(3)], c.t.dtype)
 
-    def eager_execute(self, cache, block_table, seq_lens, max_seq_len):
-        cache = cache.contiguous()
-        block_table, seq_lens = block_table.contiguous(), seq_lens.contiguous()
-        out = torch.zeros((block_table.size(0), cache.size(1), max_seq_len, cache.size(3)), dtype=cache.dtype,
-                          device=cache.device)
-        L.check(
-            L.lib().b200k_paged_gather(
-                cache.data_ptr(), block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), block_table.size(0),
-                cache.size(1), cache.size(3), cache.size(2), cache.size(0), block_table.stride(0), max_seq_len,
-                cache.stride(0), cache.stride(1), cache.element_size(), _stream(cache),
-            )
-        )
-        return out
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class kv_append(CustomOp):
     """Writes new K/V rows into the paged cache through the block table (in place).
 
@@ -766,23 +584,8 @@ class kv_append(CustomOp):
         torch._check(pos.t.dtype == torch.int32 and pos.t.dim() == 1 and pos.t.size(0) == kn.t.size(0),
                      lambda: "kv_append: positions must be int32 [num_seqs]")
 
-    def eager_execute(self, k_new, v_new, k_cache, v_cache, block_table, positions):
-        if not (k_cache.is_contiguous() and v_cache.is_contiguous()):
-            raise ValueError("kv_append: the caches are written in place and must be contiguous")
-        k_new, v_new = k_new.contiguous(), v_new.contiguous()
-        block_table, positions = block_table.contiguous(), positions.contiguous()
-        L.check(
-            L.lib().b200k_kv_append(
-                k_new.data_ptr(), v_new.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_table.data_ptr(),
-                positions.data_ptr(), k_new.size(0), k_new.size(1), k_new.size(2), k_new.size(3), k_cache.size(2),
-                k_cache.size(0), block_table.stride(0), k_cache.stride(0), k_cache.stride(1), k_cache.element_size(),
-                _status_ptr(k_cache.device), _stream(k_cache),
-            )
-        )
-        return None
 
-
-@CustomOp.register(library=LIBRARY)
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class paged_attention(CustomOp):
     """Attention forward (prefill) over a paged K/V cache.
 
@@ -816,25 +619,3 @@ class paged_attention(CustomOp):
                      lambda: "paged_attention: seq_lens must be int32 [B]")
         sel.return_tensor(_attention_out_like(q.t, "meta"))
 
-    def eager_execute(self, q, k_cache, v_cache, block_table, seq_lens, scale, is_causal):
-        o = _attention_out_like(q, q.device)
-        q = _bhsd(q)
-        k_cache, v_cache = k_cache.contiguous(), v_cache.contiguous()
-        block_table, seq_lens = block_table.contiguous(), seq_lens.contiguous()
-        a = L.PagedAttentionArgs()
-        a.q, a.k_cache, a.v_cache, a.o = q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), o.data_ptr()
-        a.block_table, a.seq_lens = block_table.data_ptr(), seq_lens.data_ptr()
-        a.batch, a.q_heads, a.kv_heads, a.seq_q = q.size(0), q.size(1), k_cache.size(1), q.size(2)
-        a.page_size, a.num_pages, a.block_table_stride = k_cache.size(2), k_cache.size(0), block_table.stride(0)
-        a.max_seq_kv = block_table.size(1) * k_cache.size(2)
-        a.head_dim = q.size(3)
-        a.q_stride_b, a.q_stride_h, a.q_stride_s = q.stride(0), q.stride(1), q.stride(2)
-        a.o_stride_b, a.o_stride_h, a.o_stride_s = o.stride(0), o.stride(1), o.stride(2)
-        a.kv_page_stride, a.kv_head_stride = k_cache.stride(0), k_cache.stride(1)
-        a.dtype = L.DTYPE_CODES[q.dtype]
-        a.causal = 1 if is_causal else 0
-        a.scale = float(scale)
-        a.status = _status_ptr(q.device)
-        a.kernel = ATTENTION_KERNEL if q.size(3) == 128 else L.ATTN_AUTO
-        L.check(L.lib().b200k_paged_attention_fwd(C.byref(a), _stream(q)))
-        return o
