@@ -37,6 +37,7 @@ struct GemmParams {
   int32_t a_mn, b_mn;
   int32_t vec_store_ok;
   int32_t tma_store_ok;  // C is 16-byte aligned with a 16-byte-multiple row pitch: epilogue uses TMA stores
+  int32_t store_bytes;   // otherwise: widest store (2, 4 or 8 bytes) that C's base and pitches allow
   // Fused all-gather of a column shard: when num_peers > 0 every output tile is written with plain
   // 16-byte stores into each peer's full matrix (peer-mapped memory) at column peer_col0.
   int32_t num_peers;
@@ -65,7 +66,9 @@ struct GemmSmem {
   static constexpr int kStagingBytes = 4 * 2 * 32 * 128;
   static constexpr int kBarOffset = kStagingOffset + kStagingBytes;
   static constexpr int kNumBars = 2 * kStages + 4;
-  static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16;
+  static constexpr int kBiasOffset = kBarOffset + kNumBars * 8 + 16;  // the tile's bias as fp32
+  static_assert(kBiasOffset % 16 == 0, "bias is read as float4");
+  static constexpr int kTotal = kBiasOffset + BN * 4;
   static constexpr int kDynamic = kTotal + 1024;  // slack for 1024-byte alignment of the tiles
 };
 
@@ -94,14 +97,23 @@ __device__ __forceinline__ __nv_bfloat16 to_out<__nv_bfloat16>(float v) {
   return __float2bfloat16_rn(v);
 }
 
+template <int ACT>
+__device__ __forceinline__ float apply_act(float x) {
+  if constexpr (ACT == B200K_ACT_RELU) return fmaxf(x, 0.f);
+  if constexpr (ACT == B200K_ACT_GELU)  // exact (erf) form, the default of aten::gelu
+    return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
+  if constexpr (ACT == B200K_ACT_SILU) return x / (1.f + __expf(-x));
+  return x;
+}
+
 __device__ __forceinline__ float apply_act(float x, int act) {
   switch (act) {
     case B200K_ACT_RELU:
-      return fmaxf(x, 0.f);
-    case B200K_ACT_GELU:  // exact (erf) form, the default of aten::gelu
-      return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
+      return apply_act<B200K_ACT_RELU>(x);
+    case B200K_ACT_GELU:
+      return apply_act<B200K_ACT_GELU>(x);
     case B200K_ACT_SILU:
-      return x / (1.f + __expf(-x));
+      return apply_act<B200K_ACT_SILU>(x);
     default:
       return x;
   }
@@ -113,59 +125,93 @@ __device__ __forceinline__ float load_bias(const void* bias, int dtype, int col)
   return __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(bias) + col));
 }
 
-// A bias of zero for calls without one (see fused_epilogue).
-static __device__ const float kZeroBias = 0.0f;
-
-// Fused epilogue on N accumulator values of one row (columns col0 .. col0 + N - 1), in place:
-// r = act(r * scale + bias).  Every lane of a warp reads the same bias element (one broadcast
-// load per column).  Afterwards the caller's own scaling must be 1.
-// No load here is guarded by a test the compiler could move it across: without a bias the pointer
-// is switched to a zero that lives in device memory, and the column index is clamped to the vector
-// instead of predicated (columns past n are never stored).  A guarded form of this loop was seen to
-// fault on a null bias in one kernel, its loads having been issued ahead of the null test.
+// acc * scale + bias, then the activation, on N accumulator values of one row, in place.  `bias` is the
+// fp32 bias of these columns in shared memory (16-byte aligned, the same for every lane, so a float4
+// read is a broadcast); afterwards the caller's own scaling must be 1.  The activation is chosen
+// outside the loop: with the choice (and a bias load that picked its data type) inside, the 64-fold
+// unrolled body made a 3000 x 4352 x 3840 product with bias take 155 us instead of 118.
 template <int N>
-__device__ __forceinline__ void fused_epilogue(uint32_t (&r)[N], float scale, const void* bias, int bias_dtype, int act,
-                                               int col0, int n) {
-  const bool has_bias = bias != nullptr;
-  const void* b = has_bias ? bias : static_cast<const void*>(&kZeroBias);
-  const int dt = has_bias ? bias_dtype : static_cast<int>(B200K_F32);
-  const int last = has_bias ? n - 1 : 0;
+__device__ __forceinline__ void fused_epilogue(uint32_t (&r)[N], float scale, const float* bias, int act) {
 #pragma unroll
-  for (int j = 0; j < N; ++j) {
-    const float x = __uint_as_float(r[j]) * scale + load_bias(b, dt, min(col0 + j, last));
-    r[j] = __float_as_uint(apply_act(x, act));
+  for (int j = 0; j < N; j += 4) {
+    const float4 b = *reinterpret_cast<const float4*>(bias + j);
+    r[j] = __float_as_uint(__uint_as_float(r[j]) * scale + b.x);
+    r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) * scale + b.y);
+    r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) * scale + b.z);
+    r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) * scale + b.w);
+  }
+  if (act == B200K_ACT_RELU) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) r[j] = __float_as_uint(apply_act<B200K_ACT_RELU>(__uint_as_float(r[j])));
+  } else if (act == B200K_ACT_GELU) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) r[j] = __float_as_uint(apply_act<B200K_ACT_GELU>(__uint_as_float(r[j])));
+  } else if (act == B200K_ACT_SILU) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) r[j] = __float_as_uint(apply_act<B200K_ACT_SILU>(__uint_as_float(r[j])));
   }
 }
 
-// Stores 32 consecutive columns of one output row.
-template <typename OutT>
-__device__ __forceinline__ void store_chunk(OutT* dst, const uint32_t (&r)[32], float scale, int valid_cols,
-                                            bool vec_ok) {
-  if (valid_cols >= 32 && vec_ok) {
-    if constexpr (sizeof(OutT) == 4) {
+// One 128-byte piece of a row of C out of N = 128 / sizeof(OutT) accumulator values, as eight 16-byte chunks.
+template <typename OutT, int N>
+__device__ __forceinline__ void pack_row(const uint32_t (&r)[N], float scale, uint4 (&v)[8]) {
+  static_assert(N * sizeof(OutT) == 128, "a piece is 128 bytes");
+  constexpr int kPer = 16 / static_cast<int>(sizeof(OutT));
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float4 v = make_float4(__uint_as_float(r[4 * i]) * scale, __uint_as_float(r[4 * i + 1]) * scale,
-                               __uint_as_float(r[4 * i + 2]) * scale, __uint_as_float(r[4 * i + 3]) * scale);
-        reinterpret_cast<float4*>(dst)[i] = v;
-      }
-    } else {
+  for (int i = 0; i < 8; ++i) {
+    union {
+      uint4 u;
+      OutT e[kPer];
+    } pk;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+    for (int j = 0; j < kPer; ++j) pk.e[j] = to_out<OutT>(__uint_as_float(r[kPer * i + j]) * scale);
+    v[i] = pk.u;
+  }
+}
+
+// Writes a staged piece (32 rows x 128 bytes, 16-byte chunks XOR-swizzled by row) to a matrix whose
+// rows are not 16-byte aligned, V bytes per lane: lanes side by side write neighbouring bytes, so an
+// instruction covers whole sectors of 1 (V = 4), 2 (V = 8) rows or half of one (V = 2).  (One row
+// per lane instead, a column per instruction, touched 32 sectors each time: a 6388 x 1446 x 1440 fp8
+// product took 129 us that way.)
+template <typename OutT, typename V>
+__device__ __forceinline__ void store_piece(OutT* c, int64_t ldc, const uint8_t* buf, int lane, int rows, int cols) {
+  constexpr int kPerRow = 128 / static_cast<int>(sizeof(V));
+  constexpr int kElems = static_cast<int>(sizeof(V) / sizeof(OutT));
+#pragma unroll 4
+  for (int u = lane; u < 32 * kPerRow; u += 32) {
+    const int lr = u / kPerRow;
+    const int byte = (u % kPerRow) * static_cast<int>(sizeof(V));
+    const V val = *reinterpret_cast<const V*>(buf + lr * 128 + (((byte >> 4) ^ (lr & 7)) << 4) + (byte & 15));
+    const int col = byte / static_cast<int>(sizeof(OutT));
+    OutT* dst = c + static_cast<int64_t>(lr) * ldc + col;
+    if (lr < rows) {
+      // a row pitch that allows V-byte stores may still end inside one (C is a column slice)
+      if (col + kElems <= cols) {
+        *reinterpret_cast<V*>(dst) = val;
+      } else {
         union {
-          uint4 u;
-          OutT h[8];
+          V v;
+          OutT e[kElems];
         } pk;
+        pk.v = val;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) pk.h[j] = to_out<OutT>(__uint_as_float(r[8 * i + j]) * scale);
-        reinterpret_cast<uint4*>(dst)[i] = pk.u;
+        for (int i = 0; i < kElems; ++i)
+          if (col + i < cols) dst[i] = pk.e[i];
       }
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (i < valid_cols) dst[i] = to_out<OutT>(__uint_as_float(r[i]) * scale);
   }
+}
+
+template <typename OutT>
+__device__ __forceinline__ void store_piece_any(OutT* c, int64_t ldc, const uint8_t* buf, int lane, int rows, int cols,
+                                                int store_bytes) {
+  if (store_bytes == 8)
+    store_piece<OutT, uint2>(c, ldc, buf, lane, rows, cols);
+  else if (sizeof(OutT) == 4 || store_bytes == 4)
+    store_piece<OutT, uint32_t>(c, ldc, buf, lane, rows, cols);
+  else if constexpr (sizeof(OutT) == 2)
+    store_piece<OutT, uint16_t>(c, ldc, buf, lane, rows, cols);
 }
 
 }  // namespace gemm_detail

@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       scale = sa * sb;
     }
     const bool fused = p.bias != nullptr || p.act != 0;  // uniform over the grid
+    float* bias_s = reinterpret_cast<float*>(smem + S::kBiasOffset);
     OutT* cbase = reinterpret_cast<OutT*>(p.c);
     uint8_t* staging = smem + S::kStagingOffset + (warp - 2) * (2 * 4096);
     uint32_t stg_count = 0;
@@ -220,68 +221,86 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       tile_coords(t - bz * tiles_per_problem, p.tiles_m, p.tiles_n, tm, tn);
       const int acc = it % kAccBufs;
       const uint32_t acc_phase = (it / kAccBufs) & 1;
+      // The tile's bias, fetched while the main loop runs (columns past n re-read the last one: never stored).
+      constexpr int kBiasPerThread = BN / 128;
+      float tile_bias[kBiasPerThread] = {};
+      const int et = static_cast<int>(threadIdx.x) - 64;  // epilogue thread 0..127
+      if (p.bias != nullptr) {
+#pragma unroll
+        for (int i = 0; i < kBiasPerThread; ++i)
+          tile_bias[i] = load_bias(p.bias, p.bias_dtype, min(tn * BN + i * 128 + et, p.n - 1));
+      }
       bool ok = mbar_wait(tfull + acc, acc_phase, abort_word);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      if (fused) {
+        // all four warps are done with the previous tile's bias, and give up together if one wait ran out
+        ok = bar_red_and(1, 128, ok);
+        if (!ok) break;
+#pragma unroll
+        for (int i = 0; i < kBiasPerThread; ++i) bias_s[i * 128 + et] = tile_bias[i];
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+      } else {
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+      }
       tc_fence_after();
 #pragma unroll
       for (int h = 0; h < MT; ++h) {
         const int row0 = tm * kTileM + h * kBM + quarter * 32;
-        const int row = row0 + lane;
         const uint32_t taddr =
             tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (MT == 1 ? acc * BN : h * BN);
-        if (p.num_peers > 0 && !p.peer_tma) {
-          // Column shard written straight into every rank's full C (own copy included): registers ->
-          // swizzled staging buffer -> each store instruction writes four full 128-byte row segments
-          // to one peer, so the NVLink traffic is made of whole lines.
-          constexpr int kCols = 128 / static_cast<int>(sizeof(OutT));
+        // 128 bytes of each of this warp's 32 rows per step: registers -> swizzled staging buffer ->
+        // C.  Two buffers per warp; a buffer is reused once its store has been read.
+        constexpr int kCols = 128 / static_cast<int>(sizeof(OutT));
+        const bool by_tma = p.tma_store_ok || p.peer_tma;
 #pragma unroll 1
-          for (int c = 0; c < BN / kCols; ++c) {
-            uint8_t* buf = staging;
-            uint4 v[8];
-            if constexpr (sizeof(OutT) == 4) {
-              uint32_t r[32];
-              tmem_ld_32x32b_x32(taddr + c * 32, r);
-              tmem_wait_ld();
-              float sc = scale;
-              if (fused) {
-                fused_epilogue<32>(r, scale, p.bias, p.bias_dtype, p.act, tn * BN + c * 32, p.n);
-                sc = 1.f;
-              }
+        for (int c = 0; c < BN / kCols; ++c) {
+          const int col = tn * BN + c * kCols;
+          if (col >= p.n) break;
+          uint8_t* buf = staging + (stg_count & 1) * 4096;
+          uint32_t r[kCols];
+          uint4 v[8];
+          if constexpr (kCols == 32)
+            tmem_ld_32x32b_x32(taddr + c * 32, r);
+          else
+            tmem_ld_32x32b_x64(taddr + c * 64, r);
+          if (by_tma && lane == 0) tma_store_wait_read<1>();
+          tmem_wait_ld();
+          if (fused) {
+            fused_epilogue<kCols>(r, scale, bias_s + c * kCols, p.act);
+            pack_row<OutT>(r, 1.f, v);
+          } else {
+            pack_row<OutT>(r, scale, v);
+          }
+          __syncwarp();  // the buffer is free: its last bulk store has been read, or its last reads by this warp are done
 #pragma unroll
-              for (int i = 0; i < 8; ++i)
-                v[i] = make_uint4(__float_as_uint(__uint_as_float(r[4 * i]) * sc),
-                                  __float_as_uint(__uint_as_float(r[4 * i + 1]) * sc),
-                                  __float_as_uint(__uint_as_float(r[4 * i + 2]) * sc),
-                                  __float_as_uint(__uint_as_float(r[4 * i + 3]) * sc));
-            } else {
-              uint32_t r[64];
-              tmem_ld_32x32b_x64(taddr + c * 64, r);
-              tmem_wait_ld();
-              float sc = scale;
-              if (fused) {
-                fused_epilogue<64>(r, scale, p.bias, p.bias_dtype, p.act, tn * BN + c * 64, p.n);
-                sc = 1.f;
-              }
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                union {
-                  uint4 u;
-                  OutT e[8];
-                } pk;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) pk.e[j] = to_out<OutT>(__uint_as_float(r[8 * i + j]) * sc);
-                v[i] = pk.u;
-              }
-            }
-            __syncwarp();  // previous chunk's reads of the staging buffer are done
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              *reinterpret_cast<uint4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4)) = v[i];
+          for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<uint4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4)) = v[i];
+          if (by_tma) {
+            // One TMA store (full 128-byte lines, clipped at the matrix edge by the tensor map).
+            // Fused all-gather: the same piece goes out once per rank, through that rank's map, as
+            // bulk stores to peer-mapped memory; the copy engine of the SM moves the data while the
+            // warp prepares the next piece.
+            fence_proxy_async_smem();
             __syncwarp();
-            const int col = tn * BN + c * kCols;  // column inside the shard
+            if (lane == 0) {
+              if (p.num_peers > 0) {
+                int pe = p.peer_first;
+                for (int i = 0; i < p.num_peers; ++i) {
+                  tma_store_2d(&peer_maps.m[pe], buf, col, row0);
+                  pe = pe + 1 == p.num_peers ? 0 : pe + 1;
+                }
+              } else {
+                tma_store_3d(&tmap_c, buf, col, row0, bz);
+              }
+              tma_store_commit();
+            }
+          } else if (p.num_peers > 0) {
+            // Column shard written straight into every rank's full C (own copy included): each store
+            // instruction writes four full 128-byte row segments to one peer, so the NVLink traffic is
+            // made of whole lines.
+            __syncwarp();
             const int chunk = lane & 7;
-            const int ecol = col + chunk * (16 / static_cast<int>(sizeof(OutT)));
+            const int ecol = col + chunk * (16 / static_cast<int>(sizeof(OutT)));  // column inside the shard
 #pragma unroll
             for (int rr = 0; rr < 8; ++rr) {
               const int lr = rr * 4 + (lane >> 3);
@@ -306,92 +325,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 }
               }
             }
-          }
-        } else if (p.tma_store_ok || p.peer_tma) {
-          // 128 bytes of each of this warp's 32 rows per step: registers -> swizzled staging
-          // buffer -> one TMA store (full 128-byte lines, clipped at the matrix edge by the
-          // tensor map).  Two buffers per warp; a buffer is reused once its store has been read.
-          // Fused all-gather: the same piece goes out once per rank, through that rank's map, as
-          // bulk stores to peer-mapped memory; the copy engine of the SM moves the data while the
-          // warp prepares the next piece.
-          constexpr int kCols = 128 / static_cast<int>(sizeof(OutT));
-#pragma unroll 1
-          for (int c = 0; c < BN / kCols; ++c) {
-            uint8_t* buf = staging + (stg_count & 1) * 4096;
-            if (lane == 0) tma_store_wait_read<1>();
+          } else {
             __syncwarp();
-            uint4 v[8];
-            if constexpr (sizeof(OutT) == 4) {
-              uint32_t r[32];
-              tmem_ld_32x32b_x32(taddr + c * 32, r);
-              tmem_wait_ld();
-              float sc = scale;
-              if (fused) {
-                fused_epilogue<32>(r, scale, p.bias, p.bias_dtype, p.act, tn * BN + c * 32, p.n);
-                sc = 1.f;
-              }
-#pragma unroll
-              for (int i = 0; i < 8; ++i)
-                v[i] = make_uint4(__float_as_uint(__uint_as_float(r[4 * i]) * sc),
-                                  __float_as_uint(__uint_as_float(r[4 * i + 1]) * sc),
-                                  __float_as_uint(__uint_as_float(r[4 * i + 2]) * sc),
-                                  __float_as_uint(__uint_as_float(r[4 * i + 3]) * sc));
-            } else {
-              uint32_t r[64];
-              tmem_ld_32x32b_x64(taddr + c * 64, r);
-              tmem_wait_ld();
-              float sc = scale;
-              if (fused) {
-                fused_epilogue<64>(r, scale, p.bias, p.bias_dtype, p.act, tn * BN + c * 64, p.n);
-                sc = 1.f;
-              }
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                union {
-                  uint4 u;
-                  OutT e[8];
-                } pk;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) pk.e[j] = to_out<OutT>(__uint_as_float(r[8 * i + j]) * sc);
-                v[i] = pk.u;
-              }
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              *reinterpret_cast<uint4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4)) = v[i];
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              if (p.num_peers > 0) {
-                int pe = p.peer_first;
-                for (int i = 0; i < p.num_peers; ++i) {
-                  tma_store_2d(&peer_maps.m[pe], buf, tn * BN + c * kCols, row0);
-                  pe = pe + 1 == p.num_peers ? 0 : pe + 1;
-                }
-              } else {
-                tma_store_3d(&tmap_c, buf, tn * BN + c * kCols, row0, bz);
-              }
-              tma_store_commit();
-            }
-            ++stg_count;
+            store_piece_any<OutT>(cbase + bz * p.c_batch_stride + static_cast<int64_t>(row0) * p.ldc + col, p.ldc, buf,
+                                  lane, p.m - row0, p.n - col, p.store_bytes);
           }
-        } else {
-#pragma unroll 2
-          for (int c = 0; c < BN / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld_32x32b_x32(taddr + c * 32, r);
-            tmem_wait_ld();
-            const int col = tn * BN + c * 32;
-            float sc = scale;
-            if (fused) {
-              fused_epilogue<32>(r, scale, p.bias, p.bias_dtype, p.act, col, p.n);
-              sc = 1.f;
-            }
-            if (row < p.m && col < p.n) {
-              store_chunk<OutT>(cbase + bz * p.c_batch_stride + static_cast<int64_t>(row) * p.ldc + col, r, sc, p.n - col,
-                                p.vec_store_ok != 0);
-            }
-          }
+          ++stg_count;
         }
       }
       tc_fence_before();
@@ -717,6 +656,9 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   if (peers.num > 0) p.vec_store_ok = 0;
 
   p.tma_store_ok = p.vec_store_ok;
+  const uint64_t c_bytes = reinterpret_cast<uintptr_t>(a.c) | static_cast<uint64_t>(a.ldc * out_es) |
+                           static_cast<uint64_t>(p.c_batch_stride * out_es);
+  p.store_bytes = c_bytes % 8 == 0 ? 8 : (c_bytes % 4 == 0 ? 4 : 2);
   CUtensorMap tc;
   memset(&tc, 0, sizeof(tc));
   if (p.tma_store_ok) {
