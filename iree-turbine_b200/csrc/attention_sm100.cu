@@ -309,19 +309,33 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
     if (warp == kKvWarp) {
       // ---------------- K / V producer: ring entries K_0 V_0 K_1 V_1 ... of every item ----------------
-      if (lane == 0) {
+      // Dense: lane 0 issues one box per tile and 64-column block.  Paged: one box per page and block,
+      // each page by a lane of its own, the page numbers read a tile ahead (one lane looking up and
+      // issuing page after page paid the latency of a table read per page: a 4 x 512-query chunk over up
+      // to 4000 keys in pages of 16 took 203 us that way).
+      const bool issuer = PAGED || lane == 0;
+      if (issuer) {
         uint32_t e = 0;  // ring entries issued so far
         bool ok = true;
-        // One 128-row K or V tile.  Dense: one box per 64-column block.  Paged: one box per page and
-        // block; a page past the sequence's length is replaced by the sequence's first page (those
-        // rows are masked; the data only has to be finite), an entry outside the pool is reported
-        // and reads as zeros (the tensor map clips it).
-        auto load_tile = [&](const CUtensorMap* tm, const Item& it, int j) {
+        const int pages_per_tile = PAGED ? kTileRows / p.page_size : 1;
+        // Page of this lane's part of tile j; a page past the sequence's length is replaced by the
+        // sequence's first page (those rows are masked; the data only has to be finite).
+        auto page_of = [&](const Item& it, int j) {
+          if (!PAGED || lane >= pages_per_tile || j >= it.nmax) return 0;
+          const int lp = j * pages_per_tile + lane;
+          const int valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
+          return __ldg(p.block_table + static_cast<int64_t>(it.batch) * p.block_table_stride + (lp < valid_pages ? lp : 0));
+        };
+        // One 128-row K or V tile.  A table entry outside the pool is reported and reads as zeros (the
+        // tensor map clips it).
+        auto load_tile = [&](const CUtensorMap* tm, const Item& it, int j, int page) {
           const uint32_t stage = e % kKvStages;
-          if (!mbar_wait(kv_empty + stage, ((e / kKvStages) & 1) ^ 1, abort_word)) return false;
+          bool got = mbar_wait(kv_empty + stage, ((e / kKvStages) & 1) ^ 1, abort_word);
+          if (PAGED) got = __all_sync(0xffffffffu, got);
+          if (!got) return false;
           uint8_t* dst = smem + L::kKvOffset + stage * kTileBytes;
           uint64_t* bar = kv_full + stage;
-          mbar_arrive_expect_tx(bar, kTileBytes);
+          if (lane == 0) mbar_arrive_expect_tx(bar, kTileBytes);
           ++e;
           if (!PAGED) {
 #pragma unroll
@@ -329,23 +343,24 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
               tma_load_4d(dst + db * kHalfTileBytes, tm, bar, db * 64, j * kTileRows, it.head / group, it.batch);
             return true;
           }
-          const int32_t* row = p.block_table + static_cast<int64_t>(it.batch) * p.block_table_stride;
-          const int pages_per_tile = kTileRows / p.page_size;
-          const int valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
-          for (int pp = 0; pp < pages_per_tile; ++pp) {
-            const int lp = j * pages_per_tile + pp;
-            const int page = __ldg(row + (lp < valid_pages ? lp : 0));
+          __syncwarp();  // the bytes are announced before any of them can arrive
+          if (lane < pages_per_tile) {
             if ((page < 0 || page >= p.num_pages) && p.status) atomicOr(p.status, kStatusDecodeBadPage);
 #pragma unroll
             for (int db = 0; db < kBlocks; ++db)
-              tma_load_4d(dst + db * kHalfTileBytes + pp * p.page_size * 128, tm, bar, db * 64, 0, it.head / group, page);
+              tma_load_4d(dst + db * kHalfTileBytes + lane * p.page_size * 128, tm, bar, db * 64, 0, it.head / group, page);
           }
           return true;
         };
         ItemWalk<PAGED> walk(p);
         Item it;
         while (ok && walk.next_busy(it)) {
-          for (int j = 0; j < it.nmax && ok; ++j) ok = load_tile(&tmap_k, it, j) && load_tile(&tmap_v, it, j);
+          int page = page_of(it, 0);
+          for (int j = 0; j < it.nmax && ok; ++j) {
+            const int page_next = page_of(it, j + 1);
+            ok = load_tile(&tmap_k, it, j, page) && load_tile(&tmap_v, it, j, page);
+            page = page_next;
+          }
         }
       }
       __syncwarp();

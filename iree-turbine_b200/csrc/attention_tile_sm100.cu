@@ -249,52 +249,71 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
     if (warp == kTmaWarp) {
       // ---------------- TMA producer ----------------
-      if (lane == 0) {
+      // Dense: lane 0 issues one box per tile and 64-column block.  Paged: one box per page and block,
+      // each page by a lane of its own, and the page numbers of the next K and V tile are read a tile
+      // ahead.  (One lane looking up and issuing page after page paid the latency of a table read per
+      // page, 8 of them per tile at page size 16: about 3 us per 128 keys where the math needs 1.)
+      const bool issuer = PAGED || lane == 0;
+      if (issuer) {
         uint32_t qc = 0, kc = 0, vc = 0;  // Q loads, K tiles, V tiles issued so far
         bool ok = true;
-        // One 128-row K or V tile.  Dense: one box per 64-column block.  Paged: one box per page and
-        // block; a page past the sequence's length is replaced by the sequence's first page (those
-        // rows are masked; the data only has to be finite), an entry outside the pool is reported
-        // and reads as zeros (the tensor map clips it).
-        auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, const Item& it, int j) {
+        const int pages_per_tile = PAGED ? kTileRows / p.page_size : 1;
+        // Page of this lane's part of tile j; a page past the sequence's length is replaced by the
+        // sequence's first page (those rows are masked; the data only has to be finite).
+        auto page_of = [&](const Item& it, int j) {
+          if (!PAGED || lane >= pages_per_tile || j >= it.n) return 0;
+          const int lp = j * pages_per_tile + lane;
+          const int valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
+          return __ldg(p.block_table + static_cast<int64_t>(it.batch) * p.block_table_stride + (lp < valid_pages ? lp : 0));
+        };
+        // One 128-row K or V tile (the caller has waited for the stage).  A table entry outside the pool
+        // is reported and reads as zeros (the tensor map clips it).
+        auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, const Item& it, int j, int page) {
+          if (lane == 0) mbar_arrive_expect_tx(bar, kTileBytes);
           if (!PAGED) {
 #pragma unroll
             for (int db = 0; db < 2; ++db)
               tma_load_4d(dst + db * kHalfTileBytes, tm, bar, db * 64, j * kTileRows, it.head / group, it.batch);
             return;
           }
-          const int32_t* row = p.block_table + static_cast<int64_t>(it.batch) * p.block_table_stride;
-          const int pages_per_tile = kTileRows / p.page_size;
-          const int valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
-          for (int pp = 0; pp < pages_per_tile; ++pp) {
-            const int lp = j * pages_per_tile + pp;
-            const int page = __ldg(row + (lp < valid_pages ? lp : 0));
+          __syncwarp();  // the bytes are announced before any of them can arrive
+          if (lane < pages_per_tile) {
             if ((page < 0 || page >= p.num_pages) && p.status) atomicOr(p.status, kStatusDecodeBadPage);
 #pragma unroll
             for (int db = 0; db < 2; ++db)
-              tma_load_4d(dst + db * kHalfTileBytes + pp * p.page_size * 128, tm, bar, db * 64, 0, it.head / group, page);
+              tma_load_4d(dst + db * kHalfTileBytes + lane * p.page_size * 128, tm, bar, db * 64, 0, it.head / group, page);
           }
         };
-        auto load_k = [&](const Item& it, int j) {
+        auto wait_free = [&](uint64_t* bar, uint32_t parity) {
+          bool got = mbar_wait(bar, parity, abort_word);
+          if (PAGED) got = __all_sync(0xffffffffu, got);
+          return got;
+        };
+        auto load_k = [&](const Item& it, int j, int page) {
           const int ks = kc % kKStages;
-          if (!mbar_wait(k_empty + ks, ((kc / kKStages) & 1) ^ 1, abort_word)) return false;
-          mbar_arrive_expect_tx(k_full + ks, kTileBytes);
-          load_tile(smem + kKOffset + ks * kTileBytes, &tmap_k, k_full + ks, it, j);
+          if (!wait_free(k_empty + ks, ((kc / kKStages) & 1) ^ 1)) return false;
+          load_tile(smem + kKOffset + ks * kTileBytes, &tmap_k, k_full + ks, it, j, page);
           ++kc;
           return true;
         };
         // Q and the first K tiles of an item.  Q's buffer is free once the previous item's last
         // score MMA has run, which is earlier than the release of its last V stage.
         auto load_head = [&](const Item& it) {
-          if (!mbar_wait(q_empty, (qc & 1) ^ 1, abort_word)) return false;
-          mbar_arrive_expect_tx(q_full, kTileBytes);
+          int pages[kKStages];
 #pragma unroll
-          for (int db = 0; db < 2; ++db)
-            tma_load_4d(smem + kQOffset + db * kHalfTileBytes, &tmap_q, q_full, db * 64, it.qtile * kTileRows, it.head,
-                        it.batch);
+          for (int jj = 0; jj < kKStages; ++jj) pages[jj] = page_of(it, jj);
+          if (!wait_free(q_empty, (qc & 1) ^ 1)) return false;
+          if (lane == 0) {
+            mbar_arrive_expect_tx(q_full, kTileBytes);
+#pragma unroll
+            for (int db = 0; db < 2; ++db)
+              tma_load_4d(smem + kQOffset + db * kHalfTileBytes, &tmap_q, q_full, db * 64, it.qtile * kTileRows, it.head,
+                          it.batch);
+          }
           ++qc;
-          for (int jj = 0; jj < kKStages && jj < it.n; ++jj)
-            if (!load_k(it, jj)) return false;
+#pragma unroll
+          for (int jj = 0; jj < kKStages; ++jj)
+            if (jj < it.n && !load_k(it, jj, pages[jj])) return false;
           return true;
         };
         auto next_item = [&](int idx, Item& nx) {  // next item of this CTA that has work; num_items if none
@@ -313,17 +332,20 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           const bool have_next = nidx < p.num_items;
           // Order within an item: V_j, then K_(j+3); a K stage is released (by the score MMA that
           // read it) earlier than a V stage.  The head of the next item goes before the last V.
+          int vpage = page_of(it, 0), kpage = page_of(it, kKStages);
           for (int j = 0; j < it.n && ok; ++j) {
+            const int vpage_next = page_of(it, j + 1), kpage_next = page_of(it, j + 1 + kKStages);
             if (j == it.n - 1 && have_next) {
               ok = load_head(nx);
               if (!ok) break;
             }
             const int vs = vc % kVStages;
-            if (!mbar_wait(v_empty + vs, ((vc / kVStages) & 1) ^ 1, abort_word)) { ok = false; break; }
-            mbar_arrive_expect_tx(v_full + vs, kTileBytes);
-            load_tile(smem + kVOffset + vs * kTileBytes, &tmap_v, v_full + vs, it, j);
+            if (!wait_free(v_empty + vs, ((vc / kVStages) & 1) ^ 1)) { ok = false; break; }
+            load_tile(smem + kVOffset + vs * kTileBytes, &tmap_v, v_full + vs, it, j, vpage);
             ++vc;
-            if (j + kKStages < it.n) ok = load_k(it, j + kKStages);
+            if (j + kKStages < it.n) ok = load_k(it, j + kKStages, kpage);
+            vpage = vpage_next;
+            kpage = kpage_next;
           }
           it = nx;
           idx = nidx;
