@@ -658,6 +658,7 @@ struct LinearFunction : torch::autograd::Function<LinearFunction> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias) {
     at::AutoDispatchBelowADInplaceOrView below;
     ctx->save_for_backward({x, w});
+    ctx->saved_data["bias"] = bias.has_value() && bias->defined();
     return call_linear_act(x, w, bias);
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
@@ -668,7 +669,8 @@ struct LinearFunction : torch::autograd::Function<LinearFunction> {
     Tensor dx, dw, db;
     if (ctx->needs_input_grad(0)) dx = call_gemm(dy, w, false, false, x.scalar_type());  // [M, N] @ [N, K]
     if (ctx->needs_input_grad(1)) dw = call_gemm(dy, x, true, false, w.scalar_type());   // [M, N]^T @ [M, K]
-    if (ctx->needs_input_grad(2)) db = dy.to(at::kFloat).sum(0).to(dy.scalar_type());
+    // an absent bias is not among the inputs that needs_input_grad counts
+    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) db = dy.to(at::kFloat).sum(0).to(dy.scalar_type());
     return {dx, dw, db};
   }
 };
