@@ -1,9 +1,10 @@
 // Decode and paged-decode attention: one query token per sequence against its KV history,
-// grouped-query heads, split over KV chunks (phase 1) and merged by a reduction kernel.
+// grouped-query heads, split over KV chunks where that pays (plan_decode) and merged inside a
+// thread-block cluster or by a reduction kernel.
 //
 // The path is HBM-bandwidth bound (about 4 flop per byte of KV), so the design goal is bytes
 // in flight, not math throughput:
-//   * a CTA owns one (sequence, kv head, KV chunk); its 4 warps each own every 4th 16-token
+//   * a CTA owns one (sequence, kv head, KV chunk); its 4 (8) warps each own every 4th (8th) 16-token
 //     tile of the chunk and run a private cp.async ring (no CTA-wide barrier in the main loop);
 //   * every global access to K/V is a 16-byte cp.async, a warp's 32 lanes covering 512
 //     contiguous bytes of a page slab; the page id comes from the block table once per tile;
@@ -18,6 +19,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -26,15 +28,12 @@ namespace b200k {
 namespace {
 
 constexpr int kTileTokens = 16;
-constexpr int kDecodeWarps = 4;
-constexpr int kDecodeThreads = kDecodeWarps * 32;
 constexpr int kDecodeStages = 3;
 // per head dim HD (128 or 64): a tile is 16 tokens x HD halves for K and the same for V
 template <int HD>
 struct DecodeTile {
   static constexpr int kRowBytes = HD * 2;
   static constexpr int kBytes = kTileTokens * kRowBytes;                        // 4 KB (HD 128) or 2 KB
-  static constexpr int kSmem = kDecodeWarps * kDecodeStages * 2 * kBytes;       // 96 KB or 48 KB
   static constexpr int kChunksPerRow = kRowBytes / 16;                          // 16-byte pieces per row
 };
 constexpr float kLog2e = 1.4426950408889634f;
@@ -51,6 +50,10 @@ struct DecodeParams {
   int32_t num_seqs, q_heads, kv_heads, group;
   int32_t page_size, num_pages, block_table_stride;
   int32_t chunk_tokens, max_chunks;
+  int32_t warps;    // per CTA: 4, two CTAs per SM; 8 where the grid leaves SMs with one CTA or none
+  int32_t stages;   // ring stages per warp: kDecodeStages, or fewer where a chunk has fewer tiles per warp
+  int32_t cluster;  // > 0: the chunks of a (sequence, kv head) are one thread-block cluster of this size, which
+                    // merges its partial results itself; 0: they go to ws_o / ws_ml and to the reduction kernel
   int32_t max_seq_len;  // seq_lens entries are clamped to [0, max_seq_len]
   int32_t* status;      // optional device status word
   int64_t kv_batch_stride, kv_head_stride, kv_page_stride;
@@ -138,29 +141,46 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+constexpr int kMaxCluster = 8;     // portable cluster size
+constexpr int kReduceThreads = 256;
+constexpr int kMergeHead = 8 * 16 * 8 + 16 * 8;  // bytes of shared memory for (max, sum) per warp and per chunk
+
+// Four dims of one output row: accumulator / sum, zero for a row without keys.
+template <typename T>
+__device__ __forceinline__ void store_out(const DecodeParams& p, int seq, int q_head, int d, float4 acc, float L,
+                                          int head_dim) {
+  const float inv_ok = L > 0.f ? 1.f : 0.f;
+  const float den = L > 0.f ? L : 1.f;
+  uint2 u;
+  u.x = pack2<T>(acc.x / den * inv_ok, acc.y / den * inv_ok);
+  u.y = pack2<T>(acc.z / den * inv_ok, acc.w / den * inv_ok);
+  T* o = reinterpret_cast<T*>(p.o) + (static_cast<int64_t>(seq) * p.q_heads + q_head) * head_dim + d;
+  *reinterpret_cast<uint2*>(o) = u;
+}
+
+__device__ __forceinline__ int clamped_len(const DecodeParams& p, int seq, bool report) {
+  const int given = __ldg(p.seq_lens + seq);
+  if (report && given > p.max_seq_len && p.status) atomicOr(p.status, kStatusDecodeLenClamped);
+  return max(0, min(given, p.max_seq_len));
+}
+
 // ------------------------------------------------------------------------------------------
 // phase 1
 // ------------------------------------------------------------------------------------------
-template <typename T, bool PAGED, int HD>
-__global__ void __launch_bounds__(kDecodeThreads, 2) decode_splitkv_kernel(const DecodeParams p) {
+template <typename T, bool PAGED, int HD, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 2 : 1) decode_splitkv_kernel(const DecodeParams p) {
+  constexpr int kDecodeWarps = WARPS;
+  constexpr int kDecodeThreads = WARPS * 32;
   constexpr int kHeadDim = HD;
   constexpr int kTileBytes = DecodeTile<HD>::kBytes;
   constexpr int kRowBytes = DecodeTile<HD>::kRowBytes;
   constexpr int kChunks = DecodeTile<HD>::kChunksPerRow;
   constexpr int kKSteps = HD / 16;  // k-steps of the score product = 16-dim slices of the head dim
-  const int chunk = blockIdx.x;
-  const int kvh = blockIdx.y;
-  const int seq = blockIdx.z;
-  // seq_lens is device data the host cannot validate: a length beyond what the grid, the workspace
-  // and the block table were sized for is cut to max_seq_len (and reported), a negative one to 0.
-  const int len_given = __ldg(p.seq_lens + seq);
-  const int len = max(0, min(len_given, p.max_seq_len));
-  if (len_given > p.max_seq_len && chunk == 0 && kvh == 0 && threadIdx.x == 0 && p.status)
-    atomicOr(p.status, kStatusDecodeLenClamped);
-  const int chunk_start = chunk * p.chunk_tokens;
-  if (chunk_start >= len) return;
-  const int chunk_end = min(len, chunk_start + p.chunk_tokens);
-  const int n_tiles = (chunk_end - chunk_start + kTileTokens - 1) / kTileTokens;
+  // Launched with programmatic stream serialization: the previous kernel's results (the appended K/V
+  // rows, the queries, the lengths) are visible from here on.  The reduction kernel may start filling
+  // idle SMs when the last CTAs of this grid have begun.
+  grid_dependency_wait();
+  grid_dependency_trigger();
 
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5;
@@ -168,11 +188,27 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) decode_splitkv_kernel(const
   const int g = lane >> 2;  // fragment row
   const int t = lane & 3;   // fragment column pair
   const int G = p.group;
-
-  uint8_t* warp_smem = smem + warp * (kDecodeStages * 2 * kTileBytes);
+  uint8_t* warp_smem = smem + warp * (p.stages * 2 * kTileBytes);
   const uint32_t warp_smem_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(warp_smem));
   const T* kbase = reinterpret_cast<const T*>(p.k);
   const T* vbase = reinterpret_cast<const T*>(p.v);
+
+  const int chunk = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z;
+  // seq_lens is device data the host cannot validate: a length beyond what the grid, the workspace
+  // and the block table were sized for is cut to max_seq_len (and reported), a negative one to 0.
+  const int len = clamped_len(p, seq, chunk == 0 && kvh == 0 && threadIdx.x == 0);
+  const int chunk_start = chunk * p.chunk_tokens;
+  // A CTA past the end of its sequence has nothing to add; in a cluster it still takes part in the merge.
+  if (chunk_start >= len && p.cluster <= 1 && (p.cluster == 0 || len > 0)) return;
+  const int chunk_end = min(len, chunk_start + p.chunk_tokens);
+  float* sm_m = reinterpret_cast<float*>(smem);                 // [warps][16]
+  float* sm_l = sm_m + kDecodeWarps * 16;                       // [warps][16]
+  float2* sm_ml = reinterpret_cast<float2*>(sm_l + kDecodeWarps * 16);  // [G] of the chunk
+  float* sm_acc = reinterpret_cast<float*>(smem + kMergeHead);  // [G][HD] of the chunk
+  float* sm_o = sm_acc + G * kHeadDim;                          // [warps][G][HD]
+  constexpr int kQuads = HD / 4;  // float4 pieces per row
+
+  const int n_tiles = max(0, (chunk_end - chunk_start + kTileTokens - 1) / kTileTokens);
 
   // Query fragments: rows = heads of the group (zero beyond G), HD / 16 k-steps of 16 dims.
   uint32_t qf[kKSteps][4];
@@ -324,11 +360,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) decode_splitkv_kernel(const
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
   __syncthreads();  // every warp is done with its ring; reuse shared memory
-  float* sm_o = reinterpret_cast<float*>(smem);                 // [warps][16][HD]
-  float* sm_m = sm_o + kDecodeWarps * 16 * kHeadDim;            // [warps][16]
-  float* sm_l = sm_m + kDecodeWarps * 16;                       // [warps][16]
   {
-    float* wo = sm_o + warp * 16 * kHeadDim;
+    float* wo = sm_o + warp * G * kHeadDim;
 #pragma unroll
     for (int i = 0; i < HD / 8; ++i) {
       const int col = i * 8 + 2 * t;
@@ -343,55 +376,161 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) decode_splitkv_kernel(const
     }
   }
   __syncthreads();
-  {
-    const int d = threadIdx.x;  // one thread per output dim (the upper half idles at HD 64)
-    for (int r = 0; r < G && d < kHeadDim; ++r) {
-      float M = -INFINITY;
+  for (int u = threadIdx.x; u < G * kQuads; u += kDecodeThreads) {
+    const int r = u / kQuads, d = (u % kQuads) * 4;
+    float M = -INFINITY;
 #pragma unroll
-      for (int w = 0; w < kDecodeWarps; ++w) M = fmaxf(M, sm_m[w * 16 + r]);
-      const float Ms = (M == -INFINITY) ? 0.f : M;
-      float L = 0.f, acc = 0.f;
+    for (int w = 0; w < kDecodeWarps; ++w) M = fmaxf(M, sm_m[w * 16 + r]);
+    const float Ms = (M == -INFINITY) ? 0.f : M;
+    float L = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int w = 0; w < kDecodeWarps; ++w) {
-        const float f = fast_exp2(sm_m[w * 16 + r] - Ms);
-        L += sm_l[w * 16 + r] * f;
-        acc += sm_o[(w * 16 + r) * kHeadDim + d] * f;
-      }
+    for (int w = 0; w < kDecodeWarps; ++w) {
+      const float f = fast_exp2(sm_m[w * 16 + r] - Ms);
+      const float4 x = *reinterpret_cast<const float4*>(sm_o + (w * G + r) * kHeadDim + d);
+      L += sm_l[w * 16 + r] * f;
+      acc.x += x.x * f;
+      acc.y += x.y * f;
+      acc.z += x.z * f;
+      acc.w += x.w * f;
+    }
+    if (p.cluster == 1) {
+      store_out<T>(p, seq, kvh * G + r, d, acc, L, kHeadDim);
+    } else if (p.cluster == 0) {
       const int64_t slot = (static_cast<int64_t>(seq) * p.q_heads + kvh * G + r) * p.max_chunks + chunk;
-      p.ws_o[slot * kHeadDim + d] = acc;
+      *reinterpret_cast<float4*>(p.ws_o + slot * kHeadDim + d) = acc;
       if (d == 0) p.ws_ml[slot] = make_float2(M, L);
+    } else {
+      *reinterpret_cast<float4*>(sm_acc + r * kHeadDim + d) = acc;
+      if (d == 0) sm_ml[r] = make_float2(M, L);
     }
   }
+  if (p.cluster <= 1) return;
+
+  // Merge over the cluster: CTA `rank` takes every cluster-th row x 4-dim piece and reads it from all
+  // CTAs that had keys through distributed shared memory, in rank order (the same bits whatever the timing).
+  cluster_sync_all();
+  {
+    const int rank = static_cast<int>(cluster_ctarank());
+    const int n_chunks = min(p.cluster, (len + p.chunk_tokens - 1) / p.chunk_tokens);
+    const uint32_t ml_addr = smem_u32(sm_ml), acc_addr = smem_u32(sm_acc);
+    for (int u = threadIdx.x * p.cluster + rank; u < G * kQuads; u += kDecodeThreads * p.cluster) {
+      const int r = u / kQuads, d = (u % kQuads) * 4;
+      float2 ml[kMaxCluster];
+      float4 x[kMaxCluster];
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c) {
+        if (c >= n_chunks) break;
+        ml[c] = ld_shared_cluster_f32x2(cluster_map_shared(ml_addr + r * 8, c));
+        x[c] = ld_shared_cluster_f32x4(cluster_map_shared(acc_addr + (r * kHeadDim + d) * 4, c));
+      }
+      float M = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c)
+        if (c < n_chunks) M = fmaxf(M, ml[c].x);
+      const float Ms = (M == -INFINITY) ? 0.f : M;
+      float L = 0.f;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c)
+        if (c < n_chunks) {
+          const float f = fast_exp2(ml[c].x - Ms);
+          L += ml[c].y * f;
+          acc.x += x[c].x * f;
+          acc.y += x[c].y * f;
+          acc.z += x[c].z * f;
+          acc.w += x[c].w * f;
+        }
+      store_out<T>(p, seq, kvh * G + r, d, acc, L, kHeadDim);
+    }
+  }
+  cluster_sync_all();  // no CTA leaves (and frees its shared memory) while a peer still reads it
 }
 
 // ------------------------------------------------------------------------------------------
 // phase 2: merge chunks
 // ------------------------------------------------------------------------------------------
+// One CTA per (sequence, query head): 8 warps take every 8th chunk each, a lane 4 (2 at HD 64) dims of
+// it, so the loads of many chunks are in flight at once.  (One thread per dim walking the chunks one
+// after another took 26 us for 7 sequences x 4 heads x 245 chunks.)
 template <typename T, int HD>
-__global__ void __launch_bounds__(HD) decode_reduce_kernel(const DecodeParams p) {
-  constexpr int kHeadDim = HD;
+__global__ void __launch_bounds__(kReduceThreads) decode_reduce_kernel(const DecodeParams p) {
+  constexpr int kPer = HD / 32;  // dims per lane
+  constexpr int kWarps = kReduceThreads / 32;
+  using Vec = typename std::conditional<HD == 128, float4, float2>::type;
+  __shared__ float wpart[kReduceThreads];      // exp2(max of chunk - max of all) of a batch of chunks
+  __shared__ float red[kWarps];
+  __shared__ Vec part[kWarps][32];
   const int qh = blockIdx.x;
   const int seq = blockIdx.y;
-  const int d = threadIdx.x;
-  const int len = max(0, min(__ldg(p.seq_lens + seq), p.max_seq_len));  // same clamp as phase 1
-  const int n_chunks = (len + p.chunk_tokens - 1) / p.chunk_tokens;      // <= max_chunks
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int len = clamped_len(p, seq, false);  // same clamp as phase 1
+  const int n_chunks = (len + p.chunk_tokens - 1) / p.chunk_tokens;  // <= max_chunks
   const int64_t slot0 = (static_cast<int64_t>(seq) * p.q_heads + qh) * p.max_chunks;
+  const float2* ml = p.ws_ml + slot0;
+  auto block_sum_or_max = [&](float v, bool is_max) {
+#pragma unroll
+    for (int i = 16; i > 0; i >>= 1) {
+      const float w = __shfl_xor_sync(0xffffffffu, v, i);
+      v = is_max ? fmaxf(v, w) : v + w;
+    }
+    __syncthreads();
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    v = red[0];
+#pragma unroll
+    for (int i = 1; i < kWarps; ++i) v = is_max ? fmaxf(v, red[i]) : v + red[i];
+    return v;
+  };
   float M = -INFINITY;
-  for (int c = 0; c < n_chunks; ++c) M = fmaxf(M, p.ws_ml[slot0 + c].x);
+  for (int c = threadIdx.x; c < n_chunks; c += kReduceThreads) M = fmaxf(M, ml[c].x);
+  M = block_sum_or_max(M, true);
   const float Ms = (M == -INFINITY) ? 0.f : M;
-  float L = 0.f, acc = 0.f;
-  for (int c = 0; c < n_chunks; ++c) {
-    const float2 ml = p.ws_ml[slot0 + c];
-    const float f = fast_exp2(ml.x - Ms);
-    L += ml.y * f;
-    acc += p.ws_o[(slot0 + c) * kHeadDim + d] * f;
+  float L = 0.f;
+  float acc[kPer] = {};
+  for (int c0 = 0; c0 < n_chunks; c0 += kReduceThreads) {
+    const int c = c0 + threadIdx.x;
+    float f = 0.f;
+    if (c < n_chunks) {
+      const float2 v = ml[c];
+      f = fast_exp2(v.x - Ms);
+      L += v.y * f;
+    }
+    __syncthreads();
+    wpart[threadIdx.x] = f;
+    __syncthreads();
+    const int n = min(kReduceThreads, n_chunks - c0);
+#pragma unroll 4
+    for (int i = warp; i < n; i += kWarps) {
+      const float w = wpart[i];
+      const Vec x = *reinterpret_cast<const Vec*>(p.ws_o + (slot0 + c0 + i) * HD + lane * kPer);
+      acc[0] += x.x * w;
+      acc[1] += x.y * w;
+      if constexpr (HD == 128) {
+        acc[2] += x.z * w;
+        acc[3] += x.w * w;
+      }
+    }
   }
-  const float out = (L > 0.f) ? acc / L : 0.f;
-  T* o = reinterpret_cast<T*>(p.o) + (static_cast<int64_t>(seq) * p.q_heads + qh) * kHeadDim + d;
-  if constexpr (sizeof(T) == 2 && std::is_same<T, __half>::value)
-    *o = __float2half_rn(out);
-  else
-    *o = __float2bfloat16_rn(out);
+  L = block_sum_or_max(L, false);
+  part[warp][lane] = *reinterpret_cast<const Vec*>(acc);
+  __syncthreads();
+  if (threadIdx.x < HD / 4) {
+    const float* all = reinterpret_cast<const float*>(part);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int d = threadIdx.x * 4;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float4 x = *reinterpret_cast<const float4*>(all + w * HD + d);
+      o.x += x.x;
+      o.y += x.y;
+      o.z += x.z;
+      o.w += x.w;
+    }
+    store_out<T>(p, seq, qh, d, o, L, HD);
+  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -452,48 +591,121 @@ int validate_decode(const b200k_decode_args& a) {
   return B200K_OK;
 }
 
+template <typename T, bool PAGED, int HD, int WARPS>
+int launch_splitkv(const DecodeParams& p, int num_seqs, cudaStream_t stream) {
+  auto kfn = decode_splitkv_kernel<T, PAGED, HD, WARPS>;
+  constexpr int kStageSmem = WARPS * 2 * DecodeTile<HD>::kBytes;
+  constexpr int kMaxMerge = kMergeHead + (WARPS + 1) * 16 * HD * static_cast<int>(sizeof(float));
+  constexpr int kMaxSmem = kDecodeStages * kStageSmem > kMaxMerge ? kDecodeStages * kStageSmem : kMaxMerge;
+  static bool configured[64] = {};
+  int rc = ensure_dynamic_smem(kfn, kMaxSmem, configured, "cudaFuncSetAttribute(decode smem)");
+  if (rc) return rc;
+  const int ring = p.stages * kStageSmem;
+  const int merge = kMergeHead + (WARPS + 1) * p.group * HD * static_cast<int>(sizeof(float));
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.cluster > 0 ? p.cluster : p.max_chunks, p.kv_heads, num_seqs);
+  cfg.blockDim = dim3(WARPS * 32, 1, 1);
+  cfg.dynamicSmemBytes = static_cast<size_t>(ring > merge ? ring : merge);
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(p.cluster > 0 ? p.cluster : 1);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.cluster > 1 ? 2 : 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kfn, p), "decode_splitkv_kernel launch");
+}
+
 template <typename T, int HD>
 int launch_decode_typed(const DecodeParams& p, bool paged, int num_seqs, cudaStream_t stream) {
-  dim3 grid(p.max_chunks, p.kv_heads, num_seqs);
-  constexpr int kSmem = DecodeTile<HD>::kSmem;
   int rc;
-  if (paged) {
-    auto kfn = decode_splitkv_kernel<T, true, HD>;
-    static bool configured[64] = {};
-    rc = ensure_dynamic_smem(kfn, kSmem, configured, "cudaFuncSetAttribute(decode smem)");
-    if (rc) return rc;
-    kfn<<<grid, kDecodeThreads, kSmem, stream>>>(p);
-  } else {
-    auto kfn = decode_splitkv_kernel<T, false, HD>;
-    static bool configured[64] = {};
-    rc = ensure_dynamic_smem(kfn, kSmem, configured, "cudaFuncSetAttribute(decode smem)");
-    if (rc) return rc;
-    kfn<<<grid, kDecodeThreads, kSmem, stream>>>(p);
-  }
-  rc = check_cuda(cudaGetLastError(), "decode_splitkv_kernel launch");
-  if (rc) return rc;
-  decode_reduce_kernel<T, HD><<<dim3(p.q_heads, num_seqs), HD, 0, stream>>>(p);
-  return check_cuda(cudaGetLastError(), "decode_reduce_kernel launch");
+  if (p.warps == 8)
+    rc = paged ? launch_splitkv<T, true, HD, 8>(p, num_seqs, stream) : launch_splitkv<T, false, HD, 8>(p, num_seqs, stream);
+  else
+    rc = paged ? launch_splitkv<T, true, HD, 4>(p, num_seqs, stream) : launch_splitkv<T, false, HD, 4>(p, num_seqs, stream);
+  if (rc || p.cluster > 0) return rc;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.q_heads, num_seqs, 1);
+  cfg.blockDim = dim3(kReduceThreads, 1, 1);
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, decode_reduce_kernel<T, HD>, p), "decode_reduce_kernel launch");
 }
 
 }  // namespace
 
-int32_t decode_default_chunk(const b200k_decode_args& a) {
-  if (a.chunk_tokens > 0) return a.chunk_tokens;
-  if (a.max_seq_len <= 0 || a.num_seqs <= 0 || a.kv_heads <= 0) return 64;
-  const int64_t want = 8ll * 148;  // enough CTAs to fill every SM several times over
-  int32_t ch = 512;
-  while (ch > 64 &&
-         static_cast<int64_t>(a.num_seqs) * a.kv_heads * ((a.max_seq_len + ch - 1) / ch) < want)
-    ch /= 2;
-  return ch;
+namespace {
+// How a problem is split (chunk_tokens 0: the library's choice).
+struct DecodePlan {
+  int32_t chunk, max_chunks;  // KV tokens per CTA, chunks of the longest sequence
+  int32_t cluster;            // see DecodeParams
+};
+
+// The rules below were read off a sweep over 26 problems (1 to 128 sequences, 1 to 16 kv heads, 67 to
+// 16000 tokens, lengths spread over a factor of 16), one chunk / clusters of 2, 4, 8 / two kernels with
+// 2 to 64 chunks, device time in a graph.  "Units" are (sequence, kv head) pairs; 296 CTAs are resident.
+//   * units fill the SMs: one chunk each (62 x 8 units of up to 238 tokens: 11 us, 23 with 2 chunks), the
+//     hardware hands out the next one where one ends.  Chunks stop at 2048 tokens (about 20 us), so that
+//     one long sequence among short ones does not run alone for long (64 x 8 units of up to 8192: 175 us
+//     unsplit, 180 at 2048, 183 at 512).
+//   * a quarter of the SM slots filled and at most 1024 tokens: one chunk as well (80 units of 469
+//     tokens: 8.0 us, 9.1 in clusters of two).
+//   * few units: the chunks of a unit form a cluster that merges them itself (8 units of 669 tokens: 3.8
+//     us, 4.9 with a second kernel), as long as the clusters are resident at once -- a cluster holds all
+//     its SMs until its last CTA is done, which costs ragged batches dearly in later waves (800 units of
+//     up to 1003 tokens: 20 us unsplit, 82 in clusters of eight) -- and chunks stay within 512 tokens.
+//   * the rest: about 400 CTAs of at least 192 tokens and the reduction kernel (7 units of 15695 tokens:
+//     43 us with 64-token chunks and the former reduction, 12.7 now).
+DecodePlan plan_decode(const b200k_decode_args& a) {
+  DecodePlan d = {64, 1, 0};
+  if (a.max_seq_len <= 0 || a.num_seqs <= 0 || a.kv_heads <= 0) return d;
+  const int64_t units = static_cast<int64_t>(a.num_seqs) * a.kv_heads;
+  const int64_t sms = num_sms(), slots = sms * 2;
+  const int64_t len = a.max_seq_len;
+  auto chunk_for = [&](int64_t n) { return static_cast<int32_t>(((len + n - 1) / n + 63) / 64 * 64); };
+  if (a.chunk_tokens > 0) {
+    d.chunk = a.chunk_tokens;
+  } else if (units >= slots || len <= 128 || (units * 4 >= slots && len <= 1024)) {
+    d.chunk = chunk_for((len + 2047) / 2048);
+  } else {
+    int64_t c = 1;
+    while (c < kMaxCluster && units * c * 2 <= sms && c * 64 < len) c *= 2;
+    if (c < kMaxCluster && units * c * 2 <= slots && chunk_for(c) > 512) c *= 2;
+    if (chunk_for(c) <= 512) {
+      d.chunk = chunk_for(c);
+    } else {
+      const int64_t n = (400 + units - 1) / units;
+      d.chunk = chunk_for(n);
+      if (d.chunk < 192) d.chunk = 192;
+      if (d.chunk > 2048) d.chunk = chunk_for((len + 2047) / 2048);
+    }
+  }
+  d.max_chunks = static_cast<int32_t>((len + d.chunk - 1) / d.chunk);
+  if (d.max_chunks <= kMaxCluster) {
+    int32_t c = 1;
+    while (c < d.max_chunks) c *= 2;
+    if (c == 1 || units * c <= slots) d.cluster = c;
+  }
+  return d;
 }
 
+uint64_t decode_slots(const b200k_decode_args& a, const DecodePlan& d) {
+  return static_cast<uint64_t>(a.num_seqs) * a.q_heads * d.max_chunks;
+}
+}  // namespace
+
+int32_t decode_default_chunk(const b200k_decode_args& a) { return plan_decode(a).chunk; }
+
 uint64_t decode_workspace_bytes(const b200k_decode_args& a) {
-  if (a.num_seqs <= 0 || a.q_heads <= 0 || a.max_seq_len <= 0) return 0;
-  const int32_t ch = decode_default_chunk(a);
-  const uint64_t max_chunks = (static_cast<uint64_t>(a.max_seq_len) + ch - 1) / ch;
-  const uint64_t slots = static_cast<uint64_t>(a.num_seqs) * a.q_heads * max_chunks;
+  if (a.num_seqs <= 0 || a.q_heads <= 0 || a.kv_heads <= 0 || a.max_seq_len <= 0) return 0;
+  const uint64_t slots = decode_slots(a, plan_decode(a));
   return slots * static_cast<uint64_t>(a.head_dim > 0 ? a.head_dim : 128) * sizeof(float) + slots * sizeof(float2);
 }
 
@@ -509,6 +721,7 @@ int launch_decode(const b200k_decode_args& a, cudaStream_t stream) {
   rc = ensure_sm100();
   if (rc) return rc;
 
+  const DecodePlan plan = plan_decode(a);
   DecodeParams p;
   p.q = a.q;
   p.k = a.k_cache;
@@ -523,15 +736,20 @@ int launch_decode(const b200k_decode_args& a, cudaStream_t stream) {
   p.page_size = a.block_table ? a.page_size : 16;
   p.num_pages = a.num_pages;
   p.block_table_stride = a.block_table_stride;
-  p.chunk_tokens = decode_default_chunk(a);
-  p.max_chunks = (a.max_seq_len + p.chunk_tokens - 1) / p.chunk_tokens;
+  p.chunk_tokens = plan.chunk;
+  p.max_chunks = plan.max_chunks;
+  p.cluster = plan.cluster;
+  const int64_t ctas = static_cast<int64_t>(p.max_chunks) * p.kv_heads * p.num_seqs;
+  p.warps = ctas <= num_sms() && p.chunk_tokens > 64 ? 8 : 4;
+  const int tiles_per_warp = (p.chunk_tokens / kTileTokens + p.warps - 1) / p.warps;
+  p.stages = tiles_per_warp < kDecodeStages ? tiles_per_warp : kDecodeStages;
   p.max_seq_len = a.max_seq_len;
   p.status = a.status;
   p.kv_batch_stride = a.kv_batch_stride;
   p.kv_head_stride = a.kv_head_stride;
   p.kv_page_stride = a.kv_page_stride;
   p.scale_log2 = a.scale * kLog2e;
-  const uint64_t slots = static_cast<uint64_t>(a.num_seqs) * a.q_heads * p.max_chunks;
+  const uint64_t slots = decode_slots(a, plan);
   p.ws_o = reinterpret_cast<float*>(a.workspace);
   p.ws_ml = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(a.workspace) + slots * a.head_dim * sizeof(float));
   if (p.max_chunks > 65535 * 32)
@@ -578,6 +796,8 @@ __global__ void kv_append_kernel(const uint8_t* __restrict__ k_new, const uint8_
                                  int32_t new_tokens, int32_t kv_heads, int32_t head_dim, int32_t page_size,
                                  int32_t num_pages, int32_t block_table_stride, int64_t kv_page_stride,
                                  int64_t kv_head_stride, int32_t elem_bytes, int32_t* status) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
   const int seq = blockIdx.z;
   const int head = blockIdx.y;
   const int row_bytes = head_dim * elem_bytes;
@@ -626,11 +846,21 @@ int launch_kv_append(const void* k_new, const void* v_new, void* k_cache, void* 
   const int warps = 4;
   int gx = (new_tokens + warps - 1) / warps;
   if (gx > 1024) gx = 1024;
-  kv_append_kernel<<<dim3(gx, kv_heads, num_seqs), warps * 32, 0, stream>>>(
-      reinterpret_cast<const uint8_t*>(k_new), reinterpret_cast<const uint8_t*>(v_new),
-      reinterpret_cast<uint8_t*>(k_cache), reinterpret_cast<uint8_t*>(v_cache), block_table, positions, new_tokens,
-      kv_heads, head_dim, page_size, num_pages, block_table_stride, kv_page_stride, kv_head_stride, elem_bytes, status);
-  return check_cuda(cudaGetLastError(), "kv_append_kernel launch");
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(gx, kv_heads, num_seqs);
+  cfg.blockDim = dim3(warps * 32, 1, 1);
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return check_cuda(
+      cudaLaunchKernelEx(&cfg, kv_append_kernel, reinterpret_cast<const uint8_t*>(k_new),
+                         reinterpret_cast<const uint8_t*>(v_new), reinterpret_cast<uint8_t*>(k_cache),
+                         reinterpret_cast<uint8_t*>(v_cache), block_table, positions, new_tokens, kv_heads, head_dim,
+                         page_size, num_pages, block_table_stride, kv_page_stride, kv_head_stride, elem_bytes, status),
+      "kv_append_kernel launch");
 }
 
 // ------------------------------------------------------------------------------------------
