@@ -4,13 +4,13 @@
 //   dP = dO V^T                            dS = P o (dP - delta),  delta[i] = sum_d dO[i, d] O[i, d]
 //   dQ = scale * dS K                      dK = scale * dS^T Q
 //
-// Three launches.  Only the forward's output O is required from the forward call; its row
-// log-sum-exp, if the caller kept it, spares the statistics sweep of the second launch:
-//   1. attn_bwd_delta_kernel: delta.
-//   2. attn_bwd_dq_kernel: one CTA per (batch, query head, tile of 128 queries).  It holds Q and dO
+// Two launches (three without the LSE).  Only the forward's output O is required from the forward call; its row
+// log-sum-exp, if the caller kept it, spares the statistics sweep of the dQ CTAs:
+//   1. attn_bwd_delta_kernel: delta.  Then attn_bwd_kernel, with two kinds of CTA:
+//   2. bwd_dq_cta: one CTA per (batch, query head, tile of 128 queries).  It holds Q and dO
 //      and sweeps the visible K/V tiles: first a statistics sweep when no LSE was given, then the
 //      gradient sweep (S, dP -> dS -> dQ += dS K).
-//   3. attn_bwd_dkv_t_kernel: one CTA per (batch, K/V head, tile of 128 keys).  It holds K and V
+//   3. bwd_dkv_cta: one CTA per (batch, K/V head, tile of 128 keys).  It holds K and V
 //      and sweeps the query tiles of every query head of the group that see these keys, with the
 //      keys as the M dimension of every product: S^T, dP^T -> P^T, dS^T -> dV += P^T dO,
 //      dK += dS^T Q.
@@ -194,10 +194,9 @@ __device__ __forceinline__ void load_tile_4d(uint8_t* dst, const CUtensorMap* tm
 // Measured per-iteration issue order of the MMA warp: dP(i), S(i+1), dQ(i).
 // ---------------------------------------------------------------------------------------------
 template <typename T, int HD>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-    attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
-                       const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                       const __grid_constant__ CUtensorMap tmap_dq, const BwdParams p) {
+__device__ __forceinline__ void bwd_dq_cta(int block, int blocks, const CUtensorMap& tmap_q, const CUtensorMap& tmap_do,
+                                           const CUtensorMap& tmap_k, const CUtensorMap& tmap_v,
+                                           const CUtensorMap& tmap_dq, const BwdParams& p) {
   static_assert(HD == 128 || HD == 64, "head dim 128 or 64");
   constexpr uint32_t kFmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBF16;
   constexpr uint32_t kIdKK = make_idesc(kFmt, kFmt, 128, 128, 0, 0);  // S, dP: 128 x 128, contraction over the head dim
@@ -231,11 +230,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   int bh, tile;
   if (p.causal) {
     int rank;
-    causal_work_item(blockIdx.x, gridDim.x / p.num_q_tiles, p.num_q_tiles, p.bh_group_q, bh, rank);
+    causal_work_item(block, blocks / p.num_q_tiles, p.num_q_tiles, p.bh_group_q, bh, rank);
     tile = p.num_q_tiles - 1 - rank;
   } else {
-    bh = blockIdx.x / p.num_q_tiles;
-    tile = blockIdx.x - bh * p.num_q_tiles;
+    bh = block / p.num_q_tiles;
+    tile = block - bh * p.num_q_tiles;
   }
   const int batch = bh / p.q_heads;
   const int head = bh - batch * p.q_heads;
@@ -277,6 +276,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_wait();
+  grid_dependency_trigger();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -586,11 +587,9 @@ constexpr int kNumDkvtBars = 9;
 constexpr int dkvt_smem_bytes() { return 6 * kTileBytes + kTVecBytes + kNumDkvtBars * 8 + 16 + 1024; }
 
 template <typename T, int HD>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-    attn_bwd_dkv_t_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
-                          const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                          const __grid_constant__ CUtensorMap tmap_dv, const __grid_constant__ CUtensorMap tmap_dk,
-                          const BwdParams p) {
+__device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtensorMap& tmap_q, const CUtensorMap& tmap_do,
+                                            const CUtensorMap& tmap_k, const CUtensorMap& tmap_v,
+                                            const CUtensorMap& tmap_dv, const CUtensorMap& tmap_dk, const BwdParams& p) {
   static_assert(HD == 128 || HD == 64, "head dim 128 or 64");
   constexpr uint32_t kFmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBF16;
   constexpr uint32_t kIdS = make_idesc(kFmt, kFmt, 128, 128, 0, 0);  // S^T, dP^T: 128 keys x 128 queries
@@ -619,10 +618,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   // causal: key tile 0 is seen by every query tile, the last one by few
   int bh, tile;
   if (p.causal) {
-    causal_work_item(blockIdx.x, gridDim.x / p.num_kv_tiles, p.num_kv_tiles, p.bh_group_kv, bh, tile);
+    causal_work_item(block, blocks / p.num_kv_tiles, p.num_kv_tiles, p.bh_group_kv, bh, tile);
   } else {
-    bh = blockIdx.x / p.num_kv_tiles;
-    tile = blockIdx.x - bh * p.num_kv_tiles;
+    bh = block / p.num_kv_tiles;
+    tile = block - bh * p.num_kv_tiles;
   }
   const int batch = bh / p.kv_heads;
   const int kvh = bh - batch * p.kv_heads;
@@ -658,6 +657,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_wait();
+  grid_dependency_trigger();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -876,6 +877,24 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   }
 }
 
+// With the forward's LSE at hand neither half needs anything from the other, and both kinds of CTA go
+// out in one launch: the dK / dV ones first (they sweep the query tiles of a whole head group, the longer
+// jobs), then the dQ ones fill the SMs they leave.  As two launches each ended in a wave of its own.
+// Without the LSE the dQ CTAs compute the row statistics the others need: two launches.
+template <typename T, int HD>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+    attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
+                    const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                    const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ CUtensorMap tmap_dk,
+                    const __grid_constant__ CUtensorMap tmap_dv, const BwdParams p, const int blocks_dkv,
+                    const int blocks_dq) {
+  const int block = blockIdx.x;
+  if (block < blocks_dkv)
+    bwd_dkv_cta<T, HD>(block, blocks_dkv, tmap_q, tmap_do, tmap_k, tmap_v, tmap_dv, tmap_dk, p);
+  else
+    bwd_dq_cta<T, HD>(block - blocks_dkv, blocks_dq, tmap_q, tmap_do, tmap_k, tmap_v, tmap_dq, p);
+}
+
 // delta[b, h, i] = sum_d dO[b, h, i, d] * O[b, h, i, d].  A row of HD 16-bit values is HD / 8 lanes
 // of 16 bytes; a warp takes 32 / (HD / 8) rows at a time and eight such groups, all loads issued
 // before the first use, so that enough bytes are in flight to run at memory speed.
@@ -890,6 +909,8 @@ __global__ void attn_bwd_delta_kernel(const T* __restrict__ o, const T* __restri
   const int sub = lane / kLanesPerRow, col = (lane % kLanesPerRow) * 8;
   const int64_t warp_id = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t row_base = warp_id * (kRowsPerPass * kPasses);
+  grid_dependency_wait();
+  grid_dependency_trigger();
   uint4 ov[kPasses], dv[kPasses];
 #pragma unroll
   for (int ps = 0; ps < kPasses; ++ps) {
@@ -933,30 +954,29 @@ int encode_bshd(CUtensorMap* out, int dtype, const void* base, int head_dim, int
 
 template <typename T, int HD>
 int launch_bwd_typed(const b200k_attention_bwd_args& a, const BwdMaps& tm, const BwdParams& p, cudaStream_t stream) {
-  auto k_dq = attn_bwd_dq_kernel<T, HD>;
-  auto k_dkv = attn_bwd_dkv_t_kernel<T, HD>;
-  static bool configured_dq[64] = {}, configured_dkv[64] = {};  // per instantiation and device ordinal
-  int rc = ensure_dynamic_smem(k_dq, dq_smem_bytes(), configured_dq, "cudaFuncSetAttribute(attention bwd dq smem)");
-  if (rc) return rc;
-  rc = ensure_dynamic_smem(k_dkv, dkvt_smem_bytes(), configured_dkv, "cudaFuncSetAttribute(attention bwd dkv smem)");
+  auto kfn = attn_bwd_kernel<T, HD>;
+  constexpr int kSmem = dq_smem_bytes() > dkvt_smem_bytes() ? dq_smem_bytes() : dkvt_smem_bytes();
+  static bool configured[64] = {};  // per instantiation and device ordinal
+  int rc = ensure_dynamic_smem(kfn, kSmem, configured, "cudaFuncSetAttribute(attention bwd smem)");
   if (rc) return rc;
   const int64_t rows = static_cast<int64_t>(a.batch) * a.q_heads * a.seq_q;
   if (rows > INT32_MAX) return set_error(B200K_ERR_BAD_SHAPE, "attention_bwd: batch * q_heads * seq_q must be below 2^31");
   const int warps_per_block = 8;
   const int64_t rows_per_block = static_cast<int64_t>(warps_per_block) * (32 / (HD / 8)) * 8;
-  attn_bwd_delta_kernel<T, HD><<<static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block),
-                             warps_per_block * 32, 0, stream>>>(
-      static_cast<const T*>(a.o), static_cast<const T*>(a.d_o), p.delta, rows, a.q_heads, a.seq_q, a.o_stride_b,
-      a.o_stride_h, a.o_stride_s, a.do_stride_b, a.do_stride_h, a.do_stride_s);
-  rc = check_cuda(cudaGetLastError(), "attn_bwd_delta_kernel launch");
+  rc = launch_pdl("attn_bwd_delta_kernel launch", attn_bwd_delta_kernel<T, HD>,
+                  dim3(static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block)), dim3(warps_per_block * 32), 0,
+                  stream, static_cast<const T*>(a.o), static_cast<const T*>(a.d_o), p.delta, rows, a.q_heads, a.seq_q,
+                  a.o_stride_b, a.o_stride_h, a.o_stride_s, a.do_stride_b, a.do_stride_h, a.do_stride_s);
   if (rc) return rc;
-  const int grid_dq = a.batch * a.q_heads * p.num_q_tiles;
-  k_dq<<<grid_dq, kBwdThreads, dq_smem_bytes(), stream>>>(tm.q, tm.d_o, tm.k, tm.v, tm.dq, p);
-  rc = check_cuda(cudaGetLastError(), "attn_bwd_dq_kernel launch");
-  if (rc) return rc;
-  const int grid_dkv = a.batch * a.kv_heads * p.num_kv_tiles;
-  k_dkv<<<grid_dkv, kBwdThreads, dkvt_smem_bytes(), stream>>>(tm.q, tm.d_o, tm.k, tm.v, tm.dv, tm.dk, p);
-  return check_cuda(cudaGetLastError(), "attn_bwd_dkv_t_kernel launch");
+  const int blocks_dq = a.batch * a.q_heads * p.num_q_tiles;
+  const int blocks_dkv = a.batch * a.kv_heads * p.num_kv_tiles;
+  auto launch = [&](int dkv, int dq) {
+    return launch_pdl("attn_bwd_kernel launch", kfn, dim3(dkv + dq), dim3(kBwdThreads), kSmem, stream, tm.q, tm.d_o, tm.k,
+                      tm.v, tm.dq, tm.dk, tm.dv, p, dkv, dq);
+  };
+  if (p.lse_in) return launch(blocks_dkv, blocks_dq);
+  rc = launch(0, blocks_dq);
+  return rc ? rc : launch(blocks_dkv, 0);
 }
 
 }  // namespace
@@ -1028,8 +1048,8 @@ int launch_attention_bwd(const b200k_attention_bwd_args& a, cudaStream_t stream)
     p.bh_group_q = group_for(p.num_q_tiles, a.batch * a.q_heads);
     p.bh_group_kv = group_for(p.num_kv_tiles, a.batch * a.kv_heads);
   }
-  if (static_cast<int64_t>(a.batch) * a.q_heads * p.num_q_tiles > INT32_MAX ||
-      static_cast<int64_t>(a.batch) * a.kv_heads * p.num_kv_tiles > INT32_MAX)
+  if (static_cast<int64_t>(a.batch) * a.q_heads * p.num_q_tiles +
+          static_cast<int64_t>(a.batch) * a.kv_heads * p.num_kv_tiles > INT32_MAX)
     return set_error(B200K_ERR_BAD_SHAPE, "attention_bwd: too many tiles");
   p.scale = a.scale;
   p.scale_log2 = a.scale * kLog2eBwd;

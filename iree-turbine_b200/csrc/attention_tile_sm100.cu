@@ -244,6 +244,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const int group = p.q_heads / p.kv_heads;
+  // (launch_pdl) everything above ran under the tail of the previous kernel
+  grid_dependency_wait();
+  grid_dependency_trigger();
 
   if (warp >= 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
@@ -704,8 +707,11 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   if (rc) return rc;
   const int sms = num_sms();
   const int grid = p.num_items < sms ? p.num_items : sms;
-  kfn<<<grid, kAttnThreads, kAttnSmem, stream>>>(tq, tk, tv, to, p);
-  return check_cuda(cudaGetLastError(), "attn_fwd_kernel launch");
+  // Launched early only when short: CTAs of an early launch land on SMs in the order these come free, which
+  // scatters the CTAs that share a head's K / V over both dies (8 x 32 x 1024 non-causal, 110 tiles per
+  // CTA: 156 us in blockIdx order, 162 launched early).
+  const int64_t tiles = static_cast<int64_t>(p.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
+  return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tq, tk, tv, to, p);
 }
 
 }  // namespace

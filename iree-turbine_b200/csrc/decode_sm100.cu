@@ -627,16 +627,8 @@ int launch_decode_typed(const DecodeParams& p, bool paged, int num_seqs, cudaStr
   else
     rc = paged ? launch_splitkv<T, true, HD, 4>(p, num_seqs, stream) : launch_splitkv<T, false, HD, 4>(p, num_seqs, stream);
   if (rc || p.cluster > 0) return rc;
-  cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.q_heads, num_seqs, 1);
-  cfg.blockDim = dim3(kReduceThreads, 1, 1);
-  cfg.stream = stream;
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return check_cuda(cudaLaunchKernelEx(&cfg, decode_reduce_kernel<T, HD>, p), "decode_reduce_kernel launch");
+  return launch_pdl("decode_reduce_kernel launch", decode_reduce_kernel<T, HD>, dim3(p.q_heads, num_seqs),
+                    dim3(kReduceThreads), 0, stream, p);
 }
 
 }  // namespace
@@ -846,21 +838,11 @@ int launch_kv_append(const void* k_new, const void* v_new, void* k_cache, void* 
   const int warps = 4;
   int gx = (new_tokens + warps - 1) / warps;
   if (gx > 1024) gx = 1024;
-  cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(gx, kv_heads, num_seqs);
-  cfg.blockDim = dim3(warps * 32, 1, 1);
-  cfg.stream = stream;
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return check_cuda(
-      cudaLaunchKernelEx(&cfg, kv_append_kernel, reinterpret_cast<const uint8_t*>(k_new),
-                         reinterpret_cast<const uint8_t*>(v_new), reinterpret_cast<uint8_t*>(k_cache),
-                         reinterpret_cast<uint8_t*>(v_cache), block_table, positions, new_tokens, kv_heads, head_dim,
-                         page_size, num_pages, block_table_stride, kv_page_stride, kv_head_stride, elem_bytes, status),
-      "kv_append_kernel launch");
+  return launch_pdl("kv_append_kernel launch", kv_append_kernel, dim3(gx, kv_heads, num_seqs), dim3(warps * 32), 0, stream,
+                    reinterpret_cast<const uint8_t*>(k_new), reinterpret_cast<const uint8_t*>(v_new),
+                    reinterpret_cast<uint8_t*>(k_cache), reinterpret_cast<uint8_t*>(v_cache), block_table, positions,
+                    new_tokens, kv_heads, head_dim, page_size, num_pages, block_table_stride, kv_page_stride,
+                    kv_head_stride, elem_bytes, status);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -369,17 +369,8 @@ int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& 
   if (rc) return rc;
   // Programmatic dependent launch: barrier set-up and the tensor-memory allocation of this kernel
   // overlap the tail of whatever runs before it in the stream (see grid_dependency_wait in the kernel).
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
-  cfg.blockDim = dim3(kGemmThreads, 1, 1);
-  cfg.dynamicSmemBytes = S::kDynamic;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return check_cuda(cudaLaunchKernelEx(&cfg, kfn, ta, tb, tc, p, pm), "gemm_nt_kernel launch");
+  return launch_pdl("gemm_nt_kernel launch", kfn, dim3(static_cast<unsigned>(grid)), dim3(kGemmThreads), S::kDynamic, stream,
+                    ta, tb, tc, p, pm);
 }
 
 template <int BN, int MT>

@@ -169,6 +169,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_wait();
+  grid_dependency_trigger();
 
   // This CTA: tile of its cluster, slice of the k-blocks by its rank.
   const int rank = static_cast<int>(cluster_ctarank());
@@ -317,19 +319,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
 }
 
-void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int grid, int split, int smem_bytes,
+void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int grid, int split, int smem_bytes,
                     cudaStream_t stream) {
   cfg = cudaLaunchConfig_t{};
   cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
   cfg.blockDim = dim3(kGemmThreads, 1, 1);
   cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
   cfg.stream = stream;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = static_cast<unsigned>(split);
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(split);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_pdl
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
 }
 
 template <int BN, int KIND, typename OutT, int EPI>
@@ -341,7 +345,7 @@ int launch_fused(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams&
   if (rc) return rc;
   const int64_t ctas = static_cast<int64_t>(p.tiles_m) * p.tiles_n * p.batch * p.split;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr;
+  cudaLaunchAttribute attr[2];
   cluster_config(cfg, attr, static_cast<int>(ctas), p.split, S::kDynamic, stream);
   return check_cuda(cudaLaunchKernelEx(&cfg, kfn, ta, tb, p), "gemm_splitk_kernel launch");
 }
@@ -375,7 +379,7 @@ int resident_clusters(int split) {
   static bool configured[64] = {};
   if (ensure_dynamic_smem(kfn, S::kDynamic, configured, "cudaFuncSetAttribute(split-K gemm smem)") != 0) return 0;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr;
+  cudaLaunchAttribute attr[2];
   cluster_config(cfg, attr, split, split, S::kDynamic, nullptr);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, kfn, &cfg) != cudaSuccess) {
