@@ -102,7 +102,17 @@ __device__ __forceinline__ float apply_act(float x) {
   if constexpr (ACT == B200K_ACT_RELU) return fmaxf(x, 0.f);
   if constexpr (ACT == B200K_ACT_GELU)  // exact (erf) form, the default of aten::gelu
     return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-  if constexpr (ACT == B200K_ACT_SILU) return x / (1.f + __expf(-x));
+  if constexpr (ACT == B200K_ACT_SILU) {
+    // x / (1 + e^-x) by a hardware reciprocal and one Newton-Raphson step, which squares its 2^-23 error
+    // away.  (The IEEE division this was before branches to a slow path per element: 2048^3 took 52 us
+    // with it, 16 without an activation.)  The exponent is capped where the result is below 2e-36 anyway,
+    // so that 1 + e^-x stays finite.
+    const float d = 1.f + __expf(fminf(-x, 87.f));
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = r * fmaf(-d, r, 2.f);
+    return x * r;
+  }
   return x;
 }
 

@@ -32,17 +32,15 @@ struct ReduceCtx {
   int rank, tm, tn, bz;
 };
 
-// CTA `rank` of a cluster of SPLIT sums rows [rank * 128 / SPLIT, (rank + 1) * 128 / SPLIT) of the
-// tile over all partial tiles, in rank order, and stores them.  A thread takes four 16-byte chunks
-// at a time and issues all their peer loads before the first add, so the latency of distributed
-// shared memory is paid once per batch, not once per chunk.
-template <int BN, int KIND, typename OutT, int EPI, int SPLIT>
-__device__ __forceinline__ void reduce_band(const ReduceCtx<OutT>& c) {
+// CTA `rank` of a cluster of SPLIT sums its share of the tile over all partial tiles, in rank order, and
+// stores it.  The shares divide the rows the matrix really has here (a product of 16 rows keeps all CTAs
+// of the cluster busy, not the one that owns the first 128 / SPLIT rows).  A thread takes four 16-byte
+// chunks at a time and issues all their peer loads before the first add, so the latency of distributed
+// shared memory is paid once per batch, not once per chunk; fewer where the share is small.
+template <int BN, int KIND, typename OutT, int EPI, int SPLIT, int BATCH>
+__device__ __forceinline__ void reduce_share(const ReduceCtx<OutT>& c, int u_begin, int u_end) {
   const GemmParams& p = c.p;
   constexpr int kChunksPerRow = BN / 4;
-  constexpr int kRows = kBM / SPLIT;
-  constexpr int kUnits = kRows * kChunksPerRow;
-  constexpr int kBatch = 4;
   float scale = 1.0f;
   if constexpr (KIND == kKindE4M3) {
     const float* sa = p.scale_a ? p.scale_a : &kUnitScale;
@@ -50,56 +48,57 @@ __device__ __forceinline__ void reduce_band(const ReduceCtx<OutT>& c) {
     scale = *sa * *sb;
   }
   OutT* cbase = reinterpret_cast<OutT*>(p.c) + c.bz * p.c_batch_stride;
-  for (int u0 = threadIdx.x; u0 < kUnits; u0 += kGemmThreads * kBatch) {
-    float4 sum[kBatch];
-    uint32_t off[kBatch];
+  for (int u0 = u_begin + static_cast<int>(threadIdx.x); u0 < u_end; u0 += kGemmThreads * BATCH) {
+    float4 sum[BATCH];
+    uint32_t off[BATCH];
+    float bias[BATCH][4];
 #pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
-      const int u = min(u0 + b * kGemmThreads, kUnits - 1);  // past the end: re-read the last unit, not stored
-      const int lr = c.rank * kRows + u / kChunksPerRow;
+    for (int b = 0; b < BATCH; ++b) {
+      const int u = min(u0 + b * kGemmThreads, u_end - 1);  // past the end: re-read the last unit, not stored
+      const int lr = u / kChunksPerRow;
       const int ch = u % kChunksPerRow;
       off[b] = static_cast<uint32_t>(lr * (BN * 4) + ((ch ^ (lr & 7)) << 4));
       sum[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if constexpr (EPI == 2) {
+        // the bias index is clamped, not predicated: every load is in bounds whatever the compiler
+        // does with its order (columns past n are not stored)
+        const int col = c.tn * BN + ch * 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bias[b][j] = load_bias(p.bias, p.bias_dtype, min(col + j, p.n - 1));
+      }
     }
-    float4 v[SPLIT][kBatch];
+    float4 v[SPLIT][BATCH];
 #pragma unroll
     for (int s = 0; s < SPLIT; ++s)
 #pragma unroll
-      for (int b = 0; b < kBatch; ++b)
+      for (int b = 0; b < BATCH; ++b)
         v[s][b] = ld_shared_cluster_f32x4(cluster_map_shared(c.smem_base + off[b], static_cast<uint32_t>(s)));
 #pragma unroll
     for (int s = 0; s < SPLIT; ++s)
 #pragma unroll
-      for (int b = 0; b < kBatch; ++b) {
+      for (int b = 0; b < BATCH; ++b) {
         sum[b].x += v[s][b].x;
         sum[b].y += v[s][b].y;
         sum[b].z += v[s][b].z;
         sum[b].w += v[s][b].w;
       }
 #pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
+    for (int b = 0; b < BATCH; ++b) {
       const int u = u0 + b * kGemmThreads;
-      if (u >= kUnits) break;
-      const int lr = c.rank * kRows + u / kChunksPerRow;
+      if (u >= u_end) break;
+      const int lr = u / kChunksPerRow;
       const int ch = u % kChunksPerRow;
       const int row = c.tm * kBM + lr;
       const int col = c.tn * BN + ch * 4;
-      if (row >= p.m || col >= p.n) continue;
+      if (col >= p.n) continue;
       uint32_t r[4] = {__float_as_uint(sum[b].x), __float_as_uint(sum[b].y), __float_as_uint(sum[b].z),
                        __float_as_uint(sum[b].w)};
-      if constexpr (EPI == 2) {
-        // the bias index is clamped, not predicated: every load is in bounds whatever the compiler
-        // does with its order (columns past n are not stored)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          r[j] = __float_as_uint(apply_act(
-              __uint_as_float(r[j]) * scale + load_bias(p.bias, p.bias_dtype, min(col + j, p.n - 1)), p.act));
-      } else if constexpr (EPI == 1) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) r[j] = __float_as_uint(apply_act(__uint_as_float(r[j]) * scale, p.act));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * scale);
+      for (int j = 0; j < 4; ++j) {
+        float x = __uint_as_float(r[j]) * scale;
+        if constexpr (EPI == 2) x += bias[b][j];
+        if constexpr (EPI >= 1) x = apply_act(x, p.act);
+        r[j] = __float_as_uint(x);
       }
       OutT* dst = cbase + static_cast<int64_t>(row) * p.ldc + col;
       if (col + 4 <= p.n && p.vec_store_ok) {
@@ -121,6 +120,16 @@ __device__ __forceinline__ void reduce_band(const ReduceCtx<OutT>& c) {
       }
     }
   }
+}
+
+template <int BN, int KIND, typename OutT, int EPI, int SPLIT>
+__device__ __forceinline__ void reduce_band(const ReduceCtx<OutT>& c) {
+  const int units = min(kBM, c.p.m - c.tm * kBM) * (BN / 4);
+  const int u_begin = units * c.rank / SPLIT, u_end = units * (c.rank + 1) / SPLIT;
+  if (u_end - u_begin > kGemmThreads)
+    reduce_share<BN, KIND, OutT, EPI, SPLIT, 4>(c, u_begin, u_end);
+  else
+    reduce_share<BN, KIND, OutT, EPI, SPLIT, 1>(c, u_begin, u_end);
 }
 
 // EPI: 0 = plain store, 1 = activation only, 2 = bias (+ activation).  Separate instantiations, so
@@ -268,10 +277,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       tc_fence_after();
       const int quarter = warp & 3;
       const int lr = quarter * 32 + lane;
+      const int rows = p.m - tm * kBM;  // rows past the matrix are not reduced
       uint8_t* prow = smem + lr * (BN * 4);
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
 #pragma unroll 2
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = 0; c < BN / 32 && quarter * 32 < rows; ++c) {
         uint32_t r[32];
         tmem_ld_32x32b_x32(taddr + c * 32, r);
         tmem_wait_ld();
