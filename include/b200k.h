@@ -417,6 +417,16 @@ int b200k_kv_append(const void* k_new, const void* v_new, void* k_cache, void* v
  */
 int b200k_quantize_e4m3(const float* x, void* y, float* scale_out, uint32_t* amax_scratch, int64_t n, void* stream);
 
+/* The same with room for one partial maximum per block (B200K_QUANTIZE_WORKSPACE_BYTES): no memset, no
+ * atomics.  A smaller workspace (4 bytes at least) takes the path of the call above; same results. */
+#define B200K_QUANTIZE_WORKSPACE_BYTES 4096u
+int b200k_quantize_e4m3_ws(const float* x, void* y, float* scale_out, void* workspace, uint64_t workspace_bytes, int64_t n,
+                           void* stream);
+
+/* out[c] = sum over r of x[r, c], summed in fp32 (the bias gradient of a linear layer).  x [rows, cols] F16 /
+ * BF16 with row pitch ld (elements), out [cols] of the same type; base, cols and ld multiples of 16 bytes. */
+int b200k_col_sum(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, int32_t dtype, void* stream);
+
 /* ---- self-test of the bounded device-side wait -------------------------------------- */
 /*
  * Every barrier wait in the kernels of this library is bounded: when one runs out the kernel sets

@@ -279,7 +279,17 @@ int b200k_selftest_bounded_wait(int32_t* status, uint32_t limit_us, void* stream
 }
 
 int b200k_quantize_e4m3(const float* x, void* y, float* scale_out, uint32_t* amax_scratch, int64_t n, void* stream) {
-  return launch_quantize_e4m3(x, y, scale_out, amax_scratch, n, static_cast<cudaStream_t>(stream));
+  return launch_quantize_e4m3(x, y, scale_out, amax_scratch, sizeof(uint32_t), n, static_cast<cudaStream_t>(stream));
+}
+
+int b200k_quantize_e4m3_ws(const float* x, void* y, float* scale_out, void* workspace, uint64_t workspace_bytes, int64_t n,
+                           void* stream) {
+  return launch_quantize_e4m3(x, y, scale_out, static_cast<uint32_t*>(workspace), workspace_bytes, n,
+                              static_cast<cudaStream_t>(stream));
+}
+
+int b200k_col_sum(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, int32_t dtype, void* stream) {
+  return launch_col_sum(x, out, rows, cols, ld, dtype, static_cast<cudaStream_t>(stream));
 }
 
 int b200k_gemm_nt_host(const b200k_gemm_args* host, const b200k_gemm_args* dev, void* stream) {

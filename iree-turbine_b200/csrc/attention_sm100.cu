@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         }
       }
     }
-    if (store_thread) tma_store_wait<0>();
+    if (store_thread) tma_store_wait_read<0>();
   } else {
     // ---------------- softmax of query tile t = warp / 4 ----------------
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));

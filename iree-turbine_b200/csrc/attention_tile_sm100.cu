@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       ++ic;
       g0 += it.n;
     }
-    if (store_thread) tma_store_wait<0>();
+    if (store_thread) tma_store_wait_read<0>();
   } else {
     // ---------------- softmax / correction: warpgroup w takes the KV steps g with (g & 1) == w ----------------
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));

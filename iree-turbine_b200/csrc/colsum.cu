@@ -1,0 +1,123 @@
+// Column sums of a 16-bit matrix in fp32 (the bias gradient of a linear layer): out[c] = sum_r x[r, c].
+//
+// HBM- or L2-bound: 2 bytes per element read once.  A cluster of eight CTAs owns 64 columns (one
+// 128-byte line per row) and splits the rows; a thread keeps 8 columns of every 32nd row of its CTA
+// in fp32, four 16-byte loads in flight.  The partial sums meet in shared memory, then across the
+// cluster through distributed shared memory in rank order: one launch, no scratch, no atomics, the
+// same bits every time.  (The torch expression it replaces, x.float().sum(0).to(x.dtype), wrote and
+// re-read the matrix in fp32: 48 us for 3000 x 4352, in three launches; this takes 7.)
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+#include "ptx.cuh"
+
+namespace b200k {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kCols = 64;
+constexpr int kCluster = 8;
+constexpr int kRowsPerPass = kThreads / 8;  // 8 lanes of 16 bytes cover a row's 64 columns
+constexpr int kUnroll = 4;
+
+__device__ __forceinline__ float2 to_float2(__half2 v) { return __half22float2(v); }
+__device__ __forceinline__ float2 to_float2(__nv_bfloat162 v) { return __bfloat1622float2(v); }
+__device__ __forceinline__ void from_float(float v, __half& o) { o = __float2half_rn(v); }
+__device__ __forceinline__ void from_float(float v, __nv_bfloat16& o) { o = __float2bfloat16_rn(v); }
+
+template <typename T, typename T2>
+__global__ void __launch_bounds__(kThreads) col_sum_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows,
+                                                           int64_t cols, int64_t ld) {
+  __shared__ float part[kThreads / 32][kCols];
+  __shared__ float total[kCols];
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int rank = static_cast<int>(cluster_ctarank());
+  const int64_t col0 = static_cast<int64_t>(blockIdx.x / kCluster) * kCols;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t col = col0 + (lane & 7) * 8;  // cols is a multiple of 8: a piece is inside or outside as a whole
+  const int64_t r_begin = rows * rank / kCluster, r_end = rows * (rank + 1) / kCluster;
+  float acc[8] = {};
+  if (col < cols) {
+    const T* px = x + col;
+    for (int64_t r = r_begin + threadIdx.x / 8; r < r_end; r += kRowsPerPass * kUnroll) {
+      uint4 v[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int64_t rr = r + u * kRowsPerPass;
+        v[u] = rr < r_end ? __ldg(reinterpret_cast<const uint4*>(px + rr * ld)) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const T2* h = reinterpret_cast<const T2*>(&v[u]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 f = to_float2(h[i]);
+          acc[2 * i] += f.x;
+          acc[2 * i + 1] += f.y;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 8);
+    acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
+    if (lane < 8) part[warp][lane * 8 + i] = acc[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < kCols) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) s += part[w][threadIdx.x];
+    total[threadIdx.x] = s;
+  }
+  cluster_sync_all();
+  // CTA `rank` finishes 8 of the 64 columns
+  if (threadIdx.x < kCols / kCluster) {
+    const int c = rank * (kCols / kCluster) + threadIdx.x;
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < kCluster; ++k) s += ld_shared_cluster_f32(cluster_map_shared(smem_u32(total + c), k));
+    if (col0 + c < cols) from_float(s, out[col0 + c]);
+  }
+  cluster_sync_all();  // no CTA leaves while a peer still reads its sums
+}
+
+template <typename T, typename T2>
+int launch(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((cols + kCols - 1) / kCols * kCluster), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kCluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return check_cuda(cudaLaunchKernelEx(&cfg, col_sum_kernel<T, T2>, static_cast<const T*>(x), static_cast<T*>(out), rows,
+                                       cols, ld),
+                    "col_sum_kernel launch");
+}
+
+}  // namespace
+
+int launch_col_sum(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, int dtype, cudaStream_t stream) {
+  if (!x || !out) return set_error(B200K_ERR_NULL, "col_sum: NULL pointer");
+  if (rows <= 0 || cols <= 0 || cols > (int64_t(1) << 31) || ld < cols)
+    return set_error(B200K_ERR_BAD_SHAPE, "col_sum: rows and cols must be positive, the row pitch at least cols");
+  if (dtype != B200K_F16 && dtype != B200K_BF16) return set_error(B200K_ERR_BAD_DTYPE, "col_sum: dtype must be F16 or BF16");
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || cols % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 1))
+    return set_error(B200K_ERR_BAD_ALIGN, "col_sum: base, row length and row pitch must be multiples of 16 bytes");
+  int rc = ensure_sm100();
+  if (rc) return rc;
+  if (dtype == B200K_F16) return launch<__half, __half2>(x, out, rows, cols, ld, stream);
+  return launch<__nv_bfloat16, __nv_bfloat162>(x, out, rows, cols, ld, stream);
+}
+
+}  // namespace b200k

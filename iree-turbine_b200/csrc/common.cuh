@@ -50,8 +50,9 @@ int launch_kv_append(const void* k_new, const void* v_new, void* k_cache, void* 
                      int32_t page_size, int32_t num_pages, int32_t block_table_stride, int64_t kv_page_stride,
                      int64_t kv_head_stride, int32_t elem_bytes, int32_t* status, cudaStream_t stream);
 int launch_bounded_wait_selftest(int32_t* status, uint32_t limit_us, cudaStream_t stream);
-int launch_quantize_e4m3(const float* x, void* y, float* scale_out, uint32_t* amax_scratch, int64_t n,
-                         cudaStream_t stream);
+int launch_quantize_e4m3(const float* x, void* y, float* scale_out, uint32_t* amax_scratch, uint64_t scratch_bytes,
+                         int64_t n, cudaStream_t stream);
+int launch_col_sum(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, int dtype, cudaStream_t stream);
 
 // Opts a kernel into more than 48 KB of dynamic shared memory.  The attribute belongs to the
 // (function, device) pair, so it is set once per device ordinal: `done` is the caller's table, one

@@ -22,10 +22,11 @@ struct GemmParams {
   int32_t* status;
   int64_t ldc;
   int32_t m, n;
-  int32_t tiles_m, tiles_n, num_kb;  // tiles_m counts MT * 128-row tiles
+  int32_t tiles_m, tiles_n, num_kb;  // tiles_m counts MT * 128-row tiles, num_kb pipeline stages along K
+  int32_t stage_bytes;               // bytes the two loads of a pipeline stage bring
   int32_t batch;                     // independent problems (tensor maps are 3-D: [batch][rows][k])
   int32_t split;                     // split-K kernel only: CTAs per tile (= cluster size) ...
-  int32_t kb_per_split;              // ... each summing this many consecutive k-blocks
+  int32_t kb_per_split;              // ... each summing this many consecutive stages
   int64_t c_batch_stride;            // elements between the C matrices of consecutive problems
   // Optional fused epilogue: y = act(acc * scale + bias[col]); bias == nullptr and act == 0 leave
   // the plain path untouched.
@@ -35,6 +36,9 @@ struct GemmParams {
   // Operand storage (generic kernel only): a_mn = A is stored [K, M] (M contiguous), b_mn = B is
   // stored [K, N] (N contiguous); 0 = the contraction dimension K is the contiguous one.
   int32_t a_mn, b_mn;
+  // MN-major and a multiple of 64 long: the tensor map is 4-D ([batch][R / 64][K][64]) and one load brings all
+  // 64-element blocks of a stage; else one 3-D load per block, which clips at R.
+  int32_t a_blocks, b_blocks;
   int32_t vec_store_ok;
   int32_t tma_store_ok;  // C is 16-byte aligned with a 16-byte-multiple row pitch: epilogue uses TMA stores
   int32_t store_bytes;   // otherwise: widest store (2, 4 or 8 bytes) that C's base and pitches allow
@@ -57,10 +61,16 @@ struct PeerMaps {
 
 template <int BN, int MT>
 struct GemmSmem {
-  static constexpr int kStages = MT == 2 ? 3 : (BN == 256 ? 4 : 6);
-  static constexpr int kABytes = MT * kBM * kBKBytes;
+  // k-blocks (128 bytes of K) per pipeline stage.  The thread that issues the MMAs spends about 50 cycles
+  // on each of a block's four and 280 more per stage on the barrier wait, the commit and the loop.  For a
+  // tile whose MMAs execute in 64 cycles or less that thread, not the tensor core or the loads, set the
+  // pace (480 cycles per block, for BN = 64 as for BN = 128), so those tiles take two blocks per stage.
+  static constexpr int kSub = MT == 1 && BN <= 128 ? 2 : 1;
+  static constexpr int kStages = MT == 2 ? 3 : (BN == 256 ? 4 : (BN == 128 ? 3 : 4));
+  static constexpr int kABytes = MT * kBM * kBKBytes;  // per k-block
   static constexpr int kBBytes = BN * kBKBytes;
-  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kBOffset = kSub * kABytes;  // a stage: A blocks, then B blocks
+  static constexpr int kStageBytes = kSub * (kABytes + kBBytes);
   // epilogue staging: per epilogue warp two 32-row x 128-byte buffers (TMA store source)
   static constexpr int kStagingOffset = kStages * kStageBytes;
   static constexpr int kStagingBytes = 4 * 2 * 32 * 128;
@@ -80,6 +90,18 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   const int r = t - group * group_size;
   tm = first_m + r % gm;
   tn = r / gm;
+}
+
+// One k-block of an MN-major operand: R rows or columns of the tile (64-element blocks 8 KB apart), 64 K-rows.
+template <int R>
+__device__ __forceinline__ void load_mn_major(uint8_t* dst, const CUtensorMap* tmap, uint64_t* bar, int r0, int k0, int bz,
+                                              bool blocks) {
+  if (blocks) {
+    tma_load_4d(dst, tmap, bar, 0, k0, r0 >> 6, bz);
+  } else {
+#pragma unroll
+    for (int b = 0; b < R / 64; ++b) tma_load_3d(dst + b * 8192, tmap, bar, r0 + b * 64, k0, bz);
+  }
 }
 
 template <typename OutT>

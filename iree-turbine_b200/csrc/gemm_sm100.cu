@@ -107,20 +107,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             break;
           }
           uint8_t* sa = smem + stage * S::kStageBytes;
-          mbar_arrive_expect_tx(full + stage, S::kStageBytes);
-          if (GEN && p.a_mn) {
+          mbar_arrive_expect_tx(full + stage, static_cast<uint32_t>(p.stage_bytes));
 #pragma unroll
-            for (int b = 0; b < kTileM / 64; ++b)
-              tma_load_3d(sa + b * 8192, &tmap_a, full + stage, tm * kTileM + b * 64, kb * kElemsPerStage, bz);
-          } else {
-            tma_load_3d(sa, &tmap_a, full + stage, kb * kElemsPerStage, tm * kTileM, bz);
-          }
-          if (GEN && p.b_mn) {
-#pragma unroll
-            for (int b = 0; b < BN / 64; ++b)
-              tma_load_3d(sa + S::kABytes + b * 8192, &tmap_b, full + stage, tn * BN + b * 64, kb * kElemsPerStage, bz);
-          } else {
-            tma_load_3d(sa + S::kABytes, &tmap_b, full + stage, kb * kElemsPerStage, tn * BN, bz);
+          for (int sub = 0; sub < S::kSub; ++sub) {
+            const int k0 = (kb * S::kSub + sub) * kElemsPerStage;
+            uint8_t* da = sa + sub * S::kABytes;
+            uint8_t* db = sa + S::kBOffset + sub * S::kBBytes;
+            if (GEN && p.a_mn) {
+              load_mn_major<kTileM>(da, &tmap_a, full + stage, tm * kTileM, k0, bz, p.a_blocks != 0);
+            } else {
+              tma_load_3d(da, &tmap_a, full + stage, k0, tm * kTileM, bz);
+            }
+            if (GEN && p.b_mn) {
+              load_mn_major<BN>(db, &tmap_b, full + stage, tn * BN, k0, bz, p.b_blocks != 0);
+            } else {
+              tma_load_3d(db, &tmap_b, full + stage, k0, tn * BN, bz);
+            }
           }
           if (++stage == S::kStages) {
             stage = 0;
@@ -169,20 +171,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
           tc_fence_after();
           const uint32_t a_lo = (GEN ? lo0_a : lo0) + stage * (S::kStageBytes >> 4);
-          const uint32_t b_lo = (GEN ? lo0_b + stage * (S::kStageBytes >> 4) : a_lo) + (S::kABytes >> 4);
+          const uint32_t b_lo = (GEN ? lo0_b + stage * (S::kStageBytes >> 4) : a_lo) + (S::kBOffset >> 4);
           const uint32_t accum0 = kb != 0 ? 1u : 0u;
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t accum = k == 0 ? accum0 : 1u;
+          for (int sk = 0; sk < 4 * S::kSub; ++sk) {
+            const int sub = sk >> 2, k = sk & 3;
+            const uint32_t accum = sk == 0 ? accum0 : 1u;
+            const uint32_t a_sub = a_lo + sub * (S::kABytes >> 4), b_sub = b_lo + sub * (S::kBBytes >> 4);
 #pragma unroll
             for (int h = 0; h < MT; ++h) {
               if constexpr (GEN) {
-                const uint64_t a_desc = desc(a_lo + h * ((kBM * kBKBytes) >> 4) + step_a * k, hi_a);
-                const uint64_t b_desc = desc(b_lo + step_b * k, hi_b);
+                const uint64_t a_desc = desc(a_sub + h * ((kBM * kBKBytes) >> 4) + step_a * k, hi_a);
+                const uint64_t b_desc = desc(b_sub + step_b * k, hi_b);
                 umma_f16_ss(d_tmem + h * BN, a_desc, b_desc, idesc, accum);
               } else {
-                const uint64_t a_desc = desc(a_lo + h * ((kBM * kBKBytes) >> 4) + 2 * k, hi);
-                const uint64_t b_desc = desc(b_lo + 2 * k, hi);
+                const uint64_t a_desc = desc(a_sub + h * ((kBM * kBKBytes) >> 4) + 2 * k, hi);
+                const uint64_t b_desc = desc(b_sub + 2 * k, hi);
                 if constexpr (KIND == kKindE4M3)
                   umma_f8_ss(d_tmem + h * BN, a_desc, b_desc, kIdesc, accum);
                 else
@@ -222,7 +226,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const int acc = it % kAccBufs;
       const uint32_t acc_phase = (it / kAccBufs) & 1;
       // The tile's bias, fetched while the main loop runs (columns past n re-read the last one: never stored).
-      constexpr int kBiasPerThread = BN / 128;
+      constexpr int kBiasPerThread = (BN + 127) / 128;
       float tile_bias[kBiasPerThread] = {};
       const int et = static_cast<int>(threadIdx.x) - 64;  // epilogue thread 0..127
       if (p.bias != nullptr) {
@@ -236,7 +240,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         ok = bar_red_and(1, 128, ok);
         if (!ok) break;
 #pragma unroll
-        for (int i = 0; i < kBiasPerThread; ++i) bias_s[i * 128 + et] = tile_bias[i];
+        for (int i = 0; i < kBiasPerThread; ++i)
+          if (BN >= 128 || et < BN) bias_s[i * 128 + et] = tile_bias[i];
         asm volatile("bar.sync 1, 128;" ::: "memory");
       } else {
         ok = __all_sync(0xffffffffu, ok);
@@ -337,7 +342,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty + acc);
     }
-    if (lane == 0) tma_store_wait<0>();  // staging memory must outlive the last stores
+    if (lane == 0) tma_store_wait_read<0>();  // staging memory must outlive the last stores (they complete before the grid does)
     __syncwarp();
   }
 
@@ -483,41 +488,74 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
     return set_error(B200K_ERR_BAD_SHAPE, "gemm_nt: unknown activation %d", a.activation);
   if (a.bias && a.bias_dtype != B200K_F32 && a.bias_dtype != B200K_F16 && a.bias_dtype != B200K_BF16)
     return set_error(B200K_ERR_BAD_DTYPE, "gemm_nt: bias must be F32, F16 or BF16");
-  if (a.tile_n != 0 && a.tile_n != 128 && a.tile_n != 256)
-    return set_error(B200K_ERR_BAD_SHAPE, "gemm_nt: tile_n must be 0, 128 or 256");
+  if (a.tile_n != 0 && a.tile_n != 64 && a.tile_n != 128 && a.tile_n != 256)
+    return set_error(B200K_ERR_BAD_SHAPE, "gemm_nt: tile_n must be 0, 64, 128 or 256");
   if (a.tile_m != 0 && a.tile_m != 128 && a.tile_m != 256)
     return set_error(B200K_ERR_BAD_SHAPE, "gemm_nt: tile_m must be 0, 128 or 256");
   int rc = ensure_sm100();
   if (rc) return rc;
 
   const int sms = num_sms();
-  // Tile choice: estimated time = waves * tile area / efficiency.  The efficiencies are the
-  // measured throughputs of the three shapes on a many-wave problem (f16 8192^3: 1039 / 1375 /
-  // 1555 TFLOP/s), relative to one another: a 128-row tile is limited by operand delivery (a
-  // 128 x 256 tile needs 96 bytes per tensor-core cycle, a 128 x 128 tile 128), a 256 x 256 tile
-  // is not.  (An earlier model with 0.67 / 0.67 / 0.72 chose 128 x 128 tiles for 4096^3, which
-  // run at 983 TFLOP/s where 256 x 256 tiles reach 1398.)
-  auto cost = [&](int bm, int bn) {
-    const int64_t tiles = ((a.m + bm - 1) / bm) * ((a.n + bn - 1) / bn) * batch;
-    const int64_t waves = (tiles + sms - 1) / sms;
-    const double eff = bm == 256 ? 0.93 : (bn == 256 ? 0.83 : 0.62);
-    return static_cast<double>(waves) * bm * bn / eff;
+  const int k_per_stage = a.in_dtype == B200K_E4M3 ? 128 : 64;
+  const int64_t num_kb = (a.k + k_per_stage - 1) / k_per_stage;
+  // Tile shape and split: the smallest estimated time, in us.  Measured on 27 shapes (rows 1 to 6000, K 300
+  // to 16000, operands from HBM, launches back to back) a launch of whole tiles takes
+  //   fixed + waves * k-blocks * per_kb,        per_kb .20 / .25 / .39 / .62 us for 128 x 64 / 128 x 128 /
+  // 128 x 256 / 256 x 256 tiles (the first three set by the issuing thread and by what an SM can pull from
+  // L2, the last by the tensor core), plus about 3 us a wave for the last one's epilogue, which nothing
+  // overlaps.  Rows that do not start on 128-byte lines cost the narrower tiles some 15 % more L2 traffic.
+  // Split-K over a cluster of s CTAs is not persistent: every wave of resident clusters pays
+  //   fixed + k-blocks / s * per_kb + (partial tiles to shared memory, two cluster barriers, reduction),
+  // the last term 1 us plus 1.4 / 2 / 4 us for a tile of 128 rows.
+  struct Shape {
+    int m, n;
+    double fixed, per_kb, wave, reduce;
+  };
+  const double lines = (a.lda * in_es) % 128 != 0 || (a.ldb * in_es) % 128 != 0 ? 1.15 : 1.0;
+  const Shape kShapes[4] = {{128, 64, 3.4, .20 * lines, 0., 1.4},
+                            {128, 128, 3.7, .25 * lines, 0., 2.},
+                            {128, 256, 4.5, .39 * lines, 0., 4.},
+                            {256, 256, 4.5, .62, 3., 0.}};
+  auto tiles_of = [&](const Shape& t) { return ((a.m + t.m - 1) / t.m) * ((a.n + t.n - 1) / t.n) * batch; };
+  auto whole_us = [&](const Shape& t) {
+    const int64_t waves = (tiles_of(t) + sms - 1) / sms;
+    return t.fixed + static_cast<double>(waves) * (num_kb * t.per_kb + t.wave);
   };
   int bm = a.tile_m, bn = a.tile_n;
   if (bm == 256 && bn == 0) bn = 256;
-  if (bn == 0) {
-    double best = cost(128, 128);
-    bn = 128;
-    int best_bm = 128;
-    if (a.n > 128 && cost(128, 256) <= best) {
-      best = cost(128, 256);
-      bn = 256;
+  double best_us = 1e30;
+  int split = 1;
+  if (bn == 0 || (a.split_k == 0 && bm != 256)) {
+    const int given_m = bm, given_n = bn;
+    for (const Shape& t : kShapes) {
+      if ((given_m != 0 && t.m != given_m) || (given_n != 0 && (t.n != given_n || t.m != (given_m ? given_m : 128)))) continue;
+      if (given_n == 0 && t.n > 64 && a.n <= t.n / 2) continue;   // the narrower tile covers it
+      if (given_m == 0 && t.m == 256 && a.m <= 128) continue;
+      if (peers.num > 0 && t.n == 64) continue;
+      const double us = whole_us(t);
+      if (us < best_us) {
+        best_us = us;
+        bm = t.m;
+        bn = t.n;
+        split = 1;
+      }
+      if (t.m != 128 || a.split_k != 0 || peers.num > 0) continue;
+      const double rows = a.m < 128 ? a.m / 128.0 : 1.0;
+      for (int s = 2; s <= 8; s *= 2) {
+        if (num_kb < 2 * s) continue;
+        const int resident = splitk_resident_clusters(t.n, s);
+        if (resident == 0) continue;
+        const int64_t waves = (tiles_of(t) + resident - 1) / resident;
+        if (waves > 4) continue;
+        const double su = static_cast<double>(waves) * (t.fixed + static_cast<double>((num_kb + s - 1) / s) * t.per_kb + 1. + rows * t.reduce);
+        if (su < best_us) {
+          best_us = su;
+          bm = 128;
+          bn = t.n;
+          split = s;
+        }
+      }
     }
-    if (bm != 128 && a.n > 128 && a.m > 128 && cost(256, 256) < best) {
-      bn = 256;
-      best_bm = 256;
-    }
-    if (bm == 0) bm = best_bm;
   }
   if (bm == 0) bm = 128;
   if (bm == 256 && bn != 256)
@@ -536,18 +574,8 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
       bn = 256;
     }
   }
-  const int k_per_stage = a.in_dtype == B200K_E4M3 ? 128 : 64;
-  const int64_t num_kb = (a.k + k_per_stage - 1) / k_per_stage;
-
-  // Split-K over a cluster (128-row tiles, gemm_splitk_sm100.cu): worth it when the whole tiles
-  // leave most SMs idle and K is long.  Estimated cycles = waves * k-blocks per CTA * cycles per
-  // k-block (measured with operands from HBM: 568 / 750 / 1250 for 128x128 / 128x256 / 256x256
-  // tiles) + the part of the epilogue nothing overlaps; a split adds the cluster launch, two
-  // cluster barriers, the partial-tile write and the reduction through peer shared memory
-  // (measured: about 4 to 6 us more than an un-split launch of the same k-blocks).
   if (a.split_k != 0 && a.split_k != 1 && a.split_k != 2 && a.split_k != 4 && a.split_k != 8)
     return set_error(B200K_ERR_BAD_SHAPE, "gemm: split_k must be 0, 1, 2, 4 or 8");
-  int split = 1;
   if (a.split_k > 1) {
     if (peers.num > 0) return set_error(B200K_ERR_BAD_SHAPE, "gemm_nt_allgather: split_k is not supported");
     if (a.tile_m == 256) return set_error(B200K_ERR_BAD_SHAPE, "gemm: split_k needs 128-row tiles (tile_m 0 or 128)");
@@ -556,60 +584,40 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
     split = a.split_k;
     if (splitk_resident_clusters(bn, split) == 0)
       return set_error(B200K_ERR_UNSUPPORTED_ARCH, "gemm: clusters of %d CTAs cannot be launched", split);
-  } else if (a.split_k == 0 && peers.num == 0) {
-    auto cycles_kb = [](int tm, int tn) { return tm == 256 ? 1250.0 : (tn == 256 ? 750.0 : 568.0); };
-    auto split_cost = [](int tn, int s) { return tn == 256 ? 10000.0 + 2000.0 * s : 8000.0 + 1200.0 * s; };
-    auto tail = [](int tm, int tn) { return tm == 256 ? 6000.0 : (tn == 256 ? 3000.0 : 1500.0); };
-    const int64_t tiles0 = ((a.m + bm - 1) / bm) * ((a.n + bn - 1) / bn) * batch;
-    const int64_t waves0 = (tiles0 + sms - 1) / sms;
-    double best = static_cast<double>(waves0) * num_kb * cycles_kb(bm, bn) + tail(bm, bn);
-    best *= 0.9;  // a split has to win clearly
-    if (tiles0 * 2 <= sms && a.tile_m != 256) {
-      for (int tn = 128; tn <= 256; tn += 128) {
-        if (a.tile_n != 0 && a.tile_n != tn) continue;
-        if (tn == 256 && a.n <= 128) continue;
-        const int64_t tiles = ((a.m + 127) / 128) * ((a.n + tn - 1) / tn) * batch;
-        for (int s = 2; s <= 8; s *= 2) {
-          if (num_kb < 4 * s) continue;  // at least four k-blocks per slice
-          const int resident = splitk_resident_clusters(tn, s);
-          if (resident == 0) continue;
-          const int64_t waves = (tiles + resident - 1) / resident;
-          const int64_t per = (num_kb + s - 1) / s;
-          const double t = static_cast<double>(waves) * per * cycles_kb(128, tn) + tail(128, tn) + split_cost(tn, s);
-          if (t < best) {
-            best = t;
-            split = s;
-            bm = 128;
-            bn = tn;
-          }
-        }
-      }
-    }
   }
   const int tiles_m = static_cast<int>((a.m + bm - 1) / bm);
   const int tiles_n = static_cast<int>((a.n + bn - 1) / bn);
 
+  // A single tile of rows loads the rows there are (whole 8-row swizzle groups), not zeros for the rest:
+  // what lies in the other rows of the stage only reaches rows or columns of the tile that are not stored.
+  auto box_rows = [](int64_t rows, int tile) {
+    return static_cast<int>(rows < tile ? (rows + 7) / 8 * 8 : tile);
+  };
+  const int box_m = a_mn ? bm : box_rows(a.m, bm), box_n = b_mn ? bn : box_rows(a.n, bn);
+  const bool a_blocks = a_mn && a.m % 64 == 0, b_blocks = b_mn && a.n % 64 == 0;
+  // Operand map.  K-major: a box is the tile's rows x 128 bytes of K.  MN-major ([K, R] storage): 64
+  // contiguous R-elements x 64 K-rows, of one 64-element block or of all blocks of the tile.
+  auto encode_operand = [&](CUtensorMap* tm, const void* base, int64_t rows, int64_t ld, int64_t batch_stride, bool mn,
+                            bool blocks, int tile, int box) {
+    const uint64_t k = static_cast<uint64_t>(a.k), r = static_cast<uint64_t>(rows), nb = static_cast<uint64_t>(batch);
+    const uint64_t pitch = static_cast<uint64_t>(ld) * in_es;
+    const uint64_t next = batch > 1 ? static_cast<uint64_t>(batch_stride) * in_es : pitch;
+    if (blocks) {
+      const uint64_t dims[4] = {64, k, r / 64, nb};
+      const uint64_t strides[3] = {pitch, 128, next};
+      const uint32_t bx[4] = {64u, 64u, static_cast<uint32_t>(tile / 64), 1u};
+      return encode_tmap(tm, a.in_dtype, 4, const_cast<void*>(base), dims, strides, bx);
+    }
+    const uint64_t dims[3] = {mn ? r : k, mn ? k : r, nb};
+    const uint64_t strides[2] = {pitch, next};
+    const uint32_t bx[3] = {static_cast<uint32_t>(mn ? 64 : k_per_stage), static_cast<uint32_t>(mn ? 64 : box), 1u};
+    return encode_tmap(tm, a.in_dtype, 3, const_cast<void*>(base), dims, strides, bx);
+  };
   CUtensorMap ta, tb;
-  {
-    // K-major: rows of the stored matrix are rows of the tile; MN-major ([K, M] storage): one box
-    // is 64 contiguous M-elements x 64 K-rows
-    uint64_t dims[3] = {static_cast<uint64_t>(a_mn ? a.m : a.k), static_cast<uint64_t>(a_mn ? a.k : a.m),
-                        static_cast<uint64_t>(batch)};
-    uint64_t strides[2] = {static_cast<uint64_t>(a.lda) * in_es,
-                           static_cast<uint64_t>(batch > 1 ? a.a_batch_stride : a.lda) * in_es};
-    uint32_t box[3] = {static_cast<uint32_t>(a_mn ? 64 : k_per_stage), static_cast<uint32_t>(a_mn ? 64 : bm), 1u};
-    rc = encode_tmap(&ta, a.in_dtype, 3, const_cast<void*>(a.a), dims, strides, box);
-    if (rc) return rc;
-  }
-  {
-    uint64_t dims[3] = {static_cast<uint64_t>(b_mn ? a.n : a.k), static_cast<uint64_t>(b_mn ? a.k : a.n),
-                        static_cast<uint64_t>(batch)};
-    uint64_t strides[2] = {static_cast<uint64_t>(a.ldb) * in_es,
-                           static_cast<uint64_t>(batch > 1 ? a.b_batch_stride : a.ldb) * in_es};
-    uint32_t box[3] = {static_cast<uint32_t>(b_mn ? 64 : k_per_stage), static_cast<uint32_t>(b_mn ? 64 : bn), 1u};
-    rc = encode_tmap(&tb, a.in_dtype, 3, const_cast<void*>(a.b), dims, strides, box);
-    if (rc) return rc;
-  }
+  rc = encode_operand(&ta, a.a, a.m, a.lda, a.a_batch_stride, a_mn, a_blocks, bm, box_m);
+  if (rc) return rc;
+  rc = encode_operand(&tb, a.b, a.n, a.ldb, a.b_batch_stride, b_mn, b_blocks, bn, box_n);
+  if (rc) return rc;
 
   GemmParams p;
   p.c = a.c;
@@ -621,17 +629,22 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   p.act = a.activation;
   p.a_mn = a_mn ? 1 : 0;
   p.b_mn = b_mn ? 1 : 0;
+  p.a_blocks = a_blocks ? 1 : 0;
+  p.b_blocks = b_blocks ? 1 : 0;
   p.ldc = a.ldc;
   p.m = static_cast<int32_t>(a.m);
   p.n = static_cast<int32_t>(a.n);
   p.tiles_m = tiles_m;
   p.tiles_n = tiles_n;
-  p.num_kb = static_cast<int32_t>(num_kb);
-  p.kb_per_split = static_cast<int32_t>((num_kb + split - 1) / split);
-  // every slice must hold at least one k-block (an empty one would leave an accumulator unwritten)
-  while (split > 1 && static_cast<int64_t>(p.kb_per_split) * (split - 1) >= num_kb) {
+  const int sub = bm == 128 && bn <= 128 ? GemmSmem<128, 1>::kSub : 1;  // k-blocks per pipeline stage
+  const int64_t num_stages = (num_kb + sub - 1) / sub;
+  p.num_kb = static_cast<int32_t>(num_stages);
+  p.stage_bytes = sub * (box_m + box_n) * kBKBytes;
+  p.kb_per_split = static_cast<int32_t>((num_stages + split - 1) / split);
+  // every slice must hold at least one stage (an empty one would leave an accumulator unwritten)
+  while (split > 1 && static_cast<int64_t>(p.kb_per_split) * (split - 1) >= num_stages) {
     split /= 2;
-    p.kb_per_split = static_cast<int32_t>((num_kb + split - 1) / split);
+    p.kb_per_split = static_cast<int32_t>((num_stages + split - 1) / split);
   }
   p.split = split;
   p.batch = static_cast<int32_t>(batch);
@@ -686,6 +699,7 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   const int grid = static_cast<int>(num_tiles < sms ? num_tiles : sms);
   if (bm == 256) return dispatch_dtype<256, 2>(a.in_dtype, a.out_dtype, ta, tb, tc, p, pm, grid, stream);
   if (bn == 256) return dispatch_dtype<256, 1>(a.in_dtype, a.out_dtype, ta, tb, tc, p, pm, grid, stream);
+  if (bn == 64) return dispatch_dtype<64, 1>(a.in_dtype, a.out_dtype, ta, tb, tc, p, pm, grid, stream);
   return dispatch_dtype<128, 1>(a.in_dtype, a.out_dtype, ta, tb, tc, p, pm, grid, stream);
 }
 }  // namespace

@@ -201,20 +201,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       for (int kb = kb_begin; kb < kb_end; ++kb) {
         if (!mbar_wait(empty + stage, phase ^ 1, abort_word)) break;
         uint8_t* sa = smem + stage * S::kStageBytes;
-        mbar_arrive_expect_tx(full + stage, S::kStageBytes);
-        if (a_mn) {
+        mbar_arrive_expect_tx(full + stage, static_cast<uint32_t>(p.stage_bytes));
 #pragma unroll
-          for (int b = 0; b < kBM / 64; ++b)
-            tma_load_3d(sa + b * 8192, &tmap_a, full + stage, tm * kBM + b * 64, kb * kElemsPerStage, bz);
-        } else {
-          tma_load_3d(sa, &tmap_a, full + stage, kb * kElemsPerStage, tm * kBM, bz);
-        }
-        if (b_mn) {
-#pragma unroll
-          for (int b = 0; b < BN / 64; ++b)
-            tma_load_3d(sa + S::kABytes + b * 8192, &tmap_b, full + stage, tn * BN + b * 64, kb * kElemsPerStage, bz);
-        } else {
-          tma_load_3d(sa + S::kABytes, &tmap_b, full + stage, kb * kElemsPerStage, tn * BN, bz);
+        for (int sub = 0; sub < S::kSub; ++sub) {
+          const int k0 = (kb * S::kSub + sub) * kElemsPerStage;
+          uint8_t* da = sa + sub * S::kABytes;
+          uint8_t* db = sa + S::kBOffset + sub * S::kBBytes;
+          if (a_mn) {
+            load_mn_major<kBM>(da, &tmap_a, full + stage, tm * kBM, k0, bz, p.a_blocks != 0);
+          } else {
+            tma_load_3d(da, &tmap_a, full + stage, k0, tm * kBM, bz);
+          }
+          if (b_mn) {
+            load_mn_major<BN>(db, &tmap_b, full + stage, tn * BN, k0, bz, p.b_blocks != 0);
+          } else {
+            tma_load_3d(db, &tmap_b, full + stage, k0, tn * BN, bz);
+          }
         }
         if (++stage == S::kStages) {
           stage = 0;
@@ -247,14 +249,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         tc_fence_after();
         const uint32_t a_lo = lo0_a + stage * (S::kStageBytes >> 4);
-        const uint32_t b_lo = lo0_b + stage * (S::kStageBytes >> 4) + (S::kABytes >> 4);
+        const uint32_t b_lo = lo0_b + stage * (S::kStageBytes >> 4) + (S::kBOffset >> 4);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t accum = (kb != kb_begin || k != 0) ? 1u : 0u;
+        for (int sk = 0; sk < 4 * S::kSub; ++sk) {
+          const uint32_t k = sk & 3;
+          const uint32_t accum = (kb != kb_begin || sk != 0) ? 1u : 0u;
+          const uint64_t a_desc = desc(a_lo + (sk >> 2) * (S::kABytes >> 4) + step_a * k, hi_a);
+          const uint64_t b_desc = desc(b_lo + (sk >> 2) * (S::kBBytes >> 4) + step_b * k, hi_b);
           if constexpr (KIND == kKindE4M3)
-            umma_f8_ss(tmem_base, desc(a_lo + step_a * k, hi_a), desc(b_lo + step_b * k, hi_b), idesc, accum);
+            umma_f8_ss(tmem_base, a_desc, b_desc, idesc, accum);
           else
-            umma_f16_ss(tmem_base, desc(a_lo + step_a * k, hi_a), desc(b_lo + step_b * k, hi_b), idesc, accum);
+            umma_f16_ss(tmem_base, a_desc, b_desc, idesc, accum);
         }
         umma_commit(empty + stage);  // frees the stage once these MMAs have read it
         if (++stage == S::kStages) {
@@ -406,18 +411,20 @@ int launch_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const gemm_
   if (p.split != 2 && p.split != 4 && p.split != 8)
     return set_error(B200K_ERR_BAD_SHAPE, "gemm (split-K): split must be 2, 4 or 8");
   if (bn == 256) return dispatch_dtype<256>(in_dtype, out_dtype, ta, tb, p, stream);
+  if (bn == 64) return dispatch_dtype<64>(in_dtype, out_dtype, ta, tb, p, stream);
   return dispatch_dtype<128>(in_dtype, out_dtype, ta, tb, p, stream);
 }
 
 int splitk_resident_clusters(int bn, int split) {
   // The CTAs of a cluster share a GPC, so fewer than SMs / split clusters fit.  Asked once per
   // device, tile width and cluster size.
-  static int cache[64][2][9] = {};  // 0 = not asked yet, -1 = cannot launch
+  static int cache[64][3][9] = {};  // 0 = not asked yet, -1 = cannot launch
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || split < 2 || split > 8) return 0;
-  int& slot = cache[dev][bn == 256 ? 1 : 0][split];
+  int& slot = cache[dev][bn == 256 ? 2 : (bn == 128 ? 1 : 0)][split];
   if (slot == 0) {
-    const int n = bn == 256 ? resident_clusters<256>(split) : resident_clusters<128>(split);
+    const int n = bn == 256 ? resident_clusters<256>(split)
+                            : (bn == 128 ? resident_clusters<128>(split) : resident_clusters<64>(split));
     slot = n > 0 ? n : -1;
   }
   return slot > 0 ? slot : 0;

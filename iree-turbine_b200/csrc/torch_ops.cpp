@@ -52,7 +52,8 @@ struct Api {
   B200K_FN(b200k_decode_attention);
   B200K_FN(b200k_paged_gather);
   B200K_FN(b200k_kv_append);
-  B200K_FN(b200k_quantize_e4m3);
+  B200K_FN(b200k_quantize_e4m3_ws);
+  B200K_FN(b200k_col_sum);
 #undef B200K_FN
 };
 
@@ -84,7 +85,8 @@ Api load_api() {
   B200K_FN(b200k_decode_attention);
   B200K_FN(b200k_paged_gather);
   B200K_FN(b200k_kv_append);
-  B200K_FN(b200k_quantize_e4m3);
+  B200K_FN(b200k_quantize_e4m3_ws);
+  B200K_FN(b200k_col_sum);
 #undef B200K_FN
   TORCH_CHECK(a.b200k_abi_version() == B200K_ABI_VERSION, path, ": ABI version ", a.b200k_abi_version(),
               ", this library expects ", B200K_ABI_VERSION);
@@ -333,11 +335,22 @@ std::tuple<Tensor, Tensor> quantize_e4m3(const Tensor& x_in) {
   const Tensor x = x_in.contiguous();
   Tensor y = empty(x.sizes(), at::kFloat8_e4m3fn, x.device());
   Tensor scale = empty({1}, at::kFloat, x.device());
-  Scratch scratch(4);
-  check(api().b200k_quantize_e4m3(static_cast<const float*>(x.data_ptr()), y.data_ptr(),
-                                  static_cast<float*>(scale.data_ptr()), static_cast<uint32_t*>(scratch.get()), x.numel(),
-                                  on.stream()));
+  Scratch ws(B200K_QUANTIZE_WORKSPACE_BYTES);
+  check(api().b200k_quantize_e4m3_ws(static_cast<const float*>(x.data_ptr()), y.data_ptr(),
+                                     static_cast<float*>(scale.data_ptr()), ws.get(), B200K_QUANTIZE_WORKSPACE_BYTES,
+                                     x.numel(), on.stream()));
   return {y, scale};
+}
+
+Tensor col_sum(const Tensor& x) {
+  OnDevice on(x.device());
+  TORCH_CHECK(x.dim() == 2 && is_half(x.scalar_type()), "col_sum: x must be a float16 or bfloat16 matrix");
+  if (x.stride(1) != 1 || x.size(0) == 0 || x.size(1) % 8 != 0 || x.stride(0) % 8 != 0 || !aligned16(x))
+    return x.to(at::kFloat).sum(0).to(x.scalar_type());  // rows that 16-byte loads cannot cover
+  Tensor out = empty({x.size(1)}, x.scalar_type(), x.device());
+  check(api().b200k_col_sum(x.data_ptr(), out.data_ptr(), x.size(0), x.size(1), x.stride(0), dtype_code(x.scalar_type()),
+                            on.stream()));
+  return out;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -654,6 +667,11 @@ Tensor call_gemm(const Tensor& a, const Tensor& b, bool ta, bool tb, at::ScalarT
   return op.call(a, b, ta, tb, out);
 }
 
+Tensor call_col_sum(const Tensor& x) {
+  static const auto op = typed_op<Tensor(const Tensor&)>("b200k::col_sum");
+  return op.call(x);
+}
+
 struct LinearFunction : torch::autograd::Function<LinearFunction> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias) {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -670,7 +688,7 @@ struct LinearFunction : torch::autograd::Function<LinearFunction> {
     if (ctx->needs_input_grad(0)) dx = call_gemm(dy, w, false, false, x.scalar_type());  // [M, N] @ [N, K]
     if (ctx->needs_input_grad(1)) dw = call_gemm(dy, x, true, false, w.scalar_type());   // [M, N]^T @ [M, K]
     // an absent bias is not among the inputs that needs_input_grad counts
-    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) db = dy.to(at::kFloat).sum(0).to(dy.scalar_type());
+    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) db = call_col_sum(dy);
     return {dx, dw, db};
   }
 };
@@ -728,6 +746,7 @@ TORCH_LIBRARY_IMPL(b200k, CUDA, m) {
   m.impl("linear", linear_cuda);
   m.impl("gemm_fp8_nt", gemm_fp8_nt);
   m.impl("quantize_e4m3", quantize_e4m3);
+  m.impl("col_sum", col_sum);
   m.impl("attention", attention);
   m.impl("attention_lse", attention_lse);
   m.impl("attention_bwd", attention_bwd);

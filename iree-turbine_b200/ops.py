@@ -222,6 +222,18 @@ class bmm(CustomOp):
 
 
 @CustomOp.register(library=LIBRARY, register_impl=False)
+class col_sum(CustomOp):
+    """Column sums of a f16 / bf16 matrix, summed in fp32: the bias gradient of ``linear``."""
+
+    signature = "col_sum(Tensor x) -> Tensor"
+
+    def select(self, sel: KernelSelection):
+        x = sel.arg_tensor(0)
+        torch._check(x.t.dim() == 2 and x.t.dtype in _HALF_TYPES, lambda: "col_sum: x must be a float16 or bfloat16 matrix")
+        sel.return_new_tensor([x.t.size(1)], x.t.dtype)
+
+
+@CustomOp.register(library=LIBRARY, register_impl=False)
 class linear_op(CustomOp):
     """``linear`` as an operator (its autograd formula is native, see ``linear`` below)."""
 

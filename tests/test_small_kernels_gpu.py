@@ -1,0 +1,71 @@
+"""Quantisation at the edges of its vector path and of its rounding, column sums at the edges of their tiles,
+GEMM tiles of 64 columns and one-load-per-operand MN-major stages."""
+
+import pytest
+import torch
+
+import iree_turbine_b200 as tb
+from iree_turbine_b200 import ops
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4096, 4099, 1 << 20, 3_000_001])
+@pytest.mark.parametrize("magnitude", [1.0, 1e-36, 1e37])
+def test_quantize_is_exact(n, magnitude):
+    x = torch.randn(n, generator=torch.Generator().manual_seed(n)) * magnitude
+    # values that sit on or next to the midpoint between two fp8 values once divided by the scale 448 / 448 = 1
+    if magnitude == 1.0 and n >= 4096:
+        grid = torch.arange(0, 127, dtype=torch.uint8).view(torch.float8_e4m3fn).float()
+        mid = (grid[1:-1] + grid[:-2]) / 2
+        x = x.clamp(-440, 440)
+        x[: mid.numel()] = mid
+        x[200:200 + mid.numel()] = torch.nextafter(mid, torch.tensor(1e9))
+        x[400:400 + mid.numel()] = -torch.nextafter(mid, torch.tensor(-1e9))
+        x[-1] = 448.0
+    y, s = torch.ops.b200k.quantize_e4m3(x.to(DEV))
+    yo, so = oracle.quantize_e4m3(x)
+    assert torch.equal(s.cpu().reshape(-1), so.reshape(-1))
+    assert torch.equal(y.cpu().view(torch.uint8), yo.view(torch.uint8))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (7, 64), (8, 56), (31, 72), (33, 520), (129, 128), (1000, 264), (4099, 1032)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_col_sum(rows, cols, dtype):
+    x = torch.randn(rows, cols + 8, generator=torch.Generator().manual_seed(5)).to(dtype).to(DEV)
+    for v in (x[:, :cols], x[:, :cols].contiguous(), x[:, 3:cols + 1]):  # pitched, dense, rows only 2-byte aligned
+        got = torch.ops.b200k.col_sum(v)
+        ref = v.double().sum(0)
+        # fp32 sum of `rows` terms (2^-24 each, of the sum of magnitudes), one rounding to the 16-bit type
+        bound = v.double().abs().sum(0) * rows * 2.0 ** -24 + ref.abs() * (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) + 1e-7
+        assert got.dtype == dtype and bool(((got.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("m,n,k,split", [(1, 64, 64, 1), (128, 64, 128, 1), (130, 65, 72, 1), (257, 200, 1000, 1), (1000, 1000, 1000, 1),
+                                         (16, 64, 512, 2), (40, 130, 1032, 4), (128, 192, 2048, 8)])
+@pytest.mark.parametrize("a_km,b_kn", [(False, False), (True, True)])
+def test_64_column_tiles(m, n, k, split, a_km, b_kn):
+    m, n = (-(-m // 8) * 8, -(-n // 8) * 8) if a_km else (m, n)
+    a, b = oracle.make_gemm_inputs(m, n, k, torch.bfloat16, seed=33)
+    out = torch.full((m, n), float("nan"), device=DEV)
+    ops._launch_gemm((a.t().contiguous() if a_km else a).to(DEV), (b.t().contiguous() if b_kn else b).to(DEV), out, None, None,
+                     tile_n=64, split_k=split, a_km=a_km, b_kn=b_kn)
+    torch.cuda.synchronize()
+    assert tb.device_status() == 0
+    oracle.assert_close_half(out, oracle.gemm_nt(a, b))
+
+
+# R % 64 == 0: one load per operand and stage; else one per 64-element block.  The last tile is partial either way.
+@pytest.mark.parametrize("m,n", [(64, 192), (320, 448), (328, 456)])
+@pytest.mark.parametrize("tile", [(128, 128), (128, 256), (256, 256)])
+def test_mn_major_operands(m, n, tile):
+    k = 200
+    a, b = oracle.make_gemm_inputs(m, n, k, torch.float16, seed=34)
+    out = torch.full((m, n), float("nan"), device=DEV)
+    ops._launch_gemm(a.t().contiguous().to(DEV), b.t().contiguous().to(DEV), out, None, None, tile_m=tile[0], tile_n=tile[1],
+                     a_km=True, b_kn=True)
+    torch.cuda.synchronize()
+    assert tb.device_status() == 0
+    oracle.assert_close_half(out, oracle.gemm_nt(a, b))
