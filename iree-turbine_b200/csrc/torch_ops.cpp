@@ -249,7 +249,7 @@ Tensor run_gemm(const Tensor& a_in, const Tensor& b_in, OptType out_dtype, bool 
   g.activation = activation;
   Tensor bias;
   if (bias_in.defined()) {
-    TORCH_CHECK(bias_in.numel() == g.n, "linear_act: bias must be [N]");
+    TORCH_CHECK(bias_in.numel() >= g.n, "linear_act: bias must be [N]");
     bias = bias_in.contiguous();
     g.bias = bias.data_ptr();
     g.bias_dtype = dtype_code(bias.scalar_type());
@@ -380,7 +380,7 @@ void check_attention(const Tensor& q, const Tensor& k, const Tensor& v) {
   TORCH_CHECK(q.scalar_type() == k.scalar_type() && q.scalar_type() == v.scalar_type(),
               "attention: q, k, v must share a dtype");
   TORCH_CHECK(k.sizes() == v.sizes(), "attention: k and v must have the same shape");
-  TORCH_CHECK(q.size(0) == k.size(0) && q.size(3) == k.size(3), "attention: q and k do not match");
+  TORCH_CHECK(q.size(0) <= k.size(0) && q.size(3) == k.size(3), "attention: q and k do not match");
 }
 
 Tensor run_attention(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, double scale, bool causal, float* lse,
@@ -503,12 +503,13 @@ void launch_decode(b200k_decode_args& a, const OnDevice& on) {
   check(api().b200k_decode_attention(&a, on.stream()));
 }
 
+// Tables and caches kept for more sequences than the call decodes are fine: the first ones are used.
 void check_decode(const char* op, const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& lens) {
   TORCH_CHECK(q.dim() == 3 && kc.dim() == 4, op, ": q must be 3-D and the K/V caches 4-D");
   TORCH_CHECK(q.scalar_type() == kc.scalar_type() && q.scalar_type() == vc.scalar_type(), op,
               ": q and the KV cache must share a dtype");
   TORCH_CHECK(kc.sizes() == vc.sizes() && kc.size(3) == q.size(2), op, ": cache shapes do not match");
-  TORCH_CHECK(lens.scalar_type() == at::kInt && lens.dim() == 1 && lens.size(0) == q.size(0), op,
+  TORCH_CHECK(lens.scalar_type() == at::kInt && lens.dim() == 1 && lens.size(0) >= q.size(0), op,
               ": seq_lens must be int32 [num_seqs]");
 }
 
@@ -517,7 +518,7 @@ Tensor decode_attention(const Tensor& q_in, const Tensor& k_in, const Tensor& v_
   one_device("decode_attention", q_in.device(), {&k_in, &v_in, &lens_in});
   OnDevice on(q_in.device());
   check_decode("decode_attention", q_in, k_in, v_in, lens_in);
-  TORCH_CHECK(k_in.size(0) == q_in.size(0), "decode_attention: k must have one history per sequence");
+  TORCH_CHECK(k_in.size(0) >= q_in.size(0), "decode_attention: k must have one history per sequence");
   const Tensor q = q_in.contiguous(), k = k_in.contiguous(), v = v_in.contiguous(), lens = lens_in.contiguous();
   Tensor o = empty(q.sizes(), q.scalar_type(), q.device());
   b200k_decode_args a = {};
@@ -545,7 +546,7 @@ Tensor paged_decode_attention(const Tensor& q_in, const Tensor& kc_in, const Ten
   one_device("paged_decode_attention", q_in.device(), {&kc_in, &vc_in, &bt_in, &lens_in});
   OnDevice on(q_in.device());
   check_decode("paged_decode_attention", q_in, kc_in, vc_in, lens_in);
-  TORCH_CHECK(bt_in.scalar_type() == at::kInt && bt_in.dim() == 2 && bt_in.size(0) == q_in.size(0),
+  TORCH_CHECK(bt_in.scalar_type() == at::kInt && bt_in.dim() == 2 && bt_in.size(0) >= q_in.size(0),
               "paged_decode_attention: block_table must be int32 [num_seqs, max_pages]");
   const Tensor q = q_in.contiguous(), kc = kc_in.contiguous(), vc = vc_in.contiguous(), bt = bt_in.contiguous(),
                lens = lens_in.contiguous();
@@ -611,7 +612,7 @@ Tensor paged_attention(const Tensor& q_in, const Tensor& kc_in, const Tensor& vc
   TORCH_CHECK(kc_in.dim() == 4 && kc_in.sizes() == vc_in.sizes() && kc_in.size(3) == q.size(3) &&
                   kc_in.scalar_type() == q.scalar_type() && vc_in.scalar_type() == q.scalar_type(),
               "paged_attention: caches do not match q");
-  TORCH_CHECK(bt_in.dim() == 2 && bt_in.size(0) == q.size(0) && lens_in.size(0) == q.size(0),
+  TORCH_CHECK(bt_in.dim() == 2 && bt_in.size(0) >= q.size(0) && lens_in.size(0) >= q.size(0),
               "paged_attention: block_table must be [B, max_pages] and seq_lens [B]");
   const Tensor kc = kc_in.contiguous(), vc = vc_in.contiguous(), bt = bt_in.contiguous(), lens = lens_in.contiguous();
   Tensor o = attention_out_like(q_in);
