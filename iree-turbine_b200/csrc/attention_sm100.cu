@@ -39,9 +39,9 @@
 // memory twice per K/V tile; measured, that costs less than the waiting it removes.
 //
 // Causal items: the two tiles of a pair need a different number of KV tiles (n[0] <= n[1]); tile 0
-// simply stops taking part once it is past its diagonal.  Work is dealt to CTAs in units that pair
-// the heaviest remaining pair of a head with the lightest, so every unit of a causal problem costs
-// the same.
+// simply stops taking part once it is past its diagonal.  Which CTA takes which pairs, and in what
+// order, is in attention_order.cuh.  Couples of a heavy and a light pair (see ItemWalk) are the order of
+// large causal problems.
 //
 // Softmax: running max in log2 units (scores are multiplied by scale * log2(e) inside the
 // exponent's FMA); O is only rescaled when a row's max grows by more than 2^8 (the stale max is
@@ -54,6 +54,7 @@
 // is freed and the kernel ORs a code into the caller's status word.
 #include <type_traits>
 
+#include "attention_order.cuh"
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -85,7 +86,8 @@ struct AttnSmem {
   static constexpr int kKvOffset = 2 * kTileBytes;
   static constexpr int kStageOffset = kKvOffset + kKvStages * kTileBytes;  // epilogue staging: one 64-column block
   static constexpr int kLsumOffset = kStageOffset + kHalfTileBytes;        // float [tile][max, sum][128 rows]
-  static constexpr int kBarOffset = kLsumOffset + 2 * 2 * kTileRows * 4;
+  static constexpr int kOrderOffset = kLsumOffset + 2 * 2 * kTileRows * 4;  // uint16: item order of a paged call
+  static constexpr int kBarOffset = kOrderOffset + attn_order::kSortBytes;
   // q_full[2] q_empty[2] | kv_full[4] kv_empty[4] | s_full[2][2] p_full[2][2] | o_full[2] o_free[2] | l_full[2] l_free[2] | turn[2] | pv_done[2]
   static constexpr int kNumBars = 4 + 2 * kKvStages + 8 + 4 + 4 + 2 + 2;
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16 + 1024;  // + slack for 1024-byte alignment
@@ -100,9 +102,8 @@ struct AttnParams {
   int64_t o_stride_b, o_stride_h, o_stride_s;
   int32_t batch, q_heads, kv_heads, seq_q, seq_kv;
   int32_t causal, causal_offset;
-  int32_t num_pairs;       // ceil(seq_q / 256)
-  int32_t units_per_head;  // work units per (batch, head): pairs, or (heavy, light) couples of pairs when causal
-  int32_t num_units;       // batch * q_heads * units_per_head
+  attn_order::ItemOrder order;  // items: pairs of query tiles, 256 rows
+  int32_t couples;              // pairs per head when a position stands for two of them, else 0 (see ItemWalk)
   float scale_log2;
   int32_t* status;
   float* lse;  // optional [batch, q_heads, seq_q]: ln sum_j exp(scale * s_ij), -inf for a row without keys
@@ -167,11 +168,11 @@ struct Item {
 };
 
 template <bool PAGED>
-__device__ __forceinline__ Item make_item(int bh, int pair, const AttnParams& p) {
+__device__ __forceinline__ Item make_item(int batch, int head, int pair, const AttnParams& p) {
   Item it;
   it.pair = pair;
-  it.batch = bh / p.q_heads;
-  it.head = bh - it.batch * p.q_heads;
+  it.batch = batch;
+  it.head = head;
   // (dense: the two are launch constants and the fields fold away)
   it.kv_len = p.seq_kv;
   if (PAGED) it.kv_len = max(0, min(__ldg(p.seq_lens + it.batch), p.seq_kv));
@@ -195,36 +196,36 @@ __device__ __forceinline__ Item make_item(int bh, int pair, const AttnParams& p)
   return it;
 }
 
-// The CTA's items, in the order every role walks them: units blockIdx.x, blockIdx.x + gridDim.x, ...;
-// a unit is one pair of a (batch, head), heaviest first, or -- causal -- the k-th heaviest pair
-// followed by the k-th lightest of the same head.  Units are numbered (batch, head)-major, so the
-// CTAs that run at one time work on a few neighbouring heads and share their K/V in L2.  (Giving
-// each CTA a contiguous range of units instead -- one head per CTA at a time -- puts 148 heads'
-// K/V in flight at once, more than L2 holds at S = 4096: measured 9 % slower.)
+// The CTA's items, in the order every role walks them.  With p.couples a position stands for two items,
+// the k-th heaviest pair of a head and then the k-th lightest, so that all positions cost the same and the
+// list can be head-major, which keeps the K/V traffic on a few heads.
 template <bool PAGED>
 struct ItemWalk {
   const AttnParams& p;
-  int unit, end, part;
-  __device__ ItemWalk(const AttnParams& params) : p(params), unit(blockIdx.x), end(params.num_units), part(0) {}
+  const uint16_t* table;
+  attn_order::Walk walk;
+  int light;  // second item of the couple, -1 without one
+  Item first;
+  __device__ ItemWalk(const AttnParams& params, const uint16_t* sorted) : p(params), table(sorted), light(-1) {}
   // Next item, empty ones (nmax == 0) included; false when the CTA has no more.
   __device__ __forceinline__ bool next(Item& it) {
-    while (unit < end) {
-      const int bh = unit / p.units_per_head;
-      const int s = unit - bh * p.units_per_head;
-      const int heavy = p.num_pairs - 1 - s;
-      if (part == 0) {
-        part = 1;
-        it = make_item<PAGED>(bh, heavy, p);
-        return true;
-      }
-      part = 0;
-      unit += gridDim.x;
-      if (p.causal && s < heavy) {
-        it = make_item<PAGED>(bh, s, p);
-        return true;
-      }
+    if (!PAGED && light >= 0) {
+      it = make_item<PAGED>(first.batch, first.head, light, p);
+      light = -1;
+      return true;
     }
-    return false;
+    if (walk.pos >= p.order.num_items) return false;
+    int batch, head, pair;
+    attn_order::item_at(p.order, walk.pos, table, p.q_heads, batch, head, pair);
+    if (!PAGED && p.couples > 0) {  // tile t of the order is the couple (couples - 1 - t, its mirror image)
+      const int k = p.order.tiles - 1 - pair;
+      pair = p.couples - 1 - k;
+      light = k < pair ? k : -1;
+    }
+    it = make_item<PAGED>(batch, head, pair, p);
+    first = it;
+    walk.step(p.order);
+    return true;
   }
   // Next item that has work.
   __device__ __forceinline__ bool next_busy(Item& it) {
@@ -249,6 +250,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   float* lsum = reinterpret_cast<float*>(smem + L::kLsumOffset);
+  uint16_t* table = reinterpret_cast<uint16_t*>(smem + L::kOrderOffset);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOffset);
   uint64_t* q_full = bars;            // [tile] Q tile loaded
   uint64_t* q_empty = q_full + 2;     // [tile] the item's last score MMA of that tile has read Q
@@ -307,6 +309,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   // (launch_pdl) everything above ran under the tail of the previous kernel
   grid_dependency_wait();
   grid_dependency_trigger();
+  if (PAGED && p.order.sorted) {
+    attn_order::sort_entries(table, p.order.sorted, [&](int e) {
+      const int batch = e / p.order.tiles;
+      return make_item<PAGED>(batch, 0, e - batch * p.order.tiles, p).nmax;
+    });
+  }
 
   if (warp >= 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
@@ -355,7 +363,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           }
           return true;
         };
-        ItemWalk<PAGED> walk(p);
+        ItemWalk<PAGED> walk(p, table);
         Item it;
         while (ok && walk.next_busy(it)) {
           int page = page_of(it, 0);
@@ -372,7 +380,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       if (lane == 0) {
         uint32_t ci[2] = {0, 0};  // items of each tile so far
         bool ok = true;
-        ItemWalk<PAGED> walk(p);
+        ItemWalk<PAGED> walk(p, table);
         Item it, nx;
         bool have = walk.next_busy(it);
         while (ok && have) {
@@ -475,7 +483,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         };
         auto pass_turn = [&]() { mbar_arrive(turn + (t ^ 1u)); };
         bool ok = true;
-        ItemWalk<PAGED> walk(p);
+        ItemWalk<PAGED> walk(p, table);
         Item it;
         while (ok && walk.next_busy(it)) {
           const int n = t ? it.n[1] : it.n[0];
@@ -547,7 +555,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     auto epi_barrier = [&]() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
     uint32_t ci[2] = {0, 0};  // items with work per tile so far
     bool ok = true;
-    ItemWalk<PAGED> walk(p);
+    ItemWalk<PAGED> walk(p, table);
     Item it;
     while (ok && walk.next(it)) {
 #pragma unroll 1
@@ -636,7 +644,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     const float2 scale2 = make_float2(scale_log2, scale_log2);
     uint32_t cs = 0, ci = 0;  // score tiles and items of this query tile so far
     bool ok = true;
-    ItemWalk<PAGED> walk(p);
+    ItemWalk<PAGED> walk(p, table);
     Item it;
     while (ok && walk.next_busy(it)) {
       const int n = it.n[t];
@@ -763,9 +771,9 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   int rc = ensure_dynamic_smem(kfn, AttnSmem<HD>::kTotal, configured, "cudaFuncSetAttribute(attention smem)");
   if (rc) return rc;
   const int sms = num_sms();
-  const int grid = p.num_units < sms ? p.num_units : sms;
+  const int grid = p.order.num_items < sms ? p.order.num_items : sms;
   // Launched early only when short, see the one-tile kernel.
-  const int64_t tiles = static_cast<int64_t>(p.num_units) * ((p.seq_kv + kTileRows - 1) / kTileRows);
+  const int64_t tiles = static_cast<int64_t>(p.order.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
   return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(kAttnThreads), AttnSmem<HD>::kTotal, stream, tq, tk, tv, to, p);
 }
 
@@ -780,36 +788,48 @@ int launch_any(int dtype, int head_dim, const CUtensorMap& tq, const CUtensorMap
   return launch_typed<__nv_bfloat16, 64, PAGED>(tq, tk, tv, to, p, stream);
 }
 
-// Work units: see ItemWalk.
-int fill_units(AttnParams& p, const char* who) {
-  p.num_pairs = (p.seq_q + kPairRows - 1) / kPairRows;
-  p.units_per_head = p.causal ? (p.num_pairs + 1) / 2 : p.num_pairs;
-  const int64_t units = static_cast<int64_t>(p.batch) * p.q_heads * p.units_per_head;
-  if (units > INT32_MAX) return set_error(B200K_ERR_BAD_SHAPE, "%s: too many query tiles", who);
-  p.num_units = static_cast<int32_t>(units);
-  return B200K_OK;
+// Causal couples fill the rounds over the SMs to 95 % or more: they are the better order then.
+// Serpentine pairs / couples, us: 4x32x4096 544 / 507, 8x32x2048 321 / 292, 4x32x4096 head dim 64 458 / 450;
+// where the last round is emptier, 4x8x4096 (86 %) 142 / 156, 1x16x8192 head dim 64 229 / 256.
+bool couples_fill(int64_t heads, int64_t seq_q) {
+  const int64_t pairs = (seq_q + kPairRows - 1) / kPairRows;
+  const int64_t units = heads * ((pairs + 1) / 2), sms = num_sms();
+  return units * 100 >= (units + sms - 1) / sms * sms * 95;
 }
 
-// Which kernel runs a problem (B200K_ATTN_AUTO).  Measured on B200, head dim 128, same box and
-// timing loop, one-tile / tile-pair in microseconds.  Non-causal: 8x32x1024 128 / 134, 8x32x2048
-// 472 / 473, 4x32x4096 992 / 1030, 1x16x16384 1827 / 2026.  Causal, many rounds of units: 4x32x4096
-// 539 / 510, 1x32(8)x16384 2073 / 1995, 2x32(8)x8192 1045 / 1026, but 4x32(8)x2048 155 / 173, where the
-// pair kernel's 512 units leave the last of four rounds over 148 SMs half empty, and 4x8x4096 (256
-// units, 86 % of two rounds) 152 / 158.  Causal, one or two rounds filled to 86 % (a head shard of
-// a long prefill on 8 GPUs): 1x8x8192 144 / 136, 4x4(1)x4096 80 / 76, 1x4x16384 273 / 248, 2x8x8192
-// 285 / 269, 1x16(4)x8192 281 / 266, but 4x6(2)x2048 41 / 45, 8x8x1024 40 / 41, 2x4x2048 41 / 43.
-// So: head dim 64 only exists in the pair kernel; causal problems take it when its units fill the
-// SMs to 90 % or more, or fill one round (two rounds) to 80 % with at least 24 (48) K/V tiles to
-// walk; everything else takes the one-tile kernel.
-bool choose_pair_kernel(int kernel, int head_dim, bool causal, int64_t pair_units, int64_t kv_tiles) {
-  if (head_dim != 128) return true;
-  if (kernel == B200K_ATTN_TILE_PAIR) return true;
-  if (kernel == B200K_ATTN_ONE_TILE) return false;
-  if (!causal) return false;
-  const int64_t sms = num_sms();
-  const int64_t rounds = (pair_units + sms - 1) / sms;
-  if (pair_units * 10 >= rounds * sms * 9) return true;
-  return rounds <= 2 && pair_units * 10 >= rounds * sms * 8 && kv_tiles >= (rounds == 1 ? 24 : 48);
+int fill_pair_order(AttnParams& p, const char* who, int head_dim, bool paged) {
+  const int64_t pairs = (p.seq_q + kPairRows - 1) / kPairRows;
+  const int64_t kv_bytes = static_cast<int64_t>(p.seq_kv) * head_dim * 4 * p.kv_heads / p.q_heads;
+  p.couples = 0;
+  if (p.causal && !paged && couples_fill(static_cast<int64_t>(p.batch) * p.q_heads, p.seq_q)) {
+    p.couples = static_cast<int32_t>(pairs);
+    return attn_order::fill_order(p.order, who, p.batch, p.q_heads, (pairs + 1) / 2, false, false, kv_bytes);
+  }
+  return attn_order::fill_order(p.order, who, p.batch, p.q_heads, pairs, p.causal != 0, paged, kv_bytes);
+}
+
+// Which kernel runs a problem (B200K_ATTN_AUTO); head dim 64 exists in the pair kernel only.  Measured at
+// head dim 128, one-tile / tile-pair, us.  Non-causal: 8x32x1024 128 / 134, 8x32x2048 472 / 473, 4x32x4096
+// 992 / 1030: the one-tile kernel.  Causal, couples that fill their rounds: 4x32x4096 527 / 507,
+// 1x32(8)x16384 1814 / 1788, 16x64x512 168 / 137, 2x64x5000 802 / 762 (32x32x256 70 / 72): the pair kernel.
+// Other causal problems, with the pair kernel in its better order: 2x32(8)x2000 84 / 87, 4x8x4096 137 / 142,
+// 1x4x16384 240 / 259, 16x16(4)x1024 101 / 106, 1x64(8)x6000 510 / 538 (4x4(1)x4096 78 / 75): the one-tile kernel.
+bool choose_pair_kernel(const b200k_attention_args& a) {
+  if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
+  if (a.kernel == B200K_ATTN_ONE_TILE || !a.causal) return false;
+  return couples_fill(static_cast<int64_t>(a.batch) * a.q_heads, a.seq_q);
+}
+
+// Paged: a K/V tile arrives page by page, and the pair kernel needs half as many tiles.  One-tile / tile-pair,
+// us: 4x32(8) 512 queries over up to 4000 keys 156 / 87 at page size 16, 114 / 95 at 64, 107 / 95 at 128;
+// 3x64(16) 1000 over 2000 170 / 146.  The one-tile kernel is ahead where the SMs are not filled and pages are
+// larger (1x8 2000 over 6000 81 / 98 at page size 32, 71 / 98 at 64, but 1x8 64 over 6000 at 16 96 / 81), and where
+// a pair would be half empty (16x16(4) 100 over 3000, page size 64, 45 / 54).
+bool choose_pair_kernel(const b200k_paged_attention_args& a) {
+  if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
+  if (a.kernel == B200K_ATTN_ONE_TILE) return false;
+  const int64_t items = static_cast<int64_t>(a.batch) * a.q_heads * ((a.seq_q + kTileRows - 1) / kTileRows);
+  return !((a.page_size >= 32 && items <= num_sms()) || (a.page_size >= 64 && a.seq_q <= kTileRows));
 }
 
 }  // namespace
@@ -840,12 +860,7 @@ int launch_attention_fwd(const b200k_attention_args& a, cudaStream_t stream) {
     return set_error(B200K_ERR_BAD_SHAPE, "attention_fwd: the one-tile kernel covers head_dim 128 only");
   int rc = ensure_sm100();
   if (rc) return rc;
-  {
-    const int64_t pairs = (a.seq_q + kPairRows - 1) / kPairRows;
-    const int64_t units = static_cast<int64_t>(a.batch) * a.q_heads * (a.causal ? (pairs + 1) / 2 : pairs);
-    if (!choose_pair_kernel(a.kernel, a.head_dim, a.causal != 0, units, (a.seq_kv + 127) / 128))
-      return launch_attention_fwd_tile(a, stream);
-  }
+  if (!choose_pair_kernel(a)) return launch_attention_fwd_tile(a, stream);
 
   CUtensorMap tq, tk, tv, to;
   const uint32_t box[4] = {64, kTileRows, 1, 1};
@@ -892,7 +907,7 @@ int launch_attention_fwd(const b200k_attention_args& a, cudaStream_t stream) {
   p.seq_kv = a.seq_kv;
   p.causal = a.causal ? 1 : 0;
   p.causal_offset = a.seq_kv - a.seq_q;
-  rc = fill_units(p, "attention_fwd");
+  rc = fill_pair_order(p, "attention_fwd", a.head_dim, false);
   if (rc) return rc;
   p.scale_log2 = a.scale * kLog2e;
   p.status = a.status;
@@ -934,12 +949,7 @@ int launch_paged_attention_fwd(const b200k_paged_attention_args& a, cudaStream_t
     return set_error(B200K_ERR_BAD_SHAPE, "paged_attention_fwd: the one-tile kernel covers head_dim 128 only");
   int rc = ensure_sm100();
   if (rc) return rc;
-  {
-    const int64_t pairs = (a.seq_q + kPairRows - 1) / kPairRows;
-    const int64_t units = static_cast<int64_t>(a.batch) * a.q_heads * (a.causal ? (pairs + 1) / 2 : pairs);
-    if (!choose_pair_kernel(a.kernel, a.head_dim, a.causal != 0, units, (a.max_seq_kv + 127) / 128))
-      return launch_paged_attention_fwd_tile(a, stream);
-  }
+  if (!choose_pair_kernel(a)) return launch_paged_attention_fwd_tile(a, stream);
 
   CUtensorMap tq, tk, tv, to;
   const uint32_t box[4] = {64, kTileRows, 1, 1};
@@ -980,7 +990,7 @@ int launch_paged_attention_fwd(const b200k_paged_attention_args& a, cudaStream_t
   p.seq_kv = a.max_seq_kv;
   p.causal = a.causal ? 1 : 0;
   p.causal_offset = a.max_seq_kv - a.seq_q;
-  rc = fill_units(p, "paged_attention_fwd");
+  rc = fill_pair_order(p, "paged_attention_fwd", a.head_dim, true);
   if (rc) return rc;
   p.scale_log2 = a.scale * kLog2e;
   p.status = a.status;

@@ -6,10 +6,8 @@
 // keeps both softmax warpgroups busy all the time and has the finer work granularity: it is the
 // faster of the two on non-causal problems and where the pair kernel's units fill the SMs badly.
 //
-// Persistent CTAs, one per SM.  A work item is one 128-row query tile of one (batch, head); a CTA
-// takes items blockIdx.x, blockIdx.x + gridDim.x, ... from a list ordered (batch, head)-major, so
-// CTAs that run at the same time share K/V in L2, heaviest query tiles of a head first; a causal
-// problem of a few rounds of items interleaves the tiles of all heads instead (see decode_item).
+// Persistent CTAs, one per SM.  A work item is one 128-row query tile of one (batch, head); which CTA
+// takes which items, and in what order, is in attention_order.cuh.
 //
 //   warps 0..3    softmax + correction of the even KV steps of the CTA (thread = query row)
 //   warps 4..7    the same for the odd KV steps
@@ -53,6 +51,7 @@
 // both P and the running sum, exact after the final division).
 #include <type_traits>
 
+#include "attention_order.cuh"
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -81,7 +80,8 @@ constexpr int kVOffset = kKOffset + kKStages * kTileBytes;
 constexpr int kOStageOffset = kVOffset + kVStages * kTileBytes;  // epilogue staging: one 64-column block
 constexpr int kMaxOffset = kOStageOffset + kHalfTileBytes;   // float [warpgroup][128 rows]: running max it published
 constexpr int kLsumOffset = kMaxOffset + 2 * kTileRows * 4;  // float [warpgroup][max, sum][128 rows] for the epilogue
-constexpr int kBarOffset = kLsumOffset + 2 * 2 * kTileRows * 4;
+constexpr int kOrderOffset = kLsumOffset + 2 * 2 * kTileRows * 4;  // uint16: item order of a paged call
+constexpr int kBarOffset = kOrderOffset + attn_order::kSortBytes;
 // q_full q_empty | k_full[3] k_empty[3] v_full[2] v_empty[2] | s_full[2] s_free[2] p_full[2] x_full[2] |
 // o_done[2] | o_full o_free l_full l_free
 constexpr int kNumBars = 2 + 2 * kKStages + 2 * kVStages + 8 + 2 + 4;
@@ -98,9 +98,7 @@ struct AttnParams {
   int64_t o_stride_b, o_stride_h, o_stride_s;
   int32_t batch, q_heads, kv_heads, seq_q, seq_kv;
   int32_t causal, causal_offset;
-  int32_t num_q_tiles;  // ceil(seq_q / 128)
-  int32_t num_items;    // batch * q_heads * num_q_tiles
-  int32_t interleave_heads, item_div;  // order of the item list, see decode_item
+  attn_order::ItemOrder order;  // items: query tiles of 128 rows
   float scale_log2;
   int32_t* status;
   float* lse;  // optional [batch, q_heads, seq_q]: ln sum_j exp(scale * s_ij), -inf for a row without keys
@@ -139,23 +137,11 @@ struct Item {
 };
 
 template <bool PAGED>
-__device__ __forceinline__ Item decode_item(int idx, const AttnParams& p) {
+__device__ __forceinline__ Item make_item(int batch, int head, int qtile, const AttnParams& p) {
   Item it;
-  // rank 0 = the last query tile of a head, the heaviest one of a causal problem.  The list is
-  // (batch, head)-major, except for a causal problem of a few rounds of items (p.interleave_heads, set
-  // by the host): there the heaviest tile of EVERY head comes first, then the next one, ...  A CTA
-  // takes every gridDim.x-th item, so each gets tiles of every weight and they finish together
-  // (head-major, a CTA of a one-round problem got one tile of arbitrary weight: 1 x 8 heads x 8192
-  // causal 172 -> 148 us, 4 x 4 x 4096 91 -> 84).  Longer lists are mixed well enough by the stride, and
-  // head-major keeps their K / V traffic on few heads.  One division either way: this runs in the
-  // single-thread roles between two items.
-  const int d = p.item_div;  // heads of all batches when interleaved, else query tiles per head
-  const int hi = idx / d, lo = idx - hi * d;
-  const int bh = p.interleave_heads ? lo : hi;
-  const int rank = p.interleave_heads ? hi : lo;
-  it.qtile = p.num_q_tiles - 1 - rank;
-  it.batch = bh / p.q_heads;
-  it.head = bh - it.batch * p.q_heads;
+  it.qtile = qtile;
+  it.batch = batch;
+  it.head = head;
   // (dense: the two are launch constants and the fields fold away)
   it.kv_len = p.seq_kv;
   if (PAGED) it.kv_len = max(0, min(__ldg(p.seq_lens + it.batch), p.seq_kv));
@@ -168,6 +154,13 @@ __device__ __forceinline__ Item decode_item(int idx, const AttnParams& p) {
     it.n = last_col < 0 ? 0 : min(last_col / kTileRows + 1, kv_tiles_total);
   }
   return it;
+}
+
+template <bool PAGED>
+__device__ __forceinline__ Item decode_item(int pos, const AttnParams& p, const uint16_t* table) {
+  int batch, head, qtile;
+  attn_order::item_at(p.order, pos, table, p.q_heads, batch, head, qtile);
+  return make_item<PAGED>(batch, head, qtile, p);
 }
 
 template <typename T, bool PAGED>
@@ -183,6 +176,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   float* lsum = reinterpret_cast<float*>(smem + kLsumOffset);
   float* xmax = reinterpret_cast<float*>(smem + kMaxOffset);
+  uint16_t* table = reinterpret_cast<uint16_t*>(smem + kOrderOffset);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kBarOffset);
   uint64_t* q_full = bars;
   uint64_t* q_empty = bars + 1;
@@ -247,6 +241,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   // (launch_pdl) everything above ran under the tail of the previous kernel
   grid_dependency_wait();
   grid_dependency_trigger();
+  if (PAGED && p.order.sorted) {
+    attn_order::sort_entries(table, p.order.sorted, [&](int e) {
+      const int batch = e / p.order.tiles;
+      return make_item<PAGED>(batch, 0, e - batch * p.order.tiles, p).n;
+    });
+  }
 
   if (warp >= 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
@@ -319,20 +319,21 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             if (jj < it.n && !load_k(it, jj, pages[jj])) return false;
           return true;
         };
-        auto next_item = [&](int idx, Item& nx) {  // next item of this CTA that has work; num_items if none
-          for (idx += gridDim.x; idx < p.num_items; idx += gridDim.x) {
-            nx = decode_item<PAGED>(idx, p);
-            if (nx.n > 0) return idx;
+        attn_order::Walk walk;
+        auto next_item = [&](Item& nx) {  // next item of this CTA that has work
+          while (walk.pos < p.order.num_items) {
+            nx = decode_item<PAGED>(walk.pos, p, table);
+            walk.step(p.order);
+            if (nx.n > 0) return true;
           }
-          return p.num_items;
+          return false;
         };
         Item it = {};
-        int idx = next_item(static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x), it);
-        if (idx < p.num_items) ok = load_head(it);
-        while (idx < p.num_items && ok) {
+        bool have = next_item(it);
+        if (have) ok = load_head(it);
+        while (have && ok) {
           Item nx = {};
-          const int nidx = next_item(idx, nx);
-          const bool have_next = nidx < p.num_items;
+          const bool have_next = next_item(nx);
           // Order within an item: V_j, then K_(j+3); a K stage is released (by the score MMA that
           // read it) earlier than a V stage.  The head of the next item goes before the last V.
           int vpage = page_of(it, 0), kpage = page_of(it, kKStages);
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             kpage = kpage_next;
           }
           it = nx;
-          idx = nidx;
+          have = have_next;
         }
       }
       __syncwarp();
@@ -374,8 +375,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         uint32_t kstage = 0, kpar = 0; // K ring position
         uint32_t qpar = 0;
         bool ok = true;
-        for (int idx = blockIdx.x; idx < p.num_items && ok; idx += gridDim.x) {
-          const Item it = decode_item<PAGED>(idx, p);
+        for (attn_order::Walk walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
+          const Item it = decode_item<PAGED>(walk.pos, p, table);
           if (it.n == 0) continue;
           if (!mbar_wait(q_full, qpar, abort_word)) break;
           qpar ^= 1;
@@ -413,8 +414,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         uint32_t g = 0, ic = 0;  // KV steps and items so far
         uint32_t vstage = 0, vpar = 0;
         bool ok = true;
-        for (int idx = blockIdx.x; idx < p.num_items && ok; idx += gridDim.x) {
-          const Item it = decode_item<PAGED>(idx, p);
+        for (attn_order::Walk walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
+          const Item it = decode_item<PAGED>(walk.pos, p, table);
           if (it.n == 0) continue;
           for (int j = 0; j < it.n; ++j, ++g) {
             const uint32_t buf = g & 1;
@@ -454,8 +455,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     auto epi_barrier = [&]() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
     uint32_t ic = 0, g0 = 0;  // items so far, KV steps before the current item
     bool ok = true;
-    for (int idx = blockIdx.x; idx < p.num_items && ok; idx += gridDim.x) {
-      const Item it = decode_item<PAGED>(idx, p);
+    for (attn_order::Walk walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
+      const Item it = decode_item<PAGED>(walk.pos, p, table);
       if (it.n == 0) {
         // no visible key: zeros (rare; plain stores)
         const int q_row = it.qtile * kTileRows + row_in_tile;
@@ -552,8 +553,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     const float2 scale2 = make_float2(scale_log2, scale_log2);
     uint32_t g = 0, ic = 0;  // KV steps (of both warpgroups) and items so far
     bool ok = true;
-    for (int idx = blockIdx.x; idx < p.num_items && ok; idx += gridDim.x) {
-      const Item it = decode_item<PAGED>(idx, p);
+    for (attn_order::Walk walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
+      const Item it = decode_item<PAGED>(walk.pos, p, table);
       if (it.n == 0) continue;
       const int tile_r0 = it.qtile * kTileRows;
       const int q_row = tile_r0 + row_in_tile;
@@ -706,11 +707,11 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   int rc = ensure_dynamic_smem(kfn, kAttnSmem, configured, "cudaFuncSetAttribute(attention smem)");
   if (rc) return rc;
   const int sms = num_sms();
-  const int grid = p.num_items < sms ? p.num_items : sms;
+  const int grid = p.order.num_items < sms ? p.order.num_items : sms;
   // Launched early only when short: CTAs of an early launch land on SMs in the order these come free, which
   // scatters the CTAs that share a head's K / V over both dies (8 x 32 x 1024 non-causal, 110 tiles per
   // CTA: 156 us in blockIdx order, 162 launched early).
-  const int64_t tiles = static_cast<int64_t>(p.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
+  const int64_t tiles = static_cast<int64_t>(p.order.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
   return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tq, tk, tv, to, p);
 }
 
@@ -783,12 +784,9 @@ int launch_attention_fwd_tile(const b200k_attention_args& a, cudaStream_t stream
   p.seq_kv = a.seq_kv;
   p.causal = a.causal ? 1 : 0;
   p.causal_offset = a.seq_kv - a.seq_q;
-  p.num_q_tiles = (a.seq_q + kTileRows - 1) / kTileRows;
-  const int64_t items = static_cast<int64_t>(a.batch) * a.q_heads * p.num_q_tiles;
-  if (items > INT32_MAX) return set_error(B200K_ERR_BAD_SHAPE, "attention_fwd: too many query tiles");
-  p.num_items = static_cast<int32_t>(items);
-  p.interleave_heads = (p.causal && items <= 4 * static_cast<int64_t>(num_sms())) ? 1 : 0;
-  p.item_div = p.interleave_heads ? p.num_items / p.num_q_tiles : p.num_q_tiles;
+  rc = attn_order::fill_order(p.order, "attention_fwd", a.batch, a.q_heads, (a.seq_q + kTileRows - 1) / kTileRows, a.causal != 0,
+                              false, static_cast<int64_t>(a.seq_kv) * kD * 4 * a.kv_heads / a.q_heads);
+  if (rc) return rc;
   p.scale_log2 = a.scale * kLog2e;
   p.status = a.status;
   p.lse = a.lse;
@@ -865,12 +863,9 @@ int launch_paged_attention_fwd_tile(const b200k_paged_attention_args& a, cudaStr
   p.seq_kv = a.max_seq_kv;
   p.causal = a.causal ? 1 : 0;
   p.causal_offset = a.max_seq_kv - a.seq_q;
-  p.num_q_tiles = (a.seq_q + kTileRows - 1) / kTileRows;
-  const int64_t items = static_cast<int64_t>(a.batch) * a.q_heads * p.num_q_tiles;
-  if (items > INT32_MAX) return set_error(B200K_ERR_BAD_SHAPE, "paged_attention_fwd: too many query tiles");
-  p.num_items = static_cast<int32_t>(items);
-  p.interleave_heads = (p.causal && items <= 4 * static_cast<int64_t>(num_sms())) ? 1 : 0;
-  p.item_div = p.interleave_heads ? p.num_items / p.num_q_tiles : p.num_q_tiles;
+  rc = attn_order::fill_order(p.order, "paged_attention_fwd", a.batch, a.q_heads, (a.seq_q + kTileRows - 1) / kTileRows, a.causal != 0,
+                              true, static_cast<int64_t>(a.max_seq_kv) * kD * 4 * a.kv_heads / a.q_heads);
+  if (rc) return rc;
   p.scale_log2 = a.scale * kLog2e;
   p.status = a.status;
   p.lse = nullptr;

@@ -26,7 +26,7 @@ BUILD_DIR = CSRC / "build"
 NATIVE_PATH = PKG / "_native.so"
 
 SOURCES = ["abi.cu", "gemm_sm100.cu", "gemm_splitk_sm100.cu", "attention_sm100.cu", "attention_tile_sm100.cu", "attention_bwd_sm100.cu", "decode_sm100.cu", "quant.cu", "colsum.cu", "selftest.cu"]
-HEADERS = ["common.cuh", "ptx.cuh", "gemm_common.cuh", str(REPO / "include" / "b200k.h")]
+HEADERS = ["common.cuh", "ptx.cuh", "gemm_common.cuh", "attention_order.cuh", str(REPO / "include" / "b200k.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
