@@ -71,9 +71,9 @@ struct GemmSmem {
   static constexpr int kBBytes = BN * kBKBytes;
   static constexpr int kBOffset = kSub * kABytes;  // a stage: A blocks, then B blocks
   static constexpr int kStageBytes = kSub * (kABytes + kBBytes);
-  // epilogue staging: per epilogue warp two 32-row x 128-byte buffers (TMA store source)
+  // epilogue staging: eight 32-row x 128-byte buffers (TMA store source)
   static constexpr int kStagingOffset = kStages * kStageBytes;
-  static constexpr int kStagingBytes = 4 * 2 * 32 * 128;
+  static constexpr int kStagingBytes = 8 * 32 * 128;
   static constexpr int kBarOffset = kStagingOffset + kStagingBytes;
   static constexpr int kNumBars = 2 * kStages + 4;
   static constexpr int kBiasOffset = kBarOffset + kNumBars * 8 + 16;  // the tile's bias as fp32

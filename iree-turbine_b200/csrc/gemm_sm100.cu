@@ -6,8 +6,8 @@
 // SM can pull from L2, so large problems use a 256 x 256 tile: two 128-row halves share each B
 // stage (64 bytes per cycle) at the price of a single, not double-buffered, accumulator set.
 //
-// CTA = 6 warps: warp 0 issues TMA loads, warp 1 owns tensor memory and issues the MMAs,
-// warps 2..5 drain accumulators (each warp its own 32-lane quarter of tensor memory).
+// CTA = 6 or 10 warps: warp 0 issues TMA loads, warp 1 owns tensor memory and issues the MMAs,
+// the others drain accumulators (one or two warps for each 32-lane quarter of tensor memory).
 //
 // Data layout.  A and B are K-contiguous, so both are "K-major" UMMA operands.  One pipeline
 // stage holds a 128 x 128-byte tile of A and a BN x 128-byte tile of B, written by TMA with the
@@ -30,8 +30,15 @@ using namespace gemm_detail;
 // it as R / 64 blocks of 64 K-rows x 128 bytes (128-byte swizzle), one TMA box each; the UMMA
 // descriptor has LBO = 8 KB between the 64-element blocks, SBO = 1 KB between 8-row groups, and a
 // k-step of 16 rows advances 2 KB.  A stage has the same size either way.
-template <int BN, int MT, int KIND, typename OutT, bool GEN>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+//
+// Epilogue warps: PARTS = 1, one per 32-lane quarter of tensor memory with two staging buffers, or PARTS = 2,
+// two that take turns at its pieces, with a buffer each.  Two where a warp has work of its own on a piece, a
+// bias, the error function or stores that the TMA unit cannot make (one / two, us): fp8 5000x5001x2048 97 / 64,
+// 8000x1025x1024 41 / 23, fp32 out 2000x2001x1000 21.4 / 18.6, GELU with bias 8000x1024x1024 32.6 / 29.8 and
+// 2048x2048x512 17.0 / 15.8.  One otherwise: a warp that waits for its only buffer costs 1 to 3 % (fp8 8192^3
+// 366 / 374, 4096^3 98 / 101), and SiLU is short enough for one (3000x4352x3840 80.2 / 82.7, 2048x2048x512 12.2 / 14.1).
+template <int BN, int MT, int KIND, typename OutT, bool GEN, int PARTS>
+__global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     gemm_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const GemmParams p,
                    const __grid_constant__ PeerMaps peer_maps) {
@@ -64,7 +71,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull + a, 1);
-      mbar_init(tempty + a, 4);
+      mbar_init(tempty + a, 4 * PARTS);
     }
     *abort_word = 0;
     fence_barrier_init();
@@ -206,7 +213,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     __syncwarp();
   } else {
     // ---------------- epilogue warps ----------------
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, part = PARTS == 1 ? 0 : (warp - 2) >> 2;
     float scale = 1.0f;
     if constexpr (KIND == kKindE4M3) {
       const float sa = p.scale_a ? *p.scale_a : 1.0f;
@@ -216,7 +223,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const bool fused = p.bias != nullptr || p.act != 0;  // uniform over the grid
     float* bias_s = reinterpret_cast<float*>(smem + S::kBiasOffset);
     OutT* cbase = reinterpret_cast<OutT*>(p.c);
-    uint8_t* staging = smem + S::kStagingOffset + (warp - 2) * (2 * 4096);
+    constexpr int kBufsPerWarp = 2 / PARTS;
+    uint8_t* staging = smem + S::kStagingOffset + (warp - 2) * (kBufsPerWarp * 4096);
     uint32_t stg_count = 0;
     int it = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
@@ -226,23 +234,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const int acc = it % kAccBufs;
       const uint32_t acc_phase = (it / kAccBufs) & 1;
       // The tile's bias, fetched while the main loop runs (columns past n re-read the last one: never stored).
-      constexpr int kBiasPerThread = (BN + 127) / 128;
+      constexpr int kEpiThreads = 128 * PARTS;
+      constexpr int kBiasPerThread = (BN + kEpiThreads - 1) / kEpiThreads;
       float tile_bias[kBiasPerThread] = {};
-      const int et = static_cast<int>(threadIdx.x) - 64;  // epilogue thread 0..127
+      const int et = static_cast<int>(threadIdx.x) - 64;  // epilogue thread
       if (p.bias != nullptr) {
 #pragma unroll
         for (int i = 0; i < kBiasPerThread; ++i)
-          tile_bias[i] = load_bias(p.bias, p.bias_dtype, min(tn * BN + i * 128 + et, p.n - 1));
+          tile_bias[i] = load_bias(p.bias, p.bias_dtype, min(tn * BN + i * kEpiThreads + et, p.n - 1));
       }
       bool ok = mbar_wait(tfull + acc, acc_phase, abort_word);
       if (fused) {
-        // all four warps are done with the previous tile's bias, and give up together if one wait ran out
-        ok = bar_red_and(1, 128, ok);
+        // all warps are done with the previous tile's bias, and give up together if one wait ran out
+        ok = bar_red_and(1, kEpiThreads, ok);
         if (!ok) break;
 #pragma unroll
         for (int i = 0; i < kBiasPerThread; ++i)
-          if (BN >= 128 || et < BN) bias_s[i * 128 + et] = tile_bias[i];
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+          if (BN >= kEpiThreads || et < BN) bias_s[i * kEpiThreads + et] = tile_bias[i];
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
       } else {
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -254,21 +263,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const uint32_t taddr =
             tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (MT == 1 ? acc * BN : h * BN);
         // 128 bytes of each of this warp's 32 rows per step: registers -> swizzled staging buffer ->
-        // C.  Two buffers per warp; a buffer is reused once its store has been read.
+        // C.  A buffer is reused once its store has been read.
         constexpr int kCols = 128 / static_cast<int>(sizeof(OutT));
         const bool by_tma = p.tma_store_ok || p.peer_tma;
 #pragma unroll 1
-        for (int c = 0; c < BN / kCols; ++c) {
+        for (int c = part; c < BN / kCols; c += PARTS) {
           const int col = tn * BN + c * kCols;
           if (col >= p.n) break;
-          uint8_t* buf = staging + (stg_count & 1) * 4096;
+          uint8_t* buf = staging + stg_count % kBufsPerWarp * 4096;
           uint32_t r[kCols];
           uint4 v[8];
           if constexpr (kCols == 32)
             tmem_ld_32x32b_x32(taddr + c * 32, r);
           else
             tmem_ld_32x32b_x64(taddr + c * 64, r);
-          if (by_tma && lane == 0) tma_store_wait_read<1>();
+          if (by_tma && lane == 0) tma_store_wait_read<kBufsPerWarp - 1>();
           tmem_wait_ld();
           if (fused) {
             fused_epilogue<kCols>(r, scale, bias_s + c * kCols, p.act);
@@ -364,18 +373,28 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
 }
 
-template <int BN, int MT, int KIND, typename OutT, bool GEN = false>
-int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
+template <int BN, int MT, int KIND, typename OutT, bool GEN, int PARTS>
+int launch_parts(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
                const PeerMaps& pm, int grid, cudaStream_t stream) {
   using S = GemmSmem<BN, MT>;
-  auto kfn = gemm_nt_kernel<BN, MT, KIND, OutT, GEN>;
+  auto kfn = gemm_nt_kernel<BN, MT, KIND, OutT, GEN, PARTS>;
   static bool configured[64] = {};  // per instantiation and device ordinal
   int rc = ensure_dynamic_smem(kfn, S::kDynamic, configured, "cudaFuncSetAttribute(gemm smem)");
   if (rc) return rc;
   // Programmatic dependent launch: barrier set-up and the tensor-memory allocation of this kernel
   // overlap the tail of whatever runs before it in the stream (see grid_dependency_wait in the kernel).
-  return launch_pdl("gemm_nt_kernel launch", kfn, dim3(static_cast<unsigned>(grid)), dim3(kGemmThreads), S::kDynamic, stream,
+  return launch_pdl("gemm_nt_kernel launch", kfn, dim3(static_cast<unsigned>(grid)), dim3(64 + 128 * PARTS), S::kDynamic, stream,
                     ta, tb, tc, p, pm);
+}
+
+template <int BN, int MT, int KIND, typename OutT, bool GEN = false>
+int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
+               const PeerMaps& pm, int grid, cudaStream_t stream) {
+  // which of the two: see the kernel
+  const bool by_tma = p.tma_store_ok || p.peer_tma;
+  const bool own_work = p.act == B200K_ACT_GELU || (p.bias != nullptr && p.act != B200K_ACT_SILU);
+  if (own_work || !by_tma) return launch_parts<BN, MT, KIND, OutT, GEN, 2>(ta, tb, tc, p, pm, grid, stream);
+  return launch_parts<BN, MT, KIND, OutT, GEN, 1>(ta, tb, tc, p, pm, grid, stream);
 }
 
 template <int BN, int MT>
