@@ -102,24 +102,27 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t& r0, u
                : "r"(addr));
 }
 
+// D = A B + C
 template <typename T>
-__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
-template <>
-__device__ __forceinline__ void mma_16816<__half>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0,
+                                          float c1, float c2, float c3) {
+  if constexpr (std::is_same<T, __half>::value)
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%10, %11, %12, %13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+  else
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%10, %11, %12, %13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
-template <>
-__device__ __forceinline__ void mma_16816<__nv_bfloat16>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
-                                                         uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+
+template <typename T>
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  mma_16816<T>(d, a, b0, b1, d[0], d[1], d[2], d[3]);
 }
 
 template <typename T>
@@ -306,33 +309,44 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 2 : 1) decode_splitkv
     mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
     mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
     mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
+    // The probabilities are taken relative to the maximum of their own tile, a_ rescales what was summed
+    // before and b_ this tile.  The largest one of every 16 is then exactly 1 when it is rounded to 16 bits
+    // for the product.  Relative to the running maximum one of a whole chunk is, and results were the
+    // further from those in 64 bits the longer the chunks: by 0 to 20 %, 3 % on average, over 42 problems of 1
+    // to 113 sequences and 66 to 16000 tokens.  It costs 0.1 to 0.2 us of a small call and 1 to 2 % of a large one
+    // (8 kv heads, 4 x 100..1000 tokens 6.8 / 7.0 us; 64 x 512..8192 178 / 180).
     const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
     const float ms_lo = (mn_lo == -INFINITY) ? 0.f : mn_lo;
     const float ms_hi = (mn_hi == -INFINITY) ? 0.f : mn_hi;
     const float a_lo = fast_exp2(m_lo - ms_lo), a_hi = fast_exp2(m_hi - ms_hi);
+    const float b_lo = fast_exp2(mx_lo - ms_lo), b_hi = fast_exp2(mx_hi - ms_hi);
+    const float mt_lo = (mx_lo == -INFINITY) ? 0.f : mx_lo;
+    const float mt_hi = (mx_hi == -INFINITY) ? 0.f : mx_hi;
     m_lo = mn_lo;
     m_hi = mn_hi;
     float ps_lo = 0.f, ps_hi = 0.f;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      s[i][0] = fast_exp2(s[i][0] - ms_lo);
-      s[i][1] = fast_exp2(s[i][1] - ms_lo);
-      s[i][2] = fast_exp2(s[i][2] - ms_hi);
-      s[i][3] = fast_exp2(s[i][3] - ms_hi);
+      s[i][0] = fast_exp2(s[i][0] - mt_lo);
+      s[i][1] = fast_exp2(s[i][1] - mt_lo);
+      s[i][2] = fast_exp2(s[i][2] - mt_hi);
+      s[i][3] = fast_exp2(s[i][3] - mt_hi);
       ps_lo += s[i][0] + s[i][1];
       ps_hi += s[i][2] + s[i][3];
     }
-    l_lo = l_lo * a_lo + ps_lo;
-    l_hi = l_hi * a_hi + ps_hi;
+    l_lo = l_lo * a_lo + ps_lo * b_lo;
+    l_hi = l_hi * a_hi + ps_hi * b_hi;
+    if (j > 0 && !__all_sync(0xffffffffu, a_lo == 1.f && a_hi == 1.f)) {  // a maximum grew: seldom after the first tiles
 #pragma unroll
-    for (int i = 0; i < HD / 8; ++i) {
-      o[i][0] *= a_lo;
-      o[i][1] *= a_lo;
-      o[i][2] *= a_hi;
-      o[i][3] *= a_hi;
+      for (int i = 0; i < HD / 8; ++i) {
+        o[i][0] *= a_lo;
+        o[i][1] *= a_lo;
+        o[i][2] *= a_hi;
+        o[i][3] *= a_hi;
+      }
     }
 
-    // ---- O += P V : 16 (heads) x HD (dims), k = 16 tokens ----
+    // ---- O = a O + b P V : 16 (heads) x HD (dims), k = 16 tokens ----
     uint32_t pf[4];
     pf[0] = pack2<T>(s[0][0], s[0][1]);
     pf[1] = pack2<T>(s[0][2], s[0][3]);
@@ -346,8 +360,17 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 2 : 1) decode_splitkv
         const int c = dn * 2 + (mi >> 1);
         uint32_t r0, r1, r2, r3;
         ldmatrix_x4_trans(sv + row * kRowBytes + ((c ^ (row & 7)) << 4), r0, r1, r2, r3);
-        mma_16816<T>(o[2 * dn], pf, r0, r1);
-        mma_16816<T>(o[2 * dn + 1], pf, r2, r3);
+        float pv[2][4];
+        mma_16816<T>(pv[0], pf, r0, r1, 0.f, 0.f, 0.f, 0.f);
+        mma_16816<T>(pv[1], pf, r2, r3, 0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float(&acc)[4] = o[2 * dn + i];
+          acc[0] = fmaf(pv[i][0], b_lo, acc[0]);
+          acc[1] = fmaf(pv[i][1], b_lo, acc[1]);
+          acc[2] = fmaf(pv[i][2], b_hi, acc[2]);
+          acc[3] = fmaf(pv[i][3], b_hi, acc[3]);
+        }
       }
     }
     __syncwarp();
