@@ -546,11 +546,12 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   int split = 1;
   if (bn == 0 || (a.split_k == 0 && bm != 256)) {
     const int given_m = bm, given_n = bn;
+    const int narrowest = peers.num > 0 ? 128 : 64;  // pieces to peers leave from tiles of at least 128 columns
     for (const Shape& t : kShapes) {
       if ((given_m != 0 && t.m != given_m) || (given_n != 0 && (t.n != given_n || t.m != (given_m ? given_m : 128)))) continue;
-      if (given_n == 0 && t.n > 64 && a.n <= t.n / 2) continue;   // the narrower tile covers it
+      if (given_n == 0 && t.n > narrowest && a.n <= t.n / 2) continue;  // the narrower tile covers it
       if (given_m == 0 && t.m == 256 && a.m <= 128) continue;
-      if (peers.num > 0 && t.n == 64) continue;
+      if (t.n < narrowest) continue;
       const double us = whole_us(t);
       if (us < best_us) {
         best_us = us;
