@@ -125,15 +125,18 @@ __device__ __forceinline__ float apply_act(float x) {
   if constexpr (ACT == B200K_ACT_GELU)  // exact (erf) form, the default of aten::gelu
     return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
   if constexpr (ACT == B200K_ACT_SILU) {
-    // x / (1 + e^-x) by a hardware reciprocal and one Newton-Raphson step, which squares its 2^-23 error
-    // away.  (The IEEE division this was before branches to a slow path per element: 2048^3 took 52 us
-    // with it, 16 without an activation.)  The exponent is capped where the result is below 2e-36 anyway,
-    // so that 1 + e^-x stays finite.
-    const float d = 1.f + __expf(fminf(-x, 87.f));
+    // x / (1 + e^-x): quotient by a hardware reciprocal, corrected by its own residual (Markstein 1990).  Over
+    // 524288 values of -95 to 95 not a bit differs from the IEEE division, which branches to a slow path per
+    // element (8000 x 1024 x 1024: 147 us with it, 26.6 now, 21.2 without an activation; 24.0 with the reciprocal
+    // alone refined, whose results were up to one unit further off).  Numerator and denominator are divided
+    // by 16, which keeps the reciprocal of the largest 1 + e^-x a normal number.  Where the residual is NaN
+    // (1 + e^-x or x infinite) the uncorrected quotient is the answer: a zero below -88.7, x at +infinity,
+    // NaN at -infinity.
+    const float d = fmaf(__expf(-x), 0.0625f, 0.0625f), num = x * 0.0625f;
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = r * fmaf(-d, r, 2.f);
-    return x * r;
+    const float q = num * r, residual = fmaf(-d, q, num);
+    return residual == residual ? fmaf(residual, r, q) : q;
   }
   return x;
 }

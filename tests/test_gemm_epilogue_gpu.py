@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import iree_turbine_b200 as tb
+from iree_turbine_b200 import ops
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -28,3 +29,25 @@ def test_unaligned_output_rows(m, n, out_dtype):
         assert torch.equal(y, c + bias.to(DEV))
     else:
         oracle.assert_close_half(y, ref + bias)
+
+
+# whole tiles with one epilogue (bias none: the values come through the product), with the other, and split-K
+@pytest.mark.parametrize("n,k,split", [(200, 64, 1), (1203, 8, 1), (200, 512, 2)])
+@pytest.mark.parametrize("bias_dtype", [torch.float32, torch.bfloat16])
+def test_silu_over_the_whole_range(n, k, split, bias_dtype):
+    low = torch.finfo(bias_dtype).min
+    x = torch.cat([torch.tensor([0.0, -0.0, 1.0, 20.0, 88.0, 104.0, 3e38, -20.0, -86.9, -87.4, -88.6, -88.8, -100.0, -1e4, -1e30, -1e36,
+                                 low, low / 2, 1e-30, -1e-30]), torch.linspace(-95, 95, n - 23)])
+    x = torch.cat([x, torch.tensor([float("inf"), -float("inf"), float("nan")])]).to(bias_dtype)
+    a, w = torch.zeros(3, k, dtype=torch.bfloat16, device=DEV), torch.zeros(n, k, dtype=torch.bfloat16, device=DEV)
+    out = torch.full((3, n), 7.0, device=DEV)
+    ops._launch_gemm(a, w, out, None, None, bias=x.to(DEV), activation="silu", split_k=split)
+    got, x64 = out.cpu().double(), x.double()
+    assert tb.device_status() == 0 and torch.equal(got[1].nan_to_num(), got[0].nan_to_num())
+    ref = x64 / (1.0 + torch.exp(-x64))
+    # the exponential is good to 2 + 1.173 |x| units of 2^-23, the sum and the quotient to one each; e^-x overflows
+    # beyond 88.7, where the exact result is below 3e-37 and a zero is due
+    finite = x64.isfinite()
+    bound = (4 + 1.173 * x64.abs().clamp(max=104)) * 2.0 ** -23 * ref.abs() + 3e-37
+    assert bool(((got[0] - ref).abs() <= bound)[finite].all())
+    assert got[0, -3] == float("inf") and bool(got[0, -2:].isnan().all())
