@@ -350,11 +350,12 @@ typedef struct b200k_decode_args {
                                  larger than max_seq_len and was cut to it */
 } b200k_decode_args;
 
-/* Bytes of scratch the call needs for the given problem (depends on num_seqs, q_heads,
- * head_dim, max_seq_len and chunk_tokens only). */
+/* Bytes of scratch the call needs for the given problem (depends on num_seqs, q_heads, kv_heads,
+ * head_dim, max_seq_len and chunk_tokens only, not on the lengths). */
 uint64_t b200k_decode_workspace_bytes(const b200k_decode_args* args);
 
-/* The chunk size the library would choose for chunk_tokens == 0. */
+/* The chunk size the library would choose for chunk_tokens == 0 and a sequence of max_seq_len tokens; shorter
+ * sequences may get smaller ones. */
 int32_t b200k_decode_default_chunk(const b200k_decode_args* args);
 
 int b200k_decode_attention(const b200k_decode_args* args, void* stream);

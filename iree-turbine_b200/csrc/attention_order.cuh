@@ -30,26 +30,6 @@ constexpr int kMaxSorted = 512;                   // entries of a paged call tha
 constexpr int kSortBytes = 2 * 2 * kMaxSorted;    // uint16 [order, cost][entry]
 constexpr int64_t kSharedKvBytes = 100ll << 20;   // K/V of the heads in flight, of 126 MB of L2
 
-// Quotients of the item walk, which runs in single-thread roles between two items: a multiplication instead
-// of the two dozen instructions of a division by a value known at run time only (8x32x1024 without a mask, 14
-// short items per CTA: 162 us with divisions, 157 with these).
-// floor(n / d) for 0 <= n < 2^31, d >= 1: with 2^(s-1) < d <= 2^s, m = floor(2^32 (2^s - d) / d) + 1 makes
-// (n + floor(n m / 2^32)) >> s exact: 2^32 + m exceeds 2^(32+s) / d by at most 1, which moves the quotient up
-// by at most n / 2^(32+s) < 1 / d.
-struct Divisor {
-  uint32_t d, mul, shift;
-  __host__ void set(int64_t divisor) {
-    d = static_cast<uint32_t>(divisor);
-    shift = 0;
-    while ((1ull << shift) < d) ++shift;
-    mul = static_cast<uint32_t>(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
-  }
-  __host__ __device__ __forceinline__ int quotient(int n) const {
-    const uint32_t high = static_cast<uint32_t>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * mul) >> 32);
-    return static_cast<int>((static_cast<uint32_t>(n) + high) >> shift);
-  }
-};
-
 struct ItemOrder {
   int32_t num_items;  // heads * tiles
   int32_t heads;      // batch * q_heads

@@ -54,6 +54,26 @@ int launch_quantize_e4m3(const float* x, void* y, float* scale_out, uint32_t* am
                          int64_t n, cudaStream_t stream);
 int launch_col_sum(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, int dtype, cudaStream_t stream);
 
+// Quotients by a value that the host knows: a multiplication instead of the two dozen instructions of a division.
+// They are on the path of single-thread roles and of short kernels (attention 8x32x1024 without a mask, whose CTAs
+// walk 14 short items each: 162 us with divisions, 157 with these).
+// floor(n / d) for 0 <= n < 2^31, d >= 1: with 2^(s-1) < d <= 2^s, m = floor(2^32 (2^s - d) / d) + 1 makes
+// (n + floor(n m / 2^32)) >> s exact: 2^32 + m exceeds 2^(32+s) / d by at most 1, which moves the quotient up
+// by at most n / 2^(32+s) < 1 / d.
+struct Divisor {
+  uint32_t d, mul, shift;
+  __host__ void set(int64_t divisor) {
+    d = static_cast<uint32_t>(divisor);
+    shift = 0;
+    while ((1ull << shift) < d) ++shift;
+    mul = static_cast<uint32_t>(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
+  }
+  __host__ __device__ __forceinline__ int quotient(int n) const {
+    const uint32_t high = static_cast<uint32_t>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * mul) >> 32);
+    return static_cast<int>((static_cast<uint32_t>(n) + high) >> shift);
+  }
+};
+
 // Opts a kernel into more than 48 KB of dynamic shared memory.  The attribute belongs to the
 // (function, device) pair, so it is set once per device ordinal: `done` is the caller's table, one
 // per kernel instantiation.  Setting it twice is harmless, which is why the table needs no lock.

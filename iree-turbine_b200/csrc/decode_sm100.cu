@@ -38,6 +38,24 @@ struct DecodeTile {
 };
 constexpr float kLog2e = 1.4426950408889634f;
 
+constexpr int kMaxChunk = 2048;
+
+// Tokens per chunk of a sequence of `len` tokens: `fixed`, or the `split`th part of the sequence, a multiple of 64
+// between `least` and kMaxChunk.  What counts is the length on the device: tables and caches are as long as they
+// may become, the histories in them are not (plan_decode has figures).
+struct ChunkRule {
+  int32_t fixed, split, least;
+  Divisor by_split;
+  __host__ __device__ __forceinline__ int tokens(int len) const {
+    if (fixed > 0) return fixed;
+    if (len > split * kMaxChunk) return kMaxChunk;
+    const int part = (by_split.quotient(len + split - 1) + 63) & ~63;
+    return part > least ? part : least;
+  }
+  // Cheap: true only where chunk number `i` starts past the end (chunks from `split` on are kMaxChunk long).
+  __device__ __forceinline__ bool past(int i, int len) const { return i >= split && i * (fixed > 0 ? fixed : kMaxChunk) >= len; }
+};
+
 struct DecodeParams {
   const void* q;
   const void* k;
@@ -49,7 +67,8 @@ struct DecodeParams {
   void* o;
   int32_t num_seqs, q_heads, kv_heads, group;
   int32_t page_size, num_pages, block_table_stride;
-  int32_t chunk_tokens, max_chunks;
+  ChunkRule chunk;
+  int32_t max_chunks;  // of the longest sequence
   int32_t warps;    // per CTA: 4, two CTAs per SM; 8 where the grid leaves SMs with one CTA or none
   int32_t stages;   // ring stages per warp: kDecodeStages, or fewer where a chunk has fewer tiles per warp
   int32_t cluster;  // > 0: the chunks of a (sequence, kv head) are one thread-block cluster of this size, which
@@ -200,10 +219,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 2 : 1) decode_splitkv
   // seq_lens is device data the host cannot validate: a length beyond what the grid, the workspace
   // and the block table were sized for is cut to max_seq_len (and reported), a negative one to 0.
   const int len = clamped_len(p, seq, chunk == 0 && kvh == 0 && threadIdx.x == 0);
-  const int chunk_start = chunk * p.chunk_tokens;
+  if (p.chunk.past(chunk, len) && p.cluster == 0) return;  // most CTAs of a call whose capacity is far above its lengths
+  const int chunk_tokens = p.chunk.tokens(len);
+  const int chunk_start = chunk * chunk_tokens;
   // A CTA past the end of its sequence has nothing to add; in a cluster it still takes part in the merge.
   if (chunk_start >= len && p.cluster <= 1 && (p.cluster == 0 || len > 0)) return;
-  const int chunk_end = min(len, chunk_start + p.chunk_tokens);
+  const int chunk_end = min(len, chunk_start + chunk_tokens);
   float* sm_m = reinterpret_cast<float*>(smem);                 // [warps][16]
   float* sm_l = sm_m + kDecodeWarps * 16;                       // [warps][16]
   float2* sm_ml = reinterpret_cast<float2*>(sm_l + kDecodeWarps * 16);  // [G] of the chunk
@@ -435,7 +456,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 2 : 1) decode_splitkv
   cluster_sync_all();
   {
     const int rank = static_cast<int>(cluster_ctarank());
-    const int n_chunks = min(p.cluster, (len + p.chunk_tokens - 1) / p.chunk_tokens);
+    const int n_chunks = min(p.cluster, (len + chunk_tokens - 1) / chunk_tokens);
     const uint32_t ml_addr = smem_u32(sm_ml), acc_addr = smem_u32(sm_acc);
     for (int u = threadIdx.x * p.cluster + rank; u < G * kQuads; u += kDecodeThreads * p.cluster) {
       const int r = u / kQuads, d = (u % kQuads) * 4;
@@ -490,7 +511,8 @@ __global__ void __launch_bounds__(kReduceThreads) decode_reduce_kernel(const Dec
   grid_dependency_wait();
   grid_dependency_trigger();
   const int len = clamped_len(p, seq, false);  // same clamp as phase 1
-  const int n_chunks = (len + p.chunk_tokens - 1) / p.chunk_tokens;  // <= max_chunks
+  const int chunk_tokens = p.chunk.tokens(len);
+  const int n_chunks = (len + chunk_tokens - 1) / chunk_tokens;  // <= max_chunks
   const int64_t slot0 = (static_cast<int64_t>(seq) * p.q_heads + qh) * p.max_chunks;
   const float2* ml = p.ws_ml + slot0;
   auto block_sum_or_max = [&](float v, bool is_max) {
@@ -659,13 +681,14 @@ int launch_decode_typed(const DecodeParams& p, bool paged, int num_seqs, cudaStr
 namespace {
 // How a problem is split (chunk_tokens 0: the library's choice).
 struct DecodePlan {
-  int32_t chunk, max_chunks;  // KV tokens per CTA, chunks of the longest sequence
-  int32_t cluster;            // see DecodeParams
+  ChunkRule chunk;
+  int32_t max_chunks;  // that a sequence of any length up to the capacity can have
+  int32_t cluster;     // see DecodeParams
 };
 
 // The rules below were read off a sweep over 26 problems (1 to 128 sequences, 1 to 16 kv heads, 67 to
-// 16000 tokens, lengths spread over a factor of 16), one chunk / clusters of 2, 4, 8 / two kernels with
-// 2 to 64 chunks, device time in a graph.  "Units" are (sequence, kv head) pairs; 296 CTAs are resident.
+// 16000 tokens, lengths spread over a factor of 16, tables as wide as the longest), one chunk / clusters of 2, 4, 8 / two
+// kernels with 2 to 64 chunks, device time in a graph.  "Units" are (sequence, kv head) pairs; 296 CTAs are resident.
 //   * units fill the SMs: one chunk each (62 x 8 units of up to 238 tokens: 11 us, 23 with 2 chunks), the
 //     hardware hands out the next one where one ends.  Chunks stop at 2048 tokens (about 20 us), so that
 //     one long sequence among short ones does not run alone for long (64 x 8 units of up to 8192: 175 us
@@ -678,31 +701,41 @@ struct DecodePlan {
 //     up to 1003 tokens: 20 us unsplit, 82 in clusters of eight) -- and chunks stay within 512 tokens.
 //   * the rest: about 400 CTAs of at least 192 tokens and the reduction kernel (7 units of 15695 tokens:
 //     43 us with 64-token chunks and the former reduction, 12.7 now).
+// Which rule applies and the size of the grid follow from the capacity; in the last two the size of a chunk follows from
+// the length (ChunkRule).  Cut to fit the capacity, as before, chunks left few CTAs with work (8 kv heads, tables for
+// 131072 tokens: 4 x 1000..2000 30 us, 14 now; 1 x 1000 16 / 8.5; 8 x 500..4000 36 / 22.5).
 DecodePlan plan_decode(const b200k_decode_args& a) {
-  DecodePlan d = {64, 1, 0};
+  DecodePlan d = {{64, 1, 64, {}}, 1, 0};
   if (a.max_seq_len <= 0 || a.num_seqs <= 0 || a.kv_heads <= 0) return d;
   const int64_t units = static_cast<int64_t>(a.num_seqs) * a.kv_heads;
   const int64_t sms = num_sms(), slots = sms * 2;
   const int64_t len = a.max_seq_len;
-  auto chunk_for = [&](int64_t n) { return static_cast<int32_t>(((len + n - 1) / n + 63) / 64 * 64); };
+  auto ceil_div = [](int64_t x, int64_t y) { return (x + y - 1) / y; };
+  ChunkRule& r = d.chunk;
   if (a.chunk_tokens > 0) {
-    d.chunk = a.chunk_tokens;
+    r.fixed = a.chunk_tokens;
   } else if (units >= slots || len <= 128 || (units * 4 >= slots && len <= 1024)) {
-    d.chunk = chunk_for((len + 2047) / 2048);
+    r.fixed = static_cast<int32_t>(ceil_div(ceil_div(len, ceil_div(len, kMaxChunk)), 64) * 64);
   } else {
     int64_t c = 1;
     while (c < kMaxCluster && units * c * 2 <= sms && c * 64 < len) c *= 2;
-    if (c < kMaxCluster && units * c * 2 <= slots && chunk_for(c) > 512) c *= 2;
-    if (chunk_for(c) <= 512) {
-      d.chunk = chunk_for(c);
+    if (c < kMaxCluster && units * c * 2 <= slots && len > c * 512) c *= 2;
+    r.fixed = 0;
+    if (len <= c * 512) {
+      r.split = static_cast<int32_t>(c);
     } else {
-      const int64_t n = (400 + units - 1) / units;
-      d.chunk = chunk_for(n);
-      if (d.chunk < 192) d.chunk = 192;
-      if (d.chunk > 2048) d.chunk = chunk_for((len + 2047) / 2048);
+      r.split = static_cast<int32_t>(ceil_div(400, units));
+      r.least = 192;
     }
+    r.by_split.set(r.split);
   }
-  d.max_chunks = static_cast<int32_t>((len + d.chunk - 1) / d.chunk);
+  if (r.fixed > 0) {
+    d.max_chunks = static_cast<int32_t>(ceil_div(len, r.fixed));
+  } else {
+    const int64_t most = ceil_div(len, kMaxChunk), fine = ceil_div(len, r.least);
+    const int64_t n = r.split > most ? r.split : most;
+    d.max_chunks = static_cast<int32_t>(n < fine ? n : fine);
+  }
   if (d.max_chunks <= kMaxCluster) {
     int32_t c = 1;
     while (c < d.max_chunks) c *= 2;
@@ -716,7 +749,7 @@ uint64_t decode_slots(const b200k_decode_args& a, const DecodePlan& d) {
 }
 }  // namespace
 
-int32_t decode_default_chunk(const b200k_decode_args& a) { return plan_decode(a).chunk; }
+int32_t decode_default_chunk(const b200k_decode_args& a) { return plan_decode(a).chunk.tokens(a.max_seq_len); }
 
 uint64_t decode_workspace_bytes(const b200k_decode_args& a) {
   if (a.num_seqs <= 0 || a.q_heads <= 0 || a.kv_heads <= 0 || a.max_seq_len <= 0) return 0;
@@ -751,12 +784,13 @@ int launch_decode(const b200k_decode_args& a, cudaStream_t stream) {
   p.page_size = a.block_table ? a.page_size : 16;
   p.num_pages = a.num_pages;
   p.block_table_stride = a.block_table_stride;
-  p.chunk_tokens = plan.chunk;
+  p.chunk = plan.chunk;
   p.max_chunks = plan.max_chunks;
   p.cluster = plan.cluster;
   const int64_t ctas = static_cast<int64_t>(p.max_chunks) * p.kv_heads * p.num_seqs;
-  p.warps = ctas <= num_sms() && p.chunk_tokens > 64 ? 8 : 4;
-  const int tiles_per_warp = (p.chunk_tokens / kTileTokens + p.warps - 1) / p.warps;
+  const int32_t longest = plan.chunk.tokens(a.max_seq_len);  // chunks grow with the length
+  p.warps = ctas <= num_sms() && longest > 64 ? 8 : 4;
+  const int tiles_per_warp = (longest / kTileTokens + p.warps - 1) / p.warps;
   p.stages = tiles_per_warp < kDecodeStages ? tiles_per_warp : kDecodeStages;
   p.max_seq_len = a.max_seq_len;
   p.status = a.status;

@@ -57,3 +57,42 @@ def test_the_largest_probability_of_every_tile_is_exact(chunk, dim, dtype):
     near = (ref * (1 - 4e-6)).to(dtype) != (ref * (1 + 4e-6)).to(dtype)
     assert near.float().mean() < 0.05
     assert torch.equal(got[~near], ref.to(dtype)[~near])
+
+
+def split_chunk(units, capacity, length):
+    """Tokens per chunk where the rule is "about 400 CTAs of at least 192 tokens": by the length, not by the capacity."""
+    n = -(-400 // units)
+    return 2048 if length > 2048 * n else max(192, -(-(-(-length // n)) // 64) * 64)
+
+
+# (sequences, kv heads, capacity, lengths): tables and caches with room for more than the histories in them.  8 units
+# with a cluster rule for the capacity, 8 and 32 units with the other, 160 and 320 units; lengths of 0 and 1
+# token, around a chunk and around 2048 times the number of chunks, and the capacity itself.
+@pytest.mark.parametrize("seqs,hkv,capacity,lens", [
+    (1, 8, 2048, [1000]), (4, 8, 4096, [100, 0, 1500, 4096]), (1, 8, 131072, [1000]), (4, 8, 131072, [191, 192, 193, 2500]),
+    (4, 8, 32768, [1, 0, 32768, 1000]), (20, 8, 8192, [8192, 2048, 2049, 0] + [300] * 16), (40, 8, 16384, [2047, 2048, 2049, 4097, 0] + [100] * 35),
+])
+@pytest.mark.parametrize("paged", [True, False])
+def test_capacity_above_the_lengths(seqs, hkv, capacity, lens, paged):
+    q, kc, vc, bt, sl = oracle.make_paged_decode_inputs(q_heads=2 * hkv, kv_heads=hkv, head_dim=64, lens=lens, seed=44)
+    if not paged and seqs * hkv * capacity > 1 << 22:
+        pytest.skip("the table form covers it")
+    ref = oracle.paged_decode_attention(q, kc, vc, bt, sl, 0.125)
+    q, sl = q.to(DEV), sl.to(DEV)
+    if paged:
+        table = torch.zeros(seqs, capacity // 16, dtype=torch.int32)
+        table[:, :bt.shape[1]] = bt.clamp(min=0)
+        rest = (kc.to(DEV), vc.to(DEV), table.to(DEV), sl, 0.125)
+        op = torch.ops.b200k.paged_decode_attention
+    else:
+        rest = tuple(torch.ops.b200k.paged_gather(c.to(DEV), bt.to(DEV), sl, capacity) for c in (kc, vc)) + (sl, 0.125)
+        op = torch.ops.b200k.decode_attention
+    got = op(q, *rest)
+    torch.cuda.synchronize()
+    assert tb.device_status() == 0
+    oracle.assert_close_half(got.cpu(), ref)
+    assert torch.equal(got, op(q, *rest))
+    units = seqs * hkv
+    if units < 296 and capacity > 4096:  # the same bits as with every sequence's chunk asked for by hand
+        for s, n in enumerate(lens):
+            assert torch.equal(got[s], op(q, *rest, split_chunk(units, capacity, n))[s]), (s, n)
