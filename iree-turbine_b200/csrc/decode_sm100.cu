@@ -167,15 +167,15 @@ constexpr int kMaxCluster = 8;     // portable cluster size
 constexpr int kReduceThreads = 256;
 constexpr int kMergeHead = 8 * 16 * 8 + 16 * 8;  // bytes of shared memory for (max, sum) per warp and per chunk
 
-// Four dims of one output row: accumulator / sum, zero for a row without keys.
+// Four dims of one output row: accumulator / sum, zero for a row without keys or without a positive sum, whatever
+// the accumulator holds then (scores of -infinity or NaN).
 template <typename T>
 __device__ __forceinline__ void store_out(const DecodeParams& p, int seq, int q_head, int d, float4 acc, float L,
                                           int head_dim) {
-  const float inv_ok = L > 0.f ? 1.f : 0.f;
-  const float den = L > 0.f ? L : 1.f;
+  const bool any = L > 0.f;
   uint2 u;
-  u.x = pack2<T>(acc.x / den * inv_ok, acc.y / den * inv_ok);
-  u.y = pack2<T>(acc.z / den * inv_ok, acc.w / den * inv_ok);
+  u.x = pack2<T>(any ? acc.x / L : 0.f, any ? acc.y / L : 0.f);
+  u.y = pack2<T>(any ? acc.z / L : 0.f, any ? acc.w / L : 0.f);
   T* o = reinterpret_cast<T*>(p.o) + (static_cast<int64_t>(seq) * p.q_heads + q_head) * head_dim + d;
   *reinterpret_cast<uint2*>(o) = u;
 }

@@ -96,3 +96,19 @@ def test_capacity_above_the_lengths(seqs, hkv, capacity, lens, paged):
     if units < 296 and capacity > 4096:  # the same bits as with every sequence's chunk asked for by hand
         for s, n in enumerate(lens):
             assert torch.equal(got[s], op(q, *rest, split_chunk(units, capacity, n))[s]), (s, n)
+
+
+@pytest.mark.parametrize("chunk", [64, 512, 0])  # second kernel, cluster, one chunk
+def test_rows_without_a_positive_sum_are_zero(chunk):
+    """Scores that are all -infinity or NaN give zeros, infinite values or not; the other rows are untouched."""
+    seqs, length, dim = 3, 640 if chunk else 64, 128
+    k = torch.randn(seqs, 2, length, dim, generator=torch.Generator().manual_seed(45)).half()
+    v = torch.randn(seqs, 2, length, dim, generator=torch.Generator().manual_seed(46)).half()
+    q = torch.randn(seqs, 4, dim, generator=torch.Generator().manual_seed(47)).half()
+    lens = torch.full((seqs,), length, dtype=torch.int32)
+    ref = oracle.decode_attention(q, k, v, lens, 0.1)
+    q[0], k[0], v[0] = 1.0, -float("inf"), float("inf")
+    q[1] = float("nan")
+    got = torch.ops.b200k.decode_attention(q.to(DEV), k.to(DEV), v.to(DEV), lens.to(DEV), 0.1, chunk).cpu()
+    assert torch.equal(got[:2], torch.zeros(2, 4, dim, dtype=torch.float16))
+    oracle.assert_close_half(got[2], ref[2])
