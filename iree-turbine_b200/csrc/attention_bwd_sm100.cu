@@ -367,8 +367,8 @@ __device__ __forceinline__ void bwd_dq_cta(int block, int blocks, const CUtensor
     const int q_g = row0 + r;
     const int64_t stat_idx = (static_cast<int64_t>(batch) * p.q_heads + head) * p.seq_q + q_g;
     if (q_g < p.seq_q) {
-      dl = __ldg(p.delta + stat_idx);
-      if (p.lse_in) lse2 = lse_to_log2(__ldg(p.lse_in + stat_idx));
+      dl = p.delta[stat_idx];
+      if (p.lse_in) lse2 = lse_to_log2(p.lse_in[stat_idx]);
     }
     // key j (global index) is visible to this row iff j <= col_hi
     int col_hi = -1;
@@ -747,9 +747,9 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
         if (q_g < p.seq_q) {
           const int64_t idx = (static_cast<int64_t>(batch) * p.q_heads + kvh * group + g_) * p.seq_q + q_g;
           if (tid < 128)
-            val = p.lse_in ? lse_to_log2(__ldg(p.lse_in + idx)) : __ldg(p.lse2 + idx);
+            val = p.lse_in ? lse_to_log2(p.lse_in[idx]) : p.lse2[idx];
           else
-            val = __ldg(p.delta + idx);
+            val = p.delta[idx];
         }
       }
       return val;
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 // of 16 bytes; a warp takes 32 / (HD / 8) rows at a time and eight such groups, all loads issued
 // before the first use, so that enough bytes are in flight to run at memory speed.
 template <typename T, int HD>
-__global__ void attn_bwd_delta_kernel(const T* __restrict__ o, const T* __restrict__ d_o, float* __restrict__ delta,
+__global__ void attn_bwd_delta_kernel(const T* o, const T* d_o, float* delta,
                                       int64_t rows, int q_heads, int seq_q, int64_t o_sb, int64_t o_sh, int64_t o_ss,
                                       int64_t do_sb, int64_t do_sh, int64_t do_ss) {
   constexpr int kLanesPerRow = HD / 8;

@@ -175,7 +175,7 @@ __device__ __forceinline__ Item make_item(int batch, int head, int pair, const A
   it.head = head;
   // (dense: the two are launch constants and the fields fold away)
   it.kv_len = p.seq_kv;
-  if (PAGED) it.kv_len = max(0, min(__ldg(p.seq_lens + it.batch), p.seq_kv));
+  if (PAGED) it.kv_len = max(0, min(p.seq_lens[it.batch], p.seq_kv));
   it.causal_offset = PAGED ? it.kv_len - p.seq_q : p.causal_offset;
   const int kv_tiles_total = (it.kv_len + kTileRows - 1) / kTileRows;
 #pragma unroll
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           if (!PAGED || lane >= pages_per_tile || j >= it.nmax) return 0;
           const int lp = j * pages_per_tile + lane;
           const int valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
-          return __ldg(p.block_table + static_cast<int64_t>(it.batch) * p.block_table_stride + (lp < valid_pages ? lp : 0));
+          return p.block_table[static_cast<int64_t>(it.batch) * p.block_table_stride + (lp < valid_pages ? lp : 0)];
         };
         // One 128-row K or V tile.  A table entry outside the pool is reported and reads as zeros (the
         // tensor map clips it).

@@ -27,8 +27,8 @@ __device__ __forceinline__ void from_float(float v, __half& o) { o = __float2hal
 __device__ __forceinline__ void from_float(float v, __nv_bfloat16& o) { o = __float2bfloat16_rn(v); }
 
 template <typename T, typename T2>
-__global__ void __launch_bounds__(kThreads) col_sum_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows,
-                                                           int64_t cols, int64_t ld) {
+__global__ void __launch_bounds__(kThreads) col_sum_kernel(const T* x, T* out, int64_t rows, int64_t cols,
+                                                           int64_t ld) {
   __shared__ float part[kThreads / 32][kCols];
   __shared__ float total[kCols];
   grid_dependency_wait();
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kThreads) col_sum_kernel(const T* __restrict__
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         const int64_t rr = r + u * kRowsPerPass;
-        v[u] = rr < r_end ? __ldg(reinterpret_cast<const uint4*>(px + rr * ld)) : make_uint4(0u, 0u, 0u, 0u);
+        v[u] = rr < r_end ? *reinterpret_cast<const uint4*>(px + rr * ld) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {

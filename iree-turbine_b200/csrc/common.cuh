@@ -93,7 +93,9 @@ inline int ensure_dynamic_smem(Kernel kfn, int bytes, bool (&done)[64], const ch
 // Launches a kernel with programmatic stream serialization: its CTAs may become resident and run up to
 // their grid_dependency_wait() while the previous kernel of the stream is still finishing.  Every
 // kernel launched this way waits before it touches global memory, so the completion of the last one
-// implies that of all before it.  Small kernels in a row lose the launch latency and set-up time
+// implies that of all before it.  They read it with plain loads: the non-coherent ones (ld.global.nc, what __ldg
+// and const __restrict__ pointers become) are for memory that does not change while the kernel lives, which the
+// previous kernel's results do, and the wait does not order them.  Small kernels in a row lose the launch latency and set-up time
 // between them (2 to 3 us each).
 template <typename... P, typename... A>
 inline int launch_maybe_pdl(bool early, const char* what, void (*kfn)(P...), dim3 grid, dim3 block, size_t smem,

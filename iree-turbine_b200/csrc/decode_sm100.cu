@@ -83,14 +83,14 @@ struct DecodeParams {
 // block-table entry is outside the pool.  This single function defines the paged layout for the
 // decode kernel and for the gather check kernel.
 template <bool PAGED>
-__device__ __forceinline__ int64_t kv_row_offset(const int32_t* __restrict__ block_table, int32_t block_table_stride,
+__device__ __forceinline__ int64_t kv_row_offset(const int32_t* block_table, int32_t block_table_stride,
                                                  int32_t page_size, int32_t num_pages, int64_t kv_page_stride,
                                                  int64_t kv_head_stride, int64_t kv_batch_stride, int32_t head_dim,
                                                  int32_t seq, int32_t head, int32_t token) {
   if constexpr (PAGED) {
     const int32_t logical_page = token / page_size;
     const int32_t in_page = token - logical_page * page_size;
-    const int32_t page = __ldg(block_table + static_cast<int64_t>(seq) * block_table_stride + logical_page);
+    const int32_t page = block_table[static_cast<int64_t>(seq) * block_table_stride + logical_page];
     if (page < 0 || page >= num_pages) return -1;
     return static_cast<int64_t>(page) * kv_page_stride + static_cast<int64_t>(head) * kv_head_stride +
            static_cast<int64_t>(in_page) * head_dim;
@@ -181,7 +181,7 @@ __device__ __forceinline__ void store_out(const DecodeParams& p, int seq, int q_
 }
 
 __device__ __forceinline__ int clamped_len(const DecodeParams& p, int seq, bool report) {
-  const int given = __ldg(p.seq_lens + seq);
+  const int given = p.seq_lens[seq];
   if (report && given > p.max_seq_len && p.status) atomicOr(p.status, kStatusDecodeLenClamped);
   return max(0, min(given, p.max_seq_len));
 }
@@ -581,14 +581,14 @@ __global__ void __launch_bounds__(kReduceThreads) decode_reduce_kernel(const Dec
 // ------------------------------------------------------------------------------------------
 // gather check kernel: copies rows through the block table with kv_row_offset<true>
 // ------------------------------------------------------------------------------------------
-__global__ void paged_gather_kernel(const uint8_t* __restrict__ cache, const int32_t* __restrict__ block_table,
-                                    const int32_t* __restrict__ seq_lens, uint8_t* __restrict__ out, int32_t kv_heads,
+__global__ void paged_gather_kernel(const uint8_t* cache, const int32_t* block_table, const int32_t* seq_lens,
+                                    uint8_t* out, int32_t kv_heads,
                                     int32_t head_dim, int32_t page_size, int32_t num_pages, int32_t block_table_stride,
                                     int32_t max_seq_len, int64_t kv_page_stride, int64_t kv_head_stride,
                                     int32_t elem_bytes) {
   const int seq = blockIdx.z;
   const int head = blockIdx.y;
-  const int len = min(__ldg(seq_lens + seq), max_seq_len);
+  const int len = min(seq_lens[seq], max_seq_len);
   const int row_bytes = head_dim * elem_bytes;
   const int chunks_per_row = row_bytes / 16;
   for (int token = blockIdx.x; token < len; token += gridDim.x) {
@@ -839,9 +839,8 @@ int launch_paged_gather(const void* cache, const int32_t* block_table, const int
 // function of the decode kernel).  One warp per (token, head) row; 16-byte stores; rows whose
 // block-table entry is outside the pool are dropped and reported through the status word.
 // ------------------------------------------------------------------------------------------
-__global__ void kv_append_kernel(const uint8_t* __restrict__ k_new, const uint8_t* __restrict__ v_new,
-                                 uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,
-                                 const int32_t* __restrict__ block_table, const int32_t* __restrict__ positions,
+__global__ void kv_append_kernel(const uint8_t* k_new, const uint8_t* v_new, uint8_t* k_cache, uint8_t* v_cache,
+                                 const int32_t* block_table, const int32_t* positions,
                                  int32_t new_tokens, int32_t kv_heads, int32_t head_dim, int32_t page_size,
                                  int32_t num_pages, int32_t block_table_stride, int64_t kv_page_stride,
                                  int64_t kv_head_stride, int32_t elem_bytes, int32_t* status) {
@@ -851,7 +850,7 @@ __global__ void kv_append_kernel(const uint8_t* __restrict__ k_new, const uint8_
   const int head = blockIdx.y;
   const int row_bytes = head_dim * elem_bytes;
   const int chunks_per_row = row_bytes / 16;
-  const int pos0 = __ldg(positions + seq);
+  const int pos0 = positions[seq];
   const int warps = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int t = blockIdx.x * warps + warp; t < new_tokens; t += gridDim.x * warps) {
@@ -870,8 +869,9 @@ __global__ void kv_append_kernel(const uint8_t* __restrict__ k_new, const uint8_
     uint4* kd = reinterpret_cast<uint4*>(k_cache + off * elem_bytes);
     uint4* vd = reinterpret_cast<uint4*>(v_cache + off * elem_bytes);
     for (int c = lane; c < chunks_per_row; c += 32) {
-      kd[c] = __ldg(ks + c);
-      vd[c] = __ldg(vs + c);
+      const uint4 k = ks[c], v = vs[c];
+      kd[c] = k;
+      vd[c] = v;
     }
   }
 }

@@ -155,9 +155,9 @@ __device__ __forceinline__ float apply_act(float x, int act) {
 }
 
 __device__ __forceinline__ float load_bias(const void* bias, int dtype, int col) {
-  if (dtype == B200K_F32) return __ldg(reinterpret_cast<const float*>(bias) + col);
-  if (dtype == B200K_F16) return __half2float(__ldg(reinterpret_cast<const __half*>(bias) + col));
-  return __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(bias) + col));
+  if (dtype == B200K_F32) return reinterpret_cast<const float*>(bias)[col];
+  if (dtype == B200K_F16) return __half2float(reinterpret_cast<const __half*>(bias)[col]);
+  return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[col]);
 }
 
 // acc * scale + bias, then the activation, on N accumulator values of one row, in place.  `bias` is the

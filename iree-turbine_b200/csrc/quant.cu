@@ -32,8 +32,8 @@ __device__ __forceinline__ float block_max(float m) {
 }
 
 // parts: one value per block, or (one_part) a single word that was zeroed before the launch.
-__global__ void __launch_bounds__(kQuantThreads) absmax_kernel(const float* __restrict__ x, int64_t n,
-                                                               uint32_t* __restrict__ parts, bool one_part) {
+__global__ void __launch_bounds__(kQuantThreads) absmax_kernel(const float* x, int64_t n, uint32_t* parts,
+                                                               bool one_part) {
   grid_dependency_wait();
   grid_dependency_trigger();
   float m = 0.f;
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kQuantThreads) absmax_kernel(const float* __re
     float4 v[kQuantUnroll];
 #pragma unroll
     for (int u = 0; u < kQuantUnroll; ++u)
-      v[u] = i + u * stride < n4 ? __ldg(x4 + i + u * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[u] = i + u * stride < n4 ? x4[i + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < kQuantUnroll; ++u)
       m = fmaxf(m, fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w))));
@@ -72,13 +72,13 @@ __device__ __forceinline__ uint32_t quantize_pair(float a, float b, float inv, f
   return r;
 }
 
-__global__ void __launch_bounds__(kQuantThreads) cast_e4m3_kernel(const float* __restrict__ x, uint8_t* __restrict__ y,
-                                                                  int64_t n, const uint32_t* __restrict__ parts,
-                                                                  int num_parts, float* __restrict__ scale_out) {
+__global__ void __launch_bounds__(kQuantThreads) cast_e4m3_kernel(const float* x, uint8_t* y, int64_t n,
+                                                                  const uint32_t* parts, int num_parts,
+                                                                  float* scale_out) {
   grid_dependency_wait();
   grid_dependency_trigger();
   float m = 0.f;
-  for (int i = threadIdx.x; i < num_parts; i += kQuantThreads) m = fmaxf(m, __uint_as_float(__ldg(parts + i)));
+  for (int i = threadIdx.x; i < num_parts; i += kQuantThreads) m = fmaxf(m, __uint_as_float(parts[i]));
   const float amax = block_max(m);
   const float scale = amax > 0.f ? __fdiv_rn(amax, kE4M3Max) : 1.0f;
   // a reciprocal that overflows or vanishes says nothing about the quotient: divide every value then
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kQuantThreads) cast_e4m3_kernel(const float* _
     float4 v[kQuantUnroll];
 #pragma unroll
     for (int u = 0; u < kQuantUnroll; ++u)
-      if (i + u * stride < n4) v[u] = __ldg(x4 + i + u * stride);
+      if (i + u * stride < n4) v[u] = x4[i + u * stride];
 #pragma unroll
     for (int u = 0; u < kQuantUnroll; ++u) {
       if (i + u * stride >= n4) break;
