@@ -387,8 +387,8 @@ int b200k_decode_attention_static(const b200k_decode_args* args, void* stream);
 /*
  * Gathers the K or V rows of every sequence through the block table into a contiguous buffer
  *   out[s, h, t, :] = cache[block_table[s, t / page_size], h, t % page_size, :]
- * with out laid out [num_seqs, kv_heads, max_seq_len, head_dim].  Rows t >= seq_lens[s] are
- * left untouched.  It uses the same address function as the paged decode kernel and exists so
+ * with out laid out [num_seqs, kv_heads, max_seq_len, head_dim].  Rows t >= seq_lens[s], or past the
+ * block_table_stride * page_size tokens of a table row, are left untouched.  It uses the same address function as the paged decode kernel and exists so
  * that the index arithmetic can be checked bit-for-bit against a host gather.
  */
 int b200k_paged_gather(const void* cache, const int32_t* block_table, const int32_t* seq_lens, void* out,

@@ -588,7 +588,8 @@ __global__ void paged_gather_kernel(const uint8_t* cache, const int32_t* block_t
                                     int32_t elem_bytes) {
   const int seq = blockIdx.z;
   const int head = blockIdx.y;
-  const int len = min(seq_lens[seq], max_seq_len);
+  const int64_t in_table = static_cast<int64_t>(block_table_stride) * page_size;  // a row of the table ends there
+  const int len = static_cast<int>(min(static_cast<int64_t>(min(seq_lens[seq], max_seq_len)), in_table));
   const int row_bytes = head_dim * elem_bytes;
   const int chunks_per_row = row_bytes / 16;
   for (int token = blockIdx.x; token < len; token += gridDim.x) {

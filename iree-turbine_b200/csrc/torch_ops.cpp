@@ -24,6 +24,7 @@
 #include <torch/csrc/utils/pybind.h>
 #include <torch/library.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
@@ -503,14 +504,28 @@ void launch_decode(b200k_decode_args& a, const OnDevice& on) {
   check(api().b200k_decode_attention(&a, on.stream()));
 }
 
-// Tables and caches kept for more sequences than the call decodes are fine: the first ones are used.
+// Block tables, lengths and positions are read by the kernels as int32 with one row (entry) per sequence; a table of
+// int64, torch's own default, would be taken apart into low and high words.  Those kept for more sequences than
+// the call has are fine: the first ones are used.
+void check_table(const char* op, const Tensor& t, int64_t sequences) {
+  TORCH_CHECK(t.scalar_type() == at::kInt && t.dim() == 2 && t.size(0) >= sequences, op,
+              ": block_table must be int32 [num_seqs, max_pages] for ", sequences, " sequences, got ", t.scalar_type(), " ",
+              t.sizes());
+}
+
+void check_per_sequence(const char* op, const char* name, const Tensor& t, int64_t sequences) {
+  const auto sizes = t.sizes();
+  const bool vector = std::count_if(sizes.begin(), sizes.end(), [](int64_t n) { return n != 1; }) <= 1;
+  TORCH_CHECK(t.scalar_type() == at::kInt && vector && t.numel() >= sequences, op, ": ", name,
+              " must be int32 [num_seqs] for ", sequences, " sequences, got ", t.scalar_type(), " ", sizes);
+}
+
 void check_decode(const char* op, const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& lens) {
   TORCH_CHECK(q.dim() == 3 && kc.dim() == 4, op, ": q must be 3-D and the K/V caches 4-D");
   TORCH_CHECK(q.scalar_type() == kc.scalar_type() && q.scalar_type() == vc.scalar_type(), op,
               ": q and the KV cache must share a dtype");
   TORCH_CHECK(kc.sizes() == vc.sizes() && kc.size(3) == q.size(2), op, ": cache shapes do not match");
-  TORCH_CHECK(lens.scalar_type() == at::kInt && lens.dim() == 1 && lens.size(0) >= q.size(0), op,
-              ": seq_lens must be int32 [num_seqs]");
+  check_per_sequence(op, "seq_lens", lens, q.size(0));
 }
 
 Tensor decode_attention(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& lens_in, double scale,
@@ -546,8 +561,7 @@ Tensor paged_decode_attention(const Tensor& q_in, const Tensor& kc_in, const Ten
   one_device("paged_decode_attention", q_in.device(), {&kc_in, &vc_in, &bt_in, &lens_in});
   OnDevice on(q_in.device());
   check_decode("paged_decode_attention", q_in, kc_in, vc_in, lens_in);
-  TORCH_CHECK(bt_in.scalar_type() == at::kInt && bt_in.dim() == 2 && bt_in.size(0) >= q_in.size(0),
-              "paged_decode_attention: block_table must be int32 [num_seqs, max_pages]");
+  check_table("paged_decode_attention", bt_in, q_in.size(0));
   const Tensor q = q_in.contiguous(), kc = kc_in.contiguous(), vc = vc_in.contiguous(), bt = bt_in.contiguous(),
                lens = lens_in.contiguous();
   Tensor o = empty(q.sizes(), q.scalar_type(), q.device());
@@ -578,6 +592,9 @@ Tensor paged_decode_attention(const Tensor& q_in, const Tensor& kc_in, const Ten
 Tensor paged_gather(const Tensor& cache_in, const Tensor& bt_in, const Tensor& lens_in, int64_t max_seq_len) {
   one_device("paged_gather", cache_in.device(), {&bt_in, &lens_in});
   OnDevice on(cache_in.device());
+  TORCH_CHECK(cache_in.dim() == 4, "paged_gather: cache must be [num_pages, heads, page_size, head_dim]");
+  check_table("paged_gather", bt_in, 0);
+  check_per_sequence("paged_gather", "seq_lens", lens_in, bt_in.size(0));
   const Tensor cache = cache_in.contiguous(), bt = bt_in.contiguous(), lens = lens_in.contiguous();
   Tensor out = at::zeros({bt.size(0), cache.size(1), max_seq_len, cache.size(3)}, cache.options());
   check(api().b200k_paged_gather(cache.data_ptr(), static_cast<const int32_t*>(bt.data_ptr()),
@@ -597,6 +614,8 @@ void kv_append(const Tensor& kn_in, const Tensor& vn_in, Tensor kc, Tensor vc, c
                   kn_in.size(2) == kc.size(1) && kn_in.size(3) == kc.size(3) && kn_in.scalar_type() == kc.scalar_type() &&
                   vn_in.scalar_type() == kc.scalar_type() && vc.scalar_type() == kc.scalar_type(),
               "kv_append: heads, head_dim and dtypes of new rows and caches must match");
+  check_table("kv_append", bt_in, kn_in.size(0));
+  check_per_sequence("kv_append", "positions", pos_in, kn_in.size(0));
   const Tensor kn = kn_in.contiguous(), vn = vn_in.contiguous(), bt = bt_in.contiguous(), pos = pos_in.contiguous();
   check(api().b200k_kv_append(kn.data_ptr(), vn.data_ptr(), kc.data_ptr(), vc.data_ptr(),
                               static_cast<const int32_t*>(bt.data_ptr()), static_cast<const int32_t*>(pos.data_ptr()),
@@ -612,8 +631,8 @@ Tensor paged_attention(const Tensor& q_in, const Tensor& kc_in, const Tensor& vc
   TORCH_CHECK(kc_in.dim() == 4 && kc_in.sizes() == vc_in.sizes() && kc_in.size(3) == q.size(3) &&
                   kc_in.scalar_type() == q.scalar_type() && vc_in.scalar_type() == q.scalar_type(),
               "paged_attention: caches do not match q");
-  TORCH_CHECK(bt_in.dim() == 2 && bt_in.size(0) >= q.size(0) && lens_in.size(0) >= q.size(0),
-              "paged_attention: block_table must be [B, max_pages] and seq_lens [B]");
+  check_table("paged_attention", bt_in, q.size(0));
+  check_per_sequence("paged_attention", "seq_lens", lens_in, q.size(0));
   const Tensor kc = kc_in.contiguous(), vc = vc_in.contiguous(), bt = bt_in.contiguous(), lens = lens_in.contiguous();
   Tensor o = attention_out_like(q_in);
   b200k_paged_attention_args a = {};
