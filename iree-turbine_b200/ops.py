@@ -388,7 +388,7 @@ def _attention_select(sel: KernelSelection):
     torch._check(q.t.size(3) in (64, 128) and k.t.size(3) == q.t.size(3) and v.t.size(3) == q.t.size(3),
                  lambda: "attention: head dim must be 128 or 64, the same for q, k and v")
     torch._check(k.t.shape == v.t.shape, lambda: "attention: k and v must have the same shape")
-    torch._check(q.t.size(0) == k.t.size(0), lambda: "attention: batch mismatch")
+    torch._check(q.t.size(0) <= k.t.size(0), lambda: "attention: batch mismatch")
     torch._check(q.t.size(1) % k.t.size(1) == 0, lambda: "attention: query heads must be a multiple of kv heads")
     q.specialize_dims(3)
     sel.return_tensor(_attention_out_like(q.t, "meta"))
@@ -477,6 +477,17 @@ def sdpa(q: Tensor, k: Tensor, v: Tensor, scale: Optional[float] = None, is_caus
 # ---------------------------------------------------------------------------------------------
 # decode / paged decode
 # ---------------------------------------------------------------------------------------------
+def _check_table(name: str, table: Tensor, sequences) -> None:
+    """As the CUDA implementations check it: rows kept for more sequences than the call's are fine."""
+    torch._check(table.dtype == torch.int32 and table.dim() == 2 and table.size(0) >= sequences,
+                 lambda: f"{name}: block_table must be int32 [num_seqs, max_pages]")
+
+
+def _check_per_sequence(name: str, what: str, t: Tensor, sequences) -> None:
+    torch._check(t.dtype == torch.int32 and sum(n != 1 for n in t.shape) <= 1 and t.numel() >= sequences,
+                 lambda: f"{name}: {what} must be int32 [num_seqs]")
+
+
 def _decode_common_checks(name: str, q: Tensor, kc: Tensor, vc: Tensor, lens: Tensor):
     torch._check(q.dim() == 3, lambda: f"{name}: q must be [num_seqs, q_heads, head_dim]")
     torch._check(q.dtype in _HALF_TYPES, lambda: f"{name}: dtype must be float16 or bfloat16, got {q.dtype}")
@@ -484,8 +495,7 @@ def _decode_common_checks(name: str, q: Tensor, kc: Tensor, vc: Tensor, lens: Te
     torch._check(q.size(2) in (64, 128), lambda: f"{name}: head dim must be 128 or 64")
     torch._check(kc.dim() == 4 and kc.shape == vc.shape, lambda: f"{name}: k and v caches must be 4-D and equal in shape")
     torch._check(kc.size(3) == q.size(2), lambda: f"{name}: cache head dim must equal q's")
-    torch._check(lens.dtype == torch.int32 and lens.dim() == 1 and lens.size(0) == q.size(0),
-                 lambda: f"{name}: seq_lens must be int32 [num_seqs]")
+    _check_per_sequence(name, "seq_lens", lens, q.size(0))
     torch._check(q.size(1) % kc.size(1) == 0 and q.size(1) // kc.size(1) <= 16,
                  lambda: f"{name}: query heads must be a multiple (at most 16x) of kv heads")
 
@@ -510,7 +520,7 @@ class decode_attention(CustomOp):
         sel.attr_float(4)
         sel.attr_int(5)
         _decode_common_checks("decode_attention", q.t, k.t, v.t, lens.t)
-        torch._check(k.t.size(0) == q.t.size(0), lambda: "decode_attention: k must have one history per sequence")
+        torch._check(k.t.size(0) >= q.t.size(0), lambda: "decode_attention: k must have one history per sequence")
         sel.return_new_tensor(list(q.t.shape), q.t.dtype)
 
 
@@ -537,8 +547,7 @@ class paged_decode_attention(CustomOp):
         sel.attr_float(5)
         sel.attr_int(6)
         _decode_common_checks("paged_decode_attention", q.t, kc.t, vc.t, lens.t)
-        torch._check(bt.t.dtype == torch.int32 and bt.t.dim() == 2 and bt.t.size(0) == q.t.size(0),
-                     lambda: "paged_decode_attention: block_table must be int32 [num_seqs, max_pages]")
+        _check_table("paged_decode_attention", bt.t, q.t.size(0))
         torch._check(kc.t.size(2) % 16 == 0, lambda: "paged_decode_attention: page size must be a multiple of 16")
         sel.return_new_tensor(list(q.t.shape), q.t.dtype)
 
@@ -558,8 +567,8 @@ class paged_gather(CustomOp):
         lens = sel.arg_tensor(2)
         n = sel.attr_int(3)
         torch._check(c.t.dim() == 4, lambda: "paged_gather: cache must be [num_pages, heads, page_size, head_dim]")
-        torch._check(bt.t.dtype == torch.int32 and bt.t.dim() == 2, lambda: "paged_gather: block_table must be int32 2-D")
-        torch._check(lens.t.dtype == torch.int32 and lens.t.dim() == 1, lambda: "paged_gather: seq_lens must be int32 1-D")
+        _check_table("paged_gather", bt.t, 0)
+        _check_per_sequence("paged_gather", "seq_lens", lens.t, bt.t.size(0))
         sel.return_new_tensor([bt.t.size(0), c.t.size(1), n.v, c.t.size(3)], c.t.dtype)
 
 
@@ -591,10 +600,8 @@ class kv_append(CustomOp):
                      lambda: "kv_append: dtypes of new rows and caches must match")
         torch._check(kn.t.size(2) == kc.t.size(1) and kn.t.size(3) == kc.t.size(3),
                      lambda: "kv_append: heads / head_dim of new rows and caches must match")
-        torch._check(bt.t.dtype == torch.int32 and bt.t.dim() == 2 and bt.t.size(0) == kn.t.size(0),
-                     lambda: "kv_append: block_table must be int32 [num_seqs, max_pages]")
-        torch._check(pos.t.dtype == torch.int32 and pos.t.dim() == 1 and pos.t.size(0) == kn.t.size(0),
-                     lambda: "kv_append: positions must be int32 [num_seqs]")
+        _check_table("kv_append", bt.t, kn.t.size(0))
+        _check_per_sequence("kv_append", "positions", pos.t, kn.t.size(0))
 
 
 @CustomOp.register(library=LIBRARY, register_impl=False)
@@ -625,9 +632,7 @@ class paged_attention(CustomOp):
         torch._check(kc.t.dtype == q.t.dtype and vc.t.dtype == q.t.dtype, lambda: "paged_attention: dtypes must match")
         torch._check(kc.t.size(2) in (16, 32, 64, 128), lambda: "paged_attention: page_size must be 16, 32, 64 or 128")
         torch._check(q.t.size(1) % kc.t.size(1) == 0, lambda: "paged_attention: query heads must be a multiple of kv heads")
-        torch._check(bt.t.dtype == torch.int32 and bt.t.dim() == 2 and bt.t.size(0) == q.t.size(0),
-                     lambda: "paged_attention: block_table must be int32 [B, max_pages]")
-        torch._check(lens.t.dtype == torch.int32 and lens.t.dim() == 1 and lens.t.size(0) == q.t.size(0),
-                     lambda: "paged_attention: seq_lens must be int32 [B]")
+        _check_table("paged_attention", bt.t, q.t.size(0))
+        _check_per_sequence("paged_attention", "seq_lens", lens.t, q.t.size(0))
         sel.return_tensor(_attention_out_like(q.t, "meta"))
 

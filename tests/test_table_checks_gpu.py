@@ -67,3 +67,12 @@ def test_gather_stops_where_a_table_row_ends():
     got = OP.paged_gather(kc.to(DEV), bt.to(DEV), lens.to(DEV), 128).cpu()
     ref = oracle.paged_gather(kc, bt, torch.tensor([32, 20], dtype=torch.int32), 128)
     assert torch.equal(got, ref)
+
+
+def test_dense_attention_takes_keys_of_more_sequences():
+    q, k, v = oracle.make_attention_inputs(3, 4, 2, 70, 90, 128, torch.float16, seed=55)
+    q, k, v = q[:2].to(DEV), k.to(DEV), v.to(DEV)
+    assert torch.equal(OP.attention(q, k, v, 0.1, False), OP.attention(q, k[:2], v[:2], 0.1, False))
+    decode = OP.decode_attention(q[:, :, 0].contiguous(), k, v, torch.tensor([90, 40, 3], dtype=torch.int32, device=DEV), 0.1)
+    oracle.assert_close_half(decode, oracle.decode_attention(q[:, :, 0].cpu(), k[:2].cpu(), v[:2].cpu(),
+                                                             torch.tensor([90, 40], dtype=torch.int32), 0.1))
