@@ -708,7 +708,11 @@ struct LinearFunction : torch::autograd::Function<LinearFunction> {
     if (ctx->needs_input_grad(0)) dx = call_gemm(dy, w, false, false, x.scalar_type());  // [M, N] @ [N, K]
     if (ctx->needs_input_grad(1)) dw = call_gemm(dy, x, true, false, w.scalar_type());   // [M, N]^T @ [M, K]
     // an absent bias is not among the inputs that needs_input_grad counts
-    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) db = call_col_sum(dy);
+    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) {
+      // col_sum has no derivative: where this sum is differentiated itself, torch's operators compute it
+      const bool differentiated = (at::GradMode::is_enabled() && dy.requires_grad()) || dy._fw_grad(0).defined();
+      db = differentiated ? dy.to(at::kFloat).sum(0).to(dy.scalar_type()) : call_col_sum(dy);
+    }
     return {dx, dw, db};
   }
 };

@@ -53,3 +53,17 @@ def test_attention_kernel_attribute_reaches_the_ops():
             torch.ops.b200k.attention(q, q, q, 0.1, False)
     finally:
         ops.ATTENTION_KERNEL = L.ATTN_AUTO
+
+
+def test_bias_gradient_can_be_differentiated():
+    g = torch.Generator().manual_seed(5)
+    x, w, b = (torch.randn(*s, generator=g).half().to(DEV) for s in ((40, 64), (24, 64), (24,)))
+    dy = torch.randn(40, 24, generator=g).half().to(DEV).requires_grad_()
+    b.requires_grad_()
+    db, = torch.autograd.grad(ops.linear(x, w, b), b, dy, create_graph=True)
+    plain, = torch.autograd.grad(ops.linear(x, w, b), b, dy.detach())
+    # one rounding to f16 (2^-11) of the same fp32 sum in two orders
+    oracle.assert_close_half(db, plain.float().cpu(), rtol=2.0 ** -10, atol=1e-4)
+    weight = torch.randn(24, generator=g).half().to(DEV)
+    ddy, = torch.autograd.grad(db, dy, weight)
+    assert torch.equal(ddy, weight.expand(40, 24))
