@@ -351,7 +351,14 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty + acc);
     }
-    if (lane == 0) tma_store_wait_read<0>();  // staging memory must outlive the last stores (they complete before the grid does)
+    // Staging memory must outlive the last stores; those to this GPU's memory complete before the grid does.  Stores to
+    // peers are waited for themselves: a barrier between ranks follows the kernel, and their writes must be done by then.
+    if (lane == 0) {
+      if (p.peer_tma)
+        tma_store_wait<0>();
+      else
+        tma_store_wait_read<0>();
+    }
     __syncwarp();
   }
 
