@@ -216,7 +216,7 @@ struct ItemWalk {
     }
     if (walk.pos >= p.order.num_items) return false;
     int batch, head, pair;
-    attn_order::item_at(p.order, walk.pos, table, p.q_heads, batch, head, pair);
+    attn_order::item_at<PAGED>(p.order, walk.pos, table, p.q_heads, batch, head, pair);
     if (!PAGED && p.couples > 0) {  // tile t of the order is the couple (couples - 1 - t, its mirror image)
       const int k = p.order.tiles - 1 - pair;
       pair = p.couples - 1 - k;

@@ -159,7 +159,7 @@ __device__ __forceinline__ Item make_item(int batch, int head, int qtile, const 
 template <bool PAGED>
 __device__ __forceinline__ Item decode_item(int pos, const AttnParams& p, const uint16_t* table) {
   int batch, head, qtile;
-  attn_order::item_at(p.order, pos, table, p.q_heads, batch, head, qtile);
+  attn_order::item_at<PAGED>(p.order, pos, table, p.q_heads, batch, head, qtile);
   return make_item<PAGED>(batch, head, qtile, p);
 }
 
@@ -302,9 +302,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         // Q and the first K tiles of an item.  Q's buffer is free once the previous item's last
         // score MMA has run, which is earlier than the release of its last V stage.
         auto load_head = [&](const Item& it) {
-          int pages[kKStages];
+          int pages[kKStages] = {};
+          if (PAGED) {
 #pragma unroll
-          for (int jj = 0; jj < kKStages; ++jj) pages[jj] = page_of(it, jj);
+            for (int jj = 0; jj < kKStages; ++jj) pages[jj] = page_of(it, jj);
+          }
           if (!wait_free(q_empty, (qc & 1) ^ 1)) return false;
           if (lane == 0) {
             mbar_arrive_expect_tx(q_full, kTileBytes);
@@ -314,6 +316,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
                           it.batch);
           }
           ++qc;
+          // Items of a few K tiles spend much of their time between items, and this loop is quicker there than three
+          // copies of its body, which longer items want: loop / copies, us, 8x16x3000 queries over 367 keys 105 / 109,
+          // 24x64x308 over 308 149 / 156; 2x32x2000 over 2000 132 / 130, 4x16x4096 over 4096 472 / 467.
+          if (!PAGED && it.n <= kKStages + 1) {
+#pragma unroll 1
+            for (int jj = 0; jj < kKStages && jj < it.n; ++jj)
+              if (!load_k(it, jj, 0)) return false;
+            return true;
+          }
 #pragma unroll
           for (int jj = 0; jj < kKStages; ++jj)
             if (jj < it.n && !load_k(it, jj, pages[jj])) return false;
