@@ -84,7 +84,7 @@ const char* b200k_status_string(int status);
  *   in_dtype  E4M3        -> out_dtype BF16 | F32, result multiplied by (*scale_a) * (*scale_b)
  *
  * lda / ldb / ldc are row strides in ELEMENTS.  A, B: 16-byte aligned base, row stride a
- * multiple of 16 bytes.  C: base aligned to 16 bytes, ldc * sizeof(out) a multiple of 16.
+ * multiple of 16 bytes.  C: base aligned to its element size (rows that start on 16 bytes are stored faster).
  * K tails, M tails and N tails are handled (out-of-range operand elements read as zero).
  *
  * The kernel is launched as a programmatic dependent launch: its barrier set-up and tensor-memory
@@ -104,7 +104,7 @@ typedef struct b200k_gemm_args {
   const float* scale_a; /* device scalar, E4M3 only, may be NULL (= 1.0) */
   const float* scale_b; /* device scalar, E4M3 only, may be NULL (= 1.0) */
   int32_t* status;      /* device status word, may be NULL */
-  int32_t tile_n;       /* 0 = choose; else 128 or 256 */
+  int32_t tile_n;       /* 0 = choose; else 64, 128 or 256 */
   int32_t tile_m;       /* 0 = choose; else 128 or 256 (256 needs tile_n 256 or 0) */
   /* Optional fused epilogue (the bias / activation tail of a linear layer, cf. the reference's
    * ops/templates/test_linear_trailing_optional_biased.mlir):  C = act(A B^T * scales + bias[n]).

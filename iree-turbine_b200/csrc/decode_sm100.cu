@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 2 : 1) decode_splitkv
   }
   cp_async_wait<0>();
 
-  // ---- merge the four warps' partial states and write the chunk's partial result ----
+  // ---- merge the warps' partial states: the result, or the chunk's partial one (see DecodeParams::cluster) ----
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);

@@ -36,7 +36,8 @@ using namespace gemm_detail;
 // bias, the error function or stores that the TMA unit cannot make (one / two, us): fp8 5000x5001x2048 97 / 64,
 // 8000x1025x1024 41 / 23, fp32 out 2000x2001x1000 21.4 / 18.6, GELU with bias 8000x1024x1024 32.6 / 29.8 and
 // 2048x2048x512 17.0 / 15.8.  One otherwise: a warp that waits for its only buffer costs 1 to 3 % (fp8 8192^3
-// 366 / 374, 4096^3 98 / 101), and SiLU is short enough for one (3000x4352x3840 80.2 / 82.7, 2048x2048x512 12.2 / 14.1).
+// 366 / 374, 4096^3 98 / 101), and SiLU is short enough for one (3000x4352x3840 79.6 / 79.9, 2048x2048x512 11.6 / 11.3,
+// 8000x1024x1024 24.8 / 24.8).
 template <int BN, int MT, int KIND, typename OutT, bool GEN, int PARTS>
 __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     gemm_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,

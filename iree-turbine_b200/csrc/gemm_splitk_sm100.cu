@@ -5,8 +5,8 @@
 // cluster compute the same 128 x BN output tile over consecutive slices of K with the same
 // TMA-fed operand ring and tcgen05 MMAs as the whole-tile kernel, then leave their fp32 partial
 // tiles in their own shared memory (in the drained ring).  After a cluster barrier every CTA sums
-// one band of 128 / split rows over all partials, in rank order, reading its peers through
-// distributed shared memory, applies the epilogue and writes the band.  No global scratch and no
+// its share of the rows that the matrix has in the tile over all partials, in rank order, reading its peers through
+// distributed shared memory, applies the epilogue and writes the share.  No global scratch and no
 // atomics: the result does not depend on timing and is reproducible bit for bit.
 //
 // CTA = 6 warps as in the whole-tile kernel: warp 0 TMA producer, warp 1 MMA issuer and owner of
@@ -23,7 +23,6 @@ using namespace gemm_detail;
 // Stand-in for an absent fp8 scale: the pointer is chosen first and the load is unconditional, so no
 // ordering of test and load can touch a null pointer.
 __device__ const float kUnitScale = 1.0f;
-
 
 template <typename OutT>
 struct ReduceCtx {
