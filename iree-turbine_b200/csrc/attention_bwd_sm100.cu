@@ -281,7 +281,7 @@ __device__ __forceinline__ void bwd_dq_cta(int block, int blocks, const CUtensor
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0 && total > 0) {
+    if (total > 0 && elect_one()) {
       mbar_arrive_expect_tx(fix_full, 2 * kOpBytes);
       load_tile_4d<HD>(smem + kOffQ, &tmap_q, fix_full, row0, head, batch);
       load_tile_4d<HD>(smem + kOffDO, &tmap_do, fix_full, row0, head, batch);
@@ -302,7 +302,7 @@ __device__ __forceinline__ void bwd_dq_cta(int block, int blocks, const CUtensor
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0 && total > 0) {
+    if (total > 0 && elect_one()) {
       // D[128 x 128] = A B^T, A (128 x HD, 16-bit pairs) in tensor memory at `a_tmem`, B a K-major tile
       auto mma_ts_k = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t b_addr) {
         const uint64_t b0 = make_desc_kmajor_sw128(b_addr);
@@ -662,7 +662,7 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0 && total > 0) {
+    if (total > 0 && elect_one()) {
       mbar_arrive_expect_tx(fix_full, 2 * kOpBytes);
       load_tile_4d<HD>(smem + kTK, &tmap_k, fix_full, row0, kvh, batch);
       load_tile_4d<HD>(smem + kTV, &tmap_v, fix_full, row0, kvh, batch);
@@ -679,7 +679,7 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0 && total > 0) {
+    if (total > 0 && elect_one()) {
       const uint32_t sk = smem_u32(smem + kTK), sv = smem_u32(smem + kTV);
       auto sq = [&](int b) { return smem_u32(smem + (b ? kTQ1 : kTQ0)); };
       auto sdo = [&](int b) { return smem_u32(smem + (b ? kTDO1 : kTDO0)); };

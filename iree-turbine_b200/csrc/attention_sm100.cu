@@ -320,11 +320,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
     if (warp == kKvWarp) {
       // ---------------- K / V producer: ring entries K_0 V_0 K_1 V_1 ... of every item ----------------
-      // Dense: lane 0 issues one box per tile and 64-column block.  Paged: one box per page and block,
+      // Dense: one lane issues one box per tile and 64-column block.  Paged: one box per page and block,
       // each page by a lane of its own, the page numbers read a tile ahead (one lane looking up and
       // issuing page after page paid the latency of a table read per page: a 4 x 512-query chunk over up
       // to 4000 keys in pages of 16 took 203 us that way).
-      const bool issuer = PAGED || lane == 0;
+      const bool issuer = PAGED || elect_one();
       if (issuer) {
         uint32_t e = 0;  // ring entries issued so far
         bool ok = true;
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           if (!got) return false;
           uint8_t* dst = smem + L::kKvOffset + stage * kTileBytes;
           uint64_t* bar = kv_full + stage;
-          if (lane == 0) mbar_arrive_expect_tx(bar, kTileBytes);
+          if (!PAGED || lane == 0) mbar_arrive_expect_tx(bar, kTileBytes);
           ++e;
           if (!PAGED) {
 #pragma unroll
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       __syncwarp();
     } else if (warp == kQWarp) {
       // ---------------- Q producer ----------------
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t ci[2] = {0, 0};  // items of each tile so far
         bool ok = true;
         ItemWalk<PAGED> walk(p, table);
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       // A K/V ring entry is released by BOTH threads (kv_empty counts two arrivals); a thread
       // that does not use an entry still waits for it to be loaded before it lets it go, so its
       // arrival can never be counted towards the stage's previous use.
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t t = (warp == kMmaWarp) ? 0u : 1u;
         // Scalar, latency-bound code in few registers: descriptors are a constant high word plus a
         // low word that is a precomputed base plus a small offset, and barriers are addressed as

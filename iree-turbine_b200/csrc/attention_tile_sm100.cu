@@ -252,11 +252,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
     if (warp == kTmaWarp) {
       // ---------------- TMA producer ----------------
-      // Dense: lane 0 issues one box per tile and 64-column block.  Paged: one box per page and block,
+      // Dense: one lane issues one box per tile and 64-column block.  Paged: one box per page and block,
       // each page by a lane of its own, and the page numbers of the next K and V tile are read a tile
       // ahead.  (One lane looking up and issuing page after page paid the latency of a table read per
       // page, 8 of them per tile at page size 16: about 3 us per 128 keys where the math needs 1.)
-      const bool issuer = PAGED || lane == 0;
+      const bool issuer = PAGED || elect_one();
       if (issuer) {
         uint32_t qc = 0, kc = 0, vc = 0;  // Q loads, K tiles, V tiles issued so far
         bool ok = true;
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         // One 128-row K or V tile (the caller has waited for the stage).  A table entry outside the pool
         // is reported and reads as zeros (the tensor map clips it).
         auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, const Item& it, int j, int page) {
-          if (lane == 0) mbar_arrive_expect_tx(bar, kTileBytes);
+          if (!PAGED || lane == 0) mbar_arrive_expect_tx(bar, kTileBytes);
           if (!PAGED) {
 #pragma unroll
             for (int db = 0; db < 2; ++db)
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             for (int jj = 0; jj < kKStages; ++jj) pages[jj] = page_of(it, jj);
           }
           if (!wait_free(q_empty, (qc & 1) ^ 1)) return false;
-          if (lane == 0) {
+          if (!PAGED || lane == 0) {
             mbar_arrive_expect_tx(q_full, kTileBytes);
 #pragma unroll
             for (int db = 0; db < 2; ++db)
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       // was busy nearly the whole step and every wait of one kind delayed the other.  The streams
       // are independent: each orders itself through barriers (score buffer taken by the softmax,
       // P written, stages loaded), never through issue order.
-      if (lane == 0) {
+      if (elect_one()) {
         // The issuing thread runs scalar, latency-bound code: descriptors are a constant high word
         // plus a low word that is a precomputed base plus a compile-time offset.
         const uint32_t hi_k = static_cast<uint32_t>(make_desc_kmajor_sw128(0) >> 32);
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       __syncwarp();
     } else if (warp == kPvWarp) {
       // ---------------- second MMAs: O (+)= P[g & 1] V_g ----------------
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t hi_mn = static_cast<uint32_t>(make_desc_mnmajor_sw128(0, kHalfTileBytes) >> 32);
         const uint32_t v_lo = static_cast<uint32_t>(make_desc_mnmajor_sw128(smem_u32(smem + kVOffset), kHalfTileBytes));
         auto desc = [](uint32_t lo, uint32_t hi) { return (static_cast<uint64_t>(hi) << 32) | lo; };

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
