@@ -9,7 +9,9 @@
 // exchanged between the two warpgroups; while one of them is busy with its exponentials the
 // tensor core works for the other one.
 //
-//   warps 0..3    softmax of query tile 0 (thread = one query row, the whole score row in registers)
+// Roles, with one softmax warpgroup per query tile (long items of head dim 64 have two, see two_groups; the others then
+// follow eight warps later):
+//   warps 0..3    softmax of query tile 0 (thread = one query row, the 64 scores of a half step in registers)
 //   warps 4..7    softmax of query tile 1
 //   warps 8..11   epilogue: O / rowsum -> global for both tiles, one item behind the others
 //   warp 12       TMA loads of K and V: one ring of kKvStages tiles, filled K_0 V_0 K_1 V_1 ...
@@ -17,6 +19,9 @@
 //   warp 14       TMA loads of Q (a thread of its own, so that waiting for a free Q buffer never
 //                 holds up K/V loads)
 //   warp 15       issues the MMAs of query tile 1 (one thread)
+// Two warpgroups of a tile take its half steps in turn: each has a score buffer of its own, reads the running max that
+// the other published early in the half step before, publishes its own, and keeps a partial row sum relative to the max
+// it last used; the epilogue brings the two sums to the last max.
 //
 // Tensor memory (512 columns x 128 lanes):  S[0] | S[1] (128 fp32 columns each) | O[0] | O[1]
 // (head-dim fp32 columns each).  A tile's 128 score columns are TWO buffers of 64: a K/V tile is
@@ -38,8 +43,8 @@
 // next item as soon as Q and K are there.  The score MMAs have N = 64, so Q is read from shared
 // memory twice per K/V tile; measured, that costs less than the waiting it removes.
 //
-// Causal items: the two tiles of a pair need a different number of KV tiles (n[0] <= n[1]); tile 0
-// simply stops taking part once it is past its diagonal.  Which CTA takes which pairs, and in what
+// Items count in half steps: a tile stops behind the last 64 keys that one of its rows sees.  Causal: the two tiles of a
+// pair need a different number (n[0] <= n[1]); tile 0 simply stops taking part once it is past its diagonal.  Which CTA takes which pairs, and in what
 // order, is in attention_order.cuh.  Couples of a heavy and a light pair (see ItemWalk) are the order of
 // large causal problems.
 //
@@ -61,16 +66,24 @@
 namespace b200k {
 namespace {
 
-constexpr int kAttnThreads = 512;
-constexpr int kKvWarp = 12;
-constexpr int kMmaWarp = 13;
-constexpr int kQWarp = 14;  // (warp 15 issues the MMAs of query tile 1)
-// Registers: 4 warps per SM sub-partition x 128 at launch = 512 per lane, redistributed.  A
-// setmaxnreg.inc beyond what the others gave up never completes.
-constexpr int kRegsSoftmax = 160;
-constexpr int kRegsEpilogue = 96;
-constexpr int kRegsOther = 96;
-static_assert(2 * kRegsSoftmax + kRegsEpilogue + kRegsOther <= 512, "setmaxnreg.inc would never complete");
+// Warps and registers by the number of softmax warpgroups that a query tile has; two take its half steps in turn.
+// Registers: warps per SM sub-partition x registers at launch, redistributed.  A setmaxnreg.inc beyond what the others
+// gave up never completes.
+template <int GROUPS>
+struct Roles {
+  static constexpr int kGroups = GROUPS;
+  static constexpr int kEpilogueWarp = 8 * kGroups;
+  static constexpr int kKvWarp = kEpilogueWarp + 4;
+  static constexpr int kMmaWarp = kKvWarp + 1;     // query tile 0
+  static constexpr int kQWarp = kKvWarp + 2;
+  static constexpr int kThreads = 32 * (kKvWarp + 4);  // (the last warp issues the MMAs of query tile 1)
+  static constexpr int kRegsAtLaunch = kGroups == 2 ? 80 : 128;
+  static constexpr int kRegsSoftmax = kGroups == 2 ? 96 : 160;
+  static constexpr int kRegsEpilogue = kGroups == 2 ? 48 : 96;
+  static constexpr int kRegsOther = kGroups == 2 ? 48 : 96;
+  static_assert(2 * kGroups * kRegsSoftmax + kRegsEpilogue + kRegsOther <= kRegsAtLaunch * kThreads / 128,
+                "setmaxnreg.inc would never complete");
+};
 constexpr int kTileRows = 128;           // query rows per tile, KV rows per tile
 constexpr int kPairRows = 2 * kTileRows;  // query rows per work item
 constexpr int kHalfTileBytes = kTileRows * 128;  // one 64-element column block of a tile: 16 KB
@@ -85,11 +98,13 @@ struct AttnSmem {
   static constexpr int kQOffset = 0;                             // two query tiles
   static constexpr int kKvOffset = 2 * kTileBytes;
   static constexpr int kStageOffset = kKvOffset + kKvStages * kTileBytes;  // epilogue staging: one 64-column block
-  static constexpr int kLsumOffset = kStageOffset + kHalfTileBytes;        // float [tile][max, sum][128 rows]
-  static constexpr int kOrderOffset = kLsumOffset + 2 * 2 * kTileRows * 4;  // uint16: item order of a paged call
+  static constexpr int kLsumOffset = kStageOffset + kHalfTileBytes;  // float [tile][warpgroup][max, sum][128 rows]
+  static constexpr int kMaxOffset = kLsumOffset + 2 * 2 * 2 * kTileRows * 4;  // float [tile][warpgroup][128 rows]: running max
+  static constexpr int kOrderOffset = kMaxOffset + 2 * 2 * kTileRows * 4;     // uint16: item order of a paged call
   static constexpr int kBarOffset = kOrderOffset + attn_order::kSortBytes;
-  // q_full[2] q_empty[2] | kv_full[4] kv_empty[4] | s_full[2][2] p_full[2][2] | o_full[2] o_free[2] | l_full[2] l_free[2] | turn[2] | pv_done[2]
-  static constexpr int kNumBars = 4 + 2 * kKvStages + 8 + 4 + 4 + 2 + 2;
+  // q_full[2] q_empty[2] | kv_full[4] kv_empty[4] | s_full[2][2] p_full[2][2] | o_full[2] o_free[2] | l_full[2] l_free[2] | turn[2] | pv_done[2] |
+  // x_full[2][2][4]
+  static constexpr int kNumBars = 4 + 2 * kKvStages + 8 + 4 + 4 + 2 + 2 + 16;
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16 + 1024;  // + slack for 1024-byte alignment
   // tensor memory columns
   static constexpr uint32_t kTmemS = 0;    // + 128 * tile; P over the first 64 columns
@@ -162,8 +177,8 @@ __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi)
 
 struct Item {
   int pair, head, batch;
-  int n[2];   // KV tiles query tile t visits (0: the tile has no rows or sees no key)
-  int nmax;   // max(n[0], n[1]): KV tiles loaded for the item
+  int n[2];   // half steps of 64 keys that query tile t visits (0: the tile has no rows or sees no key)
+  int nmax;   // KV tiles loaded for the item
   int kv_len, causal_offset;  // keys of this item's sequence; key j is visible to query i iff j <= i + causal_offset
 };
 
@@ -177,22 +192,22 @@ __device__ __forceinline__ Item make_item(int batch, int head, int pair, const A
   it.kv_len = p.seq_kv;
   if (PAGED) it.kv_len = max(0, min(p.seq_lens[it.batch], p.seq_kv));
   it.causal_offset = PAGED ? it.kv_len - p.seq_q : p.causal_offset;
-  const int kv_tiles_total = (it.kv_len + kTileRows - 1) / kTileRows;
+  const int halves_total = (it.kv_len + 63) / 64;
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
     const int r0 = pair * kPairRows + t * kTileRows;
     int n = 0;
     if (r0 < p.seq_q) {
       if (!p.causal) {
-        n = kv_tiles_total;
+        n = halves_total;
       } else {
-        const int last_col = r0 + kTileRows - 1 + it.causal_offset;
-        n = last_col < 0 ? 0 : min(last_col / kTileRows + 1, kv_tiles_total);
+        const int last_col = min(r0 + kTileRows, p.seq_q) - 1 + it.causal_offset;
+        n = last_col < 0 ? 0 : min(last_col / 64 + 1, halves_total);
       }
     }
     it.n[t] = n;
   }
-  it.nmax = max(it.n[0], it.n[1]);
+  it.nmax = (max(it.n[0], it.n[1]) + 1) / 2;
   return it;
 }
 
@@ -235,12 +250,14 @@ struct ItemWalk {
   }
 };
 
-template <typename T, int HD, bool PAGED>
-__global__ void __launch_bounds__(kAttnThreads, 1)
+template <typename T, int HD, int GROUPS, bool PAGED>
+__global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
     attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
                     const AttnParams p) {
   using L = AttnSmem<HD>;
+  using R = Roles<GROUPS>;
+  constexpr int kGroups = GROUPS;
   constexpr int kBlocks = L::kBlocks;
   constexpr int kTileBytes = L::kTileBytes;
   constexpr uint32_t kFmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBF16;
@@ -250,6 +267,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   float* lsum = reinterpret_cast<float*>(smem + L::kLsumOffset);
+  float* xmax = reinterpret_cast<float*>(smem + L::kMaxOffset);
   uint16_t* table = reinterpret_cast<uint16_t*>(smem + L::kOrderOffset);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOffset);
   uint64_t* q_full = bars;            // [tile] Q tile loaded
@@ -264,6 +282,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   uint64_t* l_free = l_full + 2;            // [tile] ... and read
   uint64_t* turn = l_free + 2;              // [tile] it is this tile's turn to put MMAs into the pipe
   uint64_t* pv_done = turn + 2;             // [tile] one completion per PV group (only waited for before a rescale of O)
+  uint64_t* x_full = pv_done + 2;           // [tile][warpgroup][quarter] running max after a half step published (two warpgroups)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::kNumBars);
   volatile uint32_t* abort_word = tmem_slot + 1;
 
@@ -281,7 +300,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       mbar_init(pv_done + t, 1);
       mbar_init(o_full + t, 1);
       mbar_init(o_free + t, 4);
-      mbar_init(l_full + t, 4);
+      mbar_init(l_full + t, 4 * kGroups);
+      for (int i = 0; i < 8; ++i) mbar_init(x_full + 8 * t + i, 1);
       mbar_init(l_free + t, 4);
       mbar_init(turn + t, 1);
     }
@@ -297,7 +317,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     prefetch_tmap(&tmap_v);
     prefetch_tmap(&tmap_o);
   }
-  if (warp == kMmaWarp) {
+  if (warp == R::kMmaWarp) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
@@ -316,11 +336,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     });
   }
 
-  if (warp >= 12) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-    if (warp == kKvWarp) {
+  if (warp >= R::kKvWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R::kRegsOther));
+    if (warp == R::kKvWarp) {
       // ---------------- K / V producer: ring entries K_0 V_0 K_1 V_1 ... of every item ----------------
-      // Dense: one lane issues one box per tile and 64-column block.  Paged: one box per page and block,
+      // Dense: lane 0 issues one box per tile and 64-column block.  Paged: one box per page and block,
       // each page by a lane of its own, the page numbers read a tile ahead (one lane looking up and
       // issuing page after page paid the latency of a table read per page: a 4 x 512-query chunk over up
       // to 4000 keys in pages of 16 took 203 us that way).
@@ -375,7 +395,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         }
       }
       __syncwarp();
-    } else if (warp == kQWarp) {
+    } else if (warp == R::kQWarp) {
       // ---------------- Q producer ----------------
       if (elect_one()) {
         uint32_t ci[2] = {0, 0};  // items of each tile so far
@@ -413,7 +433,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       }
       __syncwarp();
     } else {
-      // ---------------- MMA issue: warp 13 for query tile 0, warp 15 for query tile 1 ----------------
+      // ---------------- MMA issue: one warp per query tile ----------------
       // One thread per query tile, each with its own in-order stream
       //     wait P(h) : O += P(h) V[half h] : S(h + 2) : ...      (half steps of 64 keys)
       // so neither tile ever waits behind the other's barriers, and a tile that is done with an
@@ -424,7 +444,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       // that does not use an entry still waits for it to be loaded before it lets it go, so its
       // arrival can never be counted towards the stage's previous use.
       if (elect_one()) {
-        const uint32_t t = (warp == kMmaWarp) ? 0u : 1u;
+        const uint32_t t = (warp == R::kMmaWarp) ? 0u : 1u;
         // Scalar, latency-bound code in few registers: descriptors are a constant high word plus a
         // low word that is a precomputed base plus a small offset, and barriers are addressed as
         // one 32-bit base plus an index.
@@ -447,22 +467,22 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         auto commit = [&](uint32_t index) { umma_commit_addr(bar0 + 8 * index); };
         auto wait_entry = [&](uint32_t e) { return wait(kKvFull + e % kKvStages, (e / kKvStages) & 1); };
         auto free_entry = [&](uint32_t e) { commit(kKvEmpty + e % kKvStages); };  // arrives once this thread's MMAs are done
-        // S(half hb) = Q (K rows 64 hb .. 64 hb + 63 of ring entry e)^T, into columns 64 hb .. of the tile's score region
-        auto issue_scores = [&](uint32_t e, uint32_t hb) {
+        // S = Q (K rows 64 hb .. 64 hb + 63 of ring entry e)^T, into score buffer `buf` of the tile
+        auto issue_scores = [&](uint32_t e, uint32_t hb, uint32_t buf) {
           const uint32_t b0 = k_lo + (e % kKvStages) * (kTileBytes >> 4) + hb * (8192u >> 4);
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks) {  // k-steps of 16 over the head dimension (64-wide blocks)
             const uint32_t off = (ks >> 2) * (kHalfTileBytes >> 4) + 2 * (ks & 3);
-            umma_f16_ss(tmem_s + hb * 64, desc(q_lo + off, hi_k), desc(b0 + off, hi_k), kIdescS, ks > 0 ? 1u : 0u);
+            umma_f16_ss(tmem_s + buf * 64, desc(q_lo + off, hi_k), desc(b0 + off, hi_k), kIdescS, ks > 0 ? 1u : 0u);
           }
-          commit(kSFull + 2 * t + hb);
+          commit(kSFull + 2 * t + buf);
         };
-        // O (+)= P(half hb) V rows 64 hb .. of ring entry e: 4 k-steps of 16 KV rows; A = P from tensor memory
-        auto issue_pv = [&](uint32_t e, uint32_t hb, uint32_t accumulate) {
+        // O (+)= P(buffer buf) V rows 64 hb .. of ring entry e: 4 k-steps of 16 KV rows; A = P from tensor memory
+        auto issue_pv = [&](uint32_t e, uint32_t hb, uint32_t buf, uint32_t accumulate) {
           const uint32_t b0 = v_lo + (e % kKvStages) * (kTileBytes >> 4) + hb * (4u * (2048u >> 4));
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks)
-            umma_f16_ts(tmem_o, tmem_s + hb * 64 + ks * 8, desc(b0 + ks * (2048 >> 4), hi_mn), kIdescPV,
+            umma_f16_ts(tmem_o, tmem_s + buf * 64 + ks * 8, desc(b0 + ks * (2048 >> 4), hi_mn), kIdescPV,
                         ks > 0 ? 1u : accumulate);
           commit(kPvDone + t);
         };
@@ -496,9 +516,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             if (!wait(kQFull + t, cq & 1u)) break;
             ++cq;
             tc_fence_after();
-            issue_scores(e0, 0);
-            issue_scores(e0, 1);
-            if (n == 1) commit(kQEmpty + t);
+            issue_scores(e0, 0, ch & 1u);
+            if (n > 1) issue_scores(e0, 1, (ch & 1u) ^ 1u);
+            if (n <= 2) commit(kQEmpty + t);
           }
           free_entry(e0);
           for (int j = 0; j < nmax && ok; ++j) {
@@ -510,27 +530,30 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
 #pragma unroll
             for (uint32_t hb = 0; hb < 2; ++hb) {
               if (!take_turn()) { ok = false; break; }
-              if (j < n) {
-                if (j == 0 && hb == 0) {  // the accumulator is read by the epilogue of the tile's previous item
+              const int h = 2 * j + static_cast<int>(hb);
+              if (h < n) {
+                const uint32_t buf = ch & 1u;
+                if (h == 0) {  // the accumulator is read by the epilogue of the tile's previous item
                   if (!wait(kOFree + t, (co & 1u) ^ 1u)) { ok = false; break; }
                   ++co;
                 }
-                if (!wait(kPFull + 2 * t + hb, (ch >> 1) & 1u)) { ok = false; break; }
+                if (!wait(kPFull + 2 * t + buf, (ch >> 1) & 1u)) { ok = false; break; }
                 ++ch;
                 tc_fence_after();
-                issue_pv(ev, hb, (j > 0 || hb > 0) ? 1u : 0u);
-                pass_turn();
-                if (more && j + 1 < n) {
-                  issue_scores(ev + 1, hb);  // over the probabilities the PV group above has just been issued for
-                  if (j + 2 == n && hb == 1) commit(kQEmpty + t);  // that was the item's last score MMA of this tile
+                issue_pv(ev, hb, buf, h > 0 ? 1u : 0u);
+                if (kGroups == 1) pass_turn();
+                if (h + 2 < n) {
+                  issue_scores(ev + 1, hb, buf);  // over the probabilities the PV group above has just been issued for
+                  if (h + 3 == n) commit(kQEmpty + t);  // that was the item's last score MMA of this tile
                 }
-                if (j == n - 1 && hb == 1) commit(kOFull + t);
+                if (kGroups == 2) pass_turn();
+                if (h == n - 1) commit(kOFull + t);
               } else {
                 pass_turn();  // past this tile's diagonal
               }
             }
             if (!ok) break;
-            if (j < n) {
+            if (2 * j < n) {
               free_entry(ev);
               if (more) free_entry(ev + 1);
             } else {
@@ -544,16 +567,17 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       }
       __syncwarp();
     }
-  } else if (warp >= 8) {
+  } else if (warp >= R::kEpilogueWarp) {
     // ---------------- epilogue: O / rowsum -> global, one item behind ----------------
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R::kRegsEpilogue));
     const int quarter = warp & 3;
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t lane_field = static_cast<uint32_t>(quarter * 32) << 16;
     uint8_t* stage = smem + L::kStageOffset;
-    const bool store_thread = (warp == 8 && lane == 0);
+    const bool store_thread = (warp == R::kEpilogueWarp && lane == 0);
     auto epi_barrier = [&]() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-    uint32_t ci[2] = {0, 0};  // items with work per tile so far
+    uint32_t ci[2] = {0, 0};     // items with work per tile so far
+    uint32_t steps[2] = {0, 0};  // half steps per tile before the current item
     bool ok = true;
     ItemWalk<PAGED> walk(p, table);
     Item it;
@@ -581,8 +605,18 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         ok = bar_red_and(1, 128, ok);
         if (!ok) break;
         tc_fence_after();
-        const float m = lsum[(t * 2 + 0) * kTileRows + row_in_tile];
-        const float l = lsum[(t * 2 + 1) * kTileRows + row_in_tile];
+        const float* sums = lsum + t * 4 * kTileRows + row_in_tile;
+        float m = sums[0], l = sums[kTileRows];
+        if (HD == 64) {
+          // The sums of even and odd half steps, brought to the larger (that is the last) running max.  A warpgroup of
+          // two has the even ones where it took the item's first half step.
+          const int g0 = kGroups == 2 ? steps[t] & 1u : 0;
+          const float m0 = sums[g0 * 2 * kTileRows], l0 = sums[(g0 * 2 + 1) * kTileRows];
+          const float m1 = sums[(g0 ^ 1) * 2 * kTileRows], l1 = sums[((g0 ^ 1) * 2 + 1) * kTileRows];
+          m = fmaxf(m0, m1);
+          l = (m0 == -INFINITY ? 0.f : l0 * ex2(m0 - m)) + (m1 == -INFINITY ? 0.f : l1 * ex2(m1 - m));
+          steps[t] += it.n[t];
+        }
         const float inv = (l > 0.f) ? 1.0f / l : 0.f;
         if (p.lse && q_row < p.seq_q) {
           // m is in the log2 domain (scores times scale * log2 e), l is relative to it
@@ -596,19 +630,19 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           if (store_thread) tma_store_wait_read<0>();
           epi_barrier();
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
-            uint32_t r[32];
-            tmem_ld_32x32b_x32(t_o + (c2 * 2 + cc) * 32, r);
+          for (int cc = 0; cc < 4; ++cc) {
+            uint32_t r[16];
+            tmem_ld_32x32b_x16(t_o + (c2 * 4 + cc) * 16, r);
             tmem_wait_ld();
             uint8_t* blk = stage + row_in_tile * 128;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
+            for (int v = 0; v < 2; ++v) {
               uint4 u;
               u.x = pack_pair<T>(__uint_as_float(r[8 * v + 0]) * inv, __uint_as_float(r[8 * v + 1]) * inv);
               u.y = pack_pair<T>(__uint_as_float(r[8 * v + 2]) * inv, __uint_as_float(r[8 * v + 3]) * inv);
               u.z = pack_pair<T>(__uint_as_float(r[8 * v + 4]) * inv, __uint_as_float(r[8 * v + 5]) * inv);
               u.w = pack_pair<T>(__uint_as_float(r[8 * v + 6]) * inv, __uint_as_float(r[8 * v + 7]) * inv);
-              const int chunk = cc * 4 + v;
+              const int chunk = cc * 2 + v;
               *reinterpret_cast<uint4*>(blk + ((chunk ^ (row_in_tile & 7)) << 4)) = u;
             }
           }
@@ -632,17 +666,22 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     }
     if (store_thread) tma_store_wait_read<0>();
   } else {
-    // ---------------- softmax of query tile t = warp / 4 ----------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
-    const int t = warp >> 2;
+    // ---------------- softmax of query tile t = warp / 8: with two warpgroups the half steps of parity w ----------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R::kRegsSoftmax));
+    const int t = warp / (4 * kGroups);
+    const int w = kGroups == 2 ? (warp >> 2) & 1 : 0;
     const int quarter = warp & 3;
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t lane_field = static_cast<uint32_t>(quarter * 32) << 16;
-    const uint32_t t_s = tmem_base + lane_field + L::kTmemS + t * 128;  // scores, and P over their first half
+    const uint32_t t_s = tmem_base + lane_field + L::kTmemS + t * 128;  // scores [buffer], and P over their first half
     const uint32_t t_o = tmem_base + lane_field + L::kTmemO + t * HD;
+    [[maybe_unused]] float* m_mine = xmax + (2 * t + w) * kTileRows + row_in_tile;
+    [[maybe_unused]] const float* m_theirs = xmax + (2 * t + (w ^ 1)) * kTileRows + row_in_tile;
+    [[maybe_unused]] uint64_t* x_mine = x_full + (2 * t + w) * 4 + quarter;
+    [[maybe_unused]] uint64_t* x_theirs = x_full + (2 * t + (w ^ 1)) * 4 + quarter;
     const float scale_log2 = p.scale_log2;
     const float2 scale2 = make_float2(scale_log2, scale_log2);
-    uint32_t cs = 0, ci = 0;  // score tiles and items of this query tile so far
+    uint32_t cs = 0, ci = 0;  // half steps (of both warpgroups) and items of this query tile so far
     bool ok = true;
     ItemWalk<PAGED> walk(p, table);
     Item it;
@@ -653,16 +692,28 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       const int q_row = tile_r0 + row_in_tile;
       const int kv_len = it.kv_len;
       const int causal_offset = it.causal_offset;
-      float m_ref = -INFINITY;  // the max the row's P and running sum are relative to
+      float m_ref = -INFINITY;  // the max the running sum is relative to
       float2 l2 = make_float2(0.f, 0.f);
-      for (int h = 0; h < 2 * n; ++h, ++cs) {  // half steps of 64 keys, alternating between the two score buffers
-        const uint32_t hb = cs & 1u;
-        ok = mbar_wait(s_full + 2 * t + hb, (cs >> 1) & 1u, abort_word);
+      // Head dim 64 with one warpgroup: the other half steps' max and sum, kept apart and exchanged after each step, so that
+      // the result has the bits of two warpgroups (a paged call and the dense one of the same keys may differ in their number).
+      float m_other = -INFINITY;
+      float2 l2_other = make_float2(0.f, 0.f);
+      const uint32_t first = cs;
+      cs += n;
+      for (int h = kGroups == 2 ? (first ^ w) & 1u : 0; h < n; h += kGroups) {  // half steps of 64 keys
+        const uint32_t g = first + h;
+        const uint32_t buf = kGroups == 2 ? w : g & 1u;  // score buffer
+        ok = mbar_wait(s_full + 2 * t + buf, (g >> 1) & 1u, abort_word);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
         uint32_t sr[64];
-        tmem_ld_32x32b_x64(t_s + hb * 64, sr);
+        if (kGroups == 2) {  // (one instruction of 64 does not fit the registers at launch)
+          tmem_ld_32x32b_x32(t_s + buf * 64, *reinterpret_cast<uint32_t(*)[32]>(sr));
+          tmem_ld_32x32b_x32(t_s + buf * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(sr + 32));
+        } else {
+          tmem_ld_32x32b_x64(t_s + buf * 64, sr);
+        }
 
         const int col0 = h * 64;
         const bool need_mask = (p.causal && col0 + 63 > tile_r0 + causal_offset) || (col0 + 64 > kv_len);
@@ -687,17 +738,40 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           mx3 = fmax3(mx3, __uint_as_float(sr[i + 6]), __uint_as_float(sr[i + 7]));
         }
         const float m_new = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * scale_log2;
-        const bool grow = m_new > m_ref + kRescaleThreshold;  // also true for the first finite max
+        float m_prev = HD == 64 ? m_other : m_ref;
+        if (kGroups == 2) {
+          // The running max after the previous half step, published by the other warpgroup early in it.  Every
+          // phase is observed, also when the value is not needed (first half step of an item).
+          m_prev = -INFINITY;
+          if (g > 0) {
+            ok = mbar_wait(x_theirs, ((g - 1) >> 1) & 1u, abort_word);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            if (h > 0) m_prev = *m_theirs;
+          }
+        }
+        const bool grow = m_new > m_prev + kRescaleThreshold;  // also true for the first finite max
+        const float m_cur = grow ? m_new : m_prev;
+        if (kGroups == 2) {
+          *m_mine = m_cur;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(x_mine);
+        }
+        if (HD == 64 && m_prev != m_ref) {  // m_prev > m_ref: a half step of the other parity raised it
+          const float a = ex2(m_ref - m_prev);  // m_ref = -inf gives 0 (and the sum is 0 then)
+          l2.x *= a;
+          l2.y *= a;
+        }
         if (h > 0 && __any_sync(0xffffffffu, grow)) {
-          // Rescale O in place.  The PV group of the previous half step may still be running (the
-          // scores read above were issued before it): wait for its completion, the cs-th of this
-          // tile.  The next group waits for p_full below.  Rare after the first steps of an item:
-          // the max must grow by 2^8.
-          ok = mbar_wait(pv_done + t, (cs - 1u) & 1u, abort_word);
+          // Rescale O between "O += P V" of the previous half step, which may still be running (the scores read
+          // above were issued before it), and this one's, which waits for p_full below.  Rare after the first
+          // steps of an item: the max must grow by 2^8.
+          float alpha = 1.f;
+          if (grow) alpha = ex2(m_prev - m_new);  // m_prev = -inf gives 0
+          ok = mbar_wait(pv_done + t, (g - 1u) & 1u, abort_word);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
-          const float alpha = grow ? ex2(m_ref - m_new) : 1.f;  // m_ref = -inf gives 0
 #pragma unroll 1
           for (int c = 0; c < HD / 16; ++c) {
             uint32_t r[16];
@@ -710,8 +784,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           l2.x *= alpha;
           l2.y *= alpha;
         }
-        if (grow) m_ref = m_new;
-        const float m_sub = (m_ref == -INFINITY) ? 0.f : m_ref;
+        m_ref = m_cur;
+        const float m_sub = (m_cur == -INFINITY) ? 0.f : m_cur;
         const float2 negm2 = make_float2(-m_sub, -m_sub);
 
         // probabilities -> tensor memory (16-bit pairs) over the first half of the scores they came
@@ -727,21 +801,37 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             l2 = fadd2(l2, e);
             pk[i] = pack_pair<T>(e.x, e.y);
           }
-          tmem_st_32x32b_x16(t_s + hb * 64 + c * 16, pk);
+          tmem_st_32x32b_x16(t_s + buf * 64 + c * 16, pk);
         }
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full + 2 * t + hb);
+        if (lane == 0) mbar_arrive(p_full + 2 * t + buf);
+        if (HD == 64 && kGroups == 1) {
+          const float m = m_ref;
+          m_ref = m_other;
+          m_other = m;
+          const float2 l = l2;
+          l2 = l2_other;
+          l2_other = l;
+        }
       }
       if (!ok) break;
-      // hand (max, sum) of the item to the epilogue warps
+      // hand (max, sum) of this warpgroup's half steps to the epilogue warps
       ok = mbar_wait(l_free + t, (ci & 1) ^ 1, abort_word);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       ++ci;
-      lsum[(t * 2 + 0) * kTileRows + row_in_tile] = m_ref;
-      lsum[(t * 2 + 1) * kTileRows + row_in_tile] = l2.x + l2.y;
+      if (HD == 64 && kGroups == 1) {  // (m_ref, l2) belong to the half steps of n's parity
+        const int own = n & 1;
+        lsum[((t * 2 + own) * 2 + 0) * kTileRows + row_in_tile] = m_ref;
+        lsum[((t * 2 + own) * 2 + 1) * kTileRows + row_in_tile] = l2.x + l2.y;
+        lsum[((t * 2 + (own ^ 1)) * 2 + 0) * kTileRows + row_in_tile] = m_other;
+        lsum[((t * 2 + (own ^ 1)) * 2 + 1) * kTileRows + row_in_tile] = l2_other.x + l2_other.y;
+      } else {
+        lsum[((t * 2 + w) * 2 + 0) * kTileRows + row_in_tile] = m_ref;
+        lsum[((t * 2 + w) * 2 + 1) * kTileRows + row_in_tile] = l2.x + l2.y;
+      }
       __syncwarp();
       if (lane == 0) mbar_arrive(l_full + t);
     }
@@ -757,16 +847,16 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     if (threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusAttnTimeout);
     __syncthreads();
   }
-  if (warp == kMmaWarp) {
+  if (warp == R::kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
 }
 
-template <typename T, int HD, bool PAGED>
+template <typename T, int HD, int GROUPS, bool PAGED>
 int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
                  const AttnParams& p, cudaStream_t stream) {
-  auto kfn = attn_fwd_kernel<T, HD, PAGED>;
+  auto kfn = attn_fwd_kernel<T, HD, GROUPS, PAGED>;
   static bool configured[64] = {};  // per instantiation and device ordinal
   int rc = ensure_dynamic_smem(kfn, AttnSmem<HD>::kTotal, configured, "cudaFuncSetAttribute(attention smem)");
   if (rc) return rc;
@@ -774,18 +864,34 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   const int grid = p.order.num_items < sms ? p.order.num_items : sms;
   // Launched early only when short, see the one-tile kernel.
   const int64_t tiles = static_cast<int64_t>(p.order.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
-  return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(kAttnThreads), AttnSmem<HD>::kTotal, stream, tq, tk, tv, to, p);
+  return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(Roles<GROUPS>::kThreads), AttnSmem<HD>::kTotal, stream, tq, tk, tv, to, p);
+}
+
+// Two softmax warpgroups per query tile at head dim 64: it spends half as many tensor cycles per exponential as 128
+// does, so in a long item the exponentials are what a tile waits for, and two warps per tile and SM sub-partition get
+// through them in fewer cycles (545 per 64 columns and warp, 640 with one).  Short items pay for the hand-over of the
+// running max and for 256 more threads.  One / two, us: 4x8x2048 63.1 / 58.8, 4x32x2048 215 / 195, 1x2x8192 causal 108.5 /
+// 102.6, 2x4(1) 300 over 3000 45.1 / 41.8, paged 4x32(8) 512 over up to 4000 77.4 / 72.3; 16x16x1024 causal 79.6 / 85.9,
+// 32x8x384 30.9 / 33.5, 32x8x128 causal 10.3 / 11.2, 8x8 3000 over 200 34.7 / 37.1.  The line is a mean of 1536 keys per query.
+// Head dim 128, which waits for its score MMAs, is slower with two (4x32x4096 causal 468 / 517): more warps compete with
+// the MMA threads for issue slots.
+bool two_groups(const AttnParams& p) {
+  return 2 * static_cast<int64_t>(p.seq_kv) - (p.causal ? p.seq_q : 0) >= 2 * 1536;
 }
 
 template <bool PAGED>
 int launch_any(int dtype, int head_dim, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                const CUtensorMap& to, const AttnParams& p, cudaStream_t stream) {
   if (head_dim == 128) {
-    if (dtype == B200K_F16) return launch_typed<__half, 128, PAGED>(tq, tk, tv, to, p, stream);
-    return launch_typed<__nv_bfloat16, 128, PAGED>(tq, tk, tv, to, p, stream);
+    if (dtype == B200K_F16) return launch_typed<__half, 128, 1, PAGED>(tq, tk, tv, to, p, stream);
+    return launch_typed<__nv_bfloat16, 128, 1, PAGED>(tq, tk, tv, to, p, stream);
   }
-  if (dtype == B200K_F16) return launch_typed<__half, 64, PAGED>(tq, tk, tv, to, p, stream);
-  return launch_typed<__nv_bfloat16, 64, PAGED>(tq, tk, tv, to, p, stream);
+  if (two_groups(p)) {
+    if (dtype == B200K_F16) return launch_typed<__half, 64, 2, PAGED>(tq, tk, tv, to, p, stream);
+    return launch_typed<__nv_bfloat16, 64, 2, PAGED>(tq, tk, tv, to, p, stream);
+  }
+  if (dtype == B200K_F16) return launch_typed<__half, 64, 1, PAGED>(tq, tk, tv, to, p, stream);
+  return launch_typed<__nv_bfloat16, 64, 1, PAGED>(tq, tk, tv, to, p, stream);
 }
 
 // Causal couples fill the rounds over the SMs to 95 % or more: they are the better order then.
@@ -809,27 +915,37 @@ int fill_pair_order(AttnParams& p, const char* who, int head_dim, bool paged) {
 }
 
 // Which kernel runs a problem (B200K_ATTN_AUTO); head dim 64 exists in the pair kernel only.  Measured at
-// head dim 128, one-tile / tile-pair, us.  Non-causal: 8x32x1024 128 / 134, 8x32x2048 472 / 473, 4x32x4096
-// 992 / 1030: the one-tile kernel.  Causal, couples that fill their rounds: 4x32x4096 527 / 507,
-// 1x32(8)x16384 1814 / 1788, 16x64x512 168 / 137, 2x64x5000 802 / 762 (32x32x256 70 / 72): the pair kernel.
-// Other causal problems, with the pair kernel in its better order: 2x32(8)x2000 84 / 87, 4x8x4096 137 / 142,
-// 1x4x16384 240 / 259, 16x16(4)x1024 101 / 106, 1x64(8)x6000 510 / 538 (4x4(1)x4096 78 / 75): the one-tile kernel.
+// head dim 128, one-tile / tile-pair, us.  Without a mask all items cost the same and a pair takes 1.9 times as long as a
+// tile, so the rounds over the SMs decide: 8x32x1024 (14 / 7 rounds) 129 / 127, 4x16x4096 (14 / 7) 537 / 515, 1x16x4096
+// (4 / 2) 161 / 147, 1x8x8192 (4 / 2) 292 / 265, 4x32(8)x512 (4 / 2) 25.7 / 24.8, but 2x16x4096 (7 / 4) 287 / 308,
+// 1x8x2048 (1 / 1) 25 / 39, 24x64x308 (32 / 21) 133 / 165; over one or two tiles of keys the one-tile kernel is ahead all the
+// same (8x16x200, 2 / 1, 12.4 / 12.9; 16x16x256, 4 / 2, 17.5 / 17.7).
+// Causal, couples that fill their rounds: 4x32x4096 571 / 542, 8x32x2048 321 / 300, 16x64x512 145 / 114, 32x32x256
+// 72 / 64: the pair kernel.  Other causal problems, with the pair kernel in its better order: 2x32(8)x2000 86 / 89,
+// 4x8x4096 144 / 143, 16x16(4)x1024 93 / 98, 1x64(8)x6000 553 / 565, 1x4x8192 93 / 150, 1x32(8)x1200 23 / 27: the
+// one-tile kernel.
 bool choose_pair_kernel(const b200k_attention_args& a) {
   if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
-  if (a.kernel == B200K_ATTN_ONE_TILE || !a.causal) return false;
-  return couples_fill(static_cast<int64_t>(a.batch) * a.q_heads, a.seq_q);
+  if (a.kernel == B200K_ATTN_ONE_TILE) return false;
+  const int64_t heads = static_cast<int64_t>(a.batch) * a.q_heads, sms = num_sms();
+  if (a.causal) return couples_fill(heads, a.seq_q);
+  const int64_t tiles = heads * ((a.seq_q + kTileRows - 1) / kTileRows), pairs = heads * ((a.seq_q + kPairRows - 1) / kPairRows);
+  const int64_t tile_rounds = (tiles + sms - 1) / sms, pair_rounds = (pairs + sms - 1) / sms;
+  return a.seq_kv > 2 * kTileRows && pair_rounds * 19 <= tile_rounds * 10;
 }
 
 // Paged: a K/V tile arrives page by page, and the pair kernel needs half as many tiles.  One-tile / tile-pair,
 // us: 4x32(8) 512 queries over up to 4000 keys 156 / 87 at page size 16, 114 / 95 at 64, 107 / 95 at 128;
 // 3x64(16) 1000 over 2000 170 / 146.  The one-tile kernel is ahead where the SMs are not filled and pages are
 // larger (1x8 2000 over 6000 81 / 98 at page size 32, 71 / 98 at 64, but 1x8 64 over 6000 at 16 96 / 81), and where
-// a pair would be half empty (16x16(4) 100 over 3000, page size 64, 45 / 54).
+// a pair would be half empty (16x16(4) 100 over 3000, page size 64, 39 / 41), or the longest pairs decide (8x4(1) 1000 over
+// up to 4000, page size 64, 128 pairs, 50 / 64).
 bool choose_pair_kernel(const b200k_paged_attention_args& a) {
   if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
   if (a.kernel == B200K_ATTN_ONE_TILE) return false;
-  const int64_t items = static_cast<int64_t>(a.batch) * a.q_heads * ((a.seq_q + kTileRows - 1) / kTileRows);
-  return !((a.page_size >= 32 && items <= num_sms()) || (a.page_size >= 64 && a.seq_q <= kTileRows));
+  const int64_t heads = static_cast<int64_t>(a.batch) * a.q_heads;
+  const int64_t tiles = heads * ((a.seq_q + kTileRows - 1) / kTileRows), pairs = heads * ((a.seq_q + kPairRows - 1) / kPairRows);
+  return !((a.page_size >= 32 && tiles <= num_sms()) || (a.page_size >= 64 && (a.seq_q <= kTileRows || pairs <= num_sms())));
 }
 
 }  // namespace
