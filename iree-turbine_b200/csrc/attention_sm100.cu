@@ -915,23 +915,19 @@ int fill_pair_order(AttnParams& p, const char* who, int head_dim, bool paged) {
 }
 
 // Which kernel runs a problem (B200K_ATTN_AUTO); head dim 64 exists in the pair kernel only.  Measured at
-// head dim 128, one-tile / tile-pair, us.  Without a mask all items cost the same and a pair takes 1.9 times as long as a
-// tile, so the rounds over the SMs decide: 8x32x1024 (14 / 7 rounds) 129 / 127, 4x16x4096 (14 / 7) 537 / 515, 1x16x4096
-// (4 / 2) 161 / 147, 1x8x8192 (4 / 2) 292 / 265, 4x32(8)x512 (4 / 2) 25.7 / 24.8, but 2x16x4096 (7 / 4) 287 / 308,
-// 1x8x2048 (1 / 1) 25 / 39, 24x64x308 (32 / 21) 133 / 165; over one or two tiles of keys the one-tile kernel is ahead all the
-// same (8x16x200, 2 / 1, 12.4 / 12.9; 16x16x256, 4 / 2, 17.5 / 17.7).
+// head dim 128, one-tile / tile-pair, us.
+// Without a mask the one-tile kernel, whatever the batch: the two round probabilities against another running max, and a
+// choice by how the items fill the SMs would let a head's bits depend on the heads beside it.  What that choice would
+// give where pairs need half the rounds: 8x32x1024 129 / 127, 4x16x4096 537 / 515, 4x32(8)x512 25.7 / 24.8; elsewhere
+// pairs are slower: 2x16x4096 287 / 308, 1x8x2048 25 / 39, 24x64x308 133 / 165.
 // Causal, couples that fill their rounds: 4x32x4096 571 / 542, 8x32x2048 321 / 300, 16x64x512 145 / 114, 32x32x256
 // 72 / 64: the pair kernel.  Other causal problems, with the pair kernel in its better order: 2x32(8)x2000 86 / 89,
 // 4x8x4096 144 / 143, 16x16(4)x1024 93 / 98, 1x64(8)x6000 553 / 565, 1x4x8192 93 / 150, 1x32(8)x1200 23 / 27: the
 // one-tile kernel.
 bool choose_pair_kernel(const b200k_attention_args& a) {
   if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
-  if (a.kernel == B200K_ATTN_ONE_TILE) return false;
-  const int64_t heads = static_cast<int64_t>(a.batch) * a.q_heads, sms = num_sms();
-  if (a.causal) return couples_fill(heads, a.seq_q);
-  const int64_t tiles = heads * ((a.seq_q + kTileRows - 1) / kTileRows), pairs = heads * ((a.seq_q + kPairRows - 1) / kPairRows);
-  const int64_t tile_rounds = (tiles + sms - 1) / sms, pair_rounds = (pairs + sms - 1) / sms;
-  return a.seq_kv > 2 * kTileRows && pair_rounds * 19 <= tile_rounds * 10;
+  if (a.kernel == B200K_ATTN_ONE_TILE || !a.causal) return false;
+  return couples_fill(static_cast<int64_t>(a.batch) * a.q_heads, a.seq_q);
 }
 
 // Paged: a K/V tile arrives page by page, and the pair kernel needs half as many tiles.  One-tile / tile-pair,
