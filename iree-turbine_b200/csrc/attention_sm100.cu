@@ -613,8 +613,9 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
           const int g0 = kGroups == 2 ? steps[t] & 1u : 0;
           const float m0 = sums[g0 * 2 * kTileRows], l0 = sums[(g0 * 2 + 1) * kTileRows];
           const float m1 = sums[(g0 ^ 1) * 2 * kTileRows], l1 = sums[((g0 ^ 1) * 2 + 1) * kTileRows];
+          // A max of -inf comes with a sum of zero, or of NaN where all scores were NaN (the max passes them over).
           m = fmaxf(m0, m1);
-          l = (m0 == -INFINITY ? 0.f : l0 * ex2(m0 - m)) + (m1 == -INFINITY ? 0.f : l1 * ex2(m1 - m));
+          l = (m0 == -INFINITY ? l0 : l0 * ex2(m0 - m)) + (m1 == -INFINITY ? l1 : l1 * ex2(m1 - m));
           steps[t] += it.n[t];
         }
         const float inv = (l > 0.f) ? 1.0f / l : 0.f;

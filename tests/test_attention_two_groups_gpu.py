@@ -52,6 +52,20 @@ def test_dense(b, h, hkv, sq, skv, causal, dtype, ramp):
     assert tb.device_status() == 0
 
 
+@pytest.mark.parametrize("skv", [64, 100, 128, 129, 300, 1700])
+@pytest.mark.parametrize("first,last", [(0, 64), (64, 128), (0, 10000), (10, 11)])
+def test_nan_keys(skv, first, last):
+    """A NaN among the keys reaches output and statistic of every row, whichever half steps it is in."""
+    q, k, v = (normal((1, 2, s, 64), i, torch.bfloat16) for i, s in enumerate((5, skv, skv)))
+    k[:, :, first:last] = float("nan")
+    out, lse = torch.ops.b200k.attention_lse(q, k, v, 0.1, False)
+    if first < skv:
+        assert bool(out.isnan().all()) and not bool(lse.isfinite().any())
+    else:
+        assert bool(out.isfinite().all()) and bool(lse.isfinite().all())
+    assert tb.device_status() == 0
+
+
 @pytest.mark.parametrize("page", [16, 128])
 def test_paged(page):
     lens, sq, h, hkv = [3000, 65, 0, 1601, 2990], 200, 4, 2
