@@ -876,7 +876,13 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
 // 32x8x384 30.9 / 33.5, 32x8x128 causal 10.3 / 11.2, 8x8 3000 over 200 34.7 / 37.1.  The line is a mean of 1536 keys per query.
 // Head dim 128, which waits for its score MMAs, is slower with two (4x32x4096 causal 468 / 517): more warps compete with
 // the MMA threads for issue slots.
+// Paged: the lengths are device data.  The capacity of the table says nothing about them (a first chunk of 300 queries in
+// tables for 8192, 8x32(8): 24.7 / 28.7; 512: 33.3 / 36.9; 1200: 35.0 / 36.9), but a sequence has at least its queries:
+// from 1536 of them on, two are no slower even where those are all its keys (8x32(8) 1500 147.5 / 146.0, 8x8 47.1 / 47.0).
+// Fewer queries over long histories could gain (8x8 512 over 3000 51.1 / 46.7), but nothing here tells them from short ones.
+template <bool PAGED>
 bool two_groups(const AttnParams& p) {
+  if (PAGED && p.seq_q < 1536) return false;
   return 2 * static_cast<int64_t>(p.seq_kv) - (p.causal ? p.seq_q : 0) >= 2 * 1536;
 }
 
@@ -887,7 +893,7 @@ int launch_any(int dtype, int head_dim, const CUtensorMap& tq, const CUtensorMap
     if (dtype == B200K_F16) return launch_typed<__half, 128, 1, PAGED>(tq, tk, tv, to, p, stream);
     return launch_typed<__nv_bfloat16, 128, 1, PAGED>(tq, tk, tv, to, p, stream);
   }
-  if (two_groups(p)) {
+  if (two_groups<PAGED>(p)) {
     if (dtype == B200K_F16) return launch_typed<__half, 64, 2, PAGED>(tq, tk, tv, to, p, stream);
     return launch_typed<__nv_bfloat16, 64, 2, PAGED>(tq, tk, tv, to, p, stream);
   }

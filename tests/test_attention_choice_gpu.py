@@ -1,7 +1,10 @@
 """Which forward kernel a call gets (``B200K_ATTN_AUTO``)."""
 
+import re
+
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 import iree_turbine_b200 as tb
 from iree_turbine_b200 import _launcher as L
@@ -22,6 +25,18 @@ def normal(shape, seed, dtype=torch.bfloat16):
     return torch.randn(shape, generator=g, device=DEV, dtype=dtype)
 
 
+def forward_kernel(call):
+    """Template arguments of the one attention forward kernel that `call` launches."""
+    call()  # what a first call does besides launching is not of interest
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    found = [m[1].split(", ") for m in (re.search(r"attn_fwd_kernel<(.*?)>", e.name) for e in p.events()) if m]
+    assert len(found) == 1
+    return found[0]
+
+
 # Query tiles that fill two or four rounds over 148 SMs, pairs of them one or two; one round of either; a single head.
 @pytest.mark.parametrize("b,h,hkv,sq,skv", [(1, 37, 37, 1000, 300), (4, 32, 8, 512, 512), (2, 74, 2, 257, 1000), (1, 3, 1, 700, 900)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
@@ -35,4 +50,21 @@ def test_without_a_mask_the_kernel_does_not_depend_on_the_batch(b, h, hkv, sq, s
         assert torch.equal(got[i, j], one[0, 0])
     ops.ATTENTION_KERNEL = L.ATTN_ONE_TILE
     assert torch.equal(got, torch.ops.b200k.attention(q, k, v, 0.1, False))
+    assert tb.device_status() == 0
+
+
+@pytest.mark.parametrize("sq,lens,width,groups", [(300, [300, 300], 8192, "1"), (16, [40, 2000], 8192, "1"),
+                                                  (1535, [1535, 3000], 4096, "1"), (1536, [3000, 1536], 4096, "2"),
+                                                  (1536, [2000, 1536], 2048, "1"), (2048, [2048, 2048], 131072, "2")])
+def test_paged_head_dim_64_does_not_go_by_the_width_of_the_table(sq, lens, width, groups):
+    """Two softmax warpgroups per tile are for long histories; a table says only how long one may become."""
+    page = 64
+    counts = [-(-n // page) for n in lens]
+    table = torch.zeros((len(lens), width // page), dtype=torch.int32)
+    for row, part in zip(table, torch.arange(sum(counts), dtype=torch.int32).split(counts)):
+        row[: part.numel()] = part
+    kc, vc = (normal((sum(counts), 2, page, 64), s) for s in (1, 2))
+    q, ln = normal((len(lens), 4, sq, 64), 3), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    table = table.to(DEV)
+    assert forward_kernel(lambda: torch.ops.b200k.paged_attention(q, kc, vc, table, ln, 0.3, True))[1:3] == ["64", groups]
     assert tb.device_status() == 0

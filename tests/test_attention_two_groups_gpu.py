@@ -1,14 +1,14 @@
 """Head dim 64, long items: a query tile has two softmax warpgroups that take its half steps of 64 keys in turn.
 
-Keys from 1536 on average run there, so sizes are odd and even counts of half steps around it; the ramp makes the running
-max grow by more than 2^8 in half steps of either warpgroup, so that both rescale the accumulator and each other's sums.
+Keys from 1536 on average run there (paged: and 1536 queries), so sizes are odd and even counts of half steps around it; the
+ramp makes the running max grow by more than 2^8 in half steps of either warpgroup, so that both rescale the accumulator and
+each other's sums.
 """
 
 import pytest
 import torch
 
 import iree_turbine_b200 as tb
-from iree_turbine_b200 import _launcher as L
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -67,8 +67,9 @@ def test_nan_keys(skv, first, last):
 
 
 @pytest.mark.parametrize("page", [16, 128])
-def test_paged(page):
-    lens, sq, h, hkv = [3000, 65, 0, 1601, 2990], 200, 4, 2
+@pytest.mark.parametrize("sq", [200, 1600])  # one warpgroup per tile, two
+def test_paged(page, sq):
+    lens, h, hkv = [3000, 65, 0, 1601, 2990], 4, 2
     counts = [-(-n // page) for n in lens]
     perm = torch.randperm(sum(counts), generator=torch.Generator().manual_seed(5)).to(torch.int32)
     table = torch.zeros((len(lens), max(counts)), dtype=torch.int32)
@@ -84,4 +85,3 @@ def test_paged(page):
             k, v = (c[pages, j // 2].reshape(-1, 64)[:n] for c in (kc, vc))
             check(got[i, j], q[i, j], k, v, 0.3, n - sq, dtype)
     assert tb.device_status() == 0
-    assert L.ATTN_AUTO == tb.ops.ATTENTION_KERNEL
