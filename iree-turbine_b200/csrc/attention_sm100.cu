@@ -874,6 +874,8 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
 // running max and for 256 more threads.  One / two, us: 4x8x2048 63.1 / 58.8, 4x32x2048 215 / 195, 1x2x8192 causal 108.5 /
 // 102.6, 2x4(1) 300 over 3000 45.1 / 41.8, paged 4x32(8) 512 over up to 4000 77.4 / 72.3; 16x16x1024 causal 79.6 / 85.9,
 // 32x8x384 30.9 / 33.5, 32x8x128 causal 10.3 / 11.2, 8x8 3000 over 200 34.7 / 37.1.  The line is a mean of 1536 keys per query.
+// An item of one query tile leaves the tensor core idle while its tile waits, so the hand-over is all that two add: one /
+// two, 8x32 128 over 1800 43.9 / 45.2, 1x8 16 over 3000 32.2 / 32.8; with a second tile 8x32 256 over 1800 60.9 / 56.6.
 // Head dim 128, which waits for its score MMAs, is slower with two (4x32x4096 causal 468 / 517): more warps compete with
 // the MMA threads for issue slots.
 // Paged: the lengths are device data.  The capacity of the table says nothing about them (a first chunk of 300 queries in
@@ -882,7 +884,7 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
 // Fewer queries over long histories could gain (8x8 512 over 3000 51.1 / 46.7), but nothing here tells them from short ones.
 template <bool PAGED>
 bool two_groups(const AttnParams& p) {
-  if (PAGED && p.seq_q < 1536) return false;
+  if (p.seq_q <= kTileRows || (PAGED && p.seq_q < 1536)) return false;
   return 2 * static_cast<int64_t>(p.seq_kv) - (p.causal ? p.seq_q : 0) >= 2 * 1536;
 }
 

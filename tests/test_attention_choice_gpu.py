@@ -68,3 +68,10 @@ def test_paged_head_dim_64_does_not_go_by_the_width_of_the_table(sq, lens, width
     table = table.to(DEV)
     assert forward_kernel(lambda: torch.ops.b200k.paged_attention(q, kc, vc, table, ln, 0.3, True))[1:3] == ["64", groups]
     assert tb.device_status() == 0
+
+
+@pytest.mark.parametrize("sq,skv,causal,groups", [(128, 2000, False, "1"), (1, 8000, True, "1"), (129, 1536, False, "2"),
+                                                  (129, 1535, False, "1"), (3072, 3072, True, "2"), (3071, 3071, True, "1")])
+def test_head_dim_64_two_warpgroups_need_a_second_tile(sq, skv, causal, groups):
+    q, k, v = normal((1, 2, sq, 64), 1), normal((1, 2, skv, 64), 2), normal((1, 2, skv, 64), 3)
+    assert forward_kernel(lambda: torch.ops.b200k.attention(q, k, v, 0.3, causal))[1:3] == ["64", groups]
