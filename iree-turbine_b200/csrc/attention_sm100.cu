@@ -57,6 +57,7 @@
 //
 // Every wait is bounded; when one gives up all roles drain to the common teardown, tensor memory
 // is freed and the kernel ORs a code into the caller's status word.
+#include <algorithm>
 #include <type_traits>
 
 #include "attention_order.cuh"
@@ -939,18 +940,48 @@ bool choose_pair_kernel(const b200k_attention_args& a) {
   return couples_fill(static_cast<int64_t>(a.batch) * a.q_heads, a.seq_q);
 }
 
+// Paged, one round of pairs and so at most two of single tiles: are the tiles, heaviest first in serpentine order, done
+// before the longest pair?  In K/V tiles, one more for the start of an item; a pair's lighter tile adds 0.64 of its own.
+// Lengths are device data, so all are taken as the capacity of the table: where the two sides differ by 5 % on that, the
+// queries are most of the keys, and shorter or unequal histories only make pairs worse.  (A wide table makes all tiles
+// alike, and two rounds of them lose.)
+bool tiles_finish_first(const b200k_paged_attention_args& a, int heads, int tiles_per_head) {
+  const int sms = num_sms(), tiles = heads * tiles_per_head;
+  auto cost = [&](int t) {
+    const int64_t rows = std::min<int64_t>((t + 1) * int64_t{kTileRows}, a.seq_q);
+    const int64_t keys = a.causal ? rows + a.max_seq_kv - a.seq_q : a.max_seq_kv;
+    return static_cast<double>((std::max<int64_t>(keys, 0) + kTileRows - 1) / kTileRows);
+  };
+  auto at = [&](int pos) { return cost(tiles_per_head - 1 - pos / heads) + 1; };
+  double busiest = at(0), longest = 0;
+  for (int end = heads;; end += heads) {  // the sum is largest behind the last item of a cost
+    const int i = std::min(end, sms) - 1, partner = 2 * sms - 1 - i;
+    if (partner < tiles) busiest = std::max(busiest, at(i) + at(partner));
+    if (i == sms - 1) break;
+  }
+  for (int t = 0; t < tiles_per_head; t += 2)
+    longest = std::max(longest, t + 1 < tiles_per_head ? cost(t + 1) + 0.64 * cost(t) : cost(t));
+  return busiest < 0.95 * (longest + 1);
+}
+
 // Paged: a K/V tile arrives page by page, and the pair kernel needs half as many tiles.  One-tile / tile-pair,
 // us: 4x32(8) 512 queries over up to 4000 keys 156 / 87 at page size 16, 114 / 95 at 64, 107 / 95 at 128;
 // 3x64(16) 1000 over 2000 170 / 146.  The one-tile kernel is ahead where the SMs are not filled and pages are
-// larger (1x8 2000 over 6000 81 / 98 at page size 32, 71 / 98 at 64, but 1x8 64 over 6000 at 16 96 / 81), and where
-// a pair would be half empty (16x16(4) 100 over 3000, page size 64, 39 / 41), or the longest pairs decide (8x4(1) 1000 over
-// up to 4000, page size 64, 128 pairs, 50 / 64).
+// larger (1x8 2000 over 6000 81 / 98 at page size 32, 71 / 98 at 64, but 1x8 64 over 6000 at 16 96 / 81), where
+// a pair would be half empty (16x16(4) 100 over 3000, page size 64, 39 / 41), and where one round of pairs would do but the
+// longest of them decides: at page size 64 2x16(4) 1024 of 1024 19.3 / 21.8, 1x10(2) 3000 of 3000 36.9 / 50.3, 8x2(1) 2000
+// of 2100 31.5 / 39.4, 1x40(8) 600 of 600 13.8 / 14.2, but 8x8(2) 512 over 4000 82.9 / 67.8, 3x16(2) 536 of 588 18.5 / 15.6,
+// 1x64(16) 449 over 4295 90.5 / 73.2.  (Histories of very different lengths would gain too, 2x8(1) 1235 over 2425 and 3615
+// 39.1 / 57.8, but nothing here tells them from equal ones.)
 bool choose_pair_kernel(const b200k_paged_attention_args& a) {
   if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
   if (a.kernel == B200K_ATTN_ONE_TILE) return false;
-  const int64_t heads = static_cast<int64_t>(a.batch) * a.q_heads;
-  const int64_t tiles = heads * ((a.seq_q + kTileRows - 1) / kTileRows), pairs = heads * ((a.seq_q + kPairRows - 1) / kPairRows);
-  return !((a.page_size >= 32 && tiles <= num_sms()) || (a.page_size >= 64 && (a.seq_q <= kTileRows || pairs <= num_sms())));
+  const int64_t heads = static_cast<int64_t>(a.batch) * a.q_heads, per_head = (a.seq_q + kTileRows - 1) / kTileRows;
+  const int64_t pairs = heads * ((a.seq_q + kPairRows - 1) / kPairRows);
+  if (a.page_size >= 32 && heads * per_head <= num_sms()) return false;
+  if (a.page_size < 64) return true;
+  if (a.seq_q <= kTileRows) return false;
+  return pairs > num_sms() || !tiles_finish_first(a, static_cast<int>(heads), static_cast<int>(per_head));
 }
 
 }  // namespace

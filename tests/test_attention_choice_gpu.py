@@ -53,20 +53,23 @@ def test_without_a_mask_the_kernel_does_not_depend_on_the_batch(b, h, hkv, sq, s
     assert tb.device_status() == 0
 
 
+def paged_kernel(heads, kv_heads, dim, sq, page, lens, width):
+    counts = [-(-n // page) for n in lens]
+    table = torch.zeros((len(lens), width // page), dtype=torch.int32)
+    for row, part in zip(table, torch.arange(sum(counts), dtype=torch.int32).split(counts)):
+        row[: part.numel()] = part
+    kc, vc = (normal((sum(counts), kv_heads, page, dim), s) for s in (1, 2))
+    q, ln = normal((len(lens), heads, sq, dim), 3), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    table = table.to(DEV)
+    return forward_kernel(lambda: torch.ops.b200k.paged_attention(q, kc, vc, table, ln, 0.3, True))
+
+
 @pytest.mark.parametrize("sq,lens,width,groups", [(300, [300, 300], 8192, "1"), (16, [40, 2000], 8192, "1"),
                                                   (1535, [1535, 3000], 4096, "1"), (1536, [3000, 1536], 4096, "2"),
                                                   (1536, [2000, 1536], 2048, "1"), (2048, [2048, 2048], 131072, "2")])
 def test_paged_head_dim_64_does_not_go_by_the_width_of_the_table(sq, lens, width, groups):
     """Two softmax warpgroups per tile are for long histories; a table says only how long one may become."""
-    page = 64
-    counts = [-(-n // page) for n in lens]
-    table = torch.zeros((len(lens), width // page), dtype=torch.int32)
-    for row, part in zip(table, torch.arange(sum(counts), dtype=torch.int32).split(counts)):
-        row[: part.numel()] = part
-    kc, vc = (normal((sum(counts), 2, page, 64), s) for s in (1, 2))
-    q, ln = normal((len(lens), 4, sq, 64), 3), torch.tensor(lens, dtype=torch.int32, device=DEV)
-    table = table.to(DEV)
-    assert forward_kernel(lambda: torch.ops.b200k.paged_attention(q, kc, vc, table, ln, 0.3, True))[1:3] == ["64", groups]
+    assert paged_kernel(4, 2, 64, sq, 64, lens, width)[1:3] == ["64", groups]
     assert tb.device_status() == 0
 
 
@@ -75,3 +78,15 @@ def test_paged_head_dim_64_does_not_go_by_the_width_of_the_table(sq, lens, width
 def test_head_dim_64_two_warpgroups_need_a_second_tile(sq, skv, causal, groups):
     q, k, v = normal((1, 2, sq, 64), 1), normal((1, 2, skv, 64), 2), normal((1, 2, skv, 64), 3)
     assert forward_kernel(lambda: torch.ops.b200k.attention(q, k, v, 0.3, causal))[1:3] == ["64", groups]
+
+
+# One round of pairs, two of single tiles (148 SMs): prompts, whose tiles differ in cost; nearly equal tiles; prompts in a
+# table with room to grow; small pages; one round of single tiles; a few queries.
+@pytest.mark.parametrize("h,hkv,sq,page,lens,width,pair", [
+    (16, 4, 1024, 64, [1024] * 2, 1024, False), (10, 2, 3000, 128, [3000], 3072, False), (2, 1, 2000, 64, [2100] * 8, 2112, False),
+    (8, 2, 512, 64, [4000] * 8, 4032, True), (16, 2, 536, 64, [588, 571, 554], 640, True), (64, 16, 449, 64, [4295], 4352, True),
+    (16, 4, 1024, 64, [1024] * 2, 8192, True), (16, 4, 1024, 16, [1024] * 2, 1024, True), (16, 4, 1024, 64, [1024], 1024, False),
+    (64, 8, 128, 64, [500] * 3, 512, False)])
+def test_paged_head_dim_128(h, hkv, sq, page, lens, width, pair):
+    assert (paged_kernel(h, hkv, 128, sq, page, lens, width)[1] == "128") == pair  # (the one-tile kernel has no such argument)
+    assert tb.device_status() == 0
