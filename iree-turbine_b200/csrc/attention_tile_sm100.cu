@@ -163,7 +163,7 @@ __device__ __forceinline__ Item decode_item(int pos, const AttnParams& p, const 
   return make_item<PAGED>(batch, head, qtile, p);
 }
 
-template <typename T, bool PAGED>
+template <typename T, bool PAGED, bool ELECT>
 __global__ void __launch_bounds__(kAttnThreads, 1)
     attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       // was busy nearly the whole step and every wait of one kind delayed the other.  The streams
       // are independent: each orders itself through barriers (score buffer taken by the softmax,
       // P written, stages loaded), never through issue order.
-      if (elect_one()) {
+      if (ELECT ? elect_one() : lane == 0) {
         // The issuing thread runs scalar, latency-bound code: descriptors are a constant high word
         // plus a low word that is a precomputed base plus a compile-time offset.
         const uint32_t hi_k = static_cast<uint32_t>(make_desc_kmajor_sw128(0) >> 32);
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       __syncwarp();
     } else if (warp == kPvWarp) {
       // ---------------- second MMAs: O (+)= P[g & 1] V_g ----------------
-      if (elect_one()) {
+      if (ELECT ? elect_one() : lane == 0) {
         const uint32_t hi_mn = static_cast<uint32_t>(make_desc_mnmajor_sw128(0, kHalfTileBytes) >> 32);
         const uint32_t v_lo = static_cast<uint32_t>(make_desc_mnmajor_sw128(smem_u32(smem + kVOffset), kHalfTileBytes));
         auto desc = [](uint32_t lo, uint32_t hi) { return (static_cast<uint64_t>(hi) << 32) | lo; };
@@ -710,10 +710,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   }
 }
 
-template <typename T, bool PAGED>
+template <typename T, bool PAGED, bool ELECT>
 int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
                  const AttnParams& p, cudaStream_t stream) {
-  auto kfn = attn_fwd_kernel<T, PAGED>;
+  auto kfn = attn_fwd_kernel<T, PAGED, ELECT>;
   static bool configured[64] = {};  // per instantiation and device ordinal
   int rc = ensure_dynamic_smem(kfn, kAttnSmem, configured, "cudaFuncSetAttribute(attention smem)");
   if (rc) return rc;
@@ -724,6 +724,19 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   // CTA: 156 us in blockIdx order, 162 launched early).
   const int64_t tiles = static_cast<int64_t>(p.order.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
   return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tq, tk, tv, to, p);
+}
+
+// How the two MMA threads are picked: behind elect.sync (see elect_one) items start faster, behind lane == 0 the steps of a
+// long item follow each other faster (their MMAs have N = 128 and gain nothing by the faster issue).  The line is at a mean of
+// 1024 keys per query, and of 512 where a CTA has hardly more than one item.  lane == 0 / elect.sync, us: 24x64x308
+// 165.0 / 151.8, 2x16 1024 over 256 11.2 / 10.7, 16x16(4)x1024 causal 100.3 / 94.4, 2x20x1300 causal 30.7 / 29.4, 2x32(8)x2000
+// causal 82.8 / 81.8, 8x32x1024 153.8 / 151.9; 1x12 1536 over 1024 (one round) 13.8 / 14.0, 1x24x2048 causal 35.4 / 36.6,
+// 2x16x4096 271 / 286, 1x8x8192 275 / 294, 1x8 2048 over 3072 30.0 / 32.0, 1x4x8192 causal 73.4 / 78.1.  The score thread
+// alone behind lane == 0 is between the two (272, 275, 32.2, 74.7; 24x64x308 158.5).  Paged items wait for their pages and
+// take the same time either way (4x4(1) 1000 over 4000 44.1 / 43.9).
+bool short_items(const AttnParams& p) {
+  const int64_t keys = 2 * static_cast<int64_t>(p.seq_kv) - (p.causal ? p.seq_q : 0);  // twice the mean per query
+  return 2 * static_cast<int64_t>(p.order.num_items) > 3 * num_sms() ? keys <= 2 * 1024 : keys < 2 * 512;
 }
 
 }  // namespace
@@ -804,8 +817,12 @@ int launch_attention_fwd_tile(const b200k_attention_args& a, cudaStream_t stream
   p.block_table = nullptr;
   p.seq_lens = nullptr;
   p.block_table_stride = p.page_size = p.num_pages = 0;
-  if (a.dtype == B200K_F16) return launch_typed<__half, false>(tq, tk, tv, to, p, stream);
-  return launch_typed<__nv_bfloat16, false>(tq, tk, tv, to, p, stream);
+  if (short_items(p)) {
+    if (a.dtype == B200K_F16) return launch_typed<__half, false, true>(tq, tk, tv, to, p, stream);
+    return launch_typed<__nv_bfloat16, false, true>(tq, tk, tv, to, p, stream);
+  }
+  if (a.dtype == B200K_F16) return launch_typed<__half, false, false>(tq, tk, tv, to, p, stream);
+  return launch_typed<__nv_bfloat16, false, false>(tq, tk, tv, to, p, stream);
 }
 
 // Arguments have been validated by launch_paged_attention_fwd.
@@ -885,8 +902,8 @@ int launch_paged_attention_fwd_tile(const b200k_paged_attention_args& a, cudaStr
   p.block_table_stride = a.block_table_stride;
   p.page_size = a.page_size;
   p.num_pages = a.num_pages;
-  if (a.dtype == B200K_F16) return launch_typed<__half, true>(tq, tk, tv, to, p, stream);
-  return launch_typed<__nv_bfloat16, true>(tq, tk, tv, to, p, stream);
+  if (a.dtype == B200K_F16) return launch_typed<__half, true, true>(tq, tk, tv, to, p, stream);
+  return launch_typed<__nv_bfloat16, true, true>(tq, tk, tv, to, p, stream);
 }
 
 }  // namespace b200k

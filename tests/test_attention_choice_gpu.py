@@ -53,6 +53,29 @@ def test_without_a_mask_the_kernel_does_not_depend_on_the_batch(b, h, hkv, sq, s
     assert tb.device_status() == 0
 
 
+# Short items in several rounds over the SMs, in hardly more than one, and in one; long ones; a grouped K/V head.
+@pytest.mark.parametrize("b,h,hkv,sq,skv,causal,elected", [
+    (2, 16, 16, 1024, 1024, False, "true"), (2, 16, 2, 1024, 1025, False, "false"), (1, 16, 16, 1536, 512, False, "false"),
+    (1, 16, 16, 1536, 511, False, "true"), (1, 24, 8, 2040, 2044, True, "true"), (1, 24, 8, 2060, 2060, True, "false"),
+    (1, 2, 1, 200, 5000, False, "false")])
+def test_one_tile_mma_threads(b, h, hkv, sq, skv, causal, elected):
+    """The two ways of picking the MMA threads by item length give the same bits."""
+    q, k, v = normal((b, h, sq, 128), 1), normal((b, hkv, skv, 128), 2), normal((b, hkv, skv, 128), 3)
+    ops.ATTENTION_KERNEL = L.ATTN_ONE_TILE
+    assert forward_kernel(lambda: torch.ops.b200k.attention(q, k, v, 0.1, causal)) == ["__nv_bfloat16", "false", elected]
+    got = torch.ops.b200k.attention(q, k, v, 0.1, causal)
+    one = torch.ops.b200k.attention(q[-1:, -1:], k[-1:, -1:], v[-1:, -1:], 0.1, causal)
+    assert torch.equal(got[-1, -1], one[0, 0])
+    s = (q[-1, -1].double() @ k[-1, -1].double().t()) * 0.1
+    if causal:
+        s.masked_fill_(~torch.ones_like(s, dtype=torch.bool).tril(skv - sq), -torch.inf)
+    p = torch.softmax(s, -1)
+    ref = p @ v[-1, -1].double()
+    # probabilities and output rounded to bf16 (2^-9 each, relative), the former against sums of |v|
+    assert bool(((got[-1, -1].double() - ref).abs() <= 2.0 ** -8 * (p @ v[-1, -1].double().abs() + ref.abs()) + 1e-4).all())
+    assert tb.device_status() == 0
+
+
 def paged_kernel(heads, kv_heads, dim, sq, page, lens, width):
     counts = [-(-n // page) for n in lens]
     table = torch.zeros((len(lens), width // page), dtype=torch.int32)
