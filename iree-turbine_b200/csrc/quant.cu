@@ -17,7 +17,7 @@ namespace {
 constexpr float kE4M3Max = 448.0f;
 constexpr int kQuantThreads = 256;
 constexpr int kQuantUnroll = 4;
-constexpr int kCastBlocksPerSm = 6;  // the grid's: with 69 registers and 3 per SM 8000 x 8192 takes 93.3 us instead of 89.2
+constexpr int kBlocksPerSm = 6;  // of a grid at most
 constexpr int kMaxParts = B200K_QUANTIZE_WORKSPACE_BYTES / 4;
 
 __device__ __forceinline__ float block_max(float m) {
@@ -85,9 +85,16 @@ __device__ __forceinline__ uint32_t quantize_quad(float4 v, float inv, float sca
 // Walks x from its end to its beginning: what absmax_kernel read last is what L2 still has (8000 x 8192, 262 MB against
 // 126 MB of L2).  The first batch of loads is issued before the wait for the maxima: this kernel cannot start before
 // every CTA of absmax_kernel has triggered, and each does so behind its own wait for whatever wrote x.
-__global__ void __launch_bounds__(kQuantThreads, kCastBlocksPerSm) cast_e4m3_kernel(const float* x, uint8_t* y, int64_t n,
-                                                                                    const uint32_t* parts, int num_parts,
-                                                                                    float* scale_out) {
+// BLOCKS_PER_SM bounds the registers: 40 for 6, 58 for 4.  A grid of 6 per SM needs them all resident (8000 x 8192 with
+// 69 registers and 3 per SM 93.3 us instead of 89.2).  A smaller one finds them all resident beside the CTAs of absmax_kernel
+// with 40 registers, and their first loads get in the way of its own.  Before the loads were issued early / 6 / 4, us, x
+// from L2: 2.0 M values 6.49 / 6.73 / 6.35, 2.3 M 6.65 / 7.60 / 6.76, 2.8 M 7.47 / 7.82 / 7.41, 3.2 M 7.97 / 7.89 / 8.13; x
+// from memory: 2.0 M 7.40 / 7.45 / 7.20, 2.3 M 7.79 / 8.42 / 7.62, 2.8 M 9.36 / 8.89 / 8.85, 3.2 M 9.87 / 9.19 / 9.58.  The
+// line is at 5 blocks per SM, 3.03 M values.
+template <int BLOCKS_PER_SM>
+__global__ void __launch_bounds__(kQuantThreads, BLOCKS_PER_SM) cast_e4m3_kernel(const float* x, uint8_t* y, int64_t n,
+                                                                                 const uint32_t* parts, int num_parts,
+                                                                                 float* scale_out) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kQuantThreads;
   const int64_t n4 = n / 4;
   const float4* x4 = reinterpret_cast<const float4*>(x);
@@ -138,13 +145,14 @@ int launch_quantize_e4m3(const float* x, void* y, float* scale_out, uint32_t* am
     if (rc) return rc;
   }
   const int64_t want = (n / 4 + kQuantThreads * kQuantUnroll - 1) / (kQuantThreads * kQuantUnroll);
-  int64_t cap = static_cast<int64_t>(num_sms()) * 6;
+  int64_t cap = static_cast<int64_t>(num_sms()) * kBlocksPerSm;
   if (cap > kMaxParts) cap = kMaxParts;
   const int blocks = static_cast<int>(want < 1 ? 1 : (want > cap ? cap : want));
   rc = launch_pdl("absmax_kernel launch", absmax_kernel, dim3(blocks), dim3(kQuantThreads), 0, stream, x, n, amax_scratch,
                   one_part);
   if (rc) return rc;
-  return launch_pdl("cast_e4m3_kernel launch", cast_e4m3_kernel, dim3(blocks), dim3(kQuantThreads), 0, stream, x,
+  auto cast = blocks > 5 * num_sms() ? cast_e4m3_kernel<kBlocksPerSm> : cast_e4m3_kernel<4>;
+  return launch_pdl("cast_e4m3_kernel launch", cast, dim3(blocks), dim3(kQuantThreads), 0, stream, x,
                     reinterpret_cast<uint8_t*>(y), n, amax_scratch, one_part ? 1 : blocks, scale_out);
 }
 

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4096, 4099, 1 << 20, 3_000_001])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4096, 4099, 1 << 20, 3_000_001, 3_031_047])
 @pytest.mark.parametrize("magnitude", [1.0, 1e-36, 1e37])
 def test_quantize_is_exact(n, magnitude):
     x = torch.randn(n, generator=torch.Generator().manual_seed(n)) * magnitude
