@@ -31,6 +31,23 @@ def test_quantize_is_exact(n, magnitude):
     assert torch.equal(y.cpu().view(torch.uint8), yo.view(torch.uint8))
 
 
+# 148 SMs hold 6 blocks of 4096 values each, 3637248 in one pass of the grid; then two passes, the second of one vector, and
+# several; all with values after the last vector of four.
+@pytest.mark.parametrize("n", [3_637_247, 3_637_253, 8_000_003, 20_000_001])
+def test_quantize_in_several_passes(n):
+    """The cast issues its first loads early: x is written by the kernel just before the call."""
+    base = torch.randn(n, generator=torch.Generator().manual_seed(n))
+    base[n // 3] = 30.0  # (a single largest value)
+    x, old = base.to(DEV), torch.zeros(n, device=DEV)
+    for _ in range(3):
+        old.zero_()
+        old.add_(x)
+        y, s = torch.ops.b200k.quantize_e4m3(old)
+    yo, so = oracle.quantize_e4m3(base)
+    assert torch.equal(s.cpu().reshape(-1), so.reshape(-1))
+    assert torch.equal(y.cpu().view(torch.uint8), yo.view(torch.uint8))
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 8), (7, 64), (8, 56), (31, 72), (33, 520), (129, 128), (1000, 264), (4099, 1032)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_col_sum(rows, cols, dtype):
