@@ -933,10 +933,11 @@ int fill_pair_order(AttnParams& p, const char* who, int head_dim, bool paged) {
 // Causal, couples that fill their rounds: 4x32x4096 571 / 542, 8x32x2048 321 / 300, 16x64x512 145 / 114, 32x32x256
 // 72 / 64: the pair kernel.  Other causal problems, with the pair kernel in its better order: 2x32(8)x2000 86 / 89,
 // 4x8x4096 144 / 143, 16x16(4)x1024 93 / 98, 1x64(8)x6000 553 / 565, 1x4x8192 93 / 150, 1x32(8)x1200 23 / 27: the
-// one-tile kernel.
+// one-tile kernel, as for at most 128 queries, where every pair is half empty: 32x32x128 27.9 / 33.3, 37x16x128 18.5 / 20.7,
+// 32x32 100 over 1000 97.2 / 115.7, 16x37x17 13.9 / 14.9.
 bool choose_pair_kernel(const b200k_attention_args& a) {
   if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
-  if (a.kernel == B200K_ATTN_ONE_TILE || !a.causal) return false;
+  if (a.kernel == B200K_ATTN_ONE_TILE || !a.causal || a.seq_q <= kTileRows) return false;
   return couples_fill(static_cast<int64_t>(a.batch) * a.q_heads, a.seq_q);
 }
 

@@ -53,6 +53,15 @@ def test_without_a_mask_the_kernel_does_not_depend_on_the_batch(b, h, hkv, sq, s
     assert tb.device_status() == 0
 
 
+# 148 and 296 heads, so that couples of pairs fill their rounds: from the second query tile on they go to the pair kernel.
+@pytest.mark.parametrize("b,h,sq,skv,pair", [(4, 37, 128, 128, False), (8, 37, 100, 300, False), (4, 37, 129, 129, True),
+                                             (4, 37, 512, 512, True), (3, 37, 512, 512, False)])
+def test_causal_pairs_need_a_second_tile(b, h, sq, skv, pair):
+    q, k, v = normal((b, h, sq, 128), 1), normal((b, h, skv, 128), 2), normal((b, h, skv, 128), 3)
+    assert (forward_kernel(lambda: torch.ops.b200k.attention(q, k, v, 0.1, True))[1] == "128") == pair
+    assert tb.device_status() == 0
+
+
 # Short items in several rounds over the SMs, in hardly more than one, and in one; long ones; a grouped K/V head.
 @pytest.mark.parametrize("b,h,hkv,sq,skv,causal,elected", [
     (2, 16, 16, 1024, 1024, False, "true"), (2, 16, 2, 1024, 1025, False, "false"), (1, 16, 16, 1536, 512, False, "false"),
