@@ -195,8 +195,8 @@ int b200k_gemm_nt_allgather(const b200k_gemm_allgather_args* args, void* stream)
  * two softmax warpgroups take alternate KV steps (head_dim 128 only).  B200K_ATTN_TILE_PAIR: a
  * work item is a pair of query tiles that share every K/V tile, one softmax warpgroup each; causal
  * problems are dealt out in (heavy, light) couples of equal cost.  B200K_ATTN_AUTO picks the pair
- * kernel for head_dim 64 and for causal problems whose couples fill the SMs evenly, else the
- * one-tile kernel (the measured winner in each case).  Results of the two agree within rounding
+ * kernel for head_dim 64 and for causal problems of more than 128 queries whose couples fill the SMs
+ * evenly, else the one-tile kernel (without a mask that does not depend on the batch).  Results of the two agree within rounding
  * of the 16-bit probabilities, not bitwise.
  */
 enum { B200K_ATTN_AUTO = 0, B200K_ATTN_ONE_TILE = 1, B200K_ATTN_TILE_PAIR = 2 };

@@ -5,9 +5,9 @@
 // Persistent CTAs, one per SM.  A work item is one PAIR of 128-row query tiles (256 consecutive
 // query rows) of one (batch, head).  The two tiles of a pair are independent problems that share
 // every K/V tile: each has its own score buffer, its own probabilities, its own running max / sum
-// and its own output accumulator, and each is served by its own softmax warpgroup.  Nothing is
-// exchanged between the two warpgroups; while one of them is busy with its exponentials the
-// tensor core works for the other one.
+// and its own output accumulator, and each is served by softmax warpgroups of its own.  Nothing is
+// exchanged between the two tiles; while one of them is busy with its exponentials the tensor core
+// works for the other one.
 //
 // Roles, with one softmax warpgroup per query tile (long items of head dim 64 have two, see two_groups; the others then
 // follow eight warps later):
@@ -44,9 +44,9 @@
 // memory twice per K/V tile; measured, that costs less than the waiting it removes.
 //
 // Items count in half steps: a tile stops behind the last 64 keys that one of its rows sees.  Causal: the two tiles of a
-// pair need a different number (n[0] <= n[1]); tile 0 simply stops taking part once it is past its diagonal.  Which CTA takes which pairs, and in what
-// order, is in attention_order.cuh.  Couples of a heavy and a light pair (see ItemWalk) are the order of
-// large causal problems.
+// pair need a different number (n[0] <= n[1]); tile 0 simply stops taking part once it is past its diagonal.  Which CTA
+// takes which pairs, and in what order, is in attention_order.cuh.  Couples of a heavy and a light pair (see ItemWalk) are
+// the order of large causal problems.
 //
 // Softmax: running max in log2 units (scores are multiplied by scale * log2(e) inside the
 // exponent's FMA); O is only rescaled when a row's max grows by more than 2^8 (the stale max is
@@ -69,7 +69,8 @@ namespace {
 
 // Warps and registers by the number of softmax warpgroups that a query tile has; two take its half steps in turn.
 // Registers: warps per SM sub-partition x registers at launch, redistributed.  A setmaxnreg.inc beyond what the others
-// gave up never completes.
+// gave up never completes.  With two warpgroups the budget is exactly full (4 x 96 + 48 + 48 = 6 x 80), and the compiler,
+// which has 80 registers for the whole kernel, spills 108 to 140 bytes per thread; with one it spills nothing.
 template <int GROUPS>
 struct Roles {
   static constexpr int kGroups = GROUPS;
@@ -103,8 +104,8 @@ struct AttnSmem {
   static constexpr int kMaxOffset = kLsumOffset + 2 * 2 * 2 * kTileRows * 4;  // float [tile][warpgroup][128 rows]: running max
   static constexpr int kOrderOffset = kMaxOffset + 2 * 2 * kTileRows * 4;     // uint16: item order of a paged call
   static constexpr int kBarOffset = kOrderOffset + attn_order::kSortBytes;
-  // q_full[2] q_empty[2] | kv_full[4] kv_empty[4] | s_full[2][2] p_full[2][2] | o_full[2] o_free[2] | l_full[2] l_free[2] | turn[2] | pv_done[2] |
-  // x_full[2][2][4]
+  // q_full[2] q_empty[2] | kv_full[4] kv_empty[4] | s_full[2][2] p_full[2][2] | o_full[2] o_free[2] | l_full[2] l_free[2] |
+  // turn[2] | pv_done[2] | x_full[2][2][4]
   static constexpr int kNumBars = 4 + 2 * kKvStages + 8 + 4 + 4 + 2 + 2 + 16;
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16 + 1024;  // + slack for 1024-byte alignment
   // tensor memory columns
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R::kRegsOther));
     if (warp == R::kKvWarp) {
       // ---------------- K / V producer: ring entries K_0 V_0 K_1 V_1 ... of every item ----------------
-      // Dense: lane 0 issues one box per tile and 64-column block.  Paged: one box per page and block,
+      // Dense: one lane issues one box per tile and 64-column block.  Paged: one box per page and block,
       // each page by a lane of its own, the page numbers read a tile ahead (one lane looking up and
       // issuing page after page paid the latency of a table read per page: a 4 x 512-query chunk over up
       // to 4000 keys in pages of 16 took 203 us that way).
@@ -495,7 +496,9 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
         // the causal bf16 B4 H32 S4096 problem (same box): turns 1108 TFLOP/s; no order at all 1104
         // on another box against 1151 with turns; a lock taken once the probabilities are there and
         // held for the PV MMAs 1077, held for the score MMAs as well 925; the turn handed on before
-        // the PV MMAs 1095, after the score MMAs 852.
+        // the PV MMAs 1095, after the score MMAs 852.  With two softmax warpgroups per tile (head dim 64) the turn
+        // is handed on behind the score MMAs: 1x16x8192 causal 199 us, 201 behind the PV MMAs, 1x8x2000 30.6 / 31.0, 4x32x2048
+        // 195 / 196.
         uint32_t ct = 0;  // turns taken
         auto take_turn = [&]() {
           const bool got = wait(kTurn + t, t ? (ct & 1u) : ((ct & 1u) ^ 1u));
@@ -668,7 +671,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
     }
     if (store_thread) tma_store_wait_read<0>();
   } else {
-    // ---------------- softmax of query tile t = warp / 8: with two warpgroups the half steps of parity w ----------------
+    // ---------------- softmax of query tile t: all half steps, or with two warpgroups those of parity w ----------------
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R::kRegsSoftmax));
     const int t = warp / (4 * kGroups);
     const int w = kGroups == 2 ? (warp >> 2) & 1 : 0;
@@ -866,15 +869,16 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   const int grid = p.order.num_items < sms ? p.order.num_items : sms;
   // Launched early only when short, see the one-tile kernel.
   const int64_t tiles = static_cast<int64_t>(p.order.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
-  return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(Roles<GROUPS>::kThreads), AttnSmem<HD>::kTotal, stream, tq, tk, tv, to, p);
+  return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(Roles<GROUPS>::kThreads),
+                          AttnSmem<HD>::kTotal, stream, tq, tk, tv, to, p);
 }
 
 // Two softmax warpgroups per query tile at head dim 64: it spends half as many tensor cycles per exponential as 128
 // does, so in a long item the exponentials are what a tile waits for, and two warps per tile and SM sub-partition get
 // through them in fewer cycles (545 per 64 columns and warp, 640 with one).  Short items pay for the hand-over of the
 // running max and for 256 more threads.  One / two, us: 4x8x2048 63.1 / 58.8, 4x32x2048 215 / 195, 1x2x8192 causal 108.5 /
-// 102.6, 2x4(1) 300 over 3000 45.1 / 41.8, paged 4x32(8) 512 over up to 4000 77.4 / 72.3; 16x16x1024 causal 79.6 / 85.9,
-// 32x8x384 30.9 / 33.5, 32x8x128 causal 10.3 / 11.2, 8x8 3000 over 200 34.7 / 37.1.  The line is a mean of 1536 keys per query.
+// 102.6, 2x4(1) 300 over 3000 45.1 / 41.8; 16x16x1024 causal 79.6 / 85.9, 32x8x384 30.9 / 33.5, 32x8x128 causal 10.3 /
+// 11.2, 8x8 3000 over 200 34.7 / 37.1.  The line is a mean of 1536 keys per query.
 // An item of one query tile leaves the tensor core idle while its tile waits, so the hand-over is all that two add: one /
 // two, 8x32 128 over 1800 43.9 / 45.2, 1x8 16 over 3000 32.2 / 32.8; with a second tile 8x32 256 over 1800 60.9 / 56.6.
 // Head dim 128, which waits for its score MMAs, is slower with two (4x32x4096 causal 468 / 517): more warps compete with

@@ -723,7 +723,8 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   // scatters the CTAs that share a head's K / V over both dies (8 x 32 x 1024 non-causal, 110 tiles per
   // CTA: 156 us in blockIdx order, 162 launched early).
   const int64_t tiles = static_cast<int64_t>(p.order.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
-  return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream, tq, tk, tv, to, p);
+  return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream,
+                          tq, tk, tv, to, p);
 }
 
 // How the two MMA threads are picked: behind elect.sync (see elect_one) items start faster, behind lane == 0 the steps of a

@@ -62,7 +62,8 @@ struct PeerMaps {
 template <int BN, int MT>
 struct GemmSmem {
   // k-blocks (128 bytes of K) per pipeline stage.  The thread that issues the MMAs spends about 50 cycles
-  // on each of a block's four and 280 more per stage on the barrier wait, the commit and the loop.  For a
+  // on each of a block's four and 280 more per stage on the barrier wait, the commit and the loop (measured
+  // with that thread behind lane == 0; behind elect.sync an MMA of N = 64 takes it 49 cycles, see elect_one).  For a
   // tile whose MMAs execute in 64 cycles or less that thread, not the tensor core or the loads, set the
   // pace (480 cycles per block, for BN = 64 as for BN = 128), so those tiles take two blocks per stage.
   static constexpr int kSub = MT == 1 && BN <= 128 ? 2 : 1;

@@ -528,8 +528,8 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   // Tile shape and split: the smallest estimated time, in us.  Measured on 27 shapes (rows 1 to 6000, K 300
   // to 16000, operands from HBM, launches back to back) a launch of whole tiles takes
   //   fixed + waves * k-blocks * per_kb,        per_kb .20 / .25 / .39 / .62 us for 128 x 64 / 128 x 128 /
-  // 128 x 256 / 256 x 256 tiles (the first three set by the issuing thread and by what an SM can pull from
-  // L2, the last by the tensor core), plus about 3 us a wave for the last one's epilogue, which nothing
+  // 128 x 256 / 256 x 256 tiles (the first three set by the issuing thread, then behind lane == 0, and by what an SM
+  // can pull from L2, the last by the tensor core), plus about 3 us a wave for the last one's epilogue, which nothing
   // overlaps.  Rows that do not start on 128-byte lines cost the narrower tiles some 15 % more L2 traffic.
   // Split-K over a cluster of s CTAs is not persistent: every wave of resident clusters pays
   //   fixed + k-blocks / s * per_kb + (partial tiles to shared memory, two cluster barriers, reduction),

@@ -26,13 +26,15 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
-// True in one lane of a converged warp.  The roles of a single thread (MMA issue, TMA loads) are entered through this
-// and not through `lane == 0`: the operands of those instructions are uniform registers, and only behind elect.sync does
+// True in one lane of a converged warp.  Threads that issue MMAs or dense TMA loads are picked through this and not
+// through `lane == 0`: the operands of those instructions are uniform registers, and only behind elect.sync does
 // the compiler know that one thread runs and move them there without a detour per instruction.  Measured, cycles per
 // tcgen05.mma in a loop of one thread, lane == 0 / elect: A in tensor memory N = 64 45.5 / 32.7 (the tensor pipe's rate),
 // both in shared memory N = 32 45.6 / 40.7, N = 64 48.8 / 48.7 and N = 128 64.7 / 64.7 (the shared-memory port: 6 and 8 KB
-// at 128 B per cycle).  Kernels, us: attention 4x32x4096 causal 488 / 468, 4x32(8)x4096 causal 537 / 496, 24x64x308 144 /
-// 134; its backward 2x32(8)x2000 243 / 235; products 1024^3 6.7 / 6.0, fp8 4096^3 71 / 63, 16x4096x4096 11.8 / 10.8.
+// at 128 B per cycle).  Kernels, us: attention 4x32x4096 causal 539 / 513, 16x64x512 causal 142 / 123, 24x64x308 165 / 152;
+// its backward 2x32(8)x2000 252 / 238; products 1024^3 6.4 / 5.6, 256x256x16384 12.3 / 11.2; none where memory or the
+// shared-memory port decides (2048^3, 4096^3, 16x4096x4096).  Two places keep `lane == 0`, which was faster there: the MMA
+// threads for long items of the one-tile attention kernel and the TMA thread of the split-K GEMM.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
