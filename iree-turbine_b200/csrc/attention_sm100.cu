@@ -931,12 +931,12 @@ int fill_pair_order(AttnParams& p, const char* who, int head_dim, bool paged) {
 // Which kernel runs a problem (B200K_ATTN_AUTO); head dim 64 exists in the pair kernel only.  Measured at
 // head dim 128, one-tile / tile-pair, us.
 // Without a mask the one-tile kernel, whatever the batch: the two round probabilities against another running max, and a
-// choice by how the items fill the SMs would let a head's bits depend on the heads beside it.  What that choice would
-// give where pairs need half the rounds: 8x32x1024 129 / 127, 4x16x4096 537 / 515, 4x32(8)x512 25.7 / 24.8; elsewhere
-// pairs are slower: 2x16x4096 287 / 308, 1x8x2048 25 / 39, 24x64x308 133 / 165.
-// Causal, couples that fill their rounds: 4x32x4096 571 / 542, 8x32x2048 321 / 300, 16x64x512 145 / 114, 32x32x256
-// 72 / 64: the pair kernel.  Other causal problems, with the pair kernel in its better order: 2x32(8)x2000 86 / 89,
-// 4x8x4096 144 / 143, 16x16(4)x1024 93 / 98, 1x64(8)x6000 553 / 565, 1x4x8192 93 / 150, 1x32(8)x1200 23 / 27: the
+// choice by how the items fill the SMs would let a head's bits depend on the heads beside it.  It would gain little even
+// where pairs need half the rounds: 4x16x4096 511 / 507, 1x8x8192 264 / 257, but 8x32x1024 136 / 142, 1x16x4096 136 / 141,
+// 4x32(8)x512 25.7 / 26.0; elsewhere pairs are slower: 2x16x4096 252 / 283, 1x8x2048 21.7 / 35.8, 24x64x308 143 / 183.
+// Causal, couples that fill their rounds: 4x32x4096 555 / 527, 8x32x2048 336 / 308, 16x64x512 160 / 117, 32x32x256
+// 67 / 57: the pair kernel.  Other causal problems, with the pair kernel in its better order: 2x32(8)x2000 74 / 73,
+// 4x8x4096 144 / 144, 16x16(4)x1024 92 / 97, 1x64(8)x6000 569 / 577, 1x4x8192 67 / 123, 1x32(8)x1200 20.5 / 24.4: the
 // one-tile kernel, as for at most 128 queries, where every pair is half empty: 32x32x128 27.9 / 33.3, 37x16x128 18.5 / 20.7,
 // 32x32 100 over 1000 97.2 / 115.7, 16x37x17 13.9 / 14.9.
 bool choose_pair_kernel(const b200k_attention_args& a) {
