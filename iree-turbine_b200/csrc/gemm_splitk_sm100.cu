@@ -194,9 +194,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    // (lane 0, unlike the MMA issuer below: a share is a few stages that wait for memory, and picking this thread by
-    // elect.sync as well took 1 to 2 % longer: us, lane 0 / elect.sync, 200x1960x4304 11.52 / 11.65, fp8 10.72 / 10.92,
-    // 1x4096x4096 9.62 / 9.77, 16x4096x4096 10.01 / 10.16, 128x4096x14336 28.5 / 28.8; only 256x1024x4096 was faster, 8.35 / 8.05, 8.77 with neither)
+    // (lane 0, unlike the MMA issuer below: picking this thread by elect.sync as well took 1 to 2 % longer on most products of
+    // few rows.  us, lane 0 / elect.sync: 200x1960x4304 11.52 / 11.65, fp8 10.72 / 10.92, 1x4096x4096 9.62 / 9.77,
+    // 16x4096x4096 10.01 / 10.16, 128x4096x14336 28.5 / 28.8; but 5x5360x11600 28.2 / 27.9, 256x1024x4096 8.42 / 8.18)
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
