@@ -40,7 +40,7 @@ struct GemmParams {
   // 64-element blocks of a stage; else one 3-D load per block, which clips at R.
   int32_t a_blocks, b_blocks;
   int32_t vec_store_ok;
-  int32_t tma_store_ok;  // C is 16-byte aligned with a 16-byte-multiple row pitch: epilogue uses TMA stores
+  int32_t tma_store_ok;  // C's base, row pitch and row length are multiples of 16 bytes: epilogue uses TMA stores
   int32_t store_bytes;   // otherwise: widest store (2, 4 or 8 bytes) that C's base and pitches allow
   // Fused all-gather of a column shard: when num_peers > 0 every output tile is written with plain
   // 16-byte stores into each peer's full matrix (peer-mapped memory) at column peer_col0.

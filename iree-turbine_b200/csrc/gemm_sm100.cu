@@ -687,7 +687,8 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   for (int i = 0; i < 8; ++i) p.peers[i] = peers.c[i];
   if (peers.num > 0) p.vec_store_ok = 0;
 
-  p.tma_store_ok = p.vec_store_ok;
+  // the TMA unit clips a store at whole 16-byte pieces: where n ends inside one, it would write past column n
+  p.tma_store_ok = p.vec_store_ok && (a.n * out_es) % 16 == 0;
   const uint64_t c_bytes = reinterpret_cast<uintptr_t>(a.c) | static_cast<uint64_t>(a.ldc * out_es) |
                            static_cast<uint64_t>(p.c_batch_stride * out_es);
   p.store_bytes = c_bytes % 8 == 0 ? 8 : (c_bytes % 4 == 0 ? 4 : 2);

@@ -51,3 +51,15 @@ def test_silu_over_the_whole_range(n, k, split, bias_dtype):
     bound = (4 + 1.173 * x64.abs().clamp(max=104)) * 2.0 ** -23 * ref.abs() + 3e-37
     assert bool(((got[0] - ref).abs() <= bound)[finite].all())
     assert got[0, -3] == float("inf") and bool(got[0, -2:].isnan().all())
+
+
+# n ends 2 to 14 bytes into a 16-byte piece of a row whose pitch is a multiple of 16 bytes
+@pytest.mark.parametrize("n,ldc", [(6, 8), (33, 40), (130, 136), (515, 520)])
+@pytest.mark.parametrize("dtype,out_dtype", [(torch.float16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("tile_m,tile_n", [(128, 64), (128, 128), (128, 256), (256, 256)])
+def test_columns_past_n_are_not_written(n, ldc, dtype, out_dtype, tile_m, tile_n):
+    a, b = oracle.make_gemm_inputs(150, n, 136, dtype, seed=51)
+    c = torch.full((150, ldc), 7.0, dtype=out_dtype, device=DEV)
+    ops._launch_gemm(a.to(DEV), b.to(DEV), c[:, :n], None, None, tile_m=tile_m, tile_n=tile_n, split_k=1)
+    assert bool((c[:, n:] == 7.0).all())
+    oracle.assert_close_half(c[:, :n], oracle.gemm_nt(a, b), rtol=2e-2, atol=2e-2)
