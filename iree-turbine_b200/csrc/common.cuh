@@ -119,6 +119,27 @@ inline int launch_pdl(const char* what, void (*kfn)(P...), dim3 grid, dim3 block
   return launch_maybe_pdl(true, what, kfn, grid, block, smem, stream, static_cast<A&&>(args)...);
 }
 
+// launch_pdl in thread-block clusters of `ctas` CTAs; 1 = without.
+template <typename... P, typename... A>
+inline int launch_cluster(const char* what, void (*kfn)(P...), int ctas, dim3 grid, dim3 block, size_t smem,
+                          cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ctas > 1 ? 2 : 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kfn, static_cast<P>(args)...), what);
+}
+
 inline size_t dtype_size(int dt) {
   switch (dt) {
     case B200K_F16:

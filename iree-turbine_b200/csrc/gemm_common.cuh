@@ -11,7 +11,7 @@ namespace gemm_detail {
 constexpr int kBM = 128;
 constexpr int kBKBytes = 128;
 constexpr int kGemmThreads = 192;
-constexpr int kGroupM = 16;  // m-tiles per rasterisation group (keeps one wave's operands L2-resident)
+constexpr int kGroupRows = 2048;  // rows of a rasterisation group (keeps one wave's operands L2-resident)
 
 enum GemmKind : int { kKindF16 = 0, kKindBF16 = 1, kKindE4M3 = 2 };
 
@@ -22,8 +22,8 @@ struct GemmParams {
   int32_t* status;
   int64_t ldc;
   int32_t m, n;
-  int32_t tiles_m, tiles_n, num_kb;  // tiles_m counts MT * 128-row tiles, num_kb pipeline stages along K
-  int32_t stage_bytes;               // bytes the two loads of a pipeline stage bring
+  int32_t tiles_m, tiles_n, num_kb;  // tiles_m counts tiles of 128 rows, or 256 of a pair, num_kb pipeline stages along K
+  int32_t stage_bytes;               // bytes the loads of a pipeline stage bring, of both CTAs of a pair
   int32_t batch;                     // independent problems (tensor maps are 3-D: [batch][rows][k])
   int32_t split;                     // split-K kernel only: CTAs per tile (= cluster size) ...
   int32_t kb_per_split;              // ... each summing this many consecutive stages
@@ -59,17 +59,17 @@ struct PeerMaps {
   CUtensorMap m[8];
 };
 
-template <int BN, int MT>
+template <int BN, int CTAS>
 struct GemmSmem {
   // k-blocks (128 bytes of K) per pipeline stage.  The thread that issues the MMAs spends about 50 cycles
   // on each of a block's four and 280 more per stage on the barrier wait, the commit and the loop (measured
   // with that thread behind lane == 0; behind elect.sync an MMA of N = 64 takes it 49 cycles, see elect_one).  For a
   // tile whose MMAs execute in 64 cycles or less that thread, not the tensor core or the loads, set the
   // pace (480 cycles per block, for BN = 64 as for BN = 128), so those tiles take two blocks per stage.
-  static constexpr int kSub = MT == 1 && BN <= 128 ? 2 : 1;
-  static constexpr int kStages = MT == 2 ? 3 : (BN == 256 ? 4 : (BN == 128 ? 3 : 4));
-  static constexpr int kABytes = MT * kBM * kBKBytes;  // per k-block
-  static constexpr int kBBytes = BN * kBKBytes;
+  static constexpr int kSub = BN <= 128 ? 2 : 1;
+  static constexpr int kStages = CTAS == 2 ? 6 : (BN == 128 ? 3 : 4);
+  static constexpr int kABytes = kBM * kBKBytes;  // per k-block; a CTA of a pair holds its rows of A and its half of B
+  static constexpr int kBBytes = BN / CTAS * kBKBytes;
   static constexpr int kBOffset = kSub * kABytes;  // a stage: A blocks, then B blocks
   static constexpr int kStageBytes = kSub * (kABytes + kBBytes);
   // epilogue staging: eight 32-row x 128-byte buffers (TMA store source)
@@ -83,7 +83,9 @@ struct GemmSmem {
   static constexpr int kDynamic = kTotal + 1024;  // slack for 1024-byte alignment of the tiles
 };
 
+template <int ROWS>  // of a tile
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& tm, int& tn) {
+  constexpr int kGroupM = kGroupRows / ROWS;
   const int group_size = kGroupM * tiles_n;
   const int group = t / group_size;
   const int first_m = group * kGroupM;
@@ -93,15 +95,27 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   tn = r / gm;
 }
 
+// One box of a k-block of an operand.  CTAS == 2: counted on the barrier of the pair's leader.
+template <int CTAS>
+__device__ __forceinline__ void load_3d(uint8_t* dst, const CUtensorMap* tmap, uint64_t* bar, int c0, int c1, int c2) {
+  if constexpr (CTAS == 2)
+    tma_load_3d_pair(dst, tmap, cluster_map_shared(smem_u32(bar), 0), c0, c1, c2);
+  else
+    tma_load_3d(dst, tmap, bar, c0, c1, c2);
+}
+
 // One k-block of an MN-major operand: R rows or columns of the tile (64-element blocks 8 KB apart), 64 K-rows.
-template <int R>
+template <int R, int CTAS = 1>
 __device__ __forceinline__ void load_mn_major(uint8_t* dst, const CUtensorMap* tmap, uint64_t* bar, int r0, int k0, int bz,
                                               bool blocks) {
   if (blocks) {
-    tma_load_4d(dst, tmap, bar, 0, k0, r0 >> 6, bz);
+    if constexpr (CTAS == 2)
+      tma_load_4d_pair(dst, tmap, cluster_map_shared(smem_u32(bar), 0), 0, k0, r0 >> 6, bz);
+    else
+      tma_load_4d(dst, tmap, bar, 0, k0, r0 >> 6, bz);
   } else {
 #pragma unroll
-    for (int b = 0; b < R / 64; ++b) tma_load_3d(dst + b * 8192, tmap, bar, r0 + b * 64, k0, bz);
+    for (int b = 0; b < R / 64; ++b) load_3d<CTAS>(dst + b * 8192, tmap, bar, r0 + b * 64, k0, bz);
   }
 }
 

@@ -2,9 +2,14 @@
 // accumulators in tensor memory, persistent CTAs with double-buffered accumulators so the
 // epilogue of one tile overlaps the main loop of the next.
 //
-// Tile shapes.  A 128 x 256 tile needs 96 bytes of operands per tensor-core cycle, more than an
-// SM can pull from L2, so large problems use a 256 x 256 tile: two 128-row halves share each B
-// stage (64 bytes per cycle) at the price of a single, not double-buffered, accumulator set.
+// Tile shapes.  A CTA computes 128 x 64, 128 x 128 or 128 x 256, a pair of CTAs on two SMs 256 x 256: one
+// tcgen05.mma.cta_group::2 (M = 256) makes both tensor cores multiply the 128 rows of A that their own CTA loaded with
+// both halves of B, of which each CTA loaded one, so a pair fetches 32 KB per k-block and SM where 128 x 256 tiles fetch 48.
+// Both run their k-blocks at the tensor core's rate (512 cycles, counted inside the kernel at 2048^3, with the loads
+// and without them); what differs is the power that the traffic takes from the clock and the lines that
+// operands with odd row pitches touch.  128 x 256 / pair, us, launches back to back over changing operands: 2048^3 f16
+// 16.1 / 15.6, 2048x2048x4096 29.9 / 27.5, 3000x4352x3840 80.5 / 72, 8192^3 fp8 423 / 381 (256 x 256 tiles of one CTA,
+// with one accumulator set, which this pair took the place of: 400), 1761x6993x4272 fp8 76 / 58; but 2048x2048x512 7.05 / 7.8.
 //
 // CTA = 6 or 10 warps: warp 0 issues TMA loads, warp 1 owns tensor memory and issues the MMAs,
 // the others drain accumulators (one or two warps for each 32-lane quarter of tensor memory).
@@ -24,12 +29,24 @@ namespace {
 
 using namespace gemm_detail;
 
+template <int CTAS>
+__device__ __forceinline__ void commit(uint64_t* bar) {
+  if constexpr (CTAS == 2)
+    umma_commit_pair(bar);
+  else
+    umma_commit(bar);
+}
+
 // GEN = false: both operands K-major (A [M, K], B [N, K]); the issue path is all compile-time
 // offsets.  GEN = true (16-bit types only): either operand may be MN-major, chosen at run time
 // (p.a_mn, p.b_mn).  An MN-major operand is stored [K, R] with R contiguous; a pipeline stage holds
 // it as R / 64 blocks of 64 K-rows x 128 bytes (128-byte swizzle), one TMA box each; the UMMA
 // descriptor has LBO = 8 KB between the 64-element blocks, SBO = 1 KB between 8-row groups, and a
 // k-step of 16 rows advances 2 KB.  A stage has the same size either way.
+//
+// CTAS = 2: a pair of CTAs.  Each loads its own rows and stores its own; the leader's "stage loaded" barriers count the
+// bytes of both, its MMA thread issues for both, and its commits arrive in both.  The peer's epilogue warps report to
+// the leader's "accumulator drained" barriers.
 //
 // Epilogue warps: PARTS = 1, one per 32-lane quarter of tensor memory with two staging buffers, or PARTS = 2,
 // two that take turns at its pieces, with a buffer each.  Two where a warp has work of its own on a piece, a
@@ -38,20 +55,17 @@ using namespace gemm_detail;
 // 2048x2048x512 17.0 / 15.8.  One otherwise: a warp that waits for its only buffer costs 1 to 3 % (fp8 8192^3
 // 366 / 374, 4096^3 98 / 101), and SiLU is short enough for one (3000x4352x3840 79.6 / 79.9, 2048x2048x512 11.6 / 11.3,
 // 8000x1024x1024 24.8 / 24.8).
-template <int BN, int MT, int KIND, typename OutT, bool GEN, int PARTS>
+template <int BN, int CTAS, int KIND, typename OutT, bool GEN, int PARTS>
 __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     gemm_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const GemmParams p,
                    const __grid_constant__ PeerMaps peer_maps) {
-  using S = GemmSmem<BN, MT>;
+  using S = GemmSmem<BN, CTAS>;
   constexpr int kElemsPerStage = (KIND == kKindE4M3) ? 128 : 64;  // K elements in 128 bytes
   constexpr uint32_t kFmt = (KIND == kKindBF16) ? kFmtBF16 : (KIND == kKindF16 ? kFmtF16 : kFmtE4M3);
-  constexpr uint32_t kIdesc = make_idesc(kFmt, kFmt, kBM, BN, 0, 0);
-  constexpr uint32_t kTmemCols = 2 * BN;
-  // MT == 1: two accumulator buffers of BN columns (epilogue overlaps the next tile's main loop);
-  // MT == 2: one buffer holding the two 128-row halves side by side.
-  constexpr int kAccBufs = MT == 1 ? 2 : 1;
-  constexpr int kTileM = MT * kBM;
+  constexpr uint32_t kIdesc = make_idesc(kFmt, kFmt, CTAS * kBM, BN, 0, 0);
+  constexpr uint32_t kTmemCols = 2 * BN;  // two accumulators: the epilogue overlaps the next tile's main loop
+  constexpr int kTileM = CTAS * kBM;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -65,6 +79,9 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  const uint32_t rank = CTAS == 2 ? cluster_ctarank() : 0u;
+  const bool leader = rank == 0;
+
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::kStages; ++s) {
       mbar_init(full + s, 1);
@@ -72,7 +89,7 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull + a, 1);
-      mbar_init(tempty + a, 4 * PARTS);
+      mbar_init(tempty + a, 4 * PARTS * CTAS);
     }
     *abort_word = 0;
     fence_barrier_init();
@@ -82,11 +99,16 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     prefetch_tmap(&tmap_c);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, kTmemCols);
-    tmem_relinquish();
+    if constexpr (CTAS == 2) {
+      tmem_alloc_pair(tmem_slot, kTmemCols);
+    } else {
+      tmem_alloc(tmem_slot, kTmemCols);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (CTAS == 2) cluster_sync_all();  // the peer's barriers are there before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // Everything above touched no global memory, so under a programmatic dependent launch it ran
@@ -98,6 +120,7 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
 
   const int tiles_per_problem = p.tiles_m * p.tiles_n;
   const int num_tiles = tiles_per_problem * p.batch;  // tile t: problem t / tiles_per_problem
+  const int first_tile = blockIdx.x / CTAS, tile_step = gridDim.x / CTAS;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -105,31 +128,33 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = first_tile; t < num_tiles && ok; t += tile_step) {
         int tm, tn;
         const int bz = t / tiles_per_problem;
-        tile_coords(t - bz * tiles_per_problem, p.tiles_m, p.tiles_n, tm, tn);
+        tile_coords<kTileM>(t - bz * tiles_per_problem, p.tiles_m, p.tiles_n, tm, tn);
+        const int row0 = tm * kTileM + static_cast<int>(rank) * kBM;
+        const int col0 = tn * BN + static_cast<int>(rank) * (BN / CTAS);
         for (int kb = 0; kb < p.num_kb; ++kb) {
           if (!mbar_wait(empty + stage, phase ^ 1, abort_word)) {
             ok = false;
             break;
           }
           uint8_t* sa = smem + stage * S::kStageBytes;
-          mbar_arrive_expect_tx(full + stage, static_cast<uint32_t>(p.stage_bytes));
+          if (leader) mbar_arrive_expect_tx(full + stage, static_cast<uint32_t>(p.stage_bytes));
 #pragma unroll
           for (int sub = 0; sub < S::kSub; ++sub) {
             const int k0 = (kb * S::kSub + sub) * kElemsPerStage;
             uint8_t* da = sa + sub * S::kABytes;
             uint8_t* db = sa + S::kBOffset + sub * S::kBBytes;
             if (GEN && p.a_mn) {
-              load_mn_major<kTileM>(da, &tmap_a, full + stage, tm * kTileM, k0, bz, p.a_blocks != 0);
+              load_mn_major<kBM, CTAS>(da, &tmap_a, full + stage, row0, k0, bz, p.a_blocks != 0);
             } else {
-              tma_load_3d(da, &tmap_a, full + stage, k0, tm * kTileM, bz);
+              load_3d<CTAS>(da, &tmap_a, full + stage, k0, row0, bz);
             }
             if (GEN && p.b_mn) {
-              load_mn_major<BN>(db, &tmap_b, full + stage, tn * BN, k0, bz, p.b_blocks != 0);
+              load_mn_major<BN / CTAS, CTAS>(db, &tmap_b, full + stage, col0, k0, bz, p.b_blocks != 0);
             } else {
-              tma_load_3d(db, &tmap_b, full + stage, k0, tn * BN, bz);
+              load_3d<CTAS>(db, &tmap_b, full + stage, k0, col0, bz);
             }
           }
           if (++stage == S::kStages) {
@@ -141,8 +166,8 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (elect_one()) {
+    // ---------------- MMA issuer (of a pair: the leader's) ----------------
+    if (leader && elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -163,15 +188,15 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
       const uint32_t step_a = (GEN && p.a_mn) ? (2048u >> 4) : 2u;
       const uint32_t step_b = (GEN && p.b_mn) ? (2048u >> 4) : 2u;
       const uint32_t idesc = GEN ? (kIdesc | (p.a_mn ? 1u << 15 : 0u) | (p.b_mn ? 1u << 16 : 0u)) : kIdesc;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
-        const int acc = it % kAccBufs;
-        const uint32_t acc_phase = (it / kAccBufs) & 1;
+      for (int t = first_tile; t < num_tiles && ok; t += tile_step, ++it) {
+        const int acc = it & 1;
+        const uint32_t acc_phase = (it >> 1) & 1;
         if (!mbar_wait(tempty + acc, acc_phase ^ 1, abort_word)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (MT == 1 ? acc * BN : 0);
+        const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           if (!mbar_wait(full + stage, phase, abort_word)) {
             ok = false;
@@ -186,29 +211,27 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
             const int sub = sk >> 2, k = sk & 3;
             const uint32_t accum = sk == 0 ? accum0 : 1u;
             const uint32_t a_sub = a_lo + sub * (S::kABytes >> 4), b_sub = b_lo + sub * (S::kBBytes >> 4);
-#pragma unroll
-            for (int h = 0; h < MT; ++h) {
-              if constexpr (GEN) {
-                const uint64_t a_desc = desc(a_sub + h * ((kBM * kBKBytes) >> 4) + step_a * k, hi_a);
-                const uint64_t b_desc = desc(b_sub + step_b * k, hi_b);
-                umma_f16_ss(d_tmem + h * BN, a_desc, b_desc, idesc, accum);
-              } else {
-                const uint64_t a_desc = desc(a_sub + h * ((kBM * kBKBytes) >> 4) + 2 * k, hi);
-                const uint64_t b_desc = desc(b_sub + 2 * k, hi);
-                if constexpr (KIND == kKindE4M3)
-                  umma_f8_ss(d_tmem + h * BN, a_desc, b_desc, kIdesc, accum);
-                else
-                  umma_f16_ss(d_tmem + h * BN, a_desc, b_desc, kIdesc, accum);
-              }
+            const uint64_t a_desc = desc(a_sub + (GEN ? step_a : 2u) * k, GEN ? hi_a : hi);
+            const uint64_t b_desc = desc(b_sub + (GEN ? step_b : 2u) * k, GEN ? hi_b : hi);
+            if constexpr (CTAS == 2) {
+              if constexpr (KIND == kKindE4M3)
+                umma_pair_f8_ss(d_tmem, a_desc, b_desc, kIdesc, accum);
+              else
+                umma_pair_f16_ss(d_tmem, a_desc, b_desc, GEN ? idesc : kIdesc, accum);
+            } else {
+              if constexpr (KIND == kKindE4M3)
+                umma_f8_ss(d_tmem, a_desc, b_desc, kIdesc, accum);
+              else
+                umma_f16_ss(d_tmem, a_desc, b_desc, GEN ? idesc : kIdesc, accum);
             }
           }
-          umma_commit(empty + stage);  // frees the stage once these MMAs have read it
+          commit<CTAS>(empty + stage);  // frees the stage once these MMAs have read it
           if (++stage == S::kStages) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) umma_commit(tfull + acc);  // accumulator complete
+        if (ok) commit<CTAS>(tfull + acc);  // accumulator complete
       }
     }
     __syncwarp();
@@ -228,12 +251,12 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     uint8_t* staging = smem + S::kStagingOffset + (warp - 2) * (kBufsPerWarp * 4096);
     uint32_t stg_count = 0;
     int it = 0;
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+    for (int t = first_tile; t < num_tiles; t += tile_step, ++it) {
       int tm, tn;
       const int bz = t / tiles_per_problem;
-      tile_coords(t - bz * tiles_per_problem, p.tiles_m, p.tiles_n, tm, tn);
-      const int acc = it % kAccBufs;
-      const uint32_t acc_phase = (it / kAccBufs) & 1;
+      tile_coords<kTileM>(t - bz * tiles_per_problem, p.tiles_m, p.tiles_n, tm, tn);
+      const int acc = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
       // The tile's bias, fetched while the main loop runs (columns past n re-read the last one: never stored).
       constexpr int kEpiThreads = 128 * PARTS;
       constexpr int kBiasPerThread = (BN + kEpiThreads - 1) / kEpiThreads;
@@ -258,99 +281,100 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
         if (!ok) break;
       }
       tc_fence_after();
-#pragma unroll
-      for (int h = 0; h < MT; ++h) {
-        const int row0 = tm * kTileM + h * kBM + quarter * 32;
-        const uint32_t taddr =
-            tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (MT == 1 ? acc * BN : h * BN);
-        // 128 bytes of each of this warp's 32 rows per step: registers -> swizzled staging buffer ->
-        // C.  A buffer is reused once its store has been read.
-        constexpr int kCols = 128 / static_cast<int>(sizeof(OutT));
-        const bool by_tma = p.tma_store_ok || p.peer_tma;
+      const int row0 = tm * kTileM + static_cast<int>(rank) * kBM + quarter * 32;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+      // 128 bytes of each of this warp's 32 rows per step: registers -> swizzled staging buffer ->
+      // C.  A buffer is reused once its store has been read.
+      constexpr int kCols = 128 / static_cast<int>(sizeof(OutT));
+      const bool by_tma = p.tma_store_ok || p.peer_tma;
 #pragma unroll 1
-        for (int c = part; c < BN / kCols; c += PARTS) {
-          const int col = tn * BN + c * kCols;
-          if (col >= p.n) break;
-          uint8_t* buf = staging + stg_count % kBufsPerWarp * 4096;
-          uint32_t r[kCols];
-          uint4 v[8];
-          if constexpr (kCols == 32)
-            tmem_ld_32x32b_x32(taddr + c * 32, r);
-          else
-            tmem_ld_32x32b_x64(taddr + c * 64, r);
-          if (by_tma && lane == 0) tma_store_wait_read<kBufsPerWarp - 1>();
-          tmem_wait_ld();
-          if (fused) {
-            fused_epilogue<kCols>(r, scale, bias_s + c * kCols, p.act);
-            pack_row<OutT>(r, 1.f, v);
-          } else {
-            pack_row<OutT>(r, scale, v);
-          }
-          __syncwarp();  // the buffer is free: its last bulk store has been read, or its last reads by this warp are done
+      for (int c = part; c < BN / kCols; c += PARTS) {
+        const int col = tn * BN + c * kCols;
+        if (col >= p.n) break;
+        uint8_t* buf = staging + stg_count % kBufsPerWarp * 4096;
+        uint32_t r[kCols];
+        uint4 v[8];
+        if constexpr (kCols == 32)
+          tmem_ld_32x32b_x32(taddr + c * 32, r);
+        else
+          tmem_ld_32x32b_x64(taddr + c * 64, r);
+        if (by_tma && lane == 0) tma_store_wait_read<kBufsPerWarp - 1>();
+        tmem_wait_ld();
+        if (fused) {
+          fused_epilogue<kCols>(r, scale, bias_s + c * kCols, p.act);
+          pack_row<OutT>(r, 1.f, v);
+        } else {
+          pack_row<OutT>(r, scale, v);
+        }
+        __syncwarp();  // the buffer is free: its last bulk store has been read, or its last reads by this warp are done
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            *reinterpret_cast<uint4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4)) = v[i];
-          if (by_tma) {
-            // One TMA store (full 128-byte lines, clipped at the matrix edge by the tensor map).
-            // Fused all-gather: the same piece goes out once per rank, through that rank's map, as
-            // bulk stores to peer-mapped memory; the copy engine of the SM moves the data while the
-            // warp prepares the next piece.
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              if (p.num_peers > 0) {
+        for (int i = 0; i < 8; ++i)
+          *reinterpret_cast<uint4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4)) = v[i];
+        if (by_tma) {
+          // One TMA store (full 128-byte lines, clipped at the matrix edge by the tensor map).
+          // Fused all-gather: the same piece goes out once per rank, through that rank's map, as
+          // bulk stores to peer-mapped memory; the copy engine of the SM moves the data while the
+          // warp prepares the next piece.
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (p.num_peers > 0) {
+              int pe = p.peer_first;
+              for (int i = 0; i < p.num_peers; ++i) {
+                tma_store_2d(&peer_maps.m[pe], buf, col, row0);
+                pe = pe + 1 == p.num_peers ? 0 : pe + 1;
+              }
+            } else {
+              tma_store_3d(&tmap_c, buf, col, row0, bz);
+            }
+            tma_store_commit();
+          }
+        } else if (p.num_peers > 0) {
+          // Column shard written straight into every rank's full C (own copy included): each store
+          // instruction writes four full 128-byte row segments to one peer, so the NVLink traffic is
+          // made of whole lines.
+          __syncwarp();
+          const int chunk = lane & 7;
+          const int ecol = col + chunk * (16 / static_cast<int>(sizeof(OutT)));  // column inside the shard
+#pragma unroll
+          for (int rr = 0; rr < 8; ++rr) {
+            const int lr = rr * 4 + (lane >> 3);
+            const int grow = row0 + lr;
+            const uint4 val = *reinterpret_cast<const uint4*>(buf + lr * 128 + ((chunk ^ (lr & 7)) << 4));
+            if (grow < p.m && ecol < p.n) {
+              const int64_t off = (static_cast<int64_t>(grow) * p.peer_ldc + p.peer_col0 + ecol) *
+                                  static_cast<int64_t>(sizeof(OutT));
+              if (p.peer_mc) {
+                // one store to the multicast address: the switch writes every rank's copy
+                asm volatile("multimem.st.weak.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(
+                                 reinterpret_cast<uint8_t*>(p.peer_mc) + off),
+                             "f"(__uint_as_float(val.x)), "f"(__uint_as_float(val.y)), "f"(__uint_as_float(val.z)),
+                             "f"(__uint_as_float(val.w))
+                             : "memory");
+              } else {
                 int pe = p.peer_first;
                 for (int i = 0; i < p.num_peers; ++i) {
-                  tma_store_2d(&peer_maps.m[pe], buf, col, row0);
+                  *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.peers[pe]) + off) = val;
                   pe = pe + 1 == p.num_peers ? 0 : pe + 1;
                 }
-              } else {
-                tma_store_3d(&tmap_c, buf, col, row0, bz);
-              }
-              tma_store_commit();
-            }
-          } else if (p.num_peers > 0) {
-            // Column shard written straight into every rank's full C (own copy included): each store
-            // instruction writes four full 128-byte row segments to one peer, so the NVLink traffic is
-            // made of whole lines.
-            __syncwarp();
-            const int chunk = lane & 7;
-            const int ecol = col + chunk * (16 / static_cast<int>(sizeof(OutT)));  // column inside the shard
-#pragma unroll
-            for (int rr = 0; rr < 8; ++rr) {
-              const int lr = rr * 4 + (lane >> 3);
-              const int grow = row0 + lr;
-              const uint4 val = *reinterpret_cast<const uint4*>(buf + lr * 128 + ((chunk ^ (lr & 7)) << 4));
-              if (grow < p.m && ecol < p.n) {
-                const int64_t off = (static_cast<int64_t>(grow) * p.peer_ldc + p.peer_col0 + ecol) *
-                                    static_cast<int64_t>(sizeof(OutT));
-                if (p.peer_mc) {
-                  // one store to the multicast address: the switch writes every rank's copy
-                  asm volatile("multimem.st.weak.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(
-                                   reinterpret_cast<uint8_t*>(p.peer_mc) + off),
-                               "f"(__uint_as_float(val.x)), "f"(__uint_as_float(val.y)), "f"(__uint_as_float(val.z)),
-                               "f"(__uint_as_float(val.w))
-                               : "memory");
-                } else {
-                  int pe = p.peer_first;
-                  for (int i = 0; i < p.num_peers; ++i) {
-                    *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.peers[pe]) + off) = val;
-                    pe = pe + 1 == p.num_peers ? 0 : pe + 1;
-                  }
-                }
               }
             }
-          } else {
-            __syncwarp();
-            store_piece_any<OutT>(cbase + bz * p.c_batch_stride + static_cast<int64_t>(row0) * p.ldc + col, p.ldc, buf,
-                                  lane, p.m - row0, p.n - col, p.store_bytes);
           }
-          ++stg_count;
+        } else {
+          __syncwarp();
+          store_piece_any<OutT>(cbase + bz * p.c_batch_stride + static_cast<int64_t>(row0) * p.ldc + col, p.ldc, buf,
+                                lane, p.m - row0, p.n - col, p.store_bytes);
         }
+        ++stg_count;
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(tempty + acc);
+      if (lane == 0) {
+        if constexpr (CTAS == 2)
+          mbar_arrive_cluster(cluster_map_shared(smem_u32(tempty + acc), 0));
+        else
+          mbar_arrive(tempty + acc);
+      }
     }
     // Staging memory must outlive the last stores; those to this GPU's memory complete before the grid does.  Stores to
     // peers are waited for themselves: a barrier between ranks follows the kernel, and their writes must be done by then.
@@ -375,63 +399,67 @@ __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
     if (threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusGemmTimeout);
     __syncthreads();
   }
+  if constexpr (CTAS == 2) cluster_sync_all();  // nothing of the peer's is touched from here on
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    if constexpr (CTAS == 2)
+      tmem_dealloc_pair(tmem_base, kTmemCols);
+    else
+      tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
-template <int BN, int MT, int KIND, typename OutT, bool GEN, int PARTS>
+template <int BN, int CTAS, int KIND, typename OutT, bool GEN, int PARTS>
 int launch_parts(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
                const PeerMaps& pm, int grid, cudaStream_t stream) {
-  using S = GemmSmem<BN, MT>;
-  auto kfn = gemm_nt_kernel<BN, MT, KIND, OutT, GEN, PARTS>;
+  using S = GemmSmem<BN, CTAS>;
+  auto kfn = gemm_nt_kernel<BN, CTAS, KIND, OutT, GEN, PARTS>;
   static bool configured[64] = {};  // per instantiation and device ordinal
   int rc = ensure_dynamic_smem(kfn, S::kDynamic, configured, "cudaFuncSetAttribute(gemm smem)");
   if (rc) return rc;
   // Programmatic dependent launch: barrier set-up and the tensor-memory allocation of this kernel
   // overlap the tail of whatever runs before it in the stream (see grid_dependency_wait in the kernel).
-  return launch_pdl("gemm_nt_kernel launch", kfn, dim3(static_cast<unsigned>(grid)), dim3(64 + 128 * PARTS), S::kDynamic, stream,
-                    ta, tb, tc, p, pm);
+  return launch_cluster("gemm_nt_kernel launch", kfn, CTAS, dim3(static_cast<unsigned>(grid)), dim3(64 + 128 * PARTS), S::kDynamic, stream,
+                        ta, tb, tc, p, pm);
 }
 
-template <int BN, int MT, int KIND, typename OutT, bool GEN = false>
+template <int BN, int CTAS, int KIND, typename OutT, bool GEN = false>
 int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
                const PeerMaps& pm, int grid, cudaStream_t stream) {
   // which of the two: see the kernel
   const bool by_tma = p.tma_store_ok || p.peer_tma;
   const bool own_work = p.act == B200K_ACT_GELU || (p.bias != nullptr && p.act != B200K_ACT_SILU);
-  if (own_work || !by_tma) return launch_parts<BN, MT, KIND, OutT, GEN, 2>(ta, tb, tc, p, pm, grid, stream);
-  return launch_parts<BN, MT, KIND, OutT, GEN, 1>(ta, tb, tc, p, pm, grid, stream);
+  if (own_work || !by_tma) return launch_parts<BN, CTAS, KIND, OutT, GEN, 2>(ta, tb, tc, p, pm, grid, stream);
+  return launch_parts<BN, CTAS, KIND, OutT, GEN, 1>(ta, tb, tc, p, pm, grid, stream);
 }
 
-template <int BN, int MT>
+template <int BN, int CTAS>
 int dispatch_dtype(int in_dtype, int out_dtype, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
                    const GemmParams& p, const PeerMaps& pm, int grid, cudaStream_t stream) {
   if (p.a_mn || p.b_mn) {  // generic operand storage: 16-bit types
     if (in_dtype == B200K_F16 && out_dtype == B200K_F32)
-      return launch_one<BN, MT, kKindF16, float, true>(ta, tb, tc, p, pm, grid, stream);
+      return launch_one<BN, CTAS, kKindF16, float, true>(ta, tb, tc, p, pm, grid, stream);
     if (in_dtype == B200K_F16 && out_dtype == B200K_F16)
-      return launch_one<BN, MT, kKindF16, __half, true>(ta, tb, tc, p, pm, grid, stream);
+      return launch_one<BN, CTAS, kKindF16, __half, true>(ta, tb, tc, p, pm, grid, stream);
     if (in_dtype == B200K_BF16 && out_dtype == B200K_F32)
-      return launch_one<BN, MT, kKindBF16, float, true>(ta, tb, tc, p, pm, grid, stream);
+      return launch_one<BN, CTAS, kKindBF16, float, true>(ta, tb, tc, p, pm, grid, stream);
     if (in_dtype == B200K_BF16 && out_dtype == B200K_BF16)
-      return launch_one<BN, MT, kKindBF16, __nv_bfloat16, true>(ta, tb, tc, p, pm, grid, stream);
+      return launch_one<BN, CTAS, kKindBF16, __nv_bfloat16, true>(ta, tb, tc, p, pm, grid, stream);
     return set_error(B200K_ERR_BAD_DTYPE, "gemm: operands stored [K, M] / [K, N] need F16 or BF16 (in=%d out=%d)",
                      in_dtype, out_dtype);
   }
   if (in_dtype == B200K_F16 && out_dtype == B200K_F32)
-    return launch_one<BN, MT, kKindF16, float>(ta, tb, tc, p, pm, grid, stream);
+    return launch_one<BN, CTAS, kKindF16, float>(ta, tb, tc, p, pm, grid, stream);
   if (in_dtype == B200K_F16 && out_dtype == B200K_F16)
-    return launch_one<BN, MT, kKindF16, __half>(ta, tb, tc, p, pm, grid, stream);
+    return launch_one<BN, CTAS, kKindF16, __half>(ta, tb, tc, p, pm, grid, stream);
   if (in_dtype == B200K_BF16 && out_dtype == B200K_F32)
-    return launch_one<BN, MT, kKindBF16, float>(ta, tb, tc, p, pm, grid, stream);
+    return launch_one<BN, CTAS, kKindBF16, float>(ta, tb, tc, p, pm, grid, stream);
   if (in_dtype == B200K_BF16 && out_dtype == B200K_BF16)
-    return launch_one<BN, MT, kKindBF16, __nv_bfloat16>(ta, tb, tc, p, pm, grid, stream);
+    return launch_one<BN, CTAS, kKindBF16, __nv_bfloat16>(ta, tb, tc, p, pm, grid, stream);
   if (in_dtype == B200K_E4M3 && out_dtype == B200K_BF16)
-    return launch_one<BN, MT, kKindE4M3, __nv_bfloat16>(ta, tb, tc, p, pm, grid, stream);
+    return launch_one<BN, CTAS, kKindE4M3, __nv_bfloat16>(ta, tb, tc, p, pm, grid, stream);
   if (in_dtype == B200K_E4M3 && out_dtype == B200K_F32)
-    return launch_one<BN, MT, kKindE4M3, float>(ta, tb, tc, p, pm, grid, stream);
+    return launch_one<BN, CTAS, kKindE4M3, float>(ta, tb, tc, p, pm, grid, stream);
   return set_error(B200K_ERR_BAD_DTYPE, "gemm_nt: unsupported dtype pair in=%d out=%d", in_dtype, out_dtype);
 }
 
@@ -525,28 +553,34 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   const int sms = num_sms();
   const int k_per_stage = a.in_dtype == B200K_E4M3 ? 128 : 64;
   const int64_t num_kb = (a.k + k_per_stage - 1) / k_per_stage;
-  // Tile shape and split: the smallest estimated time, in us.  Measured on 27 shapes (rows 1 to 6000, K 300
-  // to 16000, operands from HBM, launches back to back) a launch of whole tiles takes
-  //   fixed + waves * k-blocks * per_kb,        per_kb .20 / .25 / .39 / .62 us for 128 x 64 / 128 x 128 /
-  // 128 x 256 / 256 x 256 tiles (the first three set by the issuing thread, then behind lane == 0, and by what an SM
-  // can pull from L2, the last by the tensor core), plus about 3 us a wave for the last one's epilogue, which nothing
-  // overlaps.  Rows that do not start on 128-byte lines cost the narrower tiles some 15 % more L2 traffic.
+  // Tile shape and split: the smallest estimated time, in us.  A launch of whole tiles takes
+  //   fixed + waves * (k-blocks * per_kb + wave),
+  // fitted to 27 shapes for the tiles of one CTA (rows 1 to 6000, K 300 to 16000, operands from HBM, launches back to
+  // back) and to 73 more for the 256 x 256 tiles of a pair (74 pairs to a wave).  k-blocks of 128 x 256 and pair tiles
+  // run at the tensor core's 512 cycles, at the 1.45 to 1.65 GHz that the SMs keep while all of them multiply; `wave`
+  // is the part of an epilogue that the next tile does not hide.  Operand rows that do not start on 128-byte lines cost
+  // more L2 traffic (`lines`), rows of C that the TMA unit cannot store a longer epilogue (`ragged`).  What the choice gives on
+  // the 73 shapes, against the former one with 256 x 256 tiles of one CTA, is 4.7 % in the mean (the best of all
+  // tiles for each: 5.4 %); 1761x6993x4272 fp8 80.5 -> 58.2, 5034x2320x4680 [K, N] 119 -> 95, 1979x3384x2448 35.0 -> 31.2.
   // Split-K over a cluster of s CTAs is not persistent: every wave of resident clusters pays
   //   fixed + k-blocks / s * per_kb + (partial tiles to shared memory, two cluster barriers, reduction),
   // the last term 1 us plus 1.4 / 2 / 4 us for a tile of 128 rows.
   struct Shape {
     int m, n;
-    double fixed, per_kb, wave, reduce;
+    double fixed, per_kb, lines, wave, ragged, reduce;
   };
-  const double lines = (a.lda * in_es) % 128 != 0 || (a.ldb * in_es) % 128 != 0 ? 1.15 : 1.0;
-  const Shape kShapes[4] = {{128, 64, 3.4, .20 * lines, 0., 1.4},
-                            {128, 128, 3.7, .25 * lines, 0., 2.},
-                            {128, 256, 4.5, .39 * lines, 0., 4.},
-                            {256, 256, 4.5, .62, 3., 0.}};
+  const bool lines = (a.lda * in_es) % 128 != 0 || (a.ldb * in_es) % 128 != 0;
+  const bool ragged = peers.num == 0 && ((reinterpret_cast<uintptr_t>(a.c) & 15) != 0 || (a.ldc * out_es) % 16 != 0 || (a.n * out_es) % 16 != 0);
+  const Shape kShapes[4] = {{128, 64, 3.4, .20, 1.15, 0., .5, 1.4},
+                            {128, 128, 3.7, .25, 1.15, 0., 1., 2.},
+                            {128, 256, 4.5, .39, 1.15, 0., 2., 4.},
+                            {256, 256, 4.5, .28, 1.1, 1., 3., 0.}};
+  auto per_kb = [&](const Shape& t) { return t.per_kb * (lines ? t.lines : 1.); };
   auto tiles_of = [&](const Shape& t) { return ((a.m + t.m - 1) / t.m) * ((a.n + t.n - 1) / t.n) * batch; };
   auto whole_us = [&](const Shape& t) {
-    const int64_t waves = (tiles_of(t) + sms - 1) / sms;
-    return t.fixed + static_cast<double>(waves) * (num_kb * t.per_kb + t.wave);
+    const int64_t units = t.m == 256 ? sms / 2 : sms;
+    const int64_t waves = (tiles_of(t) + units - 1) / units;
+    return t.fixed + static_cast<double>(waves) * (num_kb * per_kb(t) + t.wave + (ragged ? t.ragged : 0.));
   };
   int bm = a.tile_m, bn = a.tile_n;
   if (bm == 256 && bn == 0) bn = 256;
@@ -575,7 +609,7 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
         if (resident == 0) continue;
         const int64_t waves = (tiles_of(t) + resident - 1) / resident;
         if (waves > 4) continue;
-        const double su = static_cast<double>(waves) * (t.fixed + static_cast<double>((num_kb + s - 1) / s) * t.per_kb + 1. + rows * t.reduce);
+        const double su = static_cast<double>(waves) * (t.fixed + static_cast<double>((num_kb + s - 1) / s) * per_kb(t) + 1. + rows * t.reduce);
         if (su < best_us) {
           best_us = su;
           bm = 128;
@@ -592,7 +626,7 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   // sending the shard takes longer than computing it (measured on 4 / 8 GPUs: 104 / 56 us of math,
   // about 110 / 190 us of stores), 128-row tiles with their two accumulator sets let the stores of
   // one tile run under the main loop of the next and start after a quarter of the time of a
-  // 256 x 256 tile (4 GPUs: 214 us per step against 222).
+  // 256 x 256 tile of one CTA (4 GPUs: 214 us per step against 222).
   if (peers.num > 1 && a.tile_m == 0 && a.tile_n == 0 && a.n > 128) {
     const double send_us = static_cast<double>(peers.num - 1) * a.m * a.n * out_es / 600e3;
     const double peak_tflops = a.in_dtype == B200K_E4M3 ? 3000.0 : 1500.0;
@@ -621,7 +655,9 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   auto box_rows = [](int64_t rows, int tile) {
     return static_cast<int>(rows < tile ? (rows + 7) / 8 * 8 : tile);
   };
-  const int box_m = a_mn ? bm : box_rows(a.m, bm), box_n = b_mn ? bn : box_rows(a.n, bn);
+  const int ctas = bm == 256 ? 2 : 1;
+  const int load_m = bm / ctas, load_n = bn / ctas;  // what one CTA loads
+  const int box_m = a_mn ? load_m : box_rows(a.m, load_m), box_n = b_mn ? load_n : box_rows(a.n, load_n);
   const bool a_blocks = a_mn && a.m % 64 == 0, b_blocks = b_mn && a.n % 64 == 0;
   // Operand map.  K-major: a box is the tile's rows x 128 bytes of K.  MN-major ([K, R] storage): 64
   // contiguous R-elements x 64 K-rows, of one 64-element block or of all blocks of the tile.
@@ -642,9 +678,9 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
     return encode_tmap(tm, a.in_dtype, 3, const_cast<void*>(base), dims, strides, bx);
   };
   CUtensorMap ta, tb;
-  rc = encode_operand(&ta, a.a, a.m, a.lda, a.a_batch_stride, a_mn, a_blocks, bm, box_m);
+  rc = encode_operand(&ta, a.a, a.m, a.lda, a.a_batch_stride, a_mn, a_blocks, load_m, box_m);
   if (rc) return rc;
-  rc = encode_operand(&tb, a.b, a.n, a.ldb, a.b_batch_stride, b_mn, b_blocks, bn, box_n);
+  rc = encode_operand(&tb, a.b, a.n, a.ldb, a.b_batch_stride, b_mn, b_blocks, load_n, box_n);
   if (rc) return rc;
 
   GemmParams p;
@@ -667,7 +703,7 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   const int sub = bm == 128 && bn <= 128 ? GemmSmem<128, 1>::kSub : 1;  // k-blocks per pipeline stage
   const int64_t num_stages = (num_kb + sub - 1) / sub;
   p.num_kb = static_cast<int32_t>(num_stages);
-  p.stage_bytes = sub * (box_m + box_n) * kBKBytes;
+  p.stage_bytes = ctas * sub * (box_m + box_n) * kBKBytes;
   p.kb_per_split = static_cast<int32_t>((num_stages + split - 1) / split);
   // every slice must hold at least one stage (an empty one would leave an accumulator unwritten)
   while (split > 1 && static_cast<int64_t>(p.kb_per_split) * (split - 1) >= num_stages) {
@@ -725,7 +761,8 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
     if (num_tiles * split > INT32_MAX) return set_error(B200K_ERR_BAD_SHAPE, "gemm: too many tiles");
     return launch_gemm_splitk(ta, tb, p, bn, a.in_dtype, a.out_dtype, stream);
   }
-  const int grid = static_cast<int>(num_tiles < sms ? num_tiles : sms);
+  const int units = sms / ctas;
+  const int grid = ctas * static_cast<int>(num_tiles < units ? num_tiles : units);
   if (bm == 256) return dispatch_dtype<256, 2>(a.in_dtype, a.out_dtype, ta, tb, tc, p, pm, grid, stream);
   if (bn == 256) return dispatch_dtype<256, 1>(a.in_dtype, a.out_dtype, ta, tb, tc, p, pm, grid, stream);
   if (bn == 64) return dispatch_dtype<64, 1>(a.in_dtype, a.out_dtype, ta, tb, tc, p, pm, grid, stream);

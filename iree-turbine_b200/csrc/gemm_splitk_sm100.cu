@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int tile = static_cast<int>(blockIdx.x) / p.split;
   const int bz = tile / tiles_per_problem;
   int tm, tn;
-  tile_coords(tile - bz * tiles_per_problem, p.tiles_m, p.tiles_n, tm, tn);
+  tile_coords<kBM>(tile - bz * tiles_per_problem, p.tiles_m, p.tiles_n, tm, tn);
   const int kb_begin = rank * p.kb_per_split;
   const int kb_end = min(p.num_kb, kb_begin + p.kb_per_split);
   const bool a_mn = KIND != kKindE4M3 && p.a_mn != 0;

@@ -1,0 +1,68 @@
+"""256 x 256 tiles computed by pairs of CTAs: the bits of the 128 x 256 tiles of one CTA, which the oracle checks elsewhere.
+
+Both sum every output over the same k-steps in the same order, so the comparison is exact.
+"""
+import pytest
+import torch
+
+from iree_turbine_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _operand(rows, k, dtype, stored_kn, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    t = torch.randn((k, rows) if stored_kn else (rows, k), generator=g, device=DEV)
+    return t.to(dtype)
+
+
+def _both(m, n, k, dtype, out_dtype, a_km=False, b_kn=False, ldc=None, **kw):
+    a, b = _operand(m, k, dtype, a_km, 1), _operand(n, k, dtype, b_kn, 2)
+    got = []
+    for tile_m in (256, 128):
+        c = torch.full((m, ldc or n), 7.0, dtype=out_dtype, device=DEV)
+        ops._launch_gemm(a, b, c[:, :n], None, None, tile_m=tile_m, tile_n=256, split_k=1, a_km=a_km, b_kn=b_kn, **kw)
+        got.append(c)
+    assert bool((got[0][:, n:] == 7.0).all()), "columns past n were written"
+    return got
+
+
+# one tile and less, both sides of 128 and 256 rows and columns, K tails and fewer k-blocks than stages,
+# and lists of more than 74 tiles (pairs that run several, with both accumulators)
+SIZES = [(1, 8, 8), (128, 256, 64), (129, 257, 72), (255, 120, 1000), (256, 128, 448), (300, 264, 384), (513, 1040, 200),
+         (2305, 2304, 136), (4100, 3000, 64)]
+
+
+@pytest.mark.parametrize("m,n,k", SIZES)
+@pytest.mark.parametrize("dtype,out_dtype", [(torch.float16, torch.float32), (torch.bfloat16, torch.bfloat16),
+                                             (torch.float8_e4m3fn, torch.bfloat16)])
+def test_same_bits_as_one_cta(m, n, k, dtype, out_dtype):
+    if dtype == torch.float8_e4m3fn:
+        k = -(-k // 16) * 16
+    pair, one = _both(m, n, k, dtype, out_dtype)
+    assert torch.equal(pair, one)
+
+
+@pytest.mark.parametrize("m,n,k", [(136, 264, 72), (256, 512, 512), (2304, 2312, 200)])
+@pytest.mark.parametrize("a_km,b_kn", [(False, True), (True, False), (True, True)])
+def test_storage_orders(m, n, k, a_km, b_kn):
+    pair, one = _both(m, n, k, torch.bfloat16, torch.float32, a_km=a_km, b_kn=b_kn)
+    assert torch.equal(pair, one)
+
+
+@pytest.mark.parametrize("activation", ["none", "gelu", "silu"])
+@pytest.mark.parametrize("ldc", [520, 517])
+def test_epilogues(activation, ldc):
+    """Bias and activation, rows that the TMA unit stores and rows that it cannot."""
+    bias = torch.randn(515, device=DEV)
+    pair, one = _both(2400, 515, 264, torch.float16, torch.float16, ldc=ldc, bias=bias, activation=activation)
+    assert torch.equal(pair, one)
+
+
+def test_batched_and_chosen():
+    """A batch of problems whose tiles are pairs by the library's own choice: each the bits of its own call."""
+    a, b = (torch.randn(3, 2048, 2048, device=DEV).to(torch.bfloat16) for _ in range(2))
+    out = torch.ops.b200k.bmm(a, b.transpose(1, 2))
+    for i in range(3):
+        assert torch.equal(out[i], torch.ops.b200k.gemm_nt(a[i], b[i], torch.float32))
