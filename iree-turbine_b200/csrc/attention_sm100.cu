@@ -989,6 +989,31 @@ bool choose_pair_kernel(const b200k_paged_attention_args& a) {
   return pairs > num_sms() || !tiles_finish_first(a, static_cast<int>(heads), static_cast<int>(per_head));
 }
 
+// CTAs that share the K/V tiles of each item of a call (the one-tile kernel in clusters), 1 = one CTA per item.  Few items
+// leave SMs idle while each item is one chain of K/V tiles: 2x2 164 queries over 4652 keys, page size 16, 71.8 us by one CTA
+// per item, 44.8 / 27.4 / 17.8 by clusters of 2 / 4 / 8; 1x16(4) 29 over 3244, page size 32, 42.2, 24.9 / 16.7; 2x8(8) 758 over 3239
+// 52.1, 33.7; 4x4 22 over 1221 19.2, 12.9 / 10.6 / 9.9; dense causal 2x1x2802 24.8, 19.1, 1x2x1000 12.6, 11.6 / 10.3.  A tile costs 0.85 us
+// dense and 1 to 1.6 by pages (the more loads a tile takes, the more), adding up 3.4 / 3.8 / 4.6; against that 51 calls came
+// out right but for 0.5 us.  Where it would gain less than 1 us, items stay whole: dense 7x1x459 9.0, 9.9 / 10.8, 1x8x1000
+// 13.2, 13.4; paged 2x8 370 of 436 10.8, 12.6.  All items have to be resident at once.
+// Only where the library chooses: a kernel that is asked for gives a sequence the bits of a call on it alone.  For the same
+// reason not without a mask (see choose_pair_kernel).  Head dim 64 exists in the pair kernel only.
+int split_ctas(int kernel, int head_dim, int64_t items, int64_t keys, int page_size) {
+  if (kernel != B200K_ATTN_AUTO || head_dim != 128) return 1;
+  const double tile_us = page_size == 0 ? 0.85 : page_size == 16 ? 1.6 : page_size == 32 ? 1.3 : 1.0;
+  const double whole = static_cast<double>((keys + kTileRows - 1) / kTileRows) * tile_us;
+  double best = whole - 1.;
+  int ctas = 1;
+  for (int s = 2; s <= 8; s *= 2) {
+    const double us = whole / s + 3. + .2 * s;
+    if (us < best && items <= split_resident_clusters(s)) {
+      best = us;
+      ctas = s;
+    }
+  }
+  return ctas;
+}
+
 }  // namespace
 
 int launch_attention_fwd(const b200k_attention_args& a, cudaStream_t stream) {
@@ -1017,7 +1042,9 @@ int launch_attention_fwd(const b200k_attention_args& a, cudaStream_t stream) {
     return set_error(B200K_ERR_BAD_SHAPE, "attention_fwd: the one-tile kernel covers head_dim 128 only");
   int rc = ensure_sm100();
   if (rc) return rc;
-  if (!choose_pair_kernel(a)) return launch_attention_fwd_tile(a, stream);
+  const int64_t items = static_cast<int64_t>(a.batch) * a.q_heads * ((a.seq_q + kTileRows - 1) / kTileRows);
+  const int split = a.causal ? split_ctas(a.kernel, a.head_dim, items, a.seq_kv, 0) : 1;
+  if (split > 1 || !choose_pair_kernel(a)) return launch_attention_fwd_tile(a, split, stream);
 
   CUtensorMap tq, tk, tv, to;
   const uint32_t box[4] = {64, kTileRows, 1, 1};
@@ -1106,7 +1133,9 @@ int launch_paged_attention_fwd(const b200k_paged_attention_args& a, cudaStream_t
     return set_error(B200K_ERR_BAD_SHAPE, "paged_attention_fwd: the one-tile kernel covers head_dim 128 only");
   int rc = ensure_sm100();
   if (rc) return rc;
-  if (!choose_pair_kernel(a)) return launch_paged_attention_fwd_tile(a, stream);
+  const int64_t items = static_cast<int64_t>(a.batch) * a.q_heads * ((a.seq_q + kTileRows - 1) / kTileRows);
+  const int split = split_ctas(a.kernel, a.head_dim, items, a.max_seq_kv, a.page_size);
+  if (split > 1 || !choose_pair_kernel(a)) return launch_paged_attention_fwd_tile(a, split, stream);
 
   CUtensorMap tq, tk, tv, to;
   const uint32_t box[4] = {64, kTileRows, 1, 1};

@@ -49,6 +49,7 @@
 // Softmax: running max in log2 units (scores are multiplied by scale * log2(e) inside the
 // exponent's FMA); O is only rescaled when a row's max grows by more than 2^8 (stale max used for
 // both P and the running sum, exact after the final division).
+#include <atomic>
 #include <type_traits>
 
 #include "attention_order.cuh"
@@ -92,6 +93,9 @@ constexpr uint32_t kTmemO = 384;
 constexpr int kAttnSmem = kBarOffset + kNumBars * 8 + 16 + 1024;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.0f;
+// SPLIT: adding up the partial results takes some 3 us, as long as three K/V tiles; items of fewer than this stay whole, which
+// matters where the table of a paged call is much wider than its histories.
+constexpr int kMinSharedTiles = 4;
 
 struct AttnParams {
   void* o;
@@ -133,10 +137,12 @@ __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi)
 
 struct Item {
   int qtile, head, batch, n;  // n = number of 128-row KV tiles this item visits
+  int first;                  // ... from this one on (SPLIT: this CTA's share of the item; else 0)
+  bool shared;                // SPLIT: the item is divided; else the first CTA of the cluster has it all
   int kv_len, causal_offset;  // keys of this item's sequence; key j is visible to query i iff j <= i + causal_offset
 };
 
-template <bool PAGED>
+template <bool PAGED, bool SPLIT>
 __device__ __forceinline__ Item make_item(int batch, int head, int qtile, const AttnParams& p) {
   Item it;
   it.qtile = qtile;
@@ -153,21 +159,117 @@ __device__ __forceinline__ Item make_item(int batch, int head, int qtile, const 
     const int last_col = it.qtile * kTileRows + kTileRows - 1 + it.causal_offset;
     it.n = last_col < 0 ? 0 : min(last_col / kTileRows + 1, kv_tiles_total);
   }
+  it.first = 0;
+  it.shared = false;
+  if (SPLIT) {
+    const int ctas = static_cast<int>(cluster_num_ctas()), rank = static_cast<int>(cluster_ctarank());
+    it.shared = it.n >= kMinSharedTiles;
+    if (it.shared) {
+      it.first = it.n * rank / ctas;
+      it.n = it.n * (rank + 1) / ctas - it.first;
+    } else if (rank != 0) {
+      it.n = 0;
+    }
+  }
   return it;
 }
 
-template <bool PAGED>
+template <bool PAGED, bool SPLIT>
 __device__ __forceinline__ Item decode_item(int pos, const AttnParams& p, const uint16_t* table) {
   int batch, head, qtile;
   attn_order::item_at<PAGED>(p.order, pos, table, p.q_heads, batch, head, qtile);
-  return make_item<PAGED>(batch, head, qtile, p);
+  return make_item<PAGED, SPLIT>(batch, head, qtile, p);
 }
 
-template <typename T, bool PAGED, bool ELECT>
-__global__ void __launch_bounds__(kAttnThreads, 1)
-    attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
-                    const AttnParams p) {
+// The items of a CTA: its positions of the list, or (SPLIT) the one item of its cluster.
+template <bool SPLIT>
+struct ItemWalk : attn_order::Walk {};
+template <>
+struct ItemWalk<true> {
+  int pos;
+  __device__ __forceinline__ ItemWalk() : pos(static_cast<int>(blockIdx.x / cluster_num_ctas())) {}
+  __device__ __forceinline__ void step(const attn_order::ItemOrder&) { pos = INT32_MAX; }
+};
+
+// One chunk (four columns) of one row of the SPLIT partial results: 128 rows of 512 bytes, 16-byte chunks XOR-swizzled by row.
+__device__ __forceinline__ uint32_t partial_offset(int row, int chunk) {
+  return static_cast<uint32_t>(kKOffset + row * (kD * 4) + ((chunk ^ (row & 7)) << 4));
+}
+
+// SPLIT: sums this CTA's share of the item's rows over the partial results of the cluster's CTAs, each relative to its own
+// maximum, in rank order.  Called by the eight softmax warps: a warp takes 16 / CTAS rows, a lane four columns of each, and all
+// 16 chunks of a lane are in flight at once.  (Row after row it took 5 us where two CTAs share 128 rows.)
+template <typename T, int CTAS>
+__device__ __forceinline__ void merge_rows(const Item& it, uint32_t smem_base, const AttnParams& p) {
+  constexpr int kRowsPerWarp = 16 / CTAS;
+  const int rank = static_cast<int>(cluster_ctarank()), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = it.qtile * kTileRows, rows = min(kTileRows, p.seq_q - row0), share = (rows + CTAS - 1) / CTAS;
+  const int first = rank * share, end = min(rows, first + share);
+  auto row_of = [&](int k) { return first + warp + 8 * k; };
+  // lane k * CTAS + c: (max, sum) of row k in CTA c
+  float m = -INFINITY, l = 0.f;
+  const int my_row = row_of((lane & 15) / CTAS);
+  if (my_row < end) {
+    const uint32_t peer = cluster_map_shared(smem_base, lane % CTAS) + kLsumOffset;
+    m = ld_shared_cluster_f32(peer + my_row * 4);
+    l = ld_shared_cluster_f32(peer + (kTileRows + my_row) * 4);
+  }
+  float4 v[kRowsPerWarp][CTAS];
+#pragma unroll
+  for (int k = 0; k < kRowsPerWarp; ++k)
+    if (row_of(k) < end) {
+#pragma unroll
+      for (int c = 0; c < CTAS; ++c)
+        v[k][c] = ld_shared_cluster_f32x4(cluster_map_shared(smem_base, c) + partial_offset(row_of(k), lane));
+    }
+  float mm = m;
+#pragma unroll
+  for (int o = CTAS / 2; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+  const float w = m == -INFINITY ? 0.f : ex2(m - mm);
+  const bool used = m != -INFINITY || l != 0.f;  // else it saw none of this row's keys, and its partial row may be unwritten
+  l *= w;
+#pragma unroll
+  for (int k = 0; k < kRowsPerWarp; ++k) {
+    float sum = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < CTAS; ++c) {
+      const int from = k * CTAS + c;
+      const float wc = __shfl_sync(0xffffffffu, w, from), lc = __shfl_sync(0xffffffffu, l, from);
+      if (__shfl_sync(0xffffffffu, used, from)) {
+        sum += lc;
+        acc.x += wc * v[k][c].x;
+        acc.y += wc * v[k][c].y;
+        acc.z += wc * v[k][c].z;
+        acc.w += wc * v[k][c].w;
+      }
+    }
+    const float mk = __shfl_sync(0xffffffffu, mm, k * CTAS);
+    if (row_of(k) >= end) break;
+    const float inv = (sum > 0.f) ? 1.0f / sum : 0.f;
+    const int64_t q_row = row0 + row_of(k);
+    T* orow = reinterpret_cast<T*>(p.o) + it.batch * p.o_stride_b + it.head * p.o_stride_h + q_row * p.o_stride_s;
+    reinterpret_cast<uint2*>(orow)[lane] = make_uint2(pack_pair<T>(acc.x * inv, acc.y * inv), pack_pair<T>(acc.z * inv, acc.w * inv));
+    if (p.lse && lane == 0)
+      p.lse[(static_cast<int64_t>(it.batch) * p.q_heads + it.head) * p.seq_q + q_row] =
+          (sum > 0.f) ? (mk + log2f(sum)) * 0.6931471805599453f : -INFINITY;
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void merge_partials(const Item& it, uint32_t smem_base, const AttnParams& p) {
+  const uint32_t ctas = cluster_num_ctas();
+  if (ctas == 2) merge_rows<T, 2>(it, smem_base, p);
+  if (ctas == 4) merge_rows<T, 4>(it, smem_base, p);
+  if (ctas == 8) merge_rows<T, 8>(it, smem_base, p);
+}
+
+// SPLIT: the K/V tiles of an item are divided over the CTAs of a cluster, one item per cluster.  Each CTA runs the same
+// pipeline over its share, leaves its unnormalised fp32 rows in its drained K ring and their maxima and sums beside, and after a
+// cluster barrier every CTA adds up its part of the rows that exist, in rank order.  See split_ctas for where and why.
+template <typename T, bool PAGED, bool ELECT, bool SPLIT>
+__device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CUtensorMap& tmap_k, const CUtensorMap& tmap_v,
+                                             const CUtensorMap& tmap_o, const AttnParams& p) {
   constexpr uint32_t kFmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBF16;
   constexpr uint32_t kIdescS = make_idesc(kFmt, kFmt, 128, 128, 0, 0);   // Q, K both K-major
   constexpr uint32_t kIdescPV = make_idesc(kFmt, kFmt, 128, 128, 0, 1);  // V is MN-major
@@ -244,9 +346,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   if (PAGED && p.order.sorted) {
     attn_order::sort_entries(table, p.order.sorted, [&](int e) {
       const int batch = e / p.order.tiles;
-      return make_item<PAGED>(batch, 0, e - batch * p.order.tiles, p).n;
+      return make_item<PAGED, false>(batch, 0, e - batch * p.order.tiles, p).n;
     });
   }
+
+  const bool shared_item = SPLIT && decode_item<PAGED, SPLIT>(ItemWalk<SPLIT>().pos, p, table).shared;
 
   if (warp >= 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
@@ -265,7 +369,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         // sequence's first page (those rows are masked; the data only has to be finite).
         auto page_of = [&](const Item& it, int j) {
           if (!PAGED || lane >= pages_per_tile || j >= it.n) return 0;
-          const int lp = j * pages_per_tile + lane;
+          const int lp = (it.first + j) * pages_per_tile + lane;
           const int valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
           return p.block_table[static_cast<int64_t>(it.batch) * p.block_table_stride + (lp < valid_pages ? lp : 0)];
         };
@@ -276,7 +380,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           if (!PAGED) {
 #pragma unroll
             for (int db = 0; db < 2; ++db)
-              tma_load_4d(dst + db * kHalfTileBytes, tm, bar, db * 64, j * kTileRows, it.head / group, it.batch);
+              tma_load_4d(dst + db * kHalfTileBytes, tm, bar, db * 64, (it.first + j) * kTileRows, it.head / group, it.batch);
             return;
           }
           __syncwarp();  // the bytes are announced before any of them can arrive
@@ -330,10 +434,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             if (jj < it.n && !load_k(it, jj, pages[jj])) return false;
           return true;
         };
-        attn_order::Walk walk;
+        ItemWalk<SPLIT> walk;
         auto next_item = [&](Item& nx) {  // next item of this CTA that has work
           while (walk.pos < p.order.num_items) {
-            nx = decode_item<PAGED>(walk.pos, p, table);
+            nx = decode_item<PAGED, SPLIT>(walk.pos, p, table);
             walk.step(p.order);
             if (nx.n > 0) return true;
           }
@@ -386,8 +490,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         uint32_t kstage = 0, kpar = 0; // K ring position
         uint32_t qpar = 0;
         bool ok = true;
-        for (attn_order::Walk walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
-          const Item it = decode_item<PAGED>(walk.pos, p, table);
+        for (ItemWalk<SPLIT> walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
+          const Item it = decode_item<PAGED, SPLIT>(walk.pos, p, table);
           if (it.n == 0) continue;
           if (!mbar_wait(q_full, qpar, abort_word)) break;
           qpar ^= 1;
@@ -425,8 +529,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         uint32_t g = 0, ic = 0;  // KV steps and items so far
         uint32_t vstage = 0, vpar = 0;
         bool ok = true;
-        for (attn_order::Walk walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
-          const Item it = decode_item<PAGED>(walk.pos, p, table);
+        for (ItemWalk<SPLIT> walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
+          const Item it = decode_item<PAGED, SPLIT>(walk.pos, p, table);
           if (it.n == 0) continue;
           for (int j = 0; j < it.n; ++j, ++g) {
             const uint32_t buf = g & 1;
@@ -466,8 +570,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     auto epi_barrier = [&]() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
     uint32_t ic = 0, g0 = 0;  // items so far, KV steps before the current item
     bool ok = true;
-    for (attn_order::Walk walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
-      const Item it = decode_item<PAGED>(walk.pos, p, table);
+    for (ItemWalk<SPLIT> walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
+      const Item it = decode_item<PAGED, SPLIT>(walk.pos, p, table);
+      if (SPLIT && it.n == 0 && (it.shared || cluster_ctarank() != 0)) {  // another CTA writes the item's rows
+        lsum[row_in_tile] = -INFINITY;
+        lsum[kTileRows + row_in_tile] = 0.f;
+        continue;
+      }
       if (it.n == 0) {
         // no visible key: zeros (rare; plain stores)
         const int q_row = it.qtile * kTileRows + row_in_tile;
@@ -497,6 +606,23 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       const float a0 = (m0 == -INFINITY) ? 0.f : ex2(m0 - mm);
       const float a1 = (m1 == -INFINITY) ? 0.f : ex2(m1 - mm);
       const float l = l0 * a0 + l1 * a1;
+      if (SPLIT && it.shared) {
+        const uint32_t t_part = tmem_base + lane_field + kTmemO;
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_part + cc * 32, r);
+          tmem_wait_ld();
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<uint4*>(smem + partial_offset(row_in_tile, cc * 8 + v)) =
+                make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+        }
+        // (this row's entries; both warpgroups' have been read above)
+        lsum[row_in_tile] = mm;
+        lsum[kTileRows + row_in_tile] = l;
+        continue;
+      }
       const float inv = (l > 0.f) ? 1.0f / l : 0.f;
       if (p.lse) {
         // mm is in the log2 domain (scores times scale * log2 e), l is relative to it
@@ -564,8 +690,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     const float2 scale2 = make_float2(scale_log2, scale_log2);
     uint32_t g = 0, ic = 0;  // KV steps (of both warpgroups) and items so far
     bool ok = true;
-    for (attn_order::Walk walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
-      const Item it = decode_item<PAGED>(walk.pos, p, table);
+    for (ItemWalk<SPLIT> walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
+      const Item it = decode_item<PAGED, SPLIT>(walk.pos, p, table);
       if (it.n == 0) continue;
       const int tile_r0 = it.qtile * kTileRows;
       const int q_row = tile_r0 + row_in_tile;
@@ -584,7 +710,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         tmem_ld_32x32b_x64(t_s, sr);
         tmem_ld_32x32b_x64(t_s + 64, sr + 64);
 
-        const int col0 = j * kTileRows;
+        const int col0 = (it.first + j) * kTileRows;
         const bool need_mask =
             (p.causal && col0 + kTileRows - 1 > tile_r0 + causal_offset) || (col0 + kTileRows > kv_len);
         int limit = kTileRows;  // columns [0, limit) of this tile are visible to this row
@@ -692,6 +818,21 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       if (lane == 0) mbar_arrive(l_full);
       ++ic;
     }
+    // (here and not behind the roles: these are the warps that have the registers for it)
+    if constexpr (SPLIT) {
+      if (shared_item) {
+        cluster_sync_all();  // all partial results are in place
+        merge_partials<T>(decode_item<PAGED, SPLIT>(ItemWalk<SPLIT>().pos, p, table), smem_u32(smem), p);
+      }
+    }
+  }
+
+  if constexpr (SPLIT) {
+    // Every thread of every CTA reaches both barriers, also after a wait that gave up.
+    if (shared_item) {
+      if (warp >= 8) cluster_sync_all();
+      cluster_sync_all();  // no CTA leaves while a peer still reads its shared memory
+    }
   }
 
   // ---------------- teardown ----------------
@@ -711,6 +852,22 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
 }
 
 template <typename T, bool PAGED, bool ELECT>
+__global__ void __launch_bounds__(kAttnThreads, 1)
+    attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
+                    const AttnParams p) {
+  attn_fwd_cta<T, PAGED, ELECT, false>(tmap_q, tmap_k, tmap_v, tmap_o, p);
+}
+
+template <typename T, bool PAGED>
+__global__ void __launch_bounds__(kAttnThreads, 1)
+    split_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                          const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
+                          const AttnParams p) {
+  attn_fwd_cta<T, PAGED, true, true>(tmap_q, tmap_k, tmap_v, tmap_o, p);
+}
+
+template <typename T, bool PAGED, bool ELECT>
 int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
                  const AttnParams& p, cudaStream_t stream) {
   auto kfn = attn_fwd_kernel<T, PAGED, ELECT>;
@@ -725,6 +882,18 @@ int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   const int64_t tiles = static_cast<int64_t>(p.order.num_items) * ((p.seq_kv + kTileRows - 1) / kTileRows);
   return launch_maybe_pdl(tiles <= 32 * sms, "attn_fwd_kernel launch", kfn, dim3(grid), dim3(kAttnThreads), kAttnSmem, stream,
                           tq, tk, tv, to, p);
+}
+
+template <typename T, bool PAGED>
+int launch_split(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, AttnParams p,
+                 int ctas, cudaStream_t stream) {
+  auto kfn = split_attn_fwd_kernel<T, PAGED>;
+  static bool configured[64] = {};  // per instantiation and device ordinal
+  int rc = ensure_dynamic_smem(kfn, kAttnSmem, configured, "cudaFuncSetAttribute(attention smem)");
+  if (rc) return rc;
+  p.order.sorted = 0;  // one item per cluster: any order will do
+  return launch_cluster("split_attn_fwd_kernel launch", kfn, ctas, dim3(p.order.num_items * ctas), dim3(kAttnThreads), kAttnSmem,
+                        stream, tq, tk, tv, to, p);
 }
 
 // How the two MMA threads are picked: behind elect.sync (see elect_one) items start faster, behind lane == 0 the steps of a
@@ -742,8 +911,38 @@ bool short_items(const AttnParams& p) {
 
 }  // namespace
 
-// Arguments have been validated by launch_attention_fwd.
-int launch_attention_fwd_tile(const b200k_attention_args& a, cudaStream_t stream) {
+// The CTAs of a cluster share a GPC, so fewer than SMs / ctas fit.  Asked once per device and size.
+int split_resident_clusters(int ctas) {
+  static std::atomic<int> cache[64][9] = {};  // 0 = not asked yet, -1 = cannot launch
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::atomic<int>& known = cache[dev][ctas];
+  if (known == 0) {
+    auto kfn = split_attn_fwd_kernel<__nv_bfloat16, true>;  // all instances have the same resources
+    static bool configured[64] = {};
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kAttnThreads);
+    cfg.dynamicSmemBytes = kAttnSmem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (ensure_dynamic_smem(kfn, kAttnSmem, configured, "cudaFuncSetAttribute(attention smem)") != B200K_OK ||
+        cudaOccupancyMaxActiveClusters(&n, kfn, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    known = n > 0 ? n : -1;
+  }
+  return known > 0 ? known.load() : 0;
+}
+
+// Arguments have been validated by launch_attention_fwd.  split: CTAs per item (split_ctas), 1 without.
+int launch_attention_fwd_tile(const b200k_attention_args& a, int split, cudaStream_t stream) {
   if (!a.q || !a.k || !a.v || !a.o) return set_error(B200K_ERR_NULL, "attention_fwd: q, k, v and o must be non-NULL");
   if (a.batch <= 0 || a.q_heads <= 0 || a.kv_heads <= 0 || a.seq_q <= 0 || a.seq_kv <= 0)
     return set_error(B200K_ERR_BAD_SHAPE, "attention_fwd: all dimensions must be positive");
@@ -818,6 +1017,10 @@ int launch_attention_fwd_tile(const b200k_attention_args& a, cudaStream_t stream
   p.block_table = nullptr;
   p.seq_lens = nullptr;
   p.block_table_stride = p.page_size = p.num_pages = 0;
+  if (split > 1) {
+    if (a.dtype == B200K_F16) return launch_split<__half, false>(tq, tk, tv, to, p, split, stream);
+    return launch_split<__nv_bfloat16, false>(tq, tk, tv, to, p, split, stream);
+  }
   if (short_items(p)) {
     if (a.dtype == B200K_F16) return launch_typed<__half, false, true>(tq, tk, tv, to, p, stream);
     return launch_typed<__nv_bfloat16, false, true>(tq, tk, tv, to, p, stream);
@@ -827,7 +1030,7 @@ int launch_attention_fwd_tile(const b200k_attention_args& a, cudaStream_t stream
 }
 
 // Arguments have been validated by launch_paged_attention_fwd.
-int launch_paged_attention_fwd_tile(const b200k_paged_attention_args& a, cudaStream_t stream) {
+int launch_paged_attention_fwd_tile(const b200k_paged_attention_args& a, int split, cudaStream_t stream) {
   if (!a.q || !a.k_cache || !a.v_cache || !a.o || !a.block_table || !a.seq_lens)
     return set_error(B200K_ERR_NULL, "paged_attention_fwd: q, k_cache, v_cache, o, block_table, seq_lens must be non-NULL");
   if (a.batch <= 0 || a.q_heads <= 0 || a.kv_heads <= 0 || a.seq_q <= 0 || a.max_seq_kv <= 0)
@@ -903,6 +1106,10 @@ int launch_paged_attention_fwd_tile(const b200k_paged_attention_args& a, cudaStr
   p.block_table_stride = a.block_table_stride;
   p.page_size = a.page_size;
   p.num_pages = a.num_pages;
+  if (split > 1) {
+    if (a.dtype == B200K_F16) return launch_split<__half, true>(tq, tk, tv, to, p, split, stream);
+    return launch_split<__nv_bfloat16, true>(tq, tk, tv, to, p, split, stream);
+  }
   if (a.dtype == B200K_F16) return launch_typed<__half, true, true>(tq, tk, tv, to, p, stream);
   return launch_typed<__nv_bfloat16, true, true>(tq, tk, tv, to, p, stream);
 }

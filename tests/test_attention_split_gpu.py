@@ -1,0 +1,118 @@
+"""Calls of few items, whose K/V tiles are divided over clusters: against the undivided kernel and 64-bit results.
+
+The two sum the same tiles against other running maxima and in another grouping; both round probabilities and outputs to
+bf16 or f16 once.
+"""
+import pytest
+import torch
+
+import iree_turbine_b200 as tb
+from iree_turbine_b200 import _launcher as L
+from iree_turbine_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+EPS = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+@pytest.fixture(autouse=True)
+def automatic_kernel():
+    yield
+    ops.ATTENTION_KERNEL = L.ATTN_AUTO
+
+
+def normal(shape, seed, dtype):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return torch.randn(shape, generator=g, device=DEV, dtype=dtype)
+
+
+def exact(q, k, v, scale):
+    """(output, sum of |p v|, log-sum-exp) of one sequence in 64 bits, causal, keys aligned at the end; k, v [heads, keys, dim]."""
+    group = q.size(0) // k.size(0)
+    k, v = (t.double().repeat_interleave(group, 0) for t in (k, v))
+    s = q.double() @ k.transpose(1, 2) * scale
+    s.masked_fill_(~torch.ones(s.shape[1:], dtype=torch.bool, device=DEV).tril(k.size(1) - q.size(1)), -torch.inf)
+    p = torch.softmax(s, -1).nan_to_num(0.0)
+    return p @ v, p @ v.abs(), torch.logsumexp(s, -1)
+
+
+def check(got, whole, ref, size, dtype):
+    err, err_whole = (got.double() - ref).abs(), (whole.double() - ref).abs()
+    assert bool((err <= EPS[dtype] * (size + ref.abs()) + 1e-6).all())  # one rounding of each probability, one of the output
+    assert float(err.square().mean()) <= 1.1 * float(err_whole.square().mean()) + 1e-12  # no further off than undivided
+
+
+# One item and several; one row, a tile's edges, a second tile whose rows see more; fewer tiles than are divided (4), as many,
+# one more, a number that no cluster divides; a grouped K/V head; rows that see no key
+@pytest.mark.parametrize("b,h,hkv,sq,skv", [(1, 1, 1, 1, 5000), (1, 2, 1, 128, 1100), (2, 3, 3, 129, 2049), (1, 4, 2, 300, 3000),
+                                            (1, 1, 1, 5, 400), (1, 2, 2, 700, 2000), (1, 8, 8, 1000, 1300), (1, 4, 4, 2500, 1290)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_dense_causal(b, h, hkv, sq, skv, dtype):
+    q, k, v = normal((b, h, sq, 128), 1, dtype), normal((b, hkv, skv, 128), 2, dtype), normal((b, hkv, skv, 128), 3, dtype)
+    got, lse = torch.ops.b200k.attention_lse(q, k, v, 0.1, True)
+    assert torch.equal(got, torch.ops.b200k.attention(q, k, v, 0.1, True))
+    ops.ATTENTION_KERNEL = L.ATTN_ONE_TILE
+    whole = torch.ops.b200k.attention(q, k, v, 0.1, True)
+    for i in range(b):
+        ref, size, ref_lse = exact(q[i], k[i], v[i], 0.1)
+        check(got[i], whole[i], ref, size, dtype)
+        dead = torch.isinf(ref_lse)
+        assert torch.equal(torch.isinf(lse[i]), dead) and not got[i][dead].any()
+        assert torch.allclose(lse[i][~dead].double(), ref_lse[~dead], rtol=1e-5, atol=1e-4)
+    assert tb.device_status() == 0
+
+
+# Histories far below the table's width, empty, shorter than the queries, and of unequal length
+@pytest.mark.parametrize("page", [16, 32, 64, 128])
+@pytest.mark.parametrize("lens,sq,h,hkv,width", [([3000, 0, 40, 1500, 513], 50, 2, 1, 4096), ([4652, 2326], 164, 2, 2, 4736),
+                                                 ([2000], 1, 16, 4, 2048), ([1300, 700], 260, 4, 4, 1408), ([300], 130, 8, 8, 131072)])
+def test_paged(lens, sq, h, hkv, width, page):
+    dtype = torch.bfloat16
+    counts = [max(1, -(-n // page)) for n in lens]
+    order = torch.randperm(sum(counts), generator=torch.Generator().manual_seed(4)).int()
+    table = torch.full((len(lens), width // page), -1, dtype=torch.int32)
+    for row, part in zip(table, order.split(counts)):
+        row[:part.numel()] = part
+    table, sl = table.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    kc, vc = (normal((sum(counts), hkv, page, 128), s, dtype) for s in (5, 6))
+    q = normal((len(lens), h, sq, 128), 7, dtype)
+    got = torch.ops.b200k.paged_attention(q, kc, vc, table, sl, 0.1, True)
+    ops.ATTENTION_KERNEL = L.ATTN_ONE_TILE
+    whole = torch.ops.b200k.paged_attention(q, kc, vc, table, sl, 0.1, True)
+    for i, n in enumerate(lens):
+        if n == 0:
+            assert not got[i].any()
+            continue
+        k, v = (torch.ops.b200k.paged_gather(c, table[i:i + 1], sl[i:i + 1], n)[0] for c in (kc, vc))
+        check(got[i], whole[i], *exact(q[i], k, v, 0.1)[:2], dtype)
+    assert tb.device_status() == 0
+
+
+def test_nan_and_infinite_scores():
+    """A NaN key reaches every row that sees it, whichever CTA had it; a score of infinity gives NaN as it does undivided."""
+    q, k, v = (normal((1, 1, n, 128), s, torch.bfloat16) for s, n in ((1, 40), (2, 3000), (3, 3000)))
+    k[0, 0, 2970, 5] = float("nan")
+    got = torch.ops.b200k.attention(q, k, v, 0.1, True)
+    assert bool(got[0, 0, 10:].isnan().all()) and not got[0, 0, :10].isnan().any()
+    k[0, 0, 2970, 5] = float("inf")
+    got = torch.ops.b200k.attention(q, k, v, 0.1, True)
+    ops.ATTENTION_KERNEL = L.ATTN_ONE_TILE
+    assert torch.equal(got.isnan(), torch.ops.b200k.attention(q, k, v, 0.1, True).isnan())
+    assert tb.device_status() == 0
+
+
+# Few items with long histories; too short to gain; as many items as clusters of two fit, and one more; no mask
+@pytest.mark.parametrize("b,h,sq,skv,causal,split", [(1, 2, 100, 4000, True, True), (1, 2, 100, 400, True, False), (1, 74, 100, 3000, True, True),
+                                                     (1, 75, 100, 3000, True, False), (1, 2, 100, 4000, False, False)])
+def test_which_calls(b, h, sq, skv, causal, split):
+    from torch.profiler import ProfilerActivity, profile
+    q, k, v = (normal((b, h, n, 128), s, torch.bfloat16) for s, n in ((1, sq), (2, skv), (3, skv)))
+    torch.ops.b200k.attention(q, k, v, 0.1, causal)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        torch.ops.b200k.attention(q, k, v, 0.1, causal)
+        torch.cuda.synchronize()
+    names = [e.name for e in p.events() if "attn_fwd_kernel" in e.name]
+    if not names:
+        pytest.skip("the profiler reports no kernels here")
+    assert ["split_attn" in n for n in names] == [split]
