@@ -207,7 +207,7 @@ __device__ __forceinline__ void bwd_dq_cta(int block, int blocks, const CUtensor
   auto k_off = [](int b) { return b == 0 ? kOffK : (b == 1 ? kOffK1 : kOffQ); };
   auto v_off = [](int b) { return b == 0 ? kOffV : (b == 1 ? kOffV1 : kOffDO); };
 
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kDqTiles * kTileBytes);
   uint64_t* fix_full = bars;      // Q and dO have landed in shared memory
@@ -574,17 +574,27 @@ __device__ __forceinline__ void bwd_dq_cta(int block, int blocks, const CUtensor
 // second product, and likewise dS^T over dP^T.  The row
 // statistics belong to the query, i.e. to the COLUMN here; the 128 (lse, delta) pairs of a query
 // tile are brought into shared memory once per iteration and read by broadcast.
-// MMA order (one in-order stream): dV(i) : S^T(i+1) : dK(i) : dP^T(i+1).  S^T(i+1) may overwrite
+// MMA order (one in-order stream): dV(i) : S^T(i+1) : dK(i) : dP^T(i+1), the first two by halves of the queries, one for
+// each of the two warpgroups of the algebra: dV[0] S^T[0] dV[1] S^T[1].  S^T(i+1) may overwrite
 // P^T(i) and dP^T(i+1) may overwrite dS^T(i) without a barrier because they are issued behind the
-// products that read them.  Shared memory: K, V, two Q buffers, two dO buffers (6 x 32 KB).
+// products that read them.  By halves, the chain of one (dV[h] -> S^T[h] -> P^T[h]) runs under the other's: 64 columns of S^T
+// cost 48 cycles per MMA where 128 cost 64, but as whole tiles every iteration waited some 500 cycles for its probabilities.
+// Period in CTAs that have an SM to themselves and the clock to spare, 1x8(1)x4096 causal: 2960 cycles of 2048 for the
+// products, now 2520 (2304 with these MMAs); us, whole tiles / halves: 1x8(1)x4096 409 / 351, 1x8(2)x1000 58.8 / 51.9, 1x2x2048
+// 33.2 / 29.6; with all SMs at work and the clock under the power cap 2x32(8)x2000 267 / 257, 4x32x4096 1960 / 1858,
+// 1x16x4096 without a mask 442 / 413; 13x64(8)x81 63.9 / 62.0.  (The dQ CTAs by the same halves: no difference, 2x32(8)x2000 260 / 260.)
+// Shared memory: K, V, three Q buffers, two dO buffers (7 x 32 KB), each handed
+// back by the last product that reads it, so that a tile is requested a whole iteration before its first product.
 // Tensor memory: S^T / P^T | dP^T / dS^T | dV | dK (128 columns each).
 // ---------------------------------------------------------------------------------------------
-constexpr int kTK = 0, kTV = kTileBytes, kTQ0 = 2 * kTileBytes, kTQ1 = 3 * kTileBytes, kTDO0 = 4 * kTileBytes,
-              kTDO1 = 5 * kTileBytes, kTVec = 6 * kTileBytes;  // kTVec: [2 buffers][lse2 128 | delta 128] floats
+constexpr int kTK = 0, kTV = kTileBytes, kTQ = 2 * kTileBytes, kTDO = 5 * kTileBytes,
+              kTVec = 7 * kTileBytes;  // kTVec: [2 buffers][lse2 128 | delta 128] floats
+constexpr int kQBufs = 3, kDOBufs = 2;
 constexpr int kTVecBytes = 2 * 256 * 4;
-// fix_full, ld_full[2], it_done[2], s_full, dp_full, p_full, ds_full
-constexpr int kNumDkvtBars = 9;
-constexpr int dkvt_smem_bytes() { return 6 * kTileBytes + kTVecBytes + kNumDkvtBars * 8 + 16 + 1024; }
+// fix_full, q_full[3], q_free[3], do_full[2], do_free[2], s_full[2], dp_full, p_full[2], ds_full
+constexpr int kNumDkvtBars = 17;
+// Seven tiles leave 888 bytes of the 227 KB for the alignment of the first one; the array is declared aligned, so it needs none.
+constexpr int dkvt_smem_bytes() { return 7 * kTileBytes + kTVecBytes + kNumDkvtBars * 8 + 16 + 768; }
 
 template <typename T, int HD>
 __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtensorMap& tmap_q, const CUtensorMap& tmap_do,
@@ -592,22 +602,25 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
                                             const CUtensorMap& tmap_dv, const CUtensorMap& tmap_dk, const BwdParams& p) {
   static_assert(HD == 128 || HD == 64, "head dim 128 or 64");
   constexpr uint32_t kFmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBF16;
-  constexpr uint32_t kIdS = make_idesc(kFmt, kFmt, 128, 128, 0, 0);  // S^T, dP^T: 128 keys x 128 queries
+  constexpr uint32_t kIdS = make_idesc(kFmt, kFmt, 128, 64, 0, 0);    // half of S^T: 128 keys x 64 queries
+  constexpr uint32_t kIdDP = make_idesc(kFmt, kFmt, 128, 128, 0, 0);  // dP^T: 128 keys x 128 queries
   constexpr uint32_t kIdG = make_idesc(kFmt, kFmt, 128, HD, 0, 1);   // dV, dK: 128 keys x HD, B MN-major
   constexpr int kDSteps = HD / 16;
   constexpr int kOpBytes = kRows * HD * 2;
 
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   float* vec = reinterpret_cast<float*>(smem + kTVec);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kTVec + kTVecBytes);
   uint64_t* fix_full = bars;     // K and V have landed
-  uint64_t* ld_full = bars + 1;  // [buffer] Q and dO of an iteration have landed
-  uint64_t* it_done = bars + 3;  // [buffer] every product that reads the buffer has completed
-  uint64_t* s_full = bars + 5;   // S^T is in tensor memory
-  uint64_t* dp_full = bars + 6;  // dP^T is in tensor memory
-  uint64_t* p_full = bars + 7;   // all rows of P^T stored (S^T read)
-  uint64_t* ds_full = bars + 8;  // all rows of dS^T stored (dP^T read)
+  uint64_t* q_full = bars + 1;    // [buffer] Q of an iteration has landed
+  uint64_t* q_free = bars + 4;    // [buffer] its products, S^T and dK, have completed
+  uint64_t* do_full = bars + 7;   // [buffer] dO of an iteration has landed
+  uint64_t* do_free = bars + 9;   // [buffer] its products, dP^T and dV, have completed
+  uint64_t* s_full = bars + 11;   // [half] its 64 columns of S^T are in tensor memory
+  uint64_t* dp_full = bars + 13;  // dP^T is in tensor memory
+  uint64_t* p_full = bars + 14;   // [half] all rows of its columns of P^T stored (S^T read)
+  uint64_t* ds_full = bars + 16;  // all rows of dS^T stored (dP^T read)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumDkvtBars);
   volatile uint32_t* abort_word = tmem_slot + 1;
 
@@ -633,13 +646,12 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
 
   if (threadIdx.x == 0) {
     mbar_init(fix_full, 1);
-    mbar_init(ld_full, 1);
-    mbar_init(ld_full + 1, 1);
-    mbar_init(it_done, 1);
-    mbar_init(it_done + 1, 1);
+    for (int b = 0; b < 2 * (kQBufs + kDOBufs); ++b) mbar_init(q_full + b, 1);  // q_full .. do_free
     mbar_init(s_full, 1);
+    mbar_init(s_full + 1, 1);
     mbar_init(dp_full, 1);
-    mbar_init(p_full, kSoftmaxThreads / 32);   // one arrival per warp
+    mbar_init(p_full, kSoftmaxThreads / 64);  // one arrival per warp of the half
+    mbar_init(p_full + 1, kSoftmaxThreads / 64);
     mbar_init(ds_full, kSoftmaxThreads / 32);
     *abort_word = 0;
     fence_barrier_init();
@@ -666,14 +678,24 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
       mbar_arrive_expect_tx(fix_full, 2 * kOpBytes);
       load_tile_4d<HD>(smem + kTK, &tmap_k, fix_full, row0, kvh, batch);
       load_tile_4d<HD>(smem + kTV, &tmap_v, fix_full, row0, kvh, batch);
+      int head = kvh * group, qt = qt_lo, bq = 0;
+      uint32_t ph = 1;  // parity of the wait for q_free: the first round of buffers is free
       for (int i = 0; i < total; ++i) {
         const int b = i & 1;
-        if (i >= 2 && !mbar_wait(it_done + b, ((i - 2) >> 1) & 1, abort_word)) break;
-        const int g = i / n;
-        const int qt = qt_lo + (i - g * n);
-        mbar_arrive_expect_tx(ld_full + b, 2 * kOpBytes);
-        load_tile_4d<HD>(smem + (b ? kTQ1 : kTQ0), &tmap_q, ld_full + b, qt * kRows, kvh * group + g, batch);
-        load_tile_4d<HD>(smem + (b ? kTDO1 : kTDO0), &tmap_do, ld_full + b, qt * kRows, kvh * group + g, batch);
+        if (!mbar_wait(q_free + bq, ph, abort_word)) break;
+        mbar_arrive_expect_tx(q_full + bq, kOpBytes);
+        load_tile_4d<HD>(smem + kTQ + bq * kTileBytes, &tmap_q, q_full + bq, qt * kRows, head, batch);
+        if (!mbar_wait(do_free + b, ((i >> 1) & 1) ^ 1, abort_word)) break;
+        mbar_arrive_expect_tx(do_full + b, kOpBytes);
+        load_tile_4d<HD>(smem + kTDO + b * kTileBytes, &tmap_do, do_full + b, qt * kRows, head, batch);
+        if (++qt == p.num_q_tiles) {
+          qt = qt_lo;
+          ++head;
+        }
+        if (++bq == kQBufs) {
+          bq = 0;
+          ph ^= 1;
+        }
       }
     }
     __syncwarp();
@@ -681,45 +703,68 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
     // ---------------- MMA issuer ----------------
     if (total > 0 && elect_one()) {
       const uint32_t sk = smem_u32(smem + kTK), sv = smem_u32(smem + kTV);
-      auto sq = [&](int b) { return smem_u32(smem + (b ? kTQ1 : kTQ0)); };
-      auto sdo = [&](int b) { return smem_u32(smem + (b ? kTDO1 : kTDO0)); };
+      auto sq = [&](int b) { return smem_u32(smem + kTQ) + b * kTileBytes; };
+      auto sdo = [&](int b) { return smem_u32(smem + kTDO) + b * kTileBytes; };
       // D[keys x HD] (+)= A^T-from-tensor-memory * B, B = an MN-major tile (rows = queries): 8 steps of 16 queries
       // The 16-bit A tile sits in two pieces: queries 0..63 in columns 0..31 of the region, queries
       // 64..127 in columns 64..95 (each of the two threads of a row writes over its own S columns).
-      auto mma_ts = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t b_addr, bool accumulate) {
+      // (four of them for the queries of one half: `from` = 0 or 4)
+      auto mma_ts = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t b_addr, bool accumulate, int from, int to) {
         const uint64_t b0 = make_desc_mnmajor_sw128(b_addr, kHalfBytes);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
+        for (int ks = from; ks < to; ++ks)
           umma_f16_ts(d_tmem, a_tmem + (ks >> 2) * 64 + (ks & 3) * 8, b0 + ks * (2048 >> 4), kIdG,
                       (accumulate || ks > 0) ? 1u : 0u);
       };
+      // 64 columns of S^T: the queries in rows 64 * half .. of the tile, 8 KB into each of its 64-column blocks
+      auto mma_s = [&](int half, int buf) {
+        mma_128x128x128<false, false, kDSteps>(tmem_base + kTmS + half * 64, sk, sq(buf) + half * 8192, kIdS, false);
+        umma_commit(s_full + half);
+      };
       bool ok = mbar_wait(fix_full, 0, abort_word);
-      if (ok) ok = mbar_wait(ld_full, 0, abort_word);
+      if (ok) ok = mbar_wait(q_full, 0, abort_word);
       if (ok) {
         tc_fence_after();
-        mma_128x128x128<false, false, kDSteps>(tmem_base + kTmS, sk, sq(0), kIdS, false);   // S^T(0)
-        umma_commit(s_full);
-        mma_128x128x128<false, false, kDSteps>(tmem_base + kTmDP, sv, sdo(0), kIdS, false);  // dP^T(0)
+        mma_s(0, 0);
+        mma_s(1, 0);
+        ok = mbar_wait(do_full, 0, abort_word);
+      }
+      if (ok) {
+        tc_fence_after();
+        mma_128x128x128<false, false, kDSteps>(tmem_base + kTmDP, sv, sdo(0), kIdDP, false);  // dP^T(0)
         umma_commit(dp_full);
       }
+      int bq = 0, next_q = 1;  // buffers of Q(i) and Q(i + 1)
+      uint32_t ph = 0;         // parity of the wait for Q(i + 1)
       for (int i = 0; i < total && ok; ++i) {
         const int b = i & 1;
         if (!mbar_wait(p_full, i & 1, abort_word)) break;
         tc_fence_after();
-        mma_ts(tmem_base + kTmAcc0, tmem_base + kTmS, sdo(b), i > 0);  // dV += P^T dO
+        mma_ts(tmem_base + kTmAcc0, tmem_base + kTmS, sdo(b), i > 0, 0, 4);  // dV += P^T dO, first half of the queries
         if (i + 1 < total) {
-          if (!mbar_wait(ld_full + (b ^ 1), ((i + 1) >> 1) & 1, abort_word)) break;
+          if (!mbar_wait(q_full + next_q, ph, abort_word)) break;
           tc_fence_after();
-          mma_128x128x128<false, false, kDSteps>(tmem_base + kTmS, sk, sq(b ^ 1), kIdS, false);  // S^T(i+1), behind dV(i)
-          umma_commit(s_full);
+          mma_s(0, next_q);  // S^T(i+1), behind what dV(i) reads from its columns
         }
+        if (!mbar_wait(p_full + 1, i & 1, abort_word)) break;
+        tc_fence_after();
+        mma_ts(tmem_base + kTmAcc0, tmem_base + kTmS, sdo(b), true, 4, 8);
+        umma_commit(do_free + b);
+        if (i + 1 < total) mma_s(1, next_q);
         if (!mbar_wait(ds_full, i & 1, abort_word)) break;
         tc_fence_after();
-        mma_ts(tmem_base + kTmAcc1, tmem_base + kTmDP, sq(b), i > 0);  // dK += dS^T Q
-        umma_commit(it_done + b);
+        mma_ts(tmem_base + kTmAcc1, tmem_base + kTmDP, sq(bq), i > 0, 0, 8);  // dK += dS^T Q
+        umma_commit(q_free + bq);
         if (i + 1 < total) {
-          mma_128x128x128<false, false, kDSteps>(tmem_base + kTmDP, sv, sdo(b ^ 1), kIdS, false);  // dP^T(i+1), behind dK(i)
+          if (!mbar_wait(do_full + (b ^ 1), ((i + 1) >> 1) & 1, abort_word)) break;
+          tc_fence_after();
+          mma_128x128x128<false, false, kDSteps>(tmem_base + kTmDP, sv, sdo(b ^ 1), kIdDP, false);  // dP^T(i+1), behind dK(i)
           umma_commit(dp_full);
+        }
+        bq = next_q;
+        if (++next_q == kQBufs) {
+          next_q = 0;
+          ph ^= 1;
         }
       }
     }
@@ -730,44 +775,45 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
     const int quarter = warp & 3;
     const int half = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;
-    const int tid = threadIdx.x - 64;  // 0 .. 255
+    const int tid = (threadIdx.x - 64) & 127;  // in the half
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const int key = row0 + r;
     // query q (global index) sees this key iff q >= q_min (and q < seq_q, which the statistics encode)
     const int q_min = (key < p.seq_kv) ? (p.causal ? key - p.causal_offset : INT32_MIN) : INT32_MAX;
     bool ok = true;
-    // The (lse2, delta) pairs of the 128 queries of a tile go to shared memory, one value per thread
-    // (threads 0..127 the statistic, 128..255 delta).  The values of iteration i + 1 are fetched at
-    // the top of iteration i and stored at its end, so the global-memory latency is off the chain.
-    auto fetch_stat = [&](int it) -> float {
-      float val = (tid < 128) ? INFINITY : 0.f;  // a query past the end: P = exp2(x - inf) = 0
-      if (it < total) {
-        const int g_ = it / n;
-        const int q_g = (qt_lo + (it - g_ * n)) * kRows + (tid & 127);
-        if (q_g < p.seq_q) {
-          const int64_t idx = (static_cast<int64_t>(batch) * p.q_heads + kvh * group + g_) * p.seq_q + q_g;
-          if (tid < 128)
-            val = p.lse_in ? lse_to_log2(p.lse_in[idx]) : p.lse2[idx];
-          else
-            val = p.delta[idx];
-        }
+    // The (lse2, delta) pairs of the half's 64 queries of a tile go to shared memory, one value per thread
+    // (threads 0..63 the statistic, 64..127 delta).  The values of iteration i + 1 are fetched
+    // the top of iteration i and converted and stored at its end, so the global-memory latency is off the chain.
+    const bool raw_lse = p.lse_in != nullptr;
+    const float* stat_src = tid >= 64 ? p.delta : (raw_lse ? p.lse_in : p.lse2);
+    // a query past the end: P = exp2(x - inf) = 0
+    const float stat_none = tid >= 64 ? 0.f : (raw_lse ? -INFINITY : INFINITY);
+    int64_t stat_head = (static_cast<int64_t>(batch) * p.q_heads + kvh * group) * p.seq_q;  // first query of the head
+    int stat_qt = qt_lo;                                                                    // tile fetched next
+    auto fetch_stat = [&]() -> float {
+      const int q_g = stat_qt * kRows + half * 64 + (tid & 63);
+      const float val = q_g < p.seq_q ? stat_src[stat_head + q_g] : stat_none;
+      if (++stat_qt == p.num_q_tiles) {
+        stat_qt = qt_lo;
+        stat_head += p.seq_q;
       }
       return val;
     };
+    auto convert_stat = [&](float val) { return tid < 64 && raw_lse ? lse_to_log2(val) : val; };
+    auto half_barrier = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(3 + half) : "memory"); };
     if (total > 0) {
-      vec[tid] = fetch_stat(0);
-      asm volatile("bar.sync 3, 256;" ::: "memory");
+      vec[half * 128 + tid] = convert_stat(fetch_stat());
+      half_barrier();
     }
-    for (int i = 0; i < total; ++i) {
-      const int g = i / n;
-      const int qt = qt_lo + (i - g * n);
+    int qt = qt_lo;
+    for (int i = 0; i < total; ++i, qt = qt + 1 == p.num_q_tiles ? qt_lo : qt + 1) {
       const int q_base = qt * kRows;
-      const float next_stat = fetch_stat(i + 1);
-      const float* lse_v = vec + (i & 1) * 256 + half * 64;
-      const float* dl_v = lse_v + 128;
+      const float next_stat = i + 1 < total ? fetch_stat() : 0.f;
+      const float* lse_v = vec + (i & 1) * 256 + half * 128;
+      const float* dl_v = lse_v + 64;
       const int q0 = q_base + half * 64;  // first query column of this thread
       float pf[64];
-      if (ok && !mbar_wait(s_full, i & 1, abort_word)) ok = false;
+      if (ok && !mbar_wait(s_full + half, i & 1, abort_word)) ok = false;
       if (ok) {
         tc_fence_after();
         uint32_t s64[64];
@@ -800,7 +846,7 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(p_full + half);
       if (ok && !mbar_wait(dp_full, i & 1, abort_word)) ok = false;
       if (ok) {
         tc_fence_after();
@@ -821,19 +867,19 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
-      // every thread is done with this iteration's statistics and with the other buffer (read one
+      // every thread of the half is done with this iteration's statistics and with the other buffer (read one
       // iteration ago): publish the next ones
-      vec[((i + 1) & 1) * 256 + tid] = next_stat;
-      asm volatile("bar.sync 3, 256;" ::: "memory");
+      vec[((i + 1) & 1) * 256 + half * 128 + tid] = convert_stat(next_stat);
+      half_barrier();
     }
-    if (ok && total > 0) ok = mbar_wait(it_done + ((total - 1) & 1), ((total - 1) >> 1) & 1, abort_word);
+    if (ok && total > 0) ok = mbar_wait(q_free + (total - 1) % kQBufs, ((total - 1) / kQBufs) & 1, abort_word);  // the last dK
     ok = bar_red_and(1, kSoftmaxThreads, ok);
     if (ok) {
       tc_fence_after();
       // accumulators -> 16-bit tiles in the (now unused) Q / dO buffers -> TMA stores
 #pragma unroll
       for (int o = 0; o < 2; ++o) {
-        uint8_t* stage = smem + (o == 0 ? kTQ0 : kTDO0);
+        uint8_t* stage = smem + (o == 0 ? kTQ : kTDO);
         const uint32_t acc = lane_base + (o == 0 ? kTmAcc0 : kTmAcc1);
         const float f = o == 1 ? p.scale : 1.f;  // dK carries the softmax scale
 #pragma unroll 1
@@ -857,10 +903,10 @@ __device__ __forceinline__ void bwd_dkv_cta(int block, int blocks, const CUtenso
       fence_proxy_async_smem();
       asm volatile("bar.sync 2, 256;" ::: "memory");
       if (r == 0 && half == 0) {
-        tma_store_4d(&tmap_dv, smem + kTQ0, 0, row0, kvh, batch);
-        if (HD == 128) tma_store_4d(&tmap_dv, smem + kTQ0 + kHalfBytes, 64, row0, kvh, batch);
-        tma_store_4d(&tmap_dk, smem + kTDO0, 0, row0, kvh, batch);
-        if (HD == 128) tma_store_4d(&tmap_dk, smem + kTDO0 + kHalfBytes, 64, row0, kvh, batch);
+        tma_store_4d(&tmap_dv, smem + kTQ, 0, row0, kvh, batch);
+        if (HD == 128) tma_store_4d(&tmap_dv, smem + kTQ + kHalfBytes, 64, row0, kvh, batch);
+        tma_store_4d(&tmap_dk, smem + kTDO, 0, row0, kvh, batch);
+        if (HD == 128) tma_store_4d(&tmap_dk, smem + kTDO + kHalfBytes, 64, row0, kvh, batch);
         tma_store_commit();
         tma_store_wait_read<0>();  // the staging tile has been read: the CTA may go (the writes land before the grid ends)
       }
