@@ -834,46 +834,63 @@ int launch_paged_gather(const void* cache, const int32_t* block_table, const int
   return check_cuda(cudaGetLastError(), "paged_gather_kernel launch");
 }
 
-// ------------------------------------------------------------------------------------------
-// KV-cache append: the step before decode.  Row t of new_rows[s] goes to token position
-// positions[s] + t of sequence s, through the block table, with kv_row_offset<true> (the address
-// function of the decode kernel).  One warp per (token, head) row; 16-byte stores; rows whose
-// block-table entry is outside the pool are dropped and reported through the status word.
-// ------------------------------------------------------------------------------------------
-__global__ void kv_append_kernel(const uint8_t* k_new, const uint8_t* v_new, uint8_t* k_cache, uint8_t* v_cache,
-                                 const int32_t* block_table, const int32_t* positions,
-                                 int32_t new_tokens, int32_t kv_heads, int32_t head_dim, int32_t page_size,
-                                 int32_t num_pages, int32_t block_table_stride, int64_t kv_page_stride,
-                                 int64_t kv_head_stride, int32_t elem_bytes, int32_t* status) {
+// KV-cache append: the step before decode.  Row t of a sequence's new rows [token][head][head_dim] goes to its token positions[s] + t,
+// through the block table with kv_row_offset<true>, the address function of the decode kernel; rows whose block-table entry
+// is outside the pool are dropped and reported through the status word.  A thread copies UNROLL 16-byte chunks of K and V, neighbouring
+// threads neighbouring chunks, so reads are contiguous over rows and heads and up to eight are in flight per thread.
+// HBM-bound where there are many, a launch otherwise.  With a row per warp half of the lanes were idle at head dim 128, with one
+// pair of loads in flight per thread.  us, launches in a graph, a row per warp / now: 4 x 512 tokens of 8 heads of 256 bytes (17 MB
+// moved) 5.1 / 3.2, 16 x 2048 of 16 (537 MB) 141 / 80, 8 x 300 of 4 heads of 128 bytes 3.4 / 1.9, 128 x 1 of 16 2.8 / 1.7, 14 x 18 of 2
+// 1.74 / 1.64, 1 x 1 of 8 1.56 / 1.45.
+constexpr int kAppendThreads = 256;
+
+template <int UNROLL>
+__global__ void __launch_bounds__(kAppendThreads)
+    kv_append_kernel(const uint8_t* k_new, const uint8_t* v_new, uint8_t* k_cache, uint8_t* v_cache, const int32_t* block_table,
+                     const int32_t* positions, int32_t new_tokens, int32_t kv_heads, int32_t head_dim, int32_t page_size,
+                     int32_t num_pages, int32_t block_table_stride, int64_t kv_page_stride, int64_t kv_head_stride,
+                     int32_t elem_bytes, Divisor by_chunks, Divisor by_heads, int32_t* status) {
   grid_dependency_wait();
   grid_dependency_trigger();
-  const int seq = blockIdx.z;
-  const int head = blockIdx.y;
-  const int row_bytes = head_dim * elem_bytes;
-  const int chunks_per_row = row_bytes / 16;
+  const int seq = blockIdx.y;
+  const int chunks = static_cast<int>(by_chunks.d);  // of a row
   const int pos0 = positions[seq];
-  const int warps = blockDim.x >> 5;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int t = blockIdx.x * warps + warp; t < new_tokens; t += gridDim.x * warps) {
-    const int token = pos0 + t;
-    int64_t off = -1;
-    if (pos0 >= 0 && token / page_size < block_table_stride)
-      off = kv_row_offset<true>(block_table, block_table_stride, page_size, num_pages, kv_page_stride, kv_head_stride, 0,
-                                head_dim, seq, head, token);
-    if (off < 0) {
-      if (lane == 0 && status) atomicOr(status, kStatusDecodeBadPage);
-      continue;
+  const int64_t per_token = static_cast<int64_t>(kv_heads) * chunks;
+  const int64_t total = new_tokens * per_token;  // of the sequence
+  const uint4* ks = reinterpret_cast<const uint4*>(k_new) + seq * total;
+  const uint4* vs = reinterpret_cast<const uint4*>(v_new) + seq * total;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * (UNROLL * kAppendThreads);
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * (UNROLL * kAppendThreads); base < total; base += step) {
+    // tokens before this block's chunks are split off where the chunks of a sequence are too many for the 32-bit quotients
+    const int64_t t0 = total > INT32_MAX ? base / per_token : 0;
+    const int in0 = static_cast<int>(base - t0 * per_token);
+    uint4 k[UNROLL], v[UNROLL];
+    int64_t dst[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const int local = u * kAppendThreads + static_cast<int>(threadIdx.x);
+      dst[u] = -1;
+      if (base + local >= total) continue;
+      k[u] = ks[base + local];
+      v[u] = vs[base + local];
+      const int row = by_chunks.quotient(in0 + local), chunk = in0 + local - row * chunks;
+      const int t = by_heads.quotient(row), head = row - t * kv_heads;
+      const int token = pos0 + static_cast<int>(t0) + t;
+      int64_t off = -1;
+      if (pos0 >= 0 && token / page_size < block_table_stride)
+        off = kv_row_offset<true>(block_table, block_table_stride, page_size, num_pages, kv_page_stride, kv_head_stride, 0,
+                                  head_dim, seq, head, token);
+      if (off >= 0)
+        dst[u] = off * elem_bytes + chunk * 16;
+      else if (chunk == 0 && status)
+        atomicOr(status, kStatusDecodeBadPage);
     }
-    const int64_t src = ((static_cast<int64_t>(seq) * new_tokens + t) * kv_heads + head) * row_bytes;
-    const uint4* ks = reinterpret_cast<const uint4*>(k_new + src);
-    const uint4* vs = reinterpret_cast<const uint4*>(v_new + src);
-    uint4* kd = reinterpret_cast<uint4*>(k_cache + off * elem_bytes);
-    uint4* vd = reinterpret_cast<uint4*>(v_cache + off * elem_bytes);
-    for (int c = lane; c < chunks_per_row; c += 32) {
-      const uint4 k = ks[c], v = vs[c];
-      kd[c] = k;
-      vd[c] = v;
-    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      if (dst[u] >= 0) {
+        *reinterpret_cast<uint4*>(k_cache + dst[u]) = k[u];
+        *reinterpret_cast<uint4*>(v_cache + dst[u]) = v[u];
+      }
   }
 }
 
@@ -893,14 +910,20 @@ int launch_kv_append(const void* k_new, const void* v_new, void* k_cache, void* 
     return set_error(B200K_ERR_BAD_ALIGN, "kv_append: rows, strides and bases must be multiples of 16 bytes");
   int rc = ensure_sm100();
   if (rc) return rc;
-  const int warps = 4;
-  int gx = (new_tokens + warps - 1) / warps;
-  if (gx > 1024) gx = 1024;
-  return launch_pdl("kv_append_kernel launch", kv_append_kernel, dim3(gx, kv_heads, num_seqs), dim3(warps * 32), 0, stream,
-                    reinterpret_cast<const uint8_t*>(k_new), reinterpret_cast<const uint8_t*>(v_new),
+  const int64_t row_chunks = head_dim * elem_bytes / 16, total = new_tokens * kv_heads * row_chunks;
+  if (kv_heads * row_chunks >= INT32_MAX - 4 * kAppendThreads) return set_error(B200K_ERR_BAD_SHAPE, "kv_append: a token is too large");
+  Divisor by_chunks, by_heads;
+  by_chunks.set(row_chunks);
+  by_heads.set(kv_heads);
+  // four chunks per thread once that leaves four blocks per SM, as many blocks as chunks before
+  const bool many = total * num_seqs >= static_cast<int64_t>(num_sms()) * 4 * 4 * kAppendThreads;
+  const int64_t per_block = (many ? 4 : 1) * kAppendThreads, blocks = (total + per_block - 1) / per_block;
+  auto kfn = many ? kv_append_kernel<4> : kv_append_kernel<1>;
+  return launch_pdl("kv_append_kernel launch", kfn, dim3(static_cast<unsigned>(blocks < 4096 ? blocks : 4096), num_seqs),
+                    dim3(kAppendThreads), 0, stream, reinterpret_cast<const uint8_t*>(k_new), reinterpret_cast<const uint8_t*>(v_new),
                     reinterpret_cast<uint8_t*>(k_cache), reinterpret_cast<uint8_t*>(v_cache), block_table, positions,
                     new_tokens, kv_heads, head_dim, page_size, num_pages, block_table_stride, kv_page_stride,
-                    kv_head_stride, elem_bytes, status);
+                    kv_head_stride, elem_bytes, by_chunks, by_heads, status);
 }
 
 // ------------------------------------------------------------------------------------------

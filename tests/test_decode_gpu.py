@@ -202,3 +202,21 @@ def test_kv_append_outside_pool_is_dropped_and_reported():
     k_ref, _ = oracle.kv_append(k_new[:1], k_new[:1], k_cache, v_cache, block_table[:1], positions[:1])
     k_ref, _ = oracle.kv_append(k_new[1:, :2], k_new[1:, :2], k_ref, v_cache, block_table[1:], positions[1:])
     assert torch.equal(kc.cpu(), k_ref)
+
+
+# Chunks of a row 1, 3 (no power of two), 8 and 16; a thread copies one, or four from 606208 chunks in the call on
+@pytest.mark.parametrize("seqs,tokens,heads,dim", [(1, 1, 1, 8), (3, 7, 5, 24), (2, 300, 3, 64), (5, 130, 4, 128), (4, 1200, 8, 128), (9, 900, 5, 128)])
+def test_kv_append_copies_every_chunk(seqs, tokens, heads, dim):
+    page, g = 16, torch.Generator().manual_seed(3)
+    positions = torch.randint(0, 40, (seqs,), generator=g).to(torch.int32)
+    per_seq = -(-(tokens + 40) // page)
+    table = torch.randperm(seqs * per_seq, generator=g).to(torch.int32).view(seqs, per_seq)
+    k_new, v_new = (torch.randn(seqs, tokens, heads, dim, generator=g).to(torch.bfloat16) for _ in range(2))
+    kc, vc = (torch.zeros(seqs * per_seq, heads, page, dim, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    torch.ops.b200k.kv_append(k_new.to(DEV), v_new.to(DEV), kc, vc, table.to(DEV), positions.to(DEV))
+    token = positions[:, None] + torch.arange(tokens)
+    pages, rows = table.gather(1, (token // page).long()).to(DEV).long(), (token % page).to(DEV)
+    for cache, new in ((kc, k_new), (vc, v_new)):
+        assert torch.equal(cache[pages, :, rows], new.to(DEV))
+        assert int((cache != 0).any(-1).sum()) == seqs * tokens * heads  # and nothing else
+    assert tb.device_status() == 0
