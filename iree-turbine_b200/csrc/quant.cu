@@ -1,11 +1,12 @@
 // Per-tensor e4m3 quantisation: scale = max|x| / 448,  y = e4m3_rn(x / scale).
 //
 // HBM-bound: x is read twice (the second time from L2 where it fits) and a byte per element is
-// written.  Two launches: absmax_kernel leaves one maximum per block in the workspace (no memset, no
+// written, unless registers hold x (quantize_resident_kernel).  Two launches otherwise: absmax_kernel leaves one maximum per block in the workspace (no memset, no
 // atomics), and every block of cast_e4m3_kernel reduces those few hundred values itself.  Both keep
 // four 16-byte loads per thread in flight and are launched with programmatic stream serialization, so
 // that they and the GEMM behind them overlap their set-up.  us, with the cast walking forwards behind its wait / as it is:
 // 8000 x 8192 100.0 / 89.2, 3000 x 6000 29.4 / 28.3, 1000 x 4096 10.97 / 10.57, 64 x 2048 3.79 / 3.65.
+#include <cooperative_groups.h>
 #include <cuda_fp8.h>
 
 #include "common.cuh"
@@ -20,17 +21,30 @@ constexpr int kQuantUnroll = 4;
 constexpr int kBlocksPerSm = 6;  // of a grid at most
 constexpr int kMaxParts = B200K_QUANTIZE_WORKSPACE_BYTES / 4;
 
+template <int THREADS = kQuantThreads>
 __device__ __forceinline__ float block_max(float m) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __shared__ float wm[kQuantThreads / 32];
+  __shared__ float wm[THREADS / 32];
   if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
   __syncthreads();
   m = wm[0];
 #pragma unroll
-  for (int w = 1; w < kQuantThreads / 32; ++w) m = fmaxf(m, wm[w]);
+  for (int w = 1; w < THREADS / 32; ++w) m = fmaxf(m, wm[w]);
   return m;
 }
+
+// scale = max|x| / 448 and how to multiply by its inverse
+struct Scale {
+  float scale, inv;
+  bool divide;
+  __device__ __forceinline__ explicit Scale(float amax) {
+    scale = amax > 0.f ? __fdiv_rn(amax, kE4M3Max) : 1.0f;
+    // a reciprocal that overflows or vanishes says nothing about the quotient: divide every value then
+    inv = __fdiv_rn(1.0f, scale);
+    divide = !(inv < 1e38f && inv > 1e-37f);
+  }
+};
 
 // parts: one value per block, or (one_part) a single word that was zeroed before the launch.
 __global__ void __launch_bounds__(kQuantThreads) absmax_kernel(const float* x, int64_t n, uint32_t* parts,
@@ -110,10 +124,9 @@ __global__ void __launch_bounds__(kQuantThreads, BLOCKS_PER_SM) cast_e4m3_kernel
   float m = 0.f;
   for (int k = threadIdx.x; k < num_parts; k += kQuantThreads) m = fmaxf(m, __uint_as_float(parts[k]));
   const float amax = block_max(m);
-  const float scale = amax > 0.f ? __fdiv_rn(amax, kE4M3Max) : 1.0f;
-  // a reciprocal that overflows or vanishes says nothing about the quotient: divide every value then
-  const float inv = __fdiv_rn(1.0f, scale);
-  const bool divide = !(inv < 1e38f && inv > 1e-37f);
+  const Scale q(amax);
+  const float scale = q.scale, inv = q.inv;
+  const bool divide = q.divide;
   if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
   while (i >= 0) {
 #pragma unroll
@@ -126,6 +139,60 @@ __global__ void __launch_bounds__(kQuantThreads, BLOCKS_PER_SM) cast_e4m3_kernel
   }
   for (int64_t k = n4 * 4 + i0; k < n; k += stride)
     y[k] = __nv_cvt_float_to_fp8(__fdiv_rn(x[k], scale), __NV_SATFINITE, __NV_E4M3);
+}
+
+// One launch for what registers hold: x stays in them between the maximum and the cast, over a barrier.  CLUSTER: up to eight
+// blocks of a thread-block cluster, which exchange their maxima through shared memory.  Else two blocks of every SM, launched
+// cooperatively, and the barrier of the grid; the CUDA runtime keeps its state per launch, so launches of other streams and
+// replays of a graph do not meet in it.  A cooperative launch does not start early and costs some 1.5 us more, which the second read of x
+// outweighs from 3.5 M values on.  With a product behind, us, two launches / one: cluster 16x2379x1824 (0.03 M values) 14.3 / 12.6,
+// 64x4096x4096 (0.26 M) 14.6 / 12.9, 250x2000x1040 14.2 / 12.9; cooperative 860x4096x4096 (3.5 M) 26.2 / 25.4, 1000x4096x4096 28.2 /
+// 26.6, 1180x4096x4096 37.8 / 35.3, 2772x2641x1700 36.2 / 32.8; below the line 3400x2048x1000 20.4 / 20.5, 1228x3880x1520
+// 22.9 / 24.6, 400x4096x2000 15.9 / 16.9.  1024 threads in one block per SM: no faster (3.5 M 26.1).
+constexpr int kResidentUnroll = 8;  // float4 per thread at most
+constexpr int64_t kClusterValues = 8 * 1024 * kResidentUnroll * 4;
+constexpr int64_t kCooperativeValues = 3500000;  // and more
+
+template <bool CLUSTER>
+__global__ void __launch_bounds__(CLUSTER ? 1024 : 512, CLUSTER ? 1 : 2)
+    quantize_resident_kernel(const float* x, uint8_t* y, int64_t n, uint32_t* parts, float* scale_out) {
+  constexpr int kThreads = CLUSTER ? 1024 : 512;
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads;
+  const int64_t n4 = n / 4;
+  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  float4 v[kResidentUnroll];
+#pragma unroll
+  for (int u = 0; u < kResidentUnroll; ++u)
+    v[u] = i0 + u * stride < n4 ? reinterpret_cast<const float4*>(x)[i0 + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float last = n4 * 4 + i0 < n ? x[n4 * 4 + i0] : 0.f;
+  float m = fabsf(last);
+#pragma unroll
+  for (int u = 0; u < kResidentUnroll; ++u)
+    m = fmaxf(m, fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w))));
+  m = block_max<kThreads>(m);
+  if constexpr (CLUSTER) {
+    __shared__ float mine;
+    if (threadIdx.x == 0) mine = m;
+    cluster_sync_all();
+    m = 0.f;
+    for (int c = 0; c < static_cast<int>(gridDim.x); ++c)
+      m = fmaxf(m, ld_shared_cluster_f32(cluster_map_shared(smem_u32(&mine), c)));
+  } else {
+    if (threadIdx.x == 0) parts[blockIdx.x] = __float_as_uint(m);
+    cooperative_groups::this_grid().sync();
+    m = 0.f;
+    for (int c = threadIdx.x; c < static_cast<int>(gridDim.x); c += kThreads) m = fmaxf(m, __uint_as_float(__ldcg(parts + c)));
+    m = block_max<kThreads>(m);
+  }
+  const Scale q(m);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = q.scale;
+#pragma unroll
+  for (int u = 0; u < kResidentUnroll; ++u)
+    if (i0 + u * stride < n4) reinterpret_cast<uint32_t*>(y)[i0 + u * stride] = quantize_quad(v[u], q.inv, q.scale, q.divide);
+  if (n4 * 4 + i0 < n) y[n4 * 4 + i0] = __nv_cvt_float_to_fp8(__fdiv_rn(last, q.scale), __NV_SATFINITE, __NV_E4M3);
+  if constexpr (CLUSTER) cluster_sync_all();  // no block leaves while another may still read its maximum
 }
 
 }  // namespace
@@ -143,6 +210,26 @@ int launch_quantize_e4m3(const float* x, void* y, float* scale_out, uint32_t* am
   if (one_part) {
     rc = check_cuda(cudaMemsetAsync(amax_scratch, 0, sizeof(uint32_t), stream), "quantize_e4m3: memset");
     if (rc) return rc;
+  }
+  if (!one_part && n <= kClusterValues) {
+    const int64_t blocks = (n / 4 + 1023) / 1024;
+    const int ctas = blocks <= 1 ? 1 : blocks <= 2 ? 2 : blocks <= 4 ? 4 : 8;
+    return launch_cluster("quantize_resident_kernel launch", quantize_resident_kernel<true>, ctas, dim3(ctas), dim3(1024), 0, stream,
+                          x, static_cast<uint8_t*>(y), n, amax_scratch, scale_out);
+  }
+  const int64_t resident = 2 * static_cast<int64_t>(num_sms());
+  if (!one_part && n >= kCooperativeValues && n <= resident * 512 * kResidentUnroll * 4 && resident <= kMaxParts) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(resident));
+    cfg.blockDim = dim3(512);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return check_cuda(cudaLaunchKernelEx(&cfg, quantize_resident_kernel<false>, x, static_cast<uint8_t*>(y), n, amax_scratch, scale_out),
+                      "quantize_resident_kernel launch");
   }
   const int64_t want = (n / 4 + kQuantThreads * kQuantUnroll - 1) / (kQuantThreads * kQuantUnroll);
   int64_t cap = static_cast<int64_t>(num_sms()) * kBlocksPerSm;

@@ -48,6 +48,50 @@ def test_quantize_in_several_passes(n):
     assert torch.equal(y.cpu().view(torch.uint8), yo.view(torch.uint8))
 
 
+# One launch: clusters of 1, 2, 4 and 8 blocks of 1024 threads with up to eight vectors of four each, and from 3500000 to
+# 148 * 2 * 512 * 32 values the whole grid; two launches in between and beyond.
+@pytest.mark.parametrize("n", [4096, 4097, 8192, 8197, 16390, 32_771, 262_143, 262_144, 262_145, 3_499_999, 3_500_000, 3_500_003, 4_849_663,
+                               4_849_664, 4_849_665])
+@pytest.mark.parametrize("largest", [0, 1, 2])
+def test_quantize_resident(n, largest):
+    """The largest value first, last and in the middle, x written just before the call; the same bytes on every call."""
+    base = torch.randn(n, generator=torch.Generator().manual_seed(n))
+    base[[0, n - 1, n // 2][largest]] = -30.0
+    x, new = base.to(DEV), torch.zeros(n, device=DEV)
+    yo, so = oracle.quantize_e4m3(base)
+    for _ in range(3):
+        new.zero_()
+        new.add_(x)
+        y, s = torch.ops.b200k.quantize_e4m3(new)
+        assert torch.equal(s.cpu().reshape(-1), so.reshape(-1))
+        assert torch.equal(y.cpu().view(torch.uint8), yo.view(torch.uint8))
+
+
+def test_quantize_resident_on_two_streams_and_in_a_graph():
+    """The barrier of the grid belongs to the launch: concurrent ones and replays do not meet in it."""
+    xs = [torch.randn(n, device=DEV) * f for n, f in ((4_000_000, 1.0), (3_600_001, 3.0))]
+    want = [torch.ops.b200k.quantize_e4m3(x) for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(20):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                got[i].append(torch.ops.b200k.quantize_e4m3(xs[i]))
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(y.view(torch.uint8), want[i][0].view(torch.uint8)) and torch.equal(s, want[i][1]) for y, s in got[i])
+    x = xs[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y, s = torch.ops.b200k.quantize_e4m3(x)
+    for scale in (1.0, 0.5, 2.0):
+        x.copy_(xs[0] * scale)
+        graph.replay()
+        wy, ws = torch.ops.b200k.quantize_e4m3(xs[0] * scale)
+        assert torch.equal(y.view(torch.uint8), wy.view(torch.uint8)) and torch.equal(s, ws)
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 8), (7, 64), (8, 56), (31, 72), (33, 520), (129, 128), (1000, 264), (4099, 1032)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_col_sum(rows, cols, dtype):
