@@ -556,31 +556,35 @@ int launch_gemm_impl(const b200k_gemm_args& a, const PeerTargets& peers, cudaStr
   // Tile shape and split: the smallest estimated time, in us.  A launch of whole tiles takes
   //   fixed + waves * (k-blocks * per_kb + wave),
   // fitted to 27 shapes for the tiles of one CTA (rows 1 to 6000, K 300 to 16000, operands from HBM, launches back to
-  // back) and to 73 more for the 256 x 256 tiles of a pair (74 pairs to a wave).  k-blocks of 128 x 256 and pair tiles
+  // back) and to 136 more for the 256 x 256 tiles of a pair (74 pairs to a wave).  k-blocks of 128 x 256 and pair tiles
   // run at the tensor core's 512 cycles, at the 1.45 to 1.65 GHz that the SMs keep while all of them multiply; `wave`
-  // is the part of an epilogue that the next tile does not hide.  Operand rows that do not start on 128-byte lines cost
-  // more L2 traffic (`lines`), rows of C that the TMA unit cannot store a longer epilogue (`ragged`).  What the choice gives on
-  // the 73 shapes, against the former one with 256 x 256 tiles of one CTA, is 4.7 % in the mean (the best of all
-  // tiles for each: 5.4 %); 1761x6993x4272 fp8 80.5 -> 58.2, 5034x2320x4680 [K, N] 119 -> 95, 1979x3384x2448 35.0 -> 31.2.
+  // is the part of an epilogue that the next tile does not hide, `least` what a wave takes of a pair whose few k-blocks are shorter
+  // than its epilogue (7344x2256x303 128 x 256 16.2, pair 17.8).  Operand rows that do not start on 128-byte lines cost
+  // more L2 traffic (`lines`; pairs fetch the least), rows of C that the TMA unit cannot store a longer epilogue (`ragged`).
+  // On the 136 shapes the choice is 0.6 % in the mean above the best tile for each, and 4 % below the choice without pairs;
+  // 1761x6993x4272 fp8 80.5 -> 58.2, 5034x2320x4680 [K, N] 119 -> 95, 1979x3384x2448 35.0 -> 31.2, 7750x704x696 18.6 -> 15.2; slower is
+  // 1088x3520x1345 [K, M] [K, N] 11.5 -> 12.2.  (Pairs of 256 x 128, built and taken out: 2048x1024x4096 18.7 -> 17.0, 2248x936x5110
+  // 35.7 -> 31.6, but ahead of the others on one shape in ten only.)
   // Split-K over a cluster of s CTAs is not persistent: every wave of resident clusters pays
   //   fixed + k-blocks / s * per_kb + (partial tiles to shared memory, two cluster barriers, reduction),
   // the last term 1 us plus 1.4 / 2 / 4 us for a tile of 128 rows.
   struct Shape {
     int m, n;
-    double fixed, per_kb, lines, wave, ragged, reduce;
+    double fixed, per_kb, lines, wave, least, ragged, reduce;
   };
   const bool lines = (a.lda * in_es) % 128 != 0 || (a.ldb * in_es) % 128 != 0;
   const bool ragged = peers.num == 0 && ((reinterpret_cast<uintptr_t>(a.c) & 15) != 0 || (a.ldc * out_es) % 16 != 0 || (a.n * out_es) % 16 != 0);
-  const Shape kShapes[4] = {{128, 64, 3.4, .20, 1.15, 0., .5, 1.4},
-                            {128, 128, 3.7, .25, 1.15, 0., 1., 2.},
-                            {128, 256, 4.5, .39, 1.15, 0., 2., 4.},
-                            {256, 256, 4.5, .28, 1.1, 1., 3., 0.}};
+  const Shape kShapes[4] = {{128, 64, 3.4, .20, 1.15, 0., 0., .5, 1.4},
+                            {128, 128, 3.7, .25, 1.15, 0., 0., 1., 2.},
+                            {128, 256, 4.5, .39, 1.15, 0., 0., 2., 4.},
+                            {256, 256, 4.5, .28, 1., .5, 2.4, 3., 0.}};
   auto per_kb = [&](const Shape& t) { return t.per_kb * (lines ? t.lines : 1.); };
   auto tiles_of = [&](const Shape& t) { return ((a.m + t.m - 1) / t.m) * ((a.n + t.n - 1) / t.n) * batch; };
   auto whole_us = [&](const Shape& t) {
     const int64_t units = t.m == 256 ? sms / 2 : sms;
     const int64_t waves = (tiles_of(t) + units - 1) / units;
-    return t.fixed + static_cast<double>(waves) * (num_kb * per_kb(t) + t.wave + (ragged ? t.ragged : 0.));
+    const double wave = num_kb * per_kb(t) + t.wave;
+    return t.fixed + static_cast<double>(waves) * ((wave > t.least ? wave : t.least) + (ragged ? t.ragged : 0.));
   };
   int bm = a.tile_m, bn = a.tile_n;
   if (bm == 256 && bn == 0) bn = 256;
