@@ -352,12 +352,14 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
         bool ok = true;
         const int pages_per_tile = PAGED ? kTileRows / p.page_size : 1;
         // Page of this lane's part of tile j; a page past the sequence's length is replaced by the
-        // sequence's first page (those rows are masked; the data only has to be finite).
+        // sequence's first page (those rows are masked; the data only has to be finite).  What needs a division is worked out
+        // once per item: this warp gets an issue slot in ten cycles beside the softmax.
+        const int32_t* row = nullptr;  // of the table
+        int valid_pages = 0, kvh = 0;
         auto page_of = [&](const Item& it, int j) {
           if (!PAGED || lane >= pages_per_tile || j >= it.nmax) return 0;
           const int lp = j * pages_per_tile + lane;
-          const int valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
-          return p.block_table[static_cast<int64_t>(it.batch) * p.block_table_stride + (lp < valid_pages ? lp : 0)];
+          return row[lp < valid_pages ? lp : 0];
         };
         // One 128-row K or V tile.  A table entry outside the pool is reported and reads as zeros (the
         // tensor map clips it).
@@ -373,7 +375,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
           if (!PAGED) {
 #pragma unroll
             for (int db = 0; db < kBlocks; ++db)
-              tma_load_4d(dst + db * kHalfTileBytes, tm, bar, db * 64, j * kTileRows, it.head / group, it.batch);
+              tma_load_4d(dst + db * kHalfTileBytes, tm, bar, db * 64, j * kTileRows, kvh, it.batch);
             return true;
           }
           __syncwarp();  // the bytes are announced before any of them can arrive
@@ -381,13 +383,18 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
             if ((page < 0 || page >= p.num_pages) && p.status) atomicOr(p.status, kStatusDecodeBadPage);
 #pragma unroll
             for (int db = 0; db < kBlocks; ++db)
-              tma_load_4d(dst + db * kHalfTileBytes + lane * p.page_size * 128, tm, bar, db * 64, 0, it.head / group, page);
+              tma_load_4d(dst + db * kHalfTileBytes + lane * p.page_size * 128, tm, bar, db * 64, 0, kvh, page);
           }
           return true;
         };
         ItemWalk<PAGED> walk(p, table);
         Item it;
         while (ok && walk.next_busy(it)) {
+          kvh = it.head / group;
+          if (PAGED) {
+            row = p.block_table + static_cast<int64_t>(it.batch) * p.block_table_stride;
+            valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
+          }
           int page = page_of(it, 0);
           for (int j = 0; j < it.nmax && ok; ++j) {
             const int page_next = page_of(it, j + 1);
@@ -929,16 +936,16 @@ int fill_pair_order(AttnParams& p, const char* who, int head_dim, bool paged) {
 }
 
 // Which kernel runs a problem (B200K_ATTN_AUTO); head dim 64 exists in the pair kernel only.  Measured at
-// head dim 128, one-tile / tile-pair, us.
+// head dim 128, one-tile / tile-pair, us, launches back to back.
 // Without a mask the one-tile kernel, whatever the batch: the two round probabilities against another running max, and a
-// choice by how the items fill the SMs would let a head's bits depend on the heads beside it.  It would gain little even
-// where pairs need half the rounds: 4x16x4096 511 / 507, 1x8x8192 264 / 257, but 8x32x1024 136 / 142, 1x16x4096 136 / 141,
-// 4x32(8)x512 25.7 / 26.0; elsewhere pairs are slower: 2x16x4096 252 / 283, 1x8x2048 21.7 / 35.8, 24x64x308 143 / 183.
-// Causal, couples that fill their rounds: 4x32x4096 555 / 527, 8x32x2048 336 / 308, 16x64x512 160 / 117, 32x32x256
-// 67 / 57: the pair kernel.  Other causal problems, with the pair kernel in its better order: 2x32(8)x2000 74 / 73,
-// 4x8x4096 144 / 144, 16x16(4)x1024 92 / 97, 1x64(8)x6000 569 / 577, 1x4x8192 67 / 123, 1x32(8)x1200 20.5 / 24.4: the
-// one-tile kernel, as for at most 128 queries, where every pair is half empty: 32x32x128 27.9 / 33.3, 37x16x128 18.5 / 20.7,
-// 32x32 100 over 1000 97.2 / 115.7, 16x37x17 13.9 / 14.9.
+// choice by how the items fill the SMs would let a head's bits depend on the heads beside it.  Pairs are ahead only where they need half
+// the rounds, 8x32x1024 138 / 125; equal 4x16x4096 438 / 434, 1x8x8192 245 / 243, 4x32(8)x512 25.3 / 25.6; elsewhere slower:
+// 1x16x4096 123 / 128, 2x16x4096 234 / 252, 1x8x2048 21.1 / 36.7, 24x64x308 121 / 170.
+// Causal, couples that fill their rounds: 4x32x4096 523 / 532 (the fastest of seven runs 490 / 474), 8x32x2048 290 / 279,
+// 16x64x512 150 / 113, 32x32x256 64 / 56, 4x37x1000 59.7 / 49.5: the pair kernel.  Other causal problems, with the pair kernel in its better
+// order: 2x32(8)x2000 67.7 / 73.9, 4x8x4096 128 / 133, 16x16(4)x1024 87 / 96, 1x64(8)x6000 520 / 548, 1x4x8192 62 / 122, 1x32(8)x1200
+// 20.2 / 24.8: the one-tile kernel, as for at most 128 queries, where every pair is half empty: 32x32x128 27.8 / 33.5, 37x16x128
+// 18.3 / 20.7, 32x32 100 over 1000 93.8 / 99.1, 16x37x17 17.6 / 17.9.
 bool choose_pair_kernel(const b200k_attention_args& a) {
   if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
   if (a.kernel == B200K_ATTN_ONE_TILE || !a.causal || a.seq_q <= kTileRows) return false;
@@ -970,14 +977,14 @@ bool tiles_finish_first(const b200k_paged_attention_args& a, int heads, int tile
 }
 
 // Paged: a K/V tile arrives page by page, and the pair kernel needs half as many tiles.  One-tile / tile-pair,
-// us: 4x32(8) 512 queries over up to 4000 keys 156 / 87 at page size 16, 114 / 95 at 64, 107 / 95 at 128;
-// 3x64(16) 1000 over 2000 170 / 146.  The one-tile kernel is ahead where the SMs are not filled and pages are
-// larger (1x8 2000 over 6000 81 / 98 at page size 32, 71 / 98 at 64, but 1x8 64 over 6000 at 16 96 / 81), where
-// a pair would be half empty (16x16(4) 100 over 3000, page size 64, 39 / 41), and where one round of pairs would do but the
-// longest of them decides: at page size 64 2x16(4) 1024 of 1024 19.3 / 21.8, 1x10(2) 3000 of 3000 36.9 / 50.3, 8x2(1) 2000
-// of 2100 31.5 / 39.4, 1x40(8) 600 of 600 13.8 / 14.2, but 8x8(2) 512 over 4000 82.9 / 67.8, 3x16(2) 536 of 588 18.5 / 15.6,
-// 1x64(16) 449 over 4295 90.5 / 73.2.  (Histories of very different lengths would gain too, 2x8(1) 1235 over 2425 and 3615
-// 39.1 / 57.8, but nothing here tells them from equal ones.)
+// us: 4x32(8) 512 queries over up to 4000 keys 143 / 86 at page size 16, 88 / 83 at 64, 89 / 90 at 128;
+// 3x64(16) 1000 over 2000 116 / 105.  The one-tile kernel is ahead where the SMs are not filled and pages are
+// larger (1x8 2000 over 6000 67 / 95 at page size 32, 54 / 92 at 64, but 1x8 64 over 6000 at 16 84 / 69), where
+// a pair would be half empty (16x16(4) 100 over 3000, page size 64, 58 / 72), and where one round of pairs would do but the
+// longest of them decides: at page size 64 2x16(4) 1024 of 1024 18.4 / 21.9, 1x10(2) 3000 of 3000 31.5 / 50.2, 8x2(1) 2000
+// of 2100 28.7 / 39.7, 1x40(8) 600 of 600 13.8 / 14.2, but 8x8(2) 512 over 4000 69.9 / 67.4, 3x16(2) 536 of 588 16.7 / 16.2,
+// 1x64(16) 449 over 4295 75.9 / 72.2.  (Histories of very different lengths gain too, 2x8(1) 1235 over 2425 and 3615
+// 35.2 / 59.5, 14x4 285 over 483 to 3047 31.3 / 52.4, but nothing here tells them from equal ones.)
 bool choose_pair_kernel(const b200k_paged_attention_args& a) {
   if (a.head_dim != 128 || a.kernel == B200K_ATTN_TILE_PAIR) return true;
   if (a.kernel == B200K_ATTN_ONE_TILE) return false;
@@ -992,7 +999,8 @@ bool choose_pair_kernel(const b200k_paged_attention_args& a) {
 // CTAs that share the K/V tiles of each item of a call (the one-tile kernel in clusters), 1 = one CTA per item.  Few items
 // leave SMs idle while each item is one chain of K/V tiles: 2x2 164 queries over 4652 keys, page size 16, 71.8 us by one CTA
 // per item, 44.8 / 27.4 / 17.8 by clusters of 2 / 4 / 8; 1x16(4) 29 over 3244, page size 32, 42.2, 24.9 / 16.7; 2x8(8) 758 over 3239
-// 52.1, 33.7; 4x4 22 over 1221 19.2, 12.9 / 10.6 / 9.9; dense causal 2x1x2802 24.8, 19.1, 1x2x1000 12.6, 11.6 / 10.3.  A tile costs 0.85 us
+// 52.1, 33.7; 4x4 22 over 1221 19.2, 12.9 / 10.6 / 9.9; dense causal 2x1x2802 24.8, 19.1, 1x2x1000 12.6, 11.6 / 10.3 (all with steps of
+// 128 keys; with those of 64 the chosen ones take 5 to 10 % less: 16.7, 15.1, 30.5, 18.2 of 17.8, 16.7, 33.7, 19.1).  A tile costs 0.85 us
 // dense and 1 to 1.6 by pages (the more loads a tile takes, the more), adding up 3.4 / 3.8 / 4.6; against that 51 calls came
 // out right but for 0.5 us.  Where it would gain less than 1 us, items stay whole: dense 7x1x459 9.0, 9.9 / 10.8, 1x8x1000
 // 13.2, 13.4; paged 2x8 370 of 436 10.8, 12.6.  All items have to be resident at once.

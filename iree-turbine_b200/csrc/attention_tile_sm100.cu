@@ -1,45 +1,47 @@
 // Attention forward (vanilla and causal), head dim 128, on sm_100a: the ONE-TILE kernel.
 //
 // Two kernels share the forward path (launch_attention_fwd in attention_sm100.cu chooses): this one,
-// whose work item is a single 128-row query tile served by two softmax warpgroups on alternate KV
-// steps with double-buffered score tiles, and the tile-pair kernel in attention_sm100.cu.  This one
-// keeps both softmax warpgroups busy all the time and has the finer work granularity: it is the
-// faster of the two on non-causal problems and where the pair kernel's units fill the SMs badly.
+// whose work item is a single 128-row query tile served by three softmax warpgroups in turn, and the tile-pair kernel in
+// attention_sm100.cu.  This one has the finer work granularity, reads no Q through the shared-memory port, and is the faster of the two except
+// where pairs fill the SMs (causal) or where pages make tile loads dear.
 //
 // Persistent CTAs, one per SM.  A work item is one 128-row query tile of one (batch, head); which CTA
-// takes which items, and in what order, is in attention_order.cuh.
+// takes which items, and in what order, is in attention_order.cuh.  An item is walked through in steps of 64 keys, two to a K/V tile.
 //
-//   warps 0..3    softmax + correction of the even KV steps of the CTA (thread = query row)
-//   warps 4..7    the same for the odd KV steps
-//   warps 8..11   epilogue: O / rowsum -> global, one item behind the others
-//   warp 12       TMA loads: Q of the next item, K_j (3 stages), V_j (2 stages)
-//   warp 13       issues the score MMAs (S = Q K^T) and owns tensor memory
-//   warp 14       issues the second MMAs (O += P V)
-//   warp 15       idle (completes the fourth warpgroup for the setmaxnreg register hand-off)
+//   warps 0..11   softmax + correction: warpgroup w takes the steps g of the CTA with g % 3 == w (thread = query row)
+//   warps 12..15  epilogue: O / rowsum -> global, and Q of the next item from shared to tensor memory
+//   warp 16       TMA loads: Q of the next item, K_j (3 stages), V_j (2 stages)
+//   warp 17       issues the score MMAs (S = Q K^T) and owns tensor memory
+//   warp 18       issues the second MMAs (O += P V)
+//   warp 19       idle (completes the last warpgroup for the setmaxnreg register hand-off)
 //
-// Tensor memory (512 columns x 128 lanes):  S[0] | S[1] (128 fp32 columns each) | P[0] | P[1]
-// (64 columns each: 128 16-bit probabilities per row) | O (128 fp32 columns).
-//   * Score tile g goes to S[g & 1] and is handled by softmax warpgroup g & 1, which writes P[g & 1].
-//     The two warpgroups are half a step apart: while one is in its latency-bound part (wait,
-//     tensor-memory load, row max, hand-over) the other runs its exponentials.  They share ONE
-//     running row max and ONE accumulator: early in its step a warpgroup reads the running max the
-//     other published half a step before, decides whether this tile raises it (by more than 2^8),
-//     and publishes the result; only when it does raise it is O rescaled, by that warpgroup, after
-//     "O += P V" of the previous step (the other warpgroup's) has completed and before its own P is
+// Tensor memory (480 of 512 columns x 128 lanes):  S[3] (64 fp32 columns each) | P[3] (32 columns each: 64 16-bit
+// probabilities per row) | O (128 fp32 columns) | Q (64 columns: 128 16-bit values per row).
+//   * The warpgroups are a third of a round apart: while one is in its latency-bound part (wait,
+//     tensor-memory load, row max, hand-over) the others run their exponentials.  They share ONE
+//     running row max and ONE accumulator: early in its step a warpgroup reads the running max that
+//     the one before it published, decides whether these scores raise it (by more than 2^8),
+//     and publishes the result; only when they do is O rescaled, by that warpgroup, after
+//     "O += P V" of the previous step has completed and before its own P is
 //     handed over.  Each warpgroup keeps a partial row sum relative to the running max it last saw;
-//     the epilogue brings the two to the final max and adds them.
-//   * A softmax thread holds its whole score row in registers, so a score buffer is free
-//     again early in the step, as soon as the row has been loaded: S(j+2) is issued then.  The
-//     probabilities have buffers of their own for that reason.  The tensor core is never what the
-//     softmax waits for: neither the scores of the next step nor "O += P V" of the last one is on
-//     its critical path.
-//   * Two threads issue MMAs.  A tcgen05.mma does not return until the tensor pipe has room for
-//     it, so a group of eight blocks its thread for about as long as it executes (plus some 300
-//     cycles when the pipe was idle); with one issuing thread every wait of one kind of MMA
-//     delayed the other.
+//     the epilogue brings them to the final max and adds them.
+//   * A softmax thread holds its score row in registers, so a score buffer is free
+//     again early in the step, as soon as the row has been loaded.  The probabilities have buffers of their own for that reason.  The
+//     tensor core is never what the softmax waits for.
+//   * Two threads issue MMAs, scores and P V.  Both A operands are in tensor memory: with Q in shared memory a score MMA of
+//     64 columns takes 48 cycles, this way 33.  Each of the two warps gets an issue slot in about ten cycles beside twelve
+//     softmax warps, so their loops are a few instructions per wait, MMA and commit: with barrier addresses
+//     worked out anew each time the P V thread took 1000 cycles per step of 256.
+//   * A step has one vote of the warp, at its end, over its four waits; a vote per wait cost some 100 cycles each.
 //   * One output accumulator is enough: the first "O = P V" of an item is needed a whole softmax
 //     step after the last one of the previous item, and the epilogue reads O in less than that.
-//   * P is the A operand of the second MMA straight from tensor memory.
+//
+// Before, two warpgroups took steps of 128 keys with Q in shared memory: 3990 cycles for 256 keys, their exponentials
+// at the same time and most of the rest in nobody's shadow.  Now 2200 cycles for 192 keys (1470 per 128): load 110, max 200, hand-over 290,
+// exponentials 850 to 1000 beside two other warps of the sub-partition, the rest waits that are satisfied and stores.
+// us, two warpgroups / three: 8x32x1024 151 / 146, 4x16x4096 523 / 481, 1x8x8192 267 / 248, 2x32(8)x2000 causal 80.1 / 75.2, 24x64x308 142 /
+// 129, 1x8x2048 21.3 / 20.3, 2x16x192 causal 7.44 / 6.79, 1x16x1000 causal 14.2 / 13.7; equal or up to 1.5 % slower for items of one to four tiles
+// that fill several rounds (16x16x512 47.7 / 48.5, 32x32x128 causal 28.0 / 28.3).  Long launches are under the power cap.
 //
 // Epilogue: accumulator -> registers -> 16-bit -> 128-byte-swizzled staging block (64 columns) in
 // shared memory -> TMA store, twice (rows past the end of the sequence are clipped by the tensor
@@ -59,16 +61,20 @@
 namespace b200k {
 namespace {
 
-constexpr int kAttnThreads = 512;
-constexpr int kTmaWarp = 12;
-constexpr int kScoreWarp = 13;
-constexpr int kPvWarp = 14;
-// Registers: 4 warps per SM sub-partition x 128 at launch = 512 per lane, redistributed.  A
-// setmaxnreg.inc beyond what the others gave up never completes.
-constexpr int kRegsSoftmax = 184;
+constexpr int kGroups = 3;  // softmax warpgroups
+constexpr int kEpiWarp = 4 * kGroups;
+constexpr int kTmaWarp = kEpiWarp + 4;
+constexpr int kScoreWarp = kTmaWarp + 1;
+constexpr int kPvWarp = kTmaWarp + 2;
+constexpr int kAttnThreads = 32 * (kTmaWarp + 4);
+// Registers: 5 warps per SM sub-partition x 96 at launch = 480 per lane, redistributed.  A setmaxnreg.inc beyond what the
+// others gave up never completes.  (120 for the softmax leave the epilogue or the loads too few: 200 to 600 bytes of spills.)
+constexpr int kRegsSoftmax = 112;
 constexpr int kRegsEpilogue = 80;
 constexpr int kRegsOther = 64;
-static_assert(2 * kRegsSoftmax + kRegsEpilogue + kRegsOther <= 512, "setmaxnreg.inc would never complete");
+constexpr int kRegsLaunch = 65536 / kAttnThreads / 8 * 8;
+static_assert(kGroups * kRegsSoftmax + kRegsEpilogue + kRegsOther <= (kGroups + 2) * kRegsLaunch, "setmaxnreg.inc would never complete");
+constexpr int kStep = 64;  // keys of a step
 constexpr int kTileRows = 128;  // query rows per item, KV rows per tile
 constexpr int kD = 128;
 constexpr int kHalfTileBytes = kTileRows * 128;  // one 64-element column block: 16 KB
@@ -80,16 +86,18 @@ constexpr int kKOffset = kTileBytes;
 constexpr int kVOffset = kKOffset + kKStages * kTileBytes;
 constexpr int kOStageOffset = kVOffset + kVStages * kTileBytes;  // epilogue staging: one 64-column block
 constexpr int kMaxOffset = kOStageOffset + kHalfTileBytes;   // float [warpgroup][128 rows]: running max it published
-constexpr int kLsumOffset = kMaxOffset + 2 * kTileRows * 4;  // float [warpgroup][max, sum][128 rows] for the epilogue
-constexpr int kOrderOffset = kLsumOffset + 2 * 2 * kTileRows * 4;  // uint16: item order of a paged call
+constexpr int kLsumOffset = kMaxOffset + kGroups * kTileRows * 4;  // float [warpgroup][max, sum][128 rows] for the epilogue
+constexpr int kOrderOffset = kLsumOffset + kGroups * 2 * kTileRows * 4;  // uint16: item order of a paged call
 constexpr int kBarOffset = kOrderOffset + attn_order::kSortBytes;
-// q_full q_empty | k_full[3] k_empty[3] v_full[2] v_empty[2] | s_full[2] s_free[2] p_full[2] x_full[2] |
-// o_done[2] | o_full o_free l_full l_free
-constexpr int kNumBars = 2 + 2 * kKStages + 2 * kVStages + 8 + 2 + 4;
+// q_full q_empty q_ready q_done | k_full[3] k_empty[3] v_full[2] v_empty[2] | [group] s_full s_free p_full x_full o_done |
+// o_full o_free l_full l_free
+constexpr int kNumBars = 4 + 2 * kKStages + 2 * kVStages + 5 * kGroups + 4;
 // tensor memory columns
-constexpr uint32_t kTmemS = 0;    // + 128 * buffer
-constexpr uint32_t kTmemP = 256;  // + 64 * buffer
-constexpr uint32_t kTmemO = 384;
+constexpr uint32_t kTmemS = 0;                          // + 64 * group
+constexpr uint32_t kTmemP = kTmemS + kStep * kGroups;       // + 32 * group
+constexpr uint32_t kTmemO = kTmemP + kStep / 2 * kGroups;
+constexpr uint32_t kTmemQ = kTmemO + kD;
+static_assert(kTmemQ + kD / 2 <= 512, "tensor memory");
 constexpr int kAttnSmem = kBarOffset + kNumBars * 8 + 16 + 1024;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.0f;
@@ -137,6 +145,7 @@ __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi)
 
 struct Item {
   int qtile, head, batch, n;  // n = number of 128-row KV tiles this item visits
+  int steps;                  // of 64 keys
   int first;                  // ... from this one on (SPLIT: this CTA's share of the item; else 0)
   bool shared;                // SPLIT: the item is divided; else the first CTA of the cluster has it all
   int kv_len, causal_offset;  // keys of this item's sequence; key j is visible to query i iff j <= i + causal_offset
@@ -159,6 +168,9 @@ __device__ __forceinline__ Item make_item(int batch, int head, int qtile, const 
     const int last_col = it.qtile * kTileRows + kTileRows - 1 + it.causal_offset;
     it.n = last_col < 0 ? 0 : min(last_col / kTileRows + 1, kv_tiles_total);
   }
+  int visible = it.kv_len;
+  if (p.causal) visible = min(visible, it.qtile * kTileRows + kTileRows + it.causal_offset);
+  it.steps = max(0, (visible + kStep - 1) / kStep);
   it.first = 0;
   it.shared = false;
   if (SPLIT) {
@@ -167,8 +179,9 @@ __device__ __forceinline__ Item make_item(int batch, int head, int qtile, const 
     if (it.shared) {
       it.first = it.n * rank / ctas;
       it.n = it.n * (rank + 1) / ctas - it.first;
+      it.steps = min(2 * it.n, it.steps - 2 * it.first);
     } else if (rank != 0) {
-      it.n = 0;
+      it.n = it.steps = 0;
     }
   }
   return it;
@@ -267,11 +280,11 @@ __device__ __forceinline__ void merge_partials(const Item& it, uint32_t smem_bas
 // SPLIT: the K/V tiles of an item are divided over the CTAs of a cluster, one item per cluster.  Each CTA runs the same
 // pipeline over its share, leaves its unnormalised fp32 rows in its drained K ring and their maxima and sums beside, and after a
 // cluster barrier every CTA adds up its part of the rows that exist, in rank order.  See split_ctas for where and why.
-template <typename T, bool PAGED, bool ELECT, bool SPLIT>
+template <typename T, bool PAGED, bool SHORT, bool SPLIT>
 __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CUtensorMap& tmap_k, const CUtensorMap& tmap_v,
                                              const CUtensorMap& tmap_o, const AttnParams& p) {
   constexpr uint32_t kFmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBF16;
-  constexpr uint32_t kIdescS = make_idesc(kFmt, kFmt, 128, 128, 0, 0);   // Q, K both K-major
+  constexpr uint32_t kIdescS = make_idesc(kFmt, kFmt, 128, kStep, 0, 0);   // Q, K both K-major
   constexpr uint32_t kIdescPV = make_idesc(kFmt, kFmt, 128, 128, 0, 1);  // V is MN-major
 
   extern __shared__ uint8_t smem_raw[];
@@ -282,16 +295,18 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kBarOffset);
   uint64_t* q_full = bars;
   uint64_t* q_empty = bars + 1;
-  uint64_t* k_full = bars + 2;
+  uint64_t* q_ready = bars + 2;  // Q of an item is in tensor memory
+  uint64_t* q_done = bars + 3;   // the item's last score MMA has read it there
+  uint64_t* k_full = bars + 4;
   uint64_t* k_empty = k_full + kKStages;
   uint64_t* v_full = k_empty + kKStages;
   uint64_t* v_empty = v_full + kVStages;
   uint64_t* s_full = v_empty + kVStages;  // [buffer] score tile written
-  uint64_t* s_free = s_full + 2;          // [buffer] score tile is in the softmax threads' registers
-  uint64_t* p_full = s_free + 2;          // [buffer] probabilities written
-  uint64_t* x_full = p_full + 2;          // [warpgroup] it has published the row maxima after its step
-  uint64_t* o_done = x_full + 2;          // [step parity] "O += P V" of that step complete
-  uint64_t* o_full = o_done + 2;          // last P V of an item complete
+  uint64_t* s_free = s_full + kGroups;    // [buffer] score tile is in the softmax threads' registers
+  uint64_t* p_full = s_free + kGroups;         // [buffer] probabilities written
+  uint64_t* x_full = p_full + kGroups;         // [warpgroup] it has published the row maxima after its step
+  uint64_t* o_done = x_full + kGroups;         // [step parity] "O += P V" of that step complete
+  uint64_t* o_full = o_done + kGroups;         // last P V of an item complete
   uint64_t* o_free = o_full + 1;          // epilogue has read the accumulator
   uint64_t* l_full = o_free + 1;          // row sums written
   uint64_t* l_free = l_full + 1;          // row sums read
@@ -303,7 +318,9 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    mbar_init(q_empty, 1);
+    mbar_init(q_empty, 4);
+    mbar_init(q_ready, 4);
+    mbar_init(q_done, 1);
     for (int i = 0; i < kKStages; ++i) {
       mbar_init(k_full + i, 1);
       mbar_init(k_empty + i, 1);
@@ -312,7 +329,7 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
       mbar_init(v_full + i, 1);
       mbar_init(v_empty + i, 1);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kGroups; ++i) {
       mbar_init(s_full + i, 1);
       mbar_init(s_free + i, 4);
       mbar_init(p_full + i, 4);
@@ -321,7 +338,7 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
     }
     mbar_init(o_full, 1);
     mbar_init(o_free, 4);
-    mbar_init(l_full, 8);
+    mbar_init(l_full, 4 * kGroups);
     mbar_init(l_free, 4);
     *abort_word = 0;
     fence_barrier_init();
@@ -352,7 +369,7 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
 
   const bool shared_item = SPLIT && decode_item<PAGED, SPLIT>(ItemWalk<SPLIT>().pos, p, table).shared;
 
-  if (warp >= 12) {
+  if (warp >= kTmaWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
     if (warp == kTmaWarp) {
       // ---------------- TMA producer ----------------
@@ -366,21 +383,34 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
         bool ok = true;
         const int pages_per_tile = PAGED ? kTileRows / p.page_size : 1;
         // Page of this lane's part of tile j; a page past the sequence's length is replaced by the
-        // sequence's first page (those rows are masked; the data only has to be finite).
-        auto page_of = [&](const Item& it, int j) {
+        // sequence's first page (those rows are masked; the data only has to be finite).  The row of the table and its
+        // number of pages are worked out once per item: with a division per look-up this warp, which gets an issue slot in
+        // ten cycles beside the softmax, set the pace (1x8 64 queries over 6000 keys, page size 64, 63.7 us, 53.9 now; by pairs at page size 16 74.7 / 69.4).
+        struct Pages {
+          const int32_t* row;
+          int valid, kvh;
+        };
+        auto pages_of = [&](const Item& it) {
+          Pages r = {nullptr, 0, it.head / group};
+          if (PAGED) {
+            r.row = p.block_table + static_cast<int64_t>(it.batch) * p.block_table_stride;
+            r.valid = (it.kv_len + p.page_size - 1) / p.page_size;
+          }
+          return r;
+        };
+        auto page_of = [&](const Item& it, const Pages& pages, int j) {
           if (!PAGED || lane >= pages_per_tile || j >= it.n) return 0;
           const int lp = (it.first + j) * pages_per_tile + lane;
-          const int valid_pages = (it.kv_len + p.page_size - 1) / p.page_size;
-          return p.block_table[static_cast<int64_t>(it.batch) * p.block_table_stride + (lp < valid_pages ? lp : 0)];
+          return pages.row[lp < pages.valid ? lp : 0];
         };
         // One 128-row K or V tile (the caller has waited for the stage).  A table entry outside the pool
         // is reported and reads as zeros (the tensor map clips it).
-        auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, const Item& it, int j, int page) {
+        auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, const Item& it, int kvh, int j, int page) {
           if (!PAGED || lane == 0) mbar_arrive_expect_tx(bar, kTileBytes);
           if (!PAGED) {
 #pragma unroll
             for (int db = 0; db < 2; ++db)
-              tma_load_4d(dst + db * kHalfTileBytes, tm, bar, db * 64, (it.first + j) * kTileRows, it.head / group, it.batch);
+              tma_load_4d(dst + db * kHalfTileBytes, tm, bar, db * 64, (it.first + j) * kTileRows, kvh, it.batch);
             return;
           }
           __syncwarp();  // the bytes are announced before any of them can arrive
@@ -388,7 +418,7 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
             if ((page < 0 || page >= p.num_pages) && p.status) atomicOr(p.status, kStatusDecodeBadPage);
 #pragma unroll
             for (int db = 0; db < 2; ++db)
-              tma_load_4d(dst + db * kHalfTileBytes + lane * p.page_size * 128, tm, bar, db * 64, 0, it.head / group, page);
+              tma_load_4d(dst + db * kHalfTileBytes + lane * p.page_size * 128, tm, bar, db * 64, 0, kvh, page);
           }
         };
         auto wait_free = [&](uint64_t* bar, uint32_t parity) {
@@ -396,20 +426,20 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
           if (PAGED) got = __all_sync(0xffffffffu, got);
           return got;
         };
-        auto load_k = [&](const Item& it, int j, int page) {
+        auto load_k = [&](const Item& it, int kvh, int j, int page) {
           const int ks = kc % kKStages;
           if (!wait_free(k_empty + ks, ((kc / kKStages) & 1) ^ 1)) return false;
-          load_tile(smem + kKOffset + ks * kTileBytes, &tmap_k, k_full + ks, it, j, page);
+          load_tile(smem + kKOffset + ks * kTileBytes, &tmap_k, k_full + ks, it, kvh, j, page);
           ++kc;
           return true;
         };
         // Q and the first K tiles of an item.  Q's buffer is free once the previous item's last
         // score MMA has run, which is earlier than the release of its last V stage.
-        auto load_head = [&](const Item& it) {
+        auto load_head = [&](const Item& it, const Pages& of) {
           int pages[kKStages] = {};
           if (PAGED) {
 #pragma unroll
-            for (int jj = 0; jj < kKStages; ++jj) pages[jj] = page_of(it, jj);
+            for (int jj = 0; jj < kKStages; ++jj) pages[jj] = page_of(it, of, jj);
           }
           if (!wait_free(q_empty, (qc & 1) ^ 1)) return false;
           if (!PAGED || lane == 0) {
@@ -421,17 +451,16 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
           }
           ++qc;
           // Items of a few K tiles spend much of their time between items, and this loop is quicker there than three
-          // copies of its body, which longer items want: loop / copies, us, 8x16x3000 queries over 367 keys 105 / 109,
-          // 24x64x308 over 308 149 / 156; 2x32x2000 over 2000 132 / 130, 4x16x4096 over 4096 472 / 467.
-          if (!PAGED && it.n <= kKStages + 1) {
+          // copies of its body, which longer items want (SHORT: see short_items).
+          if (SHORT && !PAGED && it.n <= kKStages + 1) {
 #pragma unroll 1
             for (int jj = 0; jj < kKStages && jj < it.n; ++jj)
-              if (!load_k(it, jj, 0)) return false;
+              if (!load_k(it, of.kvh, jj, 0)) return false;
             return true;
           }
 #pragma unroll
           for (int jj = 0; jj < kKStages; ++jj)
-            if (jj < it.n && !load_k(it, jj, pages[jj])) return false;
+            if (jj < it.n && !load_k(it, of.kvh, jj, pages[jj])) return false;
           return true;
         };
         ItemWalk<SPLIT> walk;
@@ -445,131 +474,199 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
         };
         Item it = {};
         bool have = next_item(it);
-        if (have) ok = load_head(it);
+        Pages pages = pages_of(it);
+        if (have) ok = load_head(it, pages);
         while (have && ok) {
           Item nx = {};
           const bool have_next = next_item(nx);
+          const Pages nx_pages = pages_of(nx);
           // Order within an item: V_j, then K_(j+3); a K stage is released (by the score MMA that
           // read it) earlier than a V stage.  The head of the next item goes before the last V.
-          int vpage = page_of(it, 0), kpage = page_of(it, kKStages);
+          int vpage = page_of(it, pages, 0), kpage = page_of(it, pages, kKStages);
           for (int j = 0; j < it.n && ok; ++j) {
-            const int vpage_next = page_of(it, j + 1), kpage_next = page_of(it, j + 1 + kKStages);
+            const int vpage_next = page_of(it, pages, j + 1), kpage_next = page_of(it, pages, j + 1 + kKStages);
             if (j == it.n - 1 && have_next) {
-              ok = load_head(nx);
+              ok = load_head(nx, nx_pages);
               if (!ok) break;
             }
             const int vs = vc % kVStages;
             if (!wait_free(v_empty + vs, ((vc / kVStages) & 1) ^ 1)) { ok = false; break; }
-            load_tile(smem + kVOffset + vs * kTileBytes, &tmap_v, v_full + vs, it, j, vpage);
+            load_tile(smem + kVOffset + vs * kTileBytes, &tmap_v, v_full + vs, it, pages.kvh, j, vpage);
             ++vc;
-            if (j + kKStages < it.n) ok = load_k(it, j + kKStages, kpage);
+            if (j + kKStages < it.n) ok = load_k(it, pages.kvh, j + kKStages, kpage);
             vpage = vpage_next;
             kpage = kpage_next;
           }
           it = nx;
+          pages = nx_pages;
           have = have_next;
         }
       }
       __syncwarp();
     } else if (warp == kScoreWarp) {
-      // ---------------- score MMAs: S[g & 1] = Q K_g^T for every KV step g of this CTA ----------------
-      // Two threads issue MMAs, this one and the one below.  A tcgen05.mma does not return until
-      // the tensor pipe has room for it, so a group of eight blocks its thread for about as long
-      // as it executes (plus some 300 cycles when the pipe was idle): one thread for both kinds
-      // was busy nearly the whole step and every wait of one kind delayed the other.  The streams
-      // are independent: each orders itself through barriers (score buffer taken by the softmax,
-      // P written, stages loaded), never through issue order.
-      if (ELECT ? elect_one() : lane == 0) {
+      // ---------------- score MMAs: S[g % 3] = Q K_g^T for every step g of this CTA ----------------
+      // The streams of this thread and of the one below are independent: each orders itself through barriers (score
+      // buffer taken by the softmax, P written, stages loaded), never through issue order.
+      if (elect_one()) {
         // The issuing thread runs scalar, latency-bound code: descriptors are a constant high word
         // plus a low word that is a precomputed base plus a compile-time offset.
         const uint32_t hi_k = static_cast<uint32_t>(make_desc_kmajor_sw128(0) >> 32);
-        const uint32_t q_lo = static_cast<uint32_t>(make_desc_kmajor_sw128(smem_u32(smem + kQOffset)));
         const uint32_t k_lo = static_cast<uint32_t>(make_desc_kmajor_sw128(smem_u32(smem + kKOffset)));
         auto desc = [](uint32_t lo, uint32_t hi) { return (static_cast<uint64_t>(hi) << 32) | lo; };
-        uint32_t g = 0;                // score tiles issued so far
-        uint32_t kstage = 0, kpar = 0; // K ring position
+        const uint32_t s_full_a = smem_u32(s_full), s_free_a = smem_u32(s_free), k_full_a = smem_u32(k_full), k_empty_a = smem_u32(k_empty);
+        const uint32_t q_done_a = smem_u32(q_done);
+        const uint32_t q_tm = tmem_base + kTmemQ, s_tm = tmem_base + kTmemS;
+        uint32_t bo = 0, par = 1;    // 8 * group whose score buffer is next, parity of the wait for it (free the first time)
+        uint32_t ko = 0, kpar = 0;   // 8 * K ring position
         uint32_t qpar = 0;
         bool ok = true;
+        auto issue = [&](uint32_t b0) {
+          if (!mbar_wait_addr(s_free_a + bo, par, abort_word)) return false;  // the buffer's last scores are in registers
+          tc_fence_after();
+          const uint32_t d = s_tm + bo * (kStep / 8);
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) {  // 8 k-steps of 16 over the head dimension (two 64-wide blocks)
+            const uint32_t off = (ks >> 2) * (kHalfTileBytes >> 4) + 2 * (ks & 3);
+            umma_f16_ts(d, q_tm + ks * 8, desc(b0 + off, hi_k), kIdescS, ks > 0 ? 1u : 0u);
+          }
+          umma_commit_addr(s_full_a + bo);
+          bo += 8;
+          if (bo == 8 * kGroups) {
+            bo = 0;
+            par ^= 1;
+          }
+          return true;
+        };
         for (ItemWalk<SPLIT> walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
           const Item it = decode_item<PAGED, SPLIT>(walk.pos, p, table);
           if (it.n == 0) continue;
-          if (!mbar_wait(q_full, qpar, abort_word)) break;
+          if (!mbar_wait(q_ready, qpar, abort_word)) break;
           qpar ^= 1;
-          for (int j = 0; j < it.n; ++j, ++g) {
-            const uint32_t buf = g & 1;
-            if (!mbar_wait(k_full + kstage, kpar, abort_word)) { ok = false; break; }
-            // the buffer last held tile g - 2; the softmax threads have it in registers
-            // (passes at once for the first two tiles)
-            if (!mbar_wait(s_free + buf, ((g >> 1) & 1) ^ 1, abort_word)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t b0 = k_lo + kstage * (kTileBytes >> 4);
-            const uint32_t d = tmem_base + kTmemS + buf * 128;
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {  // 8 k-steps of 16 over the head dimension (two 64-wide blocks)
-              const uint32_t off = (ks >> 2) * (kHalfTileBytes >> 4) + 2 * (ks & 3);
-              umma_f16_ss(d, desc(q_lo + off, hi_k), desc(b0 + off, hi_k), kIdescS, ks > 0 ? 1u : 0u);
-            }
-            umma_commit(s_full + buf);
-            umma_commit(k_empty + kstage);
-            if (j == it.n - 1) umma_commit(q_empty);  // Q is free once the item's last score MMA has run
-            if (++kstage == kKStages) {
-              kstage = 0;
+          for (int left = it.steps; left > 0; left -= 2) {
+            if (!mbar_wait_addr(k_full_a + ko, kpar, abort_word)) { ok = false; break; }
+            const uint32_t b0 = k_lo + ko * (kTileBytes >> 7);
+            if (!issue(b0)) { ok = false; break; }
+            if (left > 1 && !issue(b0 + ((kStep * 128) >> 4))) { ok = false; break; }
+            umma_commit_addr(k_empty_a + ko);
+            ko += 8;
+            if (ko == 8 * kKStages) {
+              ko = 0;
               kpar ^= 1;
             }
           }
+          if (ok) umma_commit_addr(q_done_a);
         }
       }
       __syncwarp();
     } else if (warp == kPvWarp) {
-      // ---------------- second MMAs: O (+)= P[g & 1] V_g ----------------
-      if (ELECT ? elect_one() : lane == 0) {
+      // ---------------- second MMAs: O (+)= P[g % 3] V_g ----------------
+      if (elect_one()) {
         const uint32_t hi_mn = static_cast<uint32_t>(make_desc_mnmajor_sw128(0, kHalfTileBytes) >> 32);
         const uint32_t v_lo = static_cast<uint32_t>(make_desc_mnmajor_sw128(smem_u32(smem + kVOffset), kHalfTileBytes));
         auto desc = [](uint32_t lo, uint32_t hi) { return (static_cast<uint64_t>(hi) << 32) | lo; };
-        uint32_t g = 0, ic = 0;  // KV steps and items so far
-        uint32_t vstage = 0, vpar = 0;
+        const uint32_t p_full_a = smem_u32(p_full), o_done_a = smem_u32(o_done), v_full_a = smem_u32(v_full), v_empty_a = smem_u32(v_empty);
+        const uint32_t p_tm = tmem_base + kTmemP, o_tm = tmem_base + kTmemO;
+        uint32_t opar = 1;         // parity of the wait for the accumulator
+        uint32_t bo = 0, par = 0;  // 8 * group whose probabilities are next
+        uint32_t vo = 0, vpar = 0; // 8 * V ring position
         bool ok = true;
+        // 4 k-steps of 16 KV rows; A = P from tensor memory, B = V (MN-major)
+        auto issue = [&](uint32_t b0, uint32_t accumulate) {
+          const uint32_t a = p_tm + bo * (kStep / 16);
+          umma_f16_ts(o_tm, a, desc(b0, hi_mn), kIdescPV, accumulate);
+#pragma unroll
+          for (int ks = 1; ks < kStep / 16; ++ks) umma_f16_ts(o_tm, a + ks * 8, desc(b0 + ks * (2048 >> 4), hi_mn), kIdescPV, 1u);
+          umma_commit_addr(o_done_a + bo);
+          bo += 8;
+          if (bo == 8 * kGroups) {
+            bo = 0;
+            par ^= 1;
+          }
+        };
         for (ItemWalk<SPLIT> walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
           const Item it = decode_item<PAGED, SPLIT>(walk.pos, p, table);
           if (it.n == 0) continue;
-          for (int j = 0; j < it.n; ++j, ++g) {
-            const uint32_t buf = g & 1;
-            if (!mbar_wait(v_full + vstage, vpar, abort_word)) { ok = false; break; }
-            if (!mbar_wait(p_full + buf, (g >> 1) & 1, abort_word)) { ok = false; break; }
-            // the accumulator is read by the epilogue of the previous item
-            if (j == 0 && !mbar_wait(o_free, (ic & 1) ^ 1, abort_word)) { ok = false; break; }
+          // the accumulator is read by the epilogue of the previous item
+          if (!mbar_wait(o_free, opar, abort_word)) break;
+          opar ^= 1;
+          uint32_t accumulate = 0;
+          for (int left = it.steps; left > 0; left -= 2) {
+            if (!mbar_wait_addr(v_full_a + vo, vpar, abort_word)) { ok = false; break; }
+            const uint32_t b0 = v_lo + vo * (kTileBytes >> 7);
+            if (!mbar_wait_addr(p_full_a + bo, par, abort_word)) { ok = false; break; }
             tc_fence_after();
-            // 8 k-steps of 16 KV rows; A = P from tensor memory, B = V (MN-major)
-            const uint32_t b0 = v_lo + vstage * (kTileBytes >> 4);
-            const uint32_t d = tmem_base + kTmemO;
-            const uint32_t a = tmem_base + kTmemP + buf * 64;
-            umma_f16_ts(d, a, desc(b0, hi_mn), kIdescPV, j == 0 ? 0u : 1u);
-#pragma unroll
-            for (int ks = 1; ks < 8; ++ks) umma_f16_ts(d, a + ks * 8, desc(b0 + ks * (2048 >> 4), hi_mn), kIdescPV, 1u);
-            umma_commit(v_empty + vstage);
-            umma_commit(o_done + buf);
-            if (j == it.n - 1) umma_commit(o_full);
-            if (++vstage == kVStages) {
-              vstage = 0;
+            issue(b0, accumulate);
+            accumulate = 1;
+            if (left > 1) {
+              if (!mbar_wait_addr(p_full_a + bo, par, abort_word)) { ok = false; break; }
+              tc_fence_after();
+              issue(b0 + ((kStep * 128) >> 4), 1u);
+            }
+            umma_commit_addr(v_empty_a + vo);
+            vo += 8;
+            if (vo == 8 * kVStages) {
+              vo = 0;
               vpar ^= 1;
             }
           }
-          ++ic;
+          if (ok) umma_commit(o_full);
         }
       }
       __syncwarp();
     }
-  } else if (warp >= 8) {
+  } else if (warp >= kEpiWarp) {
     // ---------------- epilogue: O / rowsum -> global, one item behind ----------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
     const int quarter = warp & 3;
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t lane_field = static_cast<uint32_t>(quarter * 32) << 16;
     uint8_t* stage = smem + kOStageOffset;
-    const bool store_thread = (warp == 8 && lane == 0);
+    const bool store_thread = (warp == kEpiWarp && lane == 0);
     auto epi_barrier = [&]() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-    uint32_t ic = 0, g0 = 0;  // items so far, KV steps before the current item
+    uint32_t ic = 0, g0 = 0;  // items so far, group of the current item's first step
     bool ok = true;
+    // Q of an item moves from shared to tensor memory (16-bit pairs, a row per lane, without the swizzle), so that the score MMAs
+    // read only K through the shared-memory port.  Called one item ahead.
+    uint32_t qc = 0;
+    auto copy_q = [&]() {
+      bool got = mbar_wait(q_full, qc & 1, abort_word) && mbar_wait(q_done, (qc & 1) ^ 1, abort_word);
+      got = bar_red_and(1, 128, got);
+      if (!got) return false;
+      tc_fence_after();
+#pragma unroll
+      for (int db = 0; db < 2; ++db) {
+        const uint8_t* row = smem + kQOffset + db * kHalfTileBytes + row_in_tile * 128;
+        uint32_t r[32];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint4 v = *reinterpret_cast<const uint4*>(row + ((c ^ (row_in_tile & 7)) << 4));
+          r[4 * c] = v.x;
+          r[4 * c + 1] = v.y;
+          r[4 * c + 2] = v.z;
+          r[4 * c + 3] = v.w;
+        }
+        tmem_st_32x32b_x32(tmem_base + lane_field + kTmemQ + db * 32, r);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(q_ready);
+        mbar_arrive(q_empty);
+      }
+      ++qc;
+      return true;
+    };
+    ItemWalk<SPLIT> ahead;  // the item whose Q is copied next
+    auto copy_next_q = [&]() {
+      while (ahead.pos < p.order.num_items) {
+        const int n = decode_item<PAGED, SPLIT>(ahead.pos, p, table).n;
+        ahead.step(p.order);
+        if (n > 0) return copy_q();
+      }
+      return true;
+    };
+    ok = copy_next_q();
     for (ItemWalk<SPLIT> walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
       const Item it = decode_item<PAGED, SPLIT>(walk.pos, p, table);
       if (SPLIT && it.n == 0 && (it.shared || cluster_ctarank() != 0)) {  // another CTA writes the item's rows
@@ -590,22 +687,27 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
         continue;
       }
       const uint32_t par = ic & 1;
+      ok = copy_next_q();
+      if (!ok) break;
       ok = mbar_wait(o_full, par, abort_word) && mbar_wait(l_full, par, abort_word);
       // the four warps meet at named barriers below: they give up together or not at all
       ok = bar_red_and(1, 128, ok);
       if (!ok) break;
       tc_fence_after();
-      // The two warpgroups' partial row sums, each relative to the running max the warpgroup last
-      // used; the accumulator is relative to the larger one.  They are added in the order "the
-      // warpgroup that took the item's even steps first", so that the result does not depend on
+      // The warpgroups' partial row sums, each relative to the running max the warpgroup last used; the accumulator is
+      // relative to the largest one.  They are added in the order of the item's steps, so that the result does not depend on
       // what the CTA processed before this item.
-      const int we = g0 & 1, wo = we ^ 1;
-      const float m0 = lsum[(we * 2 + 0) * kTileRows + row_in_tile], l0 = lsum[(we * 2 + 1) * kTileRows + row_in_tile];
-      const float m1 = lsum[(wo * 2 + 0) * kTileRows + row_in_tile], l1 = lsum[(wo * 2 + 1) * kTileRows + row_in_tile];
-      const float mm = fmaxf(m0, m1);
-      const float a0 = (m0 == -INFINITY) ? 0.f : ex2(m0 - mm);
-      const float a1 = (m1 == -INFINITY) ? 0.f : ex2(m1 - mm);
-      const float l = l0 * a0 + l1 * a1;
+      float m_of[kGroups], l_of[kGroups];
+      float mm = -INFINITY, l = 0.f;
+#pragma unroll
+      for (int i = 0; i < kGroups; ++i) {
+        const int w = static_cast<int>((g0 + i) % kGroups);
+        m_of[i] = lsum[(w * 2 + 0) * kTileRows + row_in_tile];
+        l_of[i] = lsum[(w * 2 + 1) * kTileRows + row_in_tile];
+        mm = fmaxf(mm, m_of[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < kGroups; ++i) l += l_of[i] * ((m_of[i] == -INFINITY) ? 0.f : ex2(m_of[i] - mm));
       if (SPLIT && it.shared) {
         const uint32_t t_part = tmem_base + lane_field + kTmemO;
 #pragma unroll
@@ -618,7 +720,7 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
             *reinterpret_cast<uint4*>(smem + partial_offset(row_in_tile, cc * 8 + v)) =
                 make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
         }
-        // (this row's entries; both warpgroups' have been read above)
+        // (this row's entries; all warpgroups' have been read above)
         lsum[row_in_tile] = mm;
         lsum[kTileRows + row_in_tile] = l;
         continue;
@@ -671,24 +773,27 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
         }
       }
       ++ic;
-      g0 += it.n;
+      g0 = (g0 + it.steps) % kGroups;
     }
     if (store_thread) tma_store_wait_read<0>();
   } else {
-    // ---------------- softmax / correction: warpgroup w takes the KV steps g with (g & 1) == w ----------------
+    // ---------------- softmax / correction: warpgroup w takes the steps g with g % 3 == w ----------------
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
     const int w = warp >> 2;  // also the score buffer and the P buffer this warpgroup works on
+    const int before = w == 0 ? kGroups - 1 : w - 1;  // the warpgroup of the previous step
     const int quarter = warp & 3;
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t lane_field = static_cast<uint32_t>(quarter * 32) << 16;
-    const uint32_t t_s = tmem_base + lane_field + kTmemS + w * 128;
-    const uint32_t t_p = tmem_base + lane_field + kTmemP + w * 64;
+    const uint32_t t_s = tmem_base + lane_field + kTmemS + w * kStep;
+    const uint32_t t_p = tmem_base + lane_field + kTmemP + w * (kStep / 2);
     const uint32_t t_o = tmem_base + lane_field + kTmemO;
     float* m_mine = xmax + w * kTileRows + row_in_tile;
-    const float* m_theirs = xmax + (w ^ 1) * kTileRows + row_in_tile;
+    const float* m_theirs = xmax + before * kTileRows + row_in_tile;
     const float scale_log2 = p.scale_log2;
     const float2 scale2 = make_float2(scale_log2, scale_log2);
-    uint32_t g = 0, ic = 0;  // KV steps (of both warpgroups) and items so far
+    uint32_t turn = 0;   // group of the current item's first step
+    uint32_t k = 0;      // steps of this warpgroup so far
+    uint32_t ic = 0;     // items so far
     bool ok = true;
     for (ItemWalk<SPLIT> walk; walk.pos < p.order.num_items && ok; walk.step(p.order)) {
       const Item it = decode_item<PAGED, SPLIT>(walk.pos, p, table);
@@ -699,51 +804,49 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
       const int causal_offset = PAGED ? it.causal_offset : p.causal_offset;
       float m_ref = -INFINITY;  // running max this warpgroup's row sum is relative to
       float2 l2 = make_float2(0.f, 0.f);
-      for (int j = 0; j < it.n; ++j, ++g) {
-        if ((g & 1u) != static_cast<uint32_t>(w)) continue;
-        const uint32_t ph = (g >> 1) & 1;  // phase of this warpgroup's own barriers in this step
+      for (int j = (w + kGroups - static_cast<int>(turn)) % kGroups; j < it.steps; j += kGroups, ++k) {
+        const uint32_t ph = k & 1;  // phase of this warpgroup's own barriers in this step
+        const uint32_t ph_before = (w == 0 ? k - 1 : k) & 1;  // ... of the previous step's
+        // (a wait that gives up leaves the step to run its course on whatever is there; the warp decides together at its end)
         ok = mbar_wait(s_full + w, ph, abort_word);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        __syncwarp();
         tc_fence_after();
-        uint32_t sr[128];
+        uint32_t sr[kStep];
         tmem_ld_32x32b_x64(t_s, sr);
-        tmem_ld_32x32b_x64(t_s + 64, sr + 64);
 
-        const int col0 = (it.first + j) * kTileRows;
+        const int col0 = it.first * kTileRows + j * kStep;
         const bool need_mask =
-            (p.causal && col0 + kTileRows - 1 > tile_r0 + causal_offset) || (col0 + kTileRows > kv_len);
-        int limit = kTileRows;  // columns [0, limit) of this tile are visible to this row
+            (p.causal && col0 + kStep - 1 > tile_r0 + causal_offset) || (col0 + kStep > kv_len);
+        int limit = kStep;  // columns [0, limit) of this step are visible to this row
         if (need_mask) {
           int vis = kv_len;
           if (p.causal) vis = min(vis, q_row + causal_offset + 1);
           limit = vis - col0;
         }
         tmem_wait_ld();
-        // the row is in registers: the tensor core may write the tile two steps ahead over it
+        // the row is in registers: the tensor core may write the next scores over it
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(s_free + w);
         if (need_mask) {
 #pragma unroll
-          for (int i = 0; i < 128; ++i)
+          for (int i = 0; i < kStep; ++i)
             if (i >= limit) sr[i] = 0xff800000u;  // -inf
         }
-        float mx0 = -INFINITY, mx1 = -INFINITY;
+        float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < 128; i += 4) {
+        for (int i = 0; i < kStep; i += 8) {
           mx0 = fmax3(mx0, __uint_as_float(sr[i]), __uint_as_float(sr[i + 1]));
           mx1 = fmax3(mx1, __uint_as_float(sr[i + 2]), __uint_as_float(sr[i + 3]));
+          mx2 = fmax3(mx2, __uint_as_float(sr[i + 4]), __uint_as_float(sr[i + 5]));
+          mx3 = fmax3(mx3, __uint_as_float(sr[i + 6]), __uint_as_float(sr[i + 7]));
         }
-        const float m_new = fmaxf(mx0, mx1) * scale_log2;
-        // The running max after the previous step, published by the other warpgroup early in that
-        // step (half a step ago).  Every phase of x_full is observed, also when the value is not
-        // needed (first step of an item).
+        const float m_new = fmaxf(fmax3(mx0, mx1, mx2), mx3) * scale_log2;
+        // The running max after the previous step, published by its warpgroup early in that step.  Every phase of x_full is
+        // observed, also when the value is not needed (first step of an item).
         float m_prev = -INFINITY;
-        if (g > 0) {
-          ok = mbar_wait(x_full + (w ^ 1), ((g - 1) >> 1) & 1, abort_word);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
+        if (w != 0 || k != 0) {
+          ok &= mbar_wait(x_full + before, ph_before, abort_word);
           if (j > 0) m_prev = *m_theirs;
         }
         const bool grow = m_new > m_prev + kRescaleThreshold;  // also true for the first finite max
@@ -752,19 +855,21 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
         __syncwarp();
         if (lane == 0) mbar_arrive(x_full + w);
         // this warpgroup's partial row sum follows the running max
-        if (m_prev != m_ref) {  // m_prev > m_ref: the other warpgroup raised it
+        if (m_prev != m_ref) {  // m_prev > m_ref: another warpgroup raised it
           const float a = ex2(m_ref - m_prev);  // m_ref = -inf gives 0 (and the sum is 0 then)
           l2.x *= a;
           l2.y *= a;
         }
         if (j > 0 && __any_sync(0xffffffffu, grow)) {
-          // Rescale O between "O += P V" of the previous step (the other warpgroup's P) and this
-          // step's.  Rare after the first steps of an item: the max must grow by 2^8.
+          // Rescale O between "O += P V" of the previous step and this step's.  Rare after the first steps of an item: the max
+          // must grow by 2^8.
           float alpha = 1.f;
           if (grow) alpha = ex2(m_prev - m_new);  // m_prev = -inf gives 0
-          ok = mbar_wait(o_done + (w ^ 1), ((g - 1) >> 1) & 1, abort_word);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
+          // (this warpgroup's own previous one first: then the barrier waited for is in the phase before the one that is
+          // meant, never two behind)
+          if (k > 0) ok &= mbar_wait(o_done + w, ph ^ 1, abort_word);
+          ok &= mbar_wait(o_done + before, ph_before, abort_word);
+          __syncwarp();
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < 8; ++c) {
@@ -781,16 +886,9 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
         m_ref = m_cur;
         const float m_sub = (m_cur == -INFINITY) ? 0.f : m_cur;
         const float2 negm2 = make_float2(-m_sub, -m_sub);
-        // this warpgroup's P buffer was last read by "O += P V" two steps ago
-        if (g >= 2) {
-          ok = mbar_wait(o_done + w, ph ^ 1, abort_word);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-        }
-
         // probabilities -> tensor memory (16-bit pairs); masked scores are -inf and give (almost) exactly 0
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < kStep / 32; ++c) {
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -800,14 +898,21 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
             l2 = fadd2(l2, e);
             pk[i] = pack_pair<T>(e.x, e.y);
           }
+          // the P buffer was last read by the "O += P V" of this warpgroup's previous step
+          if (c == 0 && k > 0) {
+            ok &= mbar_wait(o_done + w, ph ^ 1, abort_word);
+            __syncwarp();
+          }
           tmem_st_32x32b_x16(t_p + c * 16, pk);
         }
         tmem_wait_st();
         tc_fence_before();
-        __syncwarp();
+        ok = __all_sync(0xffffffffu, ok);
         if (lane == 0) mbar_arrive(p_full + w);
+        if (!ok) break;
       }
       if (!ok) break;
+      turn = (turn + it.steps) % kGroups;
       // hand (max, sum) of this warpgroup's steps to the epilogue warps
       ok = mbar_wait(l_free, (ic & 1) ^ 1, abort_word);
       ok = __all_sync(0xffffffffu, ok);
@@ -822,7 +927,7 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
     if constexpr (SPLIT) {
       if (shared_item) {
         cluster_sync_all();  // all partial results are in place
-        merge_partials<T>(decode_item<PAGED, SPLIT>(ItemWalk<SPLIT>().pos, p, table), smem_u32(smem), p);
+        if (warp < 8) merge_partials<T>(decode_item<PAGED, SPLIT>(ItemWalk<SPLIT>().pos, p, table), smem_u32(smem), p);
       }
     }
   }
@@ -830,7 +935,7 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
   if constexpr (SPLIT) {
     // Every thread of every CTA reaches both barriers, also after a wait that gave up.
     if (shared_item) {
-      if (warp >= 8) cluster_sync_all();
+      if (warp >= kEpiWarp) cluster_sync_all();
       cluster_sync_all();  // no CTA leaves while a peer still reads its shared memory
     }
   }
@@ -851,12 +956,12 @@ __device__ __forceinline__ void attn_fwd_cta(const CUtensorMap& tmap_q, const CU
   }
 }
 
-template <typename T, bool PAGED, bool ELECT>
+template <typename T, bool PAGED, bool SHORT>
 __global__ void __launch_bounds__(kAttnThreads, 1)
     attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
                     const AttnParams p) {
-  attn_fwd_cta<T, PAGED, ELECT, false>(tmap_q, tmap_k, tmap_v, tmap_o, p);
+  attn_fwd_cta<T, PAGED, SHORT, false>(tmap_q, tmap_k, tmap_v, tmap_o, p);
 }
 
 template <typename T, bool PAGED>
@@ -867,10 +972,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   attn_fwd_cta<T, PAGED, true, true>(tmap_q, tmap_k, tmap_v, tmap_o, p);
 }
 
-template <typename T, bool PAGED, bool ELECT>
+template <typename T, bool PAGED, bool SHORT>
 int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
                  const AttnParams& p, cudaStream_t stream) {
-  auto kfn = attn_fwd_kernel<T, PAGED, ELECT>;
+  auto kfn = attn_fwd_kernel<T, PAGED, SHORT>;
   static bool configured[64] = {};  // per instantiation and device ordinal
   int rc = ensure_dynamic_smem(kfn, kAttnSmem, configured, "cudaFuncSetAttribute(attention smem)");
   if (rc) return rc;
@@ -896,14 +1001,9 @@ int launch_split(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
                         stream, tq, tk, tv, to, p);
 }
 
-// How the two MMA threads are picked: behind elect.sync (see elect_one) items start faster, behind lane == 0 the steps of a
-// long item follow each other faster (their MMAs have N = 128 and gain nothing by the faster issue).  The line is at a mean of
-// 1024 keys per query, and of 512 where a CTA has hardly more than one item.  lane == 0 / elect.sync, us: 24x64x308
-// 165.0 / 151.8, 2x16 1024 over 256 11.2 / 10.7, 16x16(4)x1024 causal 100.3 / 94.4, 2x20x1300 causal 30.7 / 29.4, 2x32(8)x2000
-// causal 82.8 / 81.8, 8x32x1024 153.8 / 151.9; 1x12 1536 over 1024 (one round) 13.8 / 14.0, 1x24x2048 causal 35.4 / 36.6,
-// 2x16x4096 271 / 286, 1x8x8192 275 / 294, 1x8 2048 over 3072 30.0 / 32.0, 1x4x8192 causal 73.4 / 78.1.  The score thread
-// alone behind lane == 0 is between the two (272, 275, 32.2, 74.7; 24x64x308 158.5).  Paged items wait for their pages and
-// take the same time either way (4x4(1) 1000 over 4000 44.1 / 43.9).
+// Calls of short items carry a loop for the first loads of an item beside the unrolled form that long ones want: loop / copies, us,
+// 8x16x3000 queries over 367 keys 105 / 109, 24x64x308 149 / 156; 2x32x2000 132 / 130, 4x16x4096 472 / 467.  The line is at a mean of
+// 1024 keys per query, and of 512 where a CTA has hardly more than one item.
 bool short_items(const AttnParams& p) {
   const int64_t keys = 2 * static_cast<int64_t>(p.seq_kv) - (p.causal ? p.seq_q : 0);  // twice the mean per query
   return 2 * static_cast<int64_t>(p.order.num_items) > 3 * num_sms() ? keys <= 2 * 1024 : keys < 2 * 512;

@@ -33,8 +33,8 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // both in shared memory N = 32 45.6 / 40.7, N = 64 48.8 / 48.7 and N = 128 64.7 / 64.7 (the shared-memory port: 6 and 8 KB
 // at 128 B per cycle).  Kernels, us: attention 4x32x4096 causal 539 / 513, 16x64x512 causal 142 / 123, 24x64x308 165 / 152;
 // its backward 2x32(8)x2000 252 / 238; products 1024^3 6.4 / 5.6, 256x256x16384 12.3 / 11.2; none where memory or the
-// shared-memory port decides (2048^3, 4096^3, 16x4096x4096).  Two places keep `lane == 0`, which was faster there: the MMA
-// threads for long items of the one-tile attention kernel and the TMA thread of the split-K GEMM.
+// shared-memory port decides (2048^3, 4096^3, 16x4096x4096).  One place keeps `lane == 0`, which was
+// faster there: the TMA thread of the split-K GEMM.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
