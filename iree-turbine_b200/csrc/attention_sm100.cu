@@ -182,6 +182,9 @@ struct Item {
   int n[2];   // half steps of 64 keys that query tile t visits (0: the tile has no rows or sees no key)
   int nmax;   // KV tiles loaded for the item
   int kv_len, causal_offset;  // keys of this item's sequence; key j is visible to query i iff j <= i + causal_offset
+  // PACKED: query tile 1 is the only tile of another head, which exists unless `second` is false
+  int head1, batch1;
+  bool second;
 };
 
 template <bool PAGED>
@@ -213,10 +216,25 @@ __device__ __forceinline__ Item make_item(int batch, int head, int pair, const A
   return it;
 }
 
+// Query tile t of an item: its first row, and the head it belongs to.
+template <bool PACKED>
+__device__ __forceinline__ int first_row(const Item& it, int t) {
+  return PACKED ? 0 : it.pair * kPairRows + t * kTileRows;
+}
+template <bool PACKED>
+__device__ __forceinline__ int head_of(const Item& it, int t) {
+  return PACKED && t ? it.head1 : it.head;
+}
+template <bool PACKED>
+__device__ __forceinline__ int batch_of(const Item& it, int t) {
+  return PACKED && t ? it.batch1 : it.batch;
+}
+
 // The CTA's items, in the order every role walks them.  With p.couples a position stands for two items,
 // the k-th heaviest pair of a head and then the k-th lightest, so that all positions cost the same and the
 // list can be head-major, which keeps the K/V traffic on a few heads.
-template <bool PAGED>
+// PACKED (see packs_heads): a position stands for the only query tiles of two heads.
+template <bool PAGED, bool PACKED>
 struct ItemWalk {
   const AttnParams& p;
   const uint16_t* table;
@@ -232,6 +250,17 @@ struct ItemWalk {
       return true;
     }
     if (walk.pos >= p.order.num_items) return false;
+    if (PACKED) {
+      const int bh = 2 * walk.pos, heads = p.batch * p.q_heads;
+      const int batch = p.order.by_q_heads.quotient(bh);
+      it = make_item<PAGED>(batch, bh - batch * p.q_heads, 0, p);
+      it.second = bh + 1 < heads;
+      it.batch1 = p.order.by_q_heads.quotient(bh + 1);
+      it.head1 = bh + 1 - it.batch1 * p.q_heads;
+      it.n[1] = it.second ? it.n[0] : 0;
+      walk.step(p.order);
+      return true;
+    }
     int batch, head, pair;
     attn_order::item_at<PAGED>(p.order, walk.pos, table, p.q_heads, batch, head, pair);
     if (!PAGED && p.couples > 0) {  // tile t of the order is the couple (couples - 1 - t, its mirror image)
@@ -252,7 +281,7 @@ struct ItemWalk {
   }
 };
 
-template <typename T, int HD, int GROUPS, bool PAGED>
+template <typename T, int HD, int GROUPS, bool PAGED, bool PACKED>
 __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
     attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
@@ -387,7 +416,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
           }
           return true;
         };
-        ItemWalk<PAGED> walk(p, table);
+        ItemWalk<PAGED, PACKED> walk(p, table);
         Item it;
         while (ok && walk.next_busy(it)) {
           kvh = it.head / group;
@@ -401,6 +430,11 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
             ok = load_tile(&tmap_k, it, j, page) && load_tile(&tmap_v, it, j, page);
             page = page_next;
           }
+          if (PACKED && ok && it.second) {
+            kvh = it.head1 / group;
+            it.batch = it.batch1;
+            ok = load_tile(&tmap_k, it, 0, 0) && load_tile(&tmap_v, it, 0, 0);
+          }
         }
       }
       __syncwarp();
@@ -409,7 +443,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
       if (elect_one()) {
         uint32_t ci[2] = {0, 0};  // items of each tile so far
         bool ok = true;
-        ItemWalk<PAGED> walk(p, table);
+        ItemWalk<PAGED, PACKED> walk(p, table);
         Item it, nx;
         bool have = walk.next_busy(it);
         while (ok && have) {
@@ -423,7 +457,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
 #pragma unroll
             for (int db = 0; db < kBlocks; ++db)
               tma_load_4d(smem + L::kQOffset + t * kTileBytes + db * kHalfTileBytes, &tmap_q, q_full + t, db * 64,
-                          it.pair * kPairRows + t * kTileRows, it.head, it.batch);
+                          first_row<PACKED>(it, t), head_of<PACKED>(it, t), batch_of<PACKED>(it, t));
           }
           // A Q buffer frees up only a step or so before the next item needs it, less than a trip
           // to HBM: ask for the next item's Q tiles in L2 now, an item ahead.
@@ -433,7 +467,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
               if (nx.n[t] == 0) continue;
 #pragma unroll
               for (int db = 0; db < kBlocks; ++db)
-                tma_prefetch_4d(&tmap_q, db * 64, nx.pair * kPairRows + t * kTileRows, nx.head, nx.batch);
+                tma_prefetch_4d(&tmap_q, db * 64, first_row<PACKED>(nx, t), head_of<PACKED>(nx, t), batch_of<PACKED>(nx, t));
             }
           }
           it = nx;
@@ -514,11 +548,24 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
         };
         auto pass_turn = [&]() { mbar_arrive(turn + (t ^ 1u)); };
         bool ok = true;
-        ItemWalk<PAGED> walk(p, table);
+        ItemWalk<PAGED, PACKED> walk(p, table);
         Item it;
         while (ok && walk.next_busy(it)) {
           const int n = t ? it.n[1] : it.n[0];
           const int nmax = it.nmax;
+          // PACKED: tile 0's K and V are the item's first two entries, tile 1's the next two; each thread lets the other's go.
+          const bool both = PACKED && it.second;
+          auto skip_entries = [&](uint32_t e) {
+            for (uint32_t i = e; i < e + 2; ++i) {
+              if (!wait_entry(i)) return false;
+              mbar_arrive(kv_empty + i % kKvStages);
+            }
+            return true;
+          };
+          if (both && t == 1) {
+            if (!skip_entries(e0)) break;
+            e0 += 2;
+          }
           // The first score tile of an item needs no turn: a tile that is done with the previous
           // item starts the next one at once, whatever the other tile is still doing.  Both score
           // buffers are free: the PV groups that read the probabilities in them were issued before.
@@ -574,6 +621,10 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
             }
           }
           e0 += 2 * nmax;
+          if (both && t == 0) {
+            if (!skip_entries(e0)) break;
+            e0 += 2;
+          }
         }
       }
       __syncwarp();
@@ -590,22 +641,22 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
     uint32_t ci[2] = {0, 0};     // items with work per tile so far
     uint32_t steps[2] = {0, 0};  // half steps per tile before the current item
     bool ok = true;
-    ItemWalk<PAGED> walk(p, table);
+    ItemWalk<PAGED, PACKED> walk(p, table);
     Item it;
     while (ok && walk.next(it)) {
 #pragma unroll 1
       for (int t = 0; t < 2; ++t) {
-        const int tile_r0 = it.pair * kPairRows + t * kTileRows;
-        if (tile_r0 >= p.seq_q) continue;
+        const int tile_r0 = first_row<PACKED>(it, t), head = head_of<PACKED>(it, t), batch = batch_of<PACKED>(it, t);
+        if (tile_r0 >= p.seq_q || (PACKED && t == 1 && !it.second)) continue;
         const int q_row = tile_r0 + row_in_tile;
         if (it.n[t] == 0) {
           // no visible key: zeros (rare; plain stores)
           if (q_row < p.seq_q) {
-            T* orow = reinterpret_cast<T*>(p.o) + it.batch * p.o_stride_b + it.head * p.o_stride_h +
+            T* orow = reinterpret_cast<T*>(p.o) + batch * p.o_stride_b + head * p.o_stride_h +
                       static_cast<int64_t>(q_row) * p.o_stride_s;
 #pragma unroll
             for (int v = 0; v < HD / 8; ++v) reinterpret_cast<uint4*>(orow)[v] = make_uint4(0u, 0u, 0u, 0u);
-            if (p.lse) p.lse[(static_cast<int64_t>(it.batch) * p.q_heads + it.head) * p.seq_q + q_row] = -INFINITY;
+            if (p.lse) p.lse[(static_cast<int64_t>(batch) * p.q_heads + head) * p.seq_q + q_row] = -INFINITY;
           }
           continue;
         }
@@ -632,7 +683,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
         const float inv = (l > 0.f) ? 1.0f / l : 0.f;
         if (p.lse && q_row < p.seq_q) {
           // m is in the log2 domain (scores times scale * log2 e), l is relative to it
-          p.lse[(static_cast<int64_t>(it.batch) * p.q_heads + it.head) * p.seq_q + q_row] =
+          p.lse[(static_cast<int64_t>(batch) * p.q_heads + head) * p.seq_q + q_row] =
               (l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
         }
         const uint32_t t_o = tmem_base + lane_field + L::kTmemO + t * HD;
@@ -670,7 +721,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
           fence_proxy_async_smem();
           epi_barrier();
           if (store_thread) {
-            tma_store_4d(&tmap_o, stage, c2 * 64, tile_r0, it.head, it.batch);
+            tma_store_4d(&tmap_o, stage, c2 * 64, tile_r0, head, batch);
             tma_store_commit();
           }
         }
@@ -695,12 +746,12 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
     const float2 scale2 = make_float2(scale_log2, scale_log2);
     uint32_t cs = 0, ci = 0;  // half steps (of both warpgroups) and items of this query tile so far
     bool ok = true;
-    ItemWalk<PAGED> walk(p, table);
+    ItemWalk<PAGED, PACKED> walk(p, table);
     Item it;
     while (ok && walk.next_busy(it)) {
       const int n = it.n[t];
       if (n == 0) continue;
-      const int tile_r0 = it.pair * kPairRows + t * kTileRows;
+      const int tile_r0 = first_row<PACKED>(it, t);
       const int q_row = tile_r0 + row_in_tile;
       const int kv_len = it.kv_len;
       const int causal_offset = it.causal_offset;
@@ -865,10 +916,10 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
   }
 }
 
-template <typename T, int HD, int GROUPS, bool PAGED>
+template <typename T, int HD, int GROUPS, bool PAGED, bool PACKED = false>
 int launch_typed(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
                  const AttnParams& p, cudaStream_t stream) {
-  auto kfn = attn_fwd_kernel<T, HD, GROUPS, PAGED>;
+  auto kfn = attn_fwd_kernel<T, HD, GROUPS, PAGED, PACKED>;
   static bool configured[64] = {};  // per instantiation and device ordinal
   int rc = ensure_dynamic_smem(kfn, AttnSmem<HD>::kTotal, configured, "cudaFuncSetAttribute(attention smem)");
   if (rc) return rc;
@@ -900,6 +951,14 @@ bool two_groups(const AttnParams& p) {
   return 2 * static_cast<int64_t>(p.seq_kv) - (p.causal ? p.seq_q : 0) >= 2 * 1536;
 }
 
+// Head dim 64, queries and keys of at most one tile, more heads than SMs: an item is the only tiles of two heads, which need not
+// share K and V (with one head per item the second tile was empty, and the heads beyond the first 148 waited for a second round).
+// One head / two heads per item, us: 32x8x128 causal 9.85 / 7.75, 19x8x128 causal 9.3 / 7.6, 37x16x128 causal 17.3 / 12.9, 64x32x128 45.2 /
+// 28.3, 100x8(2)x100 causal 24.1 / 15.3, 20x8 17 over 128 8.0 / 6.9.  With no more heads than SMs each has an SM to itself.
+bool packs_heads(const AttnParams& p) {
+  return p.seq_q <= kTileRows && p.seq_kv <= kTileRows && static_cast<int64_t>(p.batch) * p.q_heads > num_sms();
+}
+
 template <bool PAGED>
 int launch_any(int dtype, int head_dim, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                const CUtensorMap& to, const AttnParams& p, cudaStream_t stream) {
@@ -910,6 +969,15 @@ int launch_any(int dtype, int head_dim, const CUtensorMap& tq, const CUtensorMap
   if (two_groups<PAGED>(p)) {
     if (dtype == B200K_F16) return launch_typed<__half, 64, 2, PAGED>(tq, tk, tv, to, p, stream);
     return launch_typed<__nv_bfloat16, 64, 2, PAGED>(tq, tk, tv, to, p, stream);
+  }
+  if constexpr (!PAGED) {
+    if (packs_heads(p)) {
+      AttnParams packed = p;
+      packed.couples = 0;
+      packed.order.num_items = (p.batch * p.q_heads + 1) / 2;
+      if (dtype == B200K_F16) return launch_typed<__half, 64, 1, false, true>(tq, tk, tv, to, packed, stream);
+      return launch_typed<__nv_bfloat16, 64, 1, false, true>(tq, tk, tv, to, packed, stream);
+    }
   }
   if (dtype == B200K_F16) return launch_typed<__half, 64, 1, PAGED>(tq, tk, tv, to, p, stream);
   return launch_typed<__nv_bfloat16, 64, 1, PAGED>(tq, tk, tv, to, p, stream);
