@@ -255,7 +255,7 @@ __device__ __forceinline__ bool mbar_wait_addr(uint32_t bar_addr, uint32_t parit
 }
 
 // ---------------------------------------------------------------------------------------
-// TMA (tiled bulk tensor copies; no cluster-wide forms are used anywhere in this library)
+// TMA (tiled bulk tensor copies; no load is multicast anywhere in this library)
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");

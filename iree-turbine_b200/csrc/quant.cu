@@ -228,8 +228,10 @@ int launch_quantize_e4m3(const float* x, void* y, float* scale_out, uint32_t* am
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, quantize_resident_kernel<false>, x, static_cast<uint8_t*>(y), n, amax_scratch, scale_out),
-                      "quantize_resident_kernel launch");
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, quantize_resident_kernel<false>, x, static_cast<uint8_t*>(y), n, amax_scratch, scale_out);
+    // a process that may use a part of the SMs only takes the two launches below
+    if (e != cudaErrorCooperativeLaunchTooLarge) return check_cuda(e, "quantize_resident_kernel launch");
+    (void)cudaGetLastError();
   }
   const int64_t want = (n / 4 + kQuantThreads * kQuantUnroll - 1) / (kQuantThreads * kQuantUnroll);
   int64_t cap = static_cast<int64_t>(num_sms()) * kBlocksPerSm;
