@@ -192,11 +192,12 @@ int b200k_gemm_nt_allgather(const b200k_gemm_allgather_args* args, void* stream)
  * (query i sees keys j <= i + seq_kv - seq_q).
  *
  * Two kernels implement the call.  B200K_ATTN_ONE_TILE: a work item is one 128-row query tile,
- * two softmax warpgroups take alternate KV steps (head_dim 128 only).  B200K_ATTN_TILE_PAIR: a
+ * three softmax warpgroups take KV steps of 64 keys in turn (head_dim 128 only).  B200K_ATTN_TILE_PAIR: a
  * work item is a pair of query tiles that share every K/V tile, one softmax warpgroup each; causal
  * problems are dealt out in (heavy, light) couples of equal cost.  B200K_ATTN_AUTO picks the pair
  * kernel for head_dim 64 and for causal problems of more than 128 queries whose couples fill the SMs
- * evenly, else the one-tile kernel (without a mask that does not depend on the batch).  Results of the two agree within rounding
+ * evenly, else the one-tile kernel (without a mask that does not depend on the batch), for causal problems of few query tiles
+ * with the KV tiles of each divided over a cluster of CTAs.  Results of the kernels agree within rounding
  * of the 16-bit probabilities, not bitwise.
  */
 enum { B200K_ATTN_AUTO = 0, B200K_ATTN_ONE_TILE = 1, B200K_ATTN_TILE_PAIR = 2 };

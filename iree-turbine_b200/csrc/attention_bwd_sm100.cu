@@ -582,7 +582,9 @@ __device__ __forceinline__ void bwd_dq_cta(int block, int blocks, const CUtensor
 // Period in CTAs that have an SM to themselves and the clock to spare, 1x8(1)x4096 causal: 2960 cycles of 2048 for the
 // products, now 2520 (2304 with these MMAs); us, whole tiles / halves: 1x8(1)x4096 409 / 351, 1x8(2)x1000 58.8 / 51.9, 1x2x2048
 // 33.2 / 29.6; with all SMs at work and the clock under the power cap 2x32(8)x2000 267 / 257, 4x32x4096 1960 / 1858,
-// 1x16x4096 without a mask 442 / 413; 13x64(8)x81 63.9 / 62.0.  (The dQ CTAs by the same halves: no difference, 2x32(8)x2000 260 / 260.)
+// 1x16x4096 without a mask 442 / 413; 13x64(8)x81 63.9 / 62.0.  (The dQ CTAs by the same halves: no difference, 2x32(8)x2000 260 / 260.
+// Sixteen warps of algebra instead of eight, 32 columns per thread: the dQ CTAs are faster, 1x16 300 queries over 4096 keys 94.7 / 87.9,
+// these are slower, 1x8(1)x4096 350 / 374, 2x32(8)x2000 257 / 265: taken back.)
 // Shared memory: K, V, three Q buffers, two dO buffers (7 x 32 KB), each handed
 // back by the last product that reads it, so that a tile is requested a whole iteration before its first product.
 // Tensor memory: S^T / P^T | dP^T / dS^T | dV | dK (128 columns each).
