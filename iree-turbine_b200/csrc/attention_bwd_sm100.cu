@@ -944,48 +944,75 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 }
 
 // delta[b, h, i] = sum_d dO[b, h, i, d] * O[b, h, i, d].  A row of HD 16-bit values is HD / 8 lanes
-// of 16 bytes; a warp takes 32 / (HD / 8) rows at a time and eight such groups, all loads issued
-// before the first use, so that enough bytes are in flight to run at memory speed.
+// of 16 bytes; a warp takes two groups of 32 / (HD / 8) rows, all loads issued before the first use.  HBM bound in large calls, latency in
+// small ones.  Eight groups per warp with two divisions for each row, 117 registers and so two blocks per SM / this, us: 2x32x2000 21.0 /
+// 15.3, 4x32x4096 66.6 / 51.1, 7x16x1135 hd64 12.3 / 9.3, 1x8x512 4.5 / 2.9; with four groups 15.5, 51.1, 9.5, 3.1.  The first row is found
+// before the wait for the kernel before this one, which takes 1 us off every backward (1x1x128 10.5 / 8.3, 3x32(8)x97 17.1 / 14.6).
+constexpr int kDeltaThreads = 256, kDeltaGroups = 2;
 template <typename T, int HD>
-__global__ void attn_bwd_delta_kernel(const T* o, const T* d_o, float* delta,
+__global__ void __launch_bounds__(kDeltaThreads, 8) attn_bwd_delta_kernel(const T* o, const T* d_o, float* delta,
                                       int64_t rows, int q_heads, int seq_q, int64_t o_sb, int64_t o_sh, int64_t o_ss,
                                       int64_t do_sb, int64_t do_sh, int64_t do_ss) {
   constexpr int kLanesPerRow = HD / 8;
-  constexpr int kRowsPerPass = 32 / kLanesPerRow;
-  constexpr int kPasses = 8;
+  constexpr int kRowsPerGroup = 32 / kLanesPerRow;
+  constexpr int kGroups = kDeltaGroups;
   const int lane = threadIdx.x & 31;
   const int sub = lane / kLanesPerRow, col = (lane % kLanesPerRow) * 8;
   const int64_t warp_id = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int64_t row_base = warp_id * (kRowsPerPass * kPasses);
+  const int64_t row_base = warp_id * (kRowsPerGroup * kGroups);
+  const T *po = nullptr, *pd = nullptr;  // the current row of this lane
+  int i = 0;
+  // Two divisions for a warp's rows, unless they belong to several heads.
+  auto locate = [&](int64_t row) {
+    const int r32 = static_cast<int>(row);  // the host keeps rows below 2^31
+    const int bh = r32 / seq_q, b = bh / q_heads, h = bh - b * q_heads;
+    i = r32 - bh * seq_q;
+    po = o + b * o_sb + h * o_sh + i * o_ss + col;
+    pd = d_o + b * do_sb + h * do_sh + i * do_ss + col;
+  };
+  if (row_base + sub < rows) locate(row_base + sub);
   grid_dependency_wait();
   grid_dependency_trigger();
-  uint4 ov[kPasses], dv[kPasses];
+  uint4 ov[kGroups], dv[kGroups];
+  // Rows of one head, as nearly always: no branch between the loads.
+  const bool plain = __all_sync(0xffffffffu, po != nullptr && i + (kGroups - 1) * kRowsPerGroup < seq_q);
+  if (plain) {
 #pragma unroll
-  for (int ps = 0; ps < kPasses; ++ps) {
-    const int64_t row = row_base + ps * kRowsPerPass + sub;
-    ov[ps] = make_uint4(0, 0, 0, 0);
-    dv[ps] = make_uint4(0, 0, 0, 0);
-    if (row < rows) {
-      const int r32 = static_cast<int>(row);  // the host keeps rows below 2^31: 32-bit divisions
-      const int bh = r32 / seq_q;
-      const int i = r32 - bh * seq_q;
-      const int b = bh / q_heads, h = bh - b * q_heads;
-      ov[ps] = *reinterpret_cast<const uint4*>(o + b * o_sb + h * o_sh + i * o_ss + col);
-      dv[ps] = *reinterpret_cast<const uint4*>(d_o + b * do_sb + h * do_sh + i * do_ss + col);
+    for (int gr = 0; gr < kGroups; ++gr) {
+      ov[gr] = *reinterpret_cast<const uint4*>(po + gr * kRowsPerGroup * o_ss);
+      dv[gr] = *reinterpret_cast<const uint4*>(pd + gr * kRowsPerGroup * do_ss);
+    }
+  } else {
+#pragma unroll
+    for (int gr = 0; gr < kGroups; ++gr) {
+      const int64_t row = row_base + gr * kRowsPerGroup + sub;
+      ov[gr] = make_uint4(0, 0, 0, 0);
+      dv[gr] = make_uint4(0, 0, 0, 0);
+      if (row < rows) {
+        locate(row);
+        ov[gr] = *reinterpret_cast<const uint4*>(po);
+        dv[gr] = *reinterpret_cast<const uint4*>(pd);
+      }
     }
   }
+  static_assert(kGroups == 2, "the exchange below is written for two groups");
+  float acc[kGroups];
 #pragma unroll
-  for (int ps = 0; ps < kPasses; ++ps) {
-    const T* oe = reinterpret_cast<const T*>(&ov[ps]);
-    const T* de = reinterpret_cast<const T*>(&dv[ps]);
-    float acc = 0.f;
+  for (int gr = 0; gr < kGroups; ++gr) {
+    const T* oe = reinterpret_cast<const T*>(&ov[gr]);
+    const T* de = reinterpret_cast<const T*>(&dv[gr]);
+    acc[gr] = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc += static_cast<float>(oe[k]) * static_cast<float>(de[k]);
-#pragma unroll
-    for (int sft = kLanesPerRow / 2; sft > 0; sft >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, sft);
-    const int64_t row = row_base + ps * kRowsPerPass + sub;
-    if (lane % kLanesPerRow == 0 && row < rows) delta[row] = acc;
+    for (int k = 0; k < 8; ++k) acc[gr] += static_cast<float>(oe[k]) * static_cast<float>(de[k]);
   }
+  // The sums over a row's lanes: partners half of them apart, a quarter and so on, each sum in the order of a plain butterfly.  At the
+  // first exchange a lane goes on with one group and its partner with the other: 4 (HD 128) or 3 shuffles for both, not 8 or 6.
+  const bool upper = (lane & (kLanesPerRow / 2)) != 0;
+  float sum = (upper ? acc[1] : acc[0]) + __shfl_xor_sync(0xffffffffu, upper ? acc[0] : acc[1], kLanesPerRow / 2);
+#pragma unroll
+  for (int sft = kLanesPerRow / 4; sft > 0; sft >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, sft);
+  const int64_t row = row_base + (upper ? kRowsPerGroup : 0) + sub;
+  if (lane % (kLanesPerRow / 2) == 0 && row < rows) delta[row] = sum;
 }
 
 struct BwdMaps {
@@ -1009,10 +1036,9 @@ int launch_bwd_typed(const b200k_attention_bwd_args& a, const BwdMaps& tm, const
   if (rc) return rc;
   const int64_t rows = static_cast<int64_t>(a.batch) * a.q_heads * a.seq_q;
   if (rows > INT32_MAX) return set_error(B200K_ERR_BAD_SHAPE, "attention_bwd: batch * q_heads * seq_q must be below 2^31");
-  const int warps_per_block = 8;
-  const int64_t rows_per_block = static_cast<int64_t>(warps_per_block) * (32 / (HD / 8)) * 8;
+  const int64_t rows_per_block = kDeltaThreads / (HD / 8) * kDeltaGroups;
   rc = launch_pdl("attn_bwd_delta_kernel launch", attn_bwd_delta_kernel<T, HD>,
-                  dim3(static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block)), dim3(warps_per_block * 32), 0,
+                  dim3(static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block)), dim3(kDeltaThreads), 0,
                   stream, static_cast<const T*>(a.o), static_cast<const T*>(a.d_o), p.delta, rows, a.q_heads, a.seq_q,
                   a.o_stride_b, a.o_stride_h, a.o_stride_s, a.do_stride_b, a.do_stride_h, a.do_stride_s);
   if (rc) return rc;

@@ -188,3 +188,17 @@ def test_bad_arguments_are_rejected():
         torch.ops.b200k.attention_bwd(q, k, k, q, q, SCALE, False)
     with pytest.raises((RuntimeError, ValueError)):
         torch.ops.b200k.attention_bwd(q, q.float(), q, q, q, SCALE, False)
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("sq", [1, 3, 4, 7, 8, 9, 130])
+def test_rows_of_several_heads_in_a_warp(sq, head_dim):
+    """The row sums of dO o O: a warp takes 4 (head dim 128) or 8 rows, of one head or of several, here with dO in another layout than O.
+    dS = P o (dP - delta) hangs on them; same tolerance as above."""
+    scale = head_dim ** -0.5
+    q, k, v = oracle.make_attention_inputs(3, 5, 5, sq, 70, head_dim=head_dim, dtype=torch.bfloat16, seed=8)
+    d_o = _d_o((3, sq, 5, head_dim), torch.bfloat16).transpose(1, 2)
+    got = _run(q, k, v, d_o, False, scale)
+    ref = oracle.attention_bwd(q, k, v, d_o, scale, False)
+    for g, r in zip(got, ref):
+        _assert_close(g, r)
