@@ -578,6 +578,54 @@ __global__ void __launch_bounds__(kReduceThreads) decode_reduce_kernel(const Dec
   }
 }
 
+// At most eight chunks: a warp per (sequence, query head), a lane 4 dims of every chunk, all of them in flight at once and no block
+// barrier.  With eight warps per row most had no chunk and 2048 rows took two rounds of blocks.  Latency bound: length, partials, store.
+// Sums in the order of the kernel above, same bits.  Whole decode, in a graph, by the kernel above / this, us: 64 sequences of 512 to 8192
+// tokens, 32(8) heads 179.0 / 174.1, 128 of 100 to 5000, 16(4) of head dim 64 67.7 / 64.7, 100 of 2000 to 2500, 64(8) 172.8 / 157.5, 256 of
+// 100 to 2200, 32(8) 220.8 / 200.8, 38 of 10000 to 16000 (8 chunks), 8 heads 315.7 / 312.8.  With more chunks the loads are no longer one flight.
+constexpr int kFewChunks = 8;
+constexpr int kReduceFewWarps = 4;
+
+template <typename T, int HD>
+__global__ void __launch_bounds__(kReduceFewWarps * 32) decode_reduce_few_kernel(const DecodeParams p, const int32_t rows) {
+  const int lane = threadIdx.x & 31;
+  const int row = blockIdx.x * kReduceFewWarps + (threadIdx.x >> 5);
+  const int seq = row / p.q_heads, qh = row - seq * p.q_heads;
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  if (row >= rows) return;
+  const int len = clamped_len(p, seq, false);  // same clamp as phase 1
+  const int chunk_tokens = p.chunk.tokens(len);
+  const int n_chunks = (len + chunk_tokens - 1) / chunk_tokens;  // <= max_chunks <= kFewChunks
+  const int64_t slot0 = static_cast<int64_t>(row) * p.max_chunks;
+  const bool owns = lane < HD / 4;
+  float4 x[kFewChunks];
+#pragma unroll
+  for (int c = 0; c < kFewChunks; ++c)
+    if (owns && c < n_chunks) x[c] = *reinterpret_cast<const float4*>(p.ws_o + (slot0 + c) * HD + lane * 4);
+  const float2 v = lane < n_chunks ? p.ws_ml[slot0 + lane] : make_float2(-INFINITY, 0.f);
+  float M = v.x;
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, i));
+  const float Ms = (M == -INFINITY) ? 0.f : M;
+  const float f = lane < n_chunks ? fast_exp2(v.x - Ms) : 0.f;
+  float L = v.y * f;
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) L += __shfl_xor_sync(0xffffffffu, L, i);
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int c = 0; c < kFewChunks; ++c) {
+    const float w = __shfl_sync(0xffffffffu, f, c);
+    if (owns && c < n_chunks) {  // rounded products, as the other kernel's one chunk per warp
+      o.x = __fadd_rn(o.x, __fmul_rn(x[c].x, w));
+      o.y = __fadd_rn(o.y, __fmul_rn(x[c].y, w));
+      o.z = __fadd_rn(o.z, __fmul_rn(x[c].z, w));
+      o.w = __fadd_rn(o.w, __fmul_rn(x[c].w, w));
+    }
+  }
+  if (owns) store_out<T>(p, seq, qh, lane * 4, o, L, HD);
+}
+
 // ------------------------------------------------------------------------------------------
 // gather check kernel: copies rows through the block table with kv_row_offset<true>
 // ------------------------------------------------------------------------------------------
@@ -673,6 +721,12 @@ int launch_decode_typed(const DecodeParams& p, bool paged, int num_seqs, cudaStr
   else
     rc = paged ? launch_splitkv<T, true, HD, 4>(p, num_seqs, stream) : launch_splitkv<T, false, HD, 4>(p, num_seqs, stream);
   if (rc || p.cluster > 0) return rc;
+  const int64_t all = static_cast<int64_t>(num_seqs) * p.q_heads;
+  if (p.max_chunks <= kFewChunks && all < INT32_MAX - kReduceFewWarps) {
+    const int32_t rows = static_cast<int32_t>(all);
+    return launch_pdl("decode_reduce_few_kernel launch", decode_reduce_few_kernel<T, HD>,
+                      dim3((rows + kReduceFewWarps - 1) / kReduceFewWarps), dim3(kReduceFewWarps * 32), 0, stream, p, rows);
+  }
   return launch_pdl("decode_reduce_kernel launch", decode_reduce_kernel<T, HD>, dim3(p.q_heads, num_seqs),
                     dim3(kReduceThreads), 0, stream, p);
 }

@@ -220,3 +220,18 @@ def test_kv_append_copies_every_chunk(seqs, tokens, heads, dim):
         assert torch.equal(cache[pages, :, rows], new.to(DEV))
         assert int((cache != 0).any(-1).sum()) == seqs * tokens * heads  # and nothing else
     assert tb.device_status() == 0
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("q_heads", [8, 24])
+def test_merge_of_up_to_eight_chunks_has_the_bits_of_the_merge_of_many(q_heads, dtype, dim):
+    """Tables of at most eight chunks are merged by a warp per row, wider ones by a block; too many heads for clusters to merge."""
+    lens = [0, 1, 64, 65, 300, 511, 512]
+    q, kc, vc, bt, sl = oracle.make_paged_decode_inputs(num_seqs=len(lens), q_heads=q_heads, kv_heads=8, head_dim=dim, lens=lens,
+                                                        dtype=dtype, seed=12)
+    assert bt.shape[1] * 16 == 512
+    wide = torch.cat([bt, torch.zeros(len(lens), 8, dtype=bt.dtype)], 1)
+    got = _paged(q, kc, vc, bt, sl, dim ** -0.5, chunk=64)
+    assert torch.equal(got, _paged(q, kc, vc, wide, sl, dim ** -0.5, chunk=64))
+    oracle.assert_close_half(got, oracle.paged_decode_attention(q, kc, vc, bt, sl, dim ** -0.5))
