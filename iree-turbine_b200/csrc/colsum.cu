@@ -2,10 +2,10 @@
 //
 // HBM- or L2-bound: 2 bytes per element read once.  A cluster of eight CTAs owns 64 columns (one
 // 128-byte line per row) and splits the rows; a thread keeps 8 columns of every 32nd row of its CTA
-// in fp32, four 16-byte loads in flight.  The partial sums meet in shared memory, then across the
+// in fp32, four or twelve 16-byte loads in flight.  The partial sums meet in shared memory, then across the
 // cluster through distributed shared memory in rank order: one launch, no scratch, no atomics, the
 // same bits every time.  (The torch expression it replaces, x.float().sum(0).to(x.dtype), wrote and
-// re-read the matrix in fp32: 48 us for 3000 x 4352, in three launches; this takes 7.)
+// re-read the matrix in fp32: 48 us for 3000 x 4352, in three launches; this takes 5.5.)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -19,14 +19,13 @@ constexpr int kThreads = 256;
 constexpr int kCols = 64;
 constexpr int kCluster = 8;
 constexpr int kRowsPerPass = kThreads / 8;  // 8 lanes of 16 bytes cover a row's 64 columns
-constexpr int kUnroll = 4;
 
 __device__ __forceinline__ float2 to_float2(__half2 v) { return __half22float2(v); }
 __device__ __forceinline__ float2 to_float2(__nv_bfloat162 v) { return __bfloat1622float2(v); }
 __device__ __forceinline__ void from_float(float v, __half& o) { o = __float2half_rn(v); }
 __device__ __forceinline__ void from_float(float v, __nv_bfloat16& o) { o = __float2bfloat16_rn(v); }
 
-template <typename T, typename T2>
+template <typename T, typename T2, int UNROLL>
 __global__ void __launch_bounds__(kThreads) col_sum_kernel(const T* x, T* out, int64_t rows, int64_t cols,
                                                            int64_t ld) {
   __shared__ float part[kThreads / 32][kCols];
@@ -41,15 +40,15 @@ __global__ void __launch_bounds__(kThreads) col_sum_kernel(const T* x, T* out, i
   float acc[8] = {};
   if (col < cols) {
     const T* px = x + col;
-    for (int64_t r = r_begin + threadIdx.x / 8; r < r_end; r += kRowsPerPass * kUnroll) {
-      uint4 v[kUnroll];
+    for (int64_t r = r_begin + threadIdx.x / 8; r < r_end; r += kRowsPerPass * UNROLL) {
+      uint4 v[UNROLL];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
+      for (int u = 0; u < UNROLL; ++u) {
         const int64_t rr = r + u * kRowsPerPass;
         v[u] = rr < r_end ? *reinterpret_cast<const uint4*>(px + rr * ld) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
+      for (int u = 0; u < UNROLL; ++u) {
         const T2* h = reinterpret_cast<const T2*>(&v[u]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -85,6 +84,16 @@ __global__ void __launch_bounds__(kThreads) col_sum_kernel(const T* x, T* out, i
   cluster_sync_all();  // no CTA leaves while a peer still reads its sums
 }
 
+// Loads in flight per thread.  Twelve from 2048 rows on, where a CTA has eight and more rows for each thread (below, most of the twelve would
+// be past the end), if its 64 registers, four blocks per SM for six, cost no second round of blocks (clusters of eight leave some SMs out), or x is
+// more than L2 holds.  Same order of the sums.  us by four / twelve: 3000x4352 6.83 / 5.46 (read from HBM 9.4 / 7.9), 2842x552 3.84 / 2.99,
+// 6000x1000 5.85 / 4.31, 2048x4096 5.55 / 5.04, 8000x8192 37.0 / 26.3, 3000x16384 24.3 / 21.7; but 1500x2048 3.54 / 3.46, 1100x8192 6.96 / 8.92,
+// 300x1024 2.52 / 2.86, 2300x4736 6.44 / 6.83, 3500x6144 7.85 / 10.1, 4096x11008 16.3 / 18.4.
+constexpr int kMany = 12, kFew = 4;
+bool many_loads(int64_t rows, int64_t cols, int64_t ctas) {
+  return rows >= 2048 && (ctas <= num_sms() * 4 * 15 / 16 || rows * cols * 2 > 96000000);
+}
+
 template <typename T, typename T2>
 int launch(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
@@ -100,9 +109,8 @@ int launch(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, cud
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return check_cuda(cudaLaunchKernelEx(&cfg, col_sum_kernel<T, T2>, static_cast<const T*>(x), static_cast<T*>(out), rows,
-                                       cols, ld),
-                    "col_sum_kernel launch");
+  auto kfn = many_loads(rows, cols, cfg.gridDim.x) ? col_sum_kernel<T, T2, kMany> : col_sum_kernel<T, T2, kFew>;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kfn, static_cast<const T*>(x), static_cast<T*>(out), rows, cols, ld), "col_sum_kernel launch");
 }
 
 }  // namespace

@@ -104,6 +104,17 @@ def test_col_sum(rows, cols, dtype):
         assert got.dtype == dtype and bool(((got.double() - ref).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("rows,cols", [(2047, 72), (2048, 72), (2049, 72), (3071, 64), (3073, 136), (2048, 4440), (2048, 4488)])
+def test_col_sum_of_many_rows(rows, cols):
+    """Twelve rows in flight per thread from 2048 rows and up to a number of columns, else four: sums in one order, so the bits of a part
+    of the columns in a pitched view are those of the whole."""
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(6)).to(torch.bfloat16).to(DEV)
+    got, ref = torch.ops.b200k.col_sum(x), x.double().sum(0)
+    bound = x.double().abs().sum(0) * rows * 2.0 ** -24 + ref.abs() * 2.0 ** -8 + 1e-7
+    assert bool(((got.double() - ref).abs() <= bound).all())
+    assert torch.equal(torch.ops.b200k.col_sum(x[:, :64]), got[:64])
+
+
 @pytest.mark.parametrize("m,n,k,split", [(1, 64, 64, 1), (128, 64, 128, 1), (130, 65, 72, 1), (257, 200, 1000, 1), (1000, 1000, 1000, 1),
                                          (16, 64, 512, 2), (40, 130, 1032, 4), (128, 192, 2048, 8)])
 @pytest.mark.parametrize("a_km,b_kn", [(False, False), (True, True)])
