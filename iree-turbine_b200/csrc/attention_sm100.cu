@@ -182,7 +182,14 @@ struct Item {
   int n[2];   // half steps of 64 keys that query tile t visits (0: the tile has no rows or sees no key)
   int nmax;   // KV tiles loaded for the item
   int kv_len, causal_offset;  // keys of this item's sequence; key j is visible to query i iff j <= i + causal_offset
-  // PACKED: query tile 1 is the only tile of another head, which exists unless `second` is false
+};
+
+// PACKED: query tile 1 is the only tile of another head, which exists unless `second` is false.  A type of its own: with these members
+// in every kernel's items the others were slower, 4x32x4096 531 / 540 us, 4x16x2048 head dim 64 68.2 / 68.8.
+template <bool PACKED>
+struct ItemOf : Item {};
+template <>
+struct ItemOf<true> : Item {
   int head1, batch1;
   bool second;
 };
@@ -218,16 +225,23 @@ __device__ __forceinline__ Item make_item(int batch, int head, int pair, const A
 
 // Query tile t of an item: its first row, and the head it belongs to.
 template <bool PACKED>
-__device__ __forceinline__ int first_row(const Item& it, int t) {
+__device__ __forceinline__ int first_row(const ItemOf<PACKED>& it, int t) {
   return PACKED ? 0 : it.pair * kPairRows + t * kTileRows;
 }
 template <bool PACKED>
-__device__ __forceinline__ int head_of(const Item& it, int t) {
-  return PACKED && t ? it.head1 : it.head;
+__device__ __forceinline__ int head_of(const ItemOf<PACKED>& it, int t) {
+  if constexpr (PACKED) return t ? it.head1 : it.head;
+  return it.head;
 }
 template <bool PACKED>
-__device__ __forceinline__ int batch_of(const Item& it, int t) {
-  return PACKED && t ? it.batch1 : it.batch;
+__device__ __forceinline__ int batch_of(const ItemOf<PACKED>& it, int t) {
+  if constexpr (PACKED) return t ? it.batch1 : it.batch;
+  return it.batch;
+}
+template <bool PACKED>
+__device__ __forceinline__ bool has_second(const ItemOf<PACKED>& it) {
+  if constexpr (PACKED) return it.second;
+  return false;
 }
 
 // The CTA's items, in the order every role walks them.  With p.couples a position stands for two items,
@@ -243,17 +257,17 @@ struct ItemWalk {
   Item first;
   __device__ ItemWalk(const AttnParams& params, const uint16_t* sorted) : p(params), table(sorted), light(-1) {}
   // Next item, empty ones (nmax == 0) included; false when the CTA has no more.
-  __device__ __forceinline__ bool next(Item& it) {
+  __device__ __forceinline__ bool next(ItemOf<PACKED>& it) {
     if (!PAGED && light >= 0) {
-      it = make_item<PAGED>(first.batch, first.head, light, p);
+      static_cast<Item&>(it) = make_item<PAGED>(first.batch, first.head, light, p);
       light = -1;
       return true;
     }
     if (walk.pos >= p.order.num_items) return false;
-    if (PACKED) {
+    if constexpr (PACKED) {
       const int bh = 2 * walk.pos, heads = p.batch * p.q_heads;
       const int batch = p.order.by_q_heads.quotient(bh);
-      it = make_item<PAGED>(batch, bh - batch * p.q_heads, 0, p);
+      static_cast<Item&>(it) = make_item<PAGED>(batch, bh - batch * p.q_heads, 0, p);
       it.second = bh + 1 < heads;
       it.batch1 = p.order.by_q_heads.quotient(bh + 1);
       it.head1 = bh + 1 - it.batch1 * p.q_heads;
@@ -268,13 +282,13 @@ struct ItemWalk {
       pair = p.couples - 1 - k;
       light = k < pair ? k : -1;
     }
-    it = make_item<PAGED>(batch, head, pair, p);
+    static_cast<Item&>(it) = make_item<PAGED>(batch, head, pair, p);
     first = it;
     walk.step(p.order);
     return true;
   }
   // Next item that has work.
-  __device__ __forceinline__ bool next_busy(Item& it) {
+  __device__ __forceinline__ bool next_busy(ItemOf<PACKED>& it) {
     while (next(it))
       if (it.nmax > 0) return true;
     return false;
@@ -417,7 +431,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
           return true;
         };
         ItemWalk<PAGED, PACKED> walk(p, table);
-        Item it;
+        ItemOf<PACKED> it;
         while (ok && walk.next_busy(it)) {
           kvh = it.head / group;
           if (PAGED) {
@@ -430,9 +444,9 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
             ok = load_tile(&tmap_k, it, j, page) && load_tile(&tmap_v, it, j, page);
             page = page_next;
           }
-          if (PACKED && ok && it.second) {
-            kvh = it.head1 / group;
-            it.batch = it.batch1;
+          if (ok && has_second(it)) {
+            kvh = head_of(it, 1) / group;
+            it.batch = batch_of(it, 1);
             ok = load_tile(&tmap_k, it, 0, 0) && load_tile(&tmap_v, it, 0, 0);
           }
         }
@@ -444,7 +458,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
         uint32_t ci[2] = {0, 0};  // items of each tile so far
         bool ok = true;
         ItemWalk<PAGED, PACKED> walk(p, table);
-        Item it, nx;
+        ItemOf<PACKED> it, nx;
         bool have = walk.next_busy(it);
         while (ok && have) {
           const bool have_next = walk.next_busy(nx);
@@ -549,12 +563,12 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
         auto pass_turn = [&]() { mbar_arrive(turn + (t ^ 1u)); };
         bool ok = true;
         ItemWalk<PAGED, PACKED> walk(p, table);
-        Item it;
+        ItemOf<PACKED> it;
         while (ok && walk.next_busy(it)) {
           const int n = t ? it.n[1] : it.n[0];
           const int nmax = it.nmax;
           // PACKED: tile 0's K and V are the item's first two entries, tile 1's the next two; each thread lets the other's go.
-          const bool both = PACKED && it.second;
+          const bool both = has_second(it);
           auto skip_entries = [&](uint32_t e) {
             for (uint32_t i = e; i < e + 2; ++i) {
               if (!wait_entry(i)) return false;
@@ -642,12 +656,12 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
     uint32_t steps[2] = {0, 0};  // half steps per tile before the current item
     bool ok = true;
     ItemWalk<PAGED, PACKED> walk(p, table);
-    Item it;
+    ItemOf<PACKED> it;
     while (ok && walk.next(it)) {
 #pragma unroll 1
       for (int t = 0; t < 2; ++t) {
         const int tile_r0 = first_row<PACKED>(it, t), head = head_of<PACKED>(it, t), batch = batch_of<PACKED>(it, t);
-        if (tile_r0 >= p.seq_q || (PACKED && t == 1 && !it.second)) continue;
+        if (tile_r0 >= p.seq_q || (PACKED && t == 1 && !has_second(it))) continue;
         const int q_row = tile_r0 + row_in_tile;
         if (it.n[t] == 0) {
           // no visible key: zeros (rare; plain stores)
@@ -747,7 +761,7 @@ __global__ void __launch_bounds__(Roles<GROUPS>::kThreads, 1)
     uint32_t cs = 0, ci = 0;  // half steps (of both warpgroups) and items of this query tile so far
     bool ok = true;
     ItemWalk<PAGED, PACKED> walk(p, table);
-    Item it;
+    ItemOf<PACKED> it;
     while (ok && walk.next_busy(it)) {
       const int n = it.n[t];
       if (n == 0) continue;
